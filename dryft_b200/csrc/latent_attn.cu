@@ -333,10 +333,18 @@ __global__ void latent_combine_kernel(const float* __restrict__ part, const int*
       if (lane + 32 * u < n_splits) w[lane + 32 * u] = ms[u] / l;
   }
   __syncthreads();
+  // a thread a latent entry, its splits requested sixteen at a time: with four entries a thread and eight splits at a time
+  // one token's 32 splits of 512 took 22 us (sixteen trips to memory)
   for (int d = threadIdx.x; d < kv_rank; d += blockDim.x) {
     float a = 0.f;
-#pragma unroll 8
-    for (int sidx = 0; sidx < n_splits; ++sidx) a = fmaf(src[sidx * stride + 2 + d], w[sidx], a);
+    for (int s0 = 0; s0 < n_splits; s0 += 16) {
+      float v[16];
+#pragma unroll
+      for (int u = 0; u < 16; ++u) v[u] = s0 + u < n_splits ? src[(s0 + u) * stride + 2 + d] : 0.f;
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        if (s0 + u < n_splits) a = fmaf(v[u], w[s0 + u], a);
+    }
     o_lat[((size_t)hd * n_tokens + n) * kv_rank + d] = from_f32<T>(a);
   }
 }
@@ -435,38 +443,77 @@ __global__ void head_gate_rows_kernel(const T* __restrict__ o, int hd, const T* 
 // path (sums in a fixed order, so a row's result does not depend on its company):
 //   latent_fold_q     q_lat[h, n, r] = sum_d q[n, h, d] * w_k[h, d, r]                      (32-bit result)
 //   latent_unfold_o   out[n, h*V + v] = T( sigmoid(gate[n, h]) * sum_r o_lat[h, n, r] * w_v[h, r, v] )
-// One block per (token, head); a thread per output entry reads along the matrices' rows.
-template <typename T>
-__global__ void latent_fold_q_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ w, float* __restrict__ q_lat,
-                                     int n_tokens, int H, int dim, int kv_rank) {
-  extern __shared__ __align__(16) float vin[];
-  const int n = blockIdx.x, h = blockIdx.y;
-  for (int d = threadIdx.x; d < dim; d += blockDim.x) vin[d] = to_f32<T>(q[((size_t)n * H + h) * q_stride + d]);
+// One block per (token, head, FOLD_COLS columns).  A thread takes VN neighbouring columns (16 bytes) of every FOLD_THREADS /
+// (FOLD_COLS / VN)-th matrix row, requested before the vector is read; the threads' sums are added in order.  One token and head of 512 x 128:
+// 3 us, where a thread per column along all rows took 18 (64 trips to memory).
+constexpr int FOLD_COLS = 128, FOLD_THREADS = 512;
+
+// out(c, sum_i vin(i) * w[i, c]) for the columns c0 .. c0 + FOLD_COLS - 1 of a [rows, cols] matrix
+template <typename T, int VN, typename In, typename Out>
+__device__ __forceinline__ void fold_columns(const T* __restrict__ w, int rows, int cols, int c0, float* vin, float* red, In in, Out out) {
+  constexpr int LR = FOLD_COLS / VN, G = FOLD_THREADS / LR, AHEAD = 16;
+  const int c = c0 + (threadIdx.x % LR) * VN, g = threadIdx.x / LR;
+  alignas(16) T wv[AHEAD][VN];
+  auto request = [&](int i0) {
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int i = i0 + u * G;
+      if (i < rows && c < cols) {
+        if (VN > 1) *reinterpret_cast<uint4*>(wv[u]) = *reinterpret_cast<const uint4*>(w + (size_t)i * cols + c);
+        else wv[u][0] = w[(size_t)i * cols + c];
+      }
+    }
+  };
+  request(g);
+  for (int i = threadIdx.x; i < rows; i += FOLD_THREADS) vin[i] = in(i);
   __syncthreads();
-  const T* wh = w + (size_t)h * dim * kv_rank;
-  for (int r = threadIdx.x; r < kv_rank; r += blockDim.x) {
-    float acc = 0.f;
-#pragma unroll 8
-    for (int d = 0; d < dim; ++d) acc = fmaf(vin[d], to_f32<T>(wh[(size_t)d * kv_rank + r]), acc);
-    q_lat[((size_t)h * n_tokens + n) * kv_rank + r] = acc;
+  float acc[VN];
+#pragma unroll
+  for (int j = 0; j < VN; ++j) acc[j] = 0.f;
+  for (int i0 = g; i0 < rows; i0 += AHEAD * G) {
+    if (i0 != g) request(i0);
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      if (i0 + u * G >= rows || c >= cols) continue;
+      const float x = vin[i0 + u * G];
+#pragma unroll
+      for (int j = 0; j < VN; ++j) acc[j] = fmaf(x, to_f32<T>(wv[u][j]), acc[j]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < VN; ++j) red[g * FOLD_COLS + (threadIdx.x % LR) * VN + j] = acc[j];
+  __syncthreads();
+  for (int j = threadIdx.x; j < FOLD_COLS && c0 + j < cols; j += FOLD_THREADS) {
+    float sum = 0.f;
+#pragma unroll
+    for (int k = 0; k < G; ++k) sum += red[k * FOLD_COLS + j];
+    out(c0 + j, sum);
   }
 }
+template <int VN> constexpr size_t fold_smem(int rows) { return sizeof(float) * ((size_t)rows + FOLD_THREADS * VN); }
 
-template <typename T>
-__global__ void latent_unfold_o_kernel(const T* __restrict__ o_lat, const T* __restrict__ w, const T* __restrict__ gate,
-                                       int gate_ld, T* __restrict__ out, int n_tokens, int H, int kv_rank, int vdim, int per_value) {
-  extern __shared__ __align__(16) float vin[];
+template <typename T, int VN>
+__global__ void __launch_bounds__(FOLD_THREADS) latent_fold_q_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ w,
+                                                                     float* __restrict__ q_lat, int n_tokens, int H, int dim, int kv_rank) {
+  extern __shared__ __align__(16) float sm_fold[];
   const int n = blockIdx.x, h = blockIdx.y;
-  for (int r = threadIdx.x; r < kv_rank; r += blockDim.x) vin[r] = to_f32<T>(o_lat[((size_t)h * n_tokens + n) * kv_rank + r]);
-  __syncthreads();
+  const T* qr = q + ((size_t)n * H + h) * q_stride;
+  float* to = q_lat + ((size_t)h * n_tokens + n) * kv_rank;
+  fold_columns<T, VN>(w + (size_t)h * dim * kv_rank, dim, kv_rank, blockIdx.z * FOLD_COLS, sm_fold, sm_fold + dim,
+                      [&](int d) { return to_f32<T>(qr[d]); }, [&](int r, float v) { to[r] = v; });
+}
+
+template <typename T, int VN>
+__global__ void __launch_bounds__(FOLD_THREADS) latent_unfold_o_kernel(const T* __restrict__ o_lat, const T* __restrict__ w,
+                                                                       const T* __restrict__ gate, int gate_ld, T* __restrict__ out,
+                                                                       int n_tokens, int H, int kv_rank, int vdim, int per_value) {
+  extern __shared__ __align__(16) float sm_fold[];
+  const int n = blockIdx.x, h = blockIdx.y;
+  const T* from = o_lat + ((size_t)h * n_tokens + n) * kv_rank;
   auto gate_of = [&](int v) { return gate ? 1.f / (1.f + expf(-to_f32<T>(gate[(size_t)n * gate_ld + (per_value ? h * vdim + v : h)]))) : 1.f; };
-  const T* wh = w + (size_t)h * kv_rank * vdim;
-  for (int v = threadIdx.x; v < vdim; v += blockDim.x) {
-    float acc = 0.f;
-#pragma unroll 8
-    for (int r = 0; r < kv_rank; ++r) acc = fmaf(vin[r], to_f32<T>(wh[(size_t)r * vdim + v]), acc);
-    out[((size_t)n * H + h) * vdim + v] = from_f32<T>(acc * gate_of(v));
-  }
+  fold_columns<T, VN>(w + (size_t)h * kv_rank * vdim, kv_rank, vdim, blockIdx.z * FOLD_COLS, sm_fold, sm_fold + kv_rank,
+                      [&](int r) { return to_f32<T>(from[r]); },
+                      [&](int v, float x) { out[((size_t)n * H + h) * vdim + v] = from_f32<T>(x * gate_of(v)); });
 }
 
 template <typename K> int opt_in(K kernel, size_t bytes) {
@@ -494,7 +541,7 @@ int launch_rows(const float* q_lat, const void* q, int q_stride, int q_rot_off, 
                                                                window, sink);
   int e = launch_status();
   if (e || n_splits <= 1) return e;
-  latent_combine_kernel<T><<<dim3(n_tokens, H), 128, 0, st>>>(part, tok_slot, (T*)o_lat, n_splits, n_tokens, H, kv_rank, sink);
+  latent_combine_kernel<T><<<dim3(n_tokens, H), kv_rank > 256 ? 512 : 256, 0, st>>>(part, tok_slot, (T*)o_lat, n_splits, n_tokens, H, kv_rank, sink);
   return launch_status();
 }
 }  // namespace
@@ -544,17 +591,40 @@ DRYFT_API int dryft_latent_attn_rows(int is_bf16, const float* q_lat, const void
 #undef DRYFT_LATENT_ROWS
 }
 
+namespace {
+template <typename T, int VN>
+int launch_fold(const void* q, int q_stride, const void* w, float* q_lat, int n_tokens, int H, int dim, int kv_rank, cudaStream_t st) {
+  const size_t smem = fold_smem<VN>(dim);
+  const int rc = opt_in(latent_fold_q_kernel<T, VN>, smem);
+  if (rc) return rc;
+  latent_fold_q_kernel<T, VN><<<dim3(n_tokens, H, (kv_rank + FOLD_COLS - 1) / FOLD_COLS), FOLD_THREADS, smem, st>>>((const T*)q, q_stride, (const T*)w,
+                                                                                                                  q_lat, n_tokens, H, dim, kv_rank);
+  return launch_status();
+}
+template <typename T, int VN>
+int launch_unfold(const void* o_lat, const void* w, const void* gate, int gate_ld, void* out, int n_tokens, int H, int kv_rank, int vdim,
+                  int per_value, cudaStream_t st) {
+  const size_t smem = fold_smem<VN>(kv_rank);
+  const int rc = opt_in(latent_unfold_o_kernel<T, VN>, smem);
+  if (rc) return rc;
+  latent_unfold_o_kernel<T, VN><<<dim3(n_tokens, H, (vdim + FOLD_COLS - 1) / FOLD_COLS), FOLD_THREADS, smem, st>>>(
+      (const T*)o_lat, (const T*)w, (const T*)gate, gate_ld, (T*)out, n_tokens, H, kv_rank, vdim, per_value);
+  return launch_status();
+}
+// 16-byte reads of the matrix: every row of every head starts on a 16-byte boundary
+template <typename T> bool fold_vec(const void* w, int cols) { return cols % (16 / sizeof(T)) == 0 && ((uintptr_t)w & 15) == 0; }
+}  // namespace
+
 DRYFT_API int dryft_latent_fold_q(int is_bf16, const void* q, int q_stride, const void* w, float* q_lat, int n_tokens, int H, int dim,
                                   int kv_rank, cudaStream_t st) {
   if (n_tokens <= 0) return 0;
   if (H <= 0 || H > 65535 || dim <= 0 || kv_rank <= 0 || dim > 12000) return DRYFT_ERR_UNSUPPORTED;
   typedef __nv_bfloat16 bf;
-  const int threads = kv_rank >= 256 ? 256 : (kv_rank >= 128 ? 128 : 64);
-  const size_t smem = sizeof(float) * (size_t)dim;
-  dim3 grid(n_tokens, H);
-  if (is_bf16) latent_fold_q_kernel<bf><<<grid, threads, smem, st>>>((const bf*)q, q_stride, (const bf*)w, q_lat, n_tokens, H, dim, kv_rank);
-  else latent_fold_q_kernel<float><<<grid, threads, smem, st>>>((const float*)q, q_stride, (const float*)w, q_lat, n_tokens, H, dim, kv_rank);
-  return launch_status();
+  if (is_bf16)
+    return fold_vec<bf>(w, kv_rank) ? launch_fold<bf, 8>(q, q_stride, w, q_lat, n_tokens, H, dim, kv_rank, st)
+                                    : launch_fold<bf, 1>(q, q_stride, w, q_lat, n_tokens, H, dim, kv_rank, st);
+  return fold_vec<float>(w, kv_rank) ? launch_fold<float, 4>(q, q_stride, w, q_lat, n_tokens, H, dim, kv_rank, st)
+                                     : launch_fold<float, 1>(q, q_stride, w, q_lat, n_tokens, H, dim, kv_rank, st);
 }
 
 DRYFT_API int dryft_latent_unfold_o(int is_bf16, const void* o_lat, const void* w, const void* gate, int gate_ld, void* out, int n_tokens,
@@ -562,16 +632,11 @@ DRYFT_API int dryft_latent_unfold_o(int is_bf16, const void* o_lat, const void* 
   if (n_tokens <= 0) return 0;
   if (H <= 0 || H > 65535 || vdim <= 0 || kv_rank <= 0 || kv_rank > 12000) return DRYFT_ERR_UNSUPPORTED;
   typedef __nv_bfloat16 bf;
-  const int threads = vdim >= 256 ? 256 : (vdim >= 128 ? 128 : 64);
-  const size_t smem = sizeof(float) * (size_t)kv_rank;
-  dim3 grid(n_tokens, H);
   if (is_bf16)
-    latent_unfold_o_kernel<bf><<<grid, threads, smem, st>>>((const bf*)o_lat, (const bf*)w, (const bf*)gate, gate_ld, (bf*)out, n_tokens, H,
-                                                            kv_rank, vdim, per_value);
-  else
-    latent_unfold_o_kernel<float><<<grid, threads, smem, st>>>((const float*)o_lat, (const float*)w, (const float*)gate, gate_ld, (float*)out,
-                                                               n_tokens, H, kv_rank, vdim, per_value);
-  return launch_status();
+    return fold_vec<bf>(w, vdim) ? launch_unfold<bf, 8>(o_lat, w, gate, gate_ld, out, n_tokens, H, kv_rank, vdim, per_value, st)
+                                 : launch_unfold<bf, 1>(o_lat, w, gate, gate_ld, out, n_tokens, H, kv_rank, vdim, per_value, st);
+  return fold_vec<float>(w, vdim) ? launch_unfold<float, 4>(o_lat, w, gate, gate_ld, out, n_tokens, H, kv_rank, vdim, per_value, st)
+                                  : launch_unfold<float, 1>(o_lat, w, gate, gate_ld, out, n_tokens, H, kv_rank, vdim, per_value, st);
 }
 
 DRYFT_API int dryft_latent_scratch_table(const int* cu_q, const int* seq_slot, int n_seqs, int* table, int max_pages, int page_size,

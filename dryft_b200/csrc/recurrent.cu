@@ -489,6 +489,108 @@ __global__ void __launch_bounds__(G_THREADS) rglru_gates_kernel(
   }
 }
 
+// The same for steps of few tokens.  There a block per gate block leaves a thread 2 nb dependent trips long (22 us for one
+// token of 16 blocks of 128 x 128); here a block takes FEW_COLS of its outputs for up to GT tokens, a thread 4 neighbouring ones
+// over every 32nd k, and the threads' sums are added in a fixed order.
+constexpr int FEW_COLS = 32, FEW_GROUPS = G_THREADS / (FEW_COLS / 4);     // 32 threads share a column's k
+
+template <typename T>
+__global__ void __launch_bounds__(G_THREADS) rglru_gates_few_kernel(
+    const T* __restrict__ proj, int ld, int x_off, const float* __restrict__ x_bias, const int* __restrict__ tok_slot,
+    const float* __restrict__ conv_w, const float* __restrict__ conv_b, int taps, const float* __restrict__ tail,
+    const float* __restrict__ w_gates, const float* __restrict__ b_a, const float* __restrict__ b_i,
+    const float* __restrict__ sp_lam, float c_mult, float* __restrict__ a_out, float* __restrict__ b_out, int n_tokens,
+    int C, int nb) {
+  extern __shared__ __align__(16) float u_s[];   // [GT][nb]
+  __shared__ float red[G_THREADS / 32][GT][2][FEW_COLS];
+  const int n0 = blockIdx.x * GT, blk = blockIdx.y, c0 = blk * nb, o0 = blockIdx.z * FEW_COLS;
+  const int K1 = taps - 1, live = min(GT, n_tokens - n0);
+  const int o = o0 + (threadIdx.x % (FEW_COLS / 4)) * 4, g = threadIdx.x / (FEW_COLS / 4);
+  const float* wg = w_gates + (size_t)blk * nb * 2 * nb;   // [k][2][o]
+  constexpr int AHEAD = 4;
+  float4 wr[AHEAD], wi[AHEAD];
+  auto request = [&](int k0) {
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int k = k0 + u * FEW_GROUPS;
+      if (k < nb && o < nb) {
+        wr[u] = *reinterpret_cast<const float4*>(wg + ((size_t)k * 2) * nb + o);
+        wi[u] = *reinterpret_cast<const float4*>(wg + ((size_t)k * 2 + 1) * nb + o);
+      }
+    }
+  };
+  request(g);
+  for (int idx = threadIdx.x; idx < live * nb; idx += G_THREADS) {
+    const int t = idx / nb, cc = idx % nb, n = n0 + t, c = c0 + cc;
+    float u = 0.f;
+    const int slot = tok_slot[n];
+    if (slot >= 0) {
+      int avail = 0;   // tokens of the same sequence right before this one in the step, up to taps-1
+      while (avail < K1 && n - avail - 1 >= 0 && tok_slot[n - avail - 1] == slot) ++avail;
+      u = conv_b[c];
+      for (int j = 0; j < taps; ++j) {
+        const int back = K1 - j;
+        float xv;
+        if (back <= avail) xv = to_f32<T>(proj[(size_t)(n - back) * ld + x_off + c]) + x_bias[c];
+        else xv = tail[((size_t)slot * K1 + (K1 - back + avail)) * C + c];
+        u = fmaf(conv_w[(size_t)c * taps + j], xv, u);
+      }
+    }
+    u_s[t * nb + cc] = u;
+  }
+  __syncthreads();
+  float acc[GT][2][4];
+#pragma unroll
+  for (int t = 0; t < GT; ++t)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[t][0][j] = acc[t][1][j] = 0.f;
+  for (int k0 = g; k0 < nb; k0 += AHEAD * FEW_GROUPS) {
+    if (k0 != g) request(k0);
+#pragma unroll
+    for (int u = 0; u < AHEAD; ++u) {
+      const int k = k0 + u * FEW_GROUPS;
+      if (k >= nb || o >= nb) continue;
+      const float r4[4] = {wr[u].x, wr[u].y, wr[u].z, wr[u].w}, i4[4] = {wi[u].x, wi[u].y, wi[u].z, wi[u].w};
+#pragma unroll
+      for (int t = 0; t < GT; ++t) {
+        if (t >= live) break;
+        const float uv = u_s[t * nb + k];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) { acc[t][0][j] = fmaf(r4[j], uv, acc[t][0][j]); acc[t][1][j] = fmaf(i4[j], uv, acc[t][1][j]); }
+      }
+    }
+  }
+  // a warp's four groups by shuffles, then the warps in order
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int t = 0; t < GT; ++t) {
+    if (t >= live) break;
+#pragma unroll
+    for (int m = 0; m < 2; ++m)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        float v = acc[t][m][j];
+        v += __shfl_xor_sync(0xffffffffu, v, 8);
+        v += __shfl_xor_sync(0xffffffffu, v, 16);
+        if (lane < 8) red[warp][t][m][lane * 4 + j] = v;
+      }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < live * FEW_COLS; i += G_THREADS) {
+    const int t = i / FEW_COLS, oo = i % FEW_COLS, n = n0 + t, c = o0 + oo;
+    if (c >= nb) continue;
+    float ar = b_a[c0 + c], ai = b_i[c0 + c];
+#pragma unroll
+    for (int w = 0; w < G_THREADS / 32; ++w) { ar += red[w][t][0][oo]; ai += red[w][t][1][oo]; }
+    const float r = 1.f / (1.f + expf(-ar)), ig = 1.f / (1.f + expf(-ai));
+    const float log_a = -c_mult * r * sp_lam[c0 + c];
+    a_out[(size_t)n * C + c0 + c] = expm1f(log_a);   // a - 1: a decay close to one keeps its distance from one
+    b_out[(size_t)n * C + c0 + c] = sqrtf(-expm1f(2.f * log_a)) * ig * u_s[t * nb + c];
+  }
+}
+// Steps of up to this many tokens (a decode step's rows): beyond it the prompt form's blocks fill the SMs.
+constexpr int FEW_TOKENS = 64;
+
 __device__ __forceinline__ float gelu_tanh_f(float z) {
   return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }
@@ -647,6 +749,16 @@ DRYFT_API int dryft_rglru_gates(int is_bf16, const void* proj, int ld, int x_off
   typedef __nv_bfloat16 bf;
   const int nb = C / n_blocks;
   const size_t smem = sizeof(float) * (size_t)GT * nb;
+  if (n_tokens <= FEW_TOKENS && nb % 4 == 0 && ((uintptr_t)w_gates & 15) == 0 && smem <= 32 * 1024) {
+    const dim3 few((n_tokens + GT - 1) / GT, n_blocks, (nb + FEW_COLS - 1) / FEW_COLS);
+    if (is_bf16)
+      rglru_gates_few_kernel<bf><<<few, G_THREADS, smem, st>>>((const bf*)proj, ld, x_off, x_bias, tok_slot, conv_w, conv_b, taps, tail,
+                                                               w_gates, b_a, b_i, sp_lam, c_mult, a_out, b_out, n_tokens, C, nb);
+    else
+      rglru_gates_few_kernel<float><<<few, G_THREADS, smem, st>>>((const float*)proj, ld, x_off, x_bias, tok_slot, conv_w, conv_b, taps,
+                                                                  tail, w_gates, b_a, b_i, sp_lam, c_mult, a_out, b_out, n_tokens, C, nb);
+    return launch_status();
+  }
   int rc = is_bf16 ? opt_in_smem(rglru_gates_kernel<bf>, smem) : opt_in_smem(rglru_gates_kernel<float>, smem);
   if (rc) return rc;
   dim3 grid((n_tokens + GT - 1) / GT, n_blocks);
