@@ -244,14 +244,53 @@ __global__ void __launch_bounds__(ROWS_THREADS) moe_rows_kernel(
   }
 }
 
-template <typename T>
-__global__ void moe_combine_kernel(const T* __restrict__ y, const float* __restrict__ wts, int top, int width, T* __restrict__ out) {
-  const int n = blockIdx.x;
-  for (int c = threadIdx.x; c < width; c += blockDim.x) {
-    float v = 0.f;
-    for (int k = 0; k < top; ++k) v = fmaf(wts[(size_t)n * top + k], to_f32<T>(y[((size_t)n * top + k) * width + c]), v);
-    out[(size_t)n * width + c] = from_f32<T>(v);
+// A thread sums 16 bytes of columns (one column where the width or the addresses are no multiple of 16 bytes): its `top`
+// rows' words are requested together, eight at a time, and added in the order of k.  2,048 tokens x 8 rows of 2,048: 12 us
+// for 75 MB, 31 with one column a thread; 8 tokens: 2 us against 13.
+constexpr int COMBINE_THREADS = 128;
+template <typename T, int V>
+__global__ void __launch_bounds__(COMBINE_THREADS) moe_combine_kernel(const T* __restrict__ y, const float* __restrict__ wts, int top, int width,
+                                                                      T* __restrict__ out) {
+  const int n = blockIdx.x, c = (blockIdx.y * COMBINE_THREADS + threadIdx.x) * V;
+  if (c >= width) return;
+  const T* from = y + (size_t)n * top * width + c;
+  float sum[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) sum[j] = 0.f;
+  for (int k0 = 0; k0 < top; k0 += 8) {
+    alignas(16) T v[8][V];
+    float w[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (k0 + k >= top) continue;
+      w[k] = wts[(size_t)n * top + k0 + k];
+      if (V * sizeof(T) == 16) *reinterpret_cast<uint4*>(v[k]) = *reinterpret_cast<const uint4*>(from + (size_t)(k0 + k) * width);
+      else v[k][0] = from[(size_t)(k0 + k) * width];
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (k0 + k >= top) continue;
+#pragma unroll
+      for (int j = 0; j < V; ++j) sum[j] = fmaf(w[k], to_f32<T>(v[k][j]), sum[j]);
+    }
   }
+  alignas(16) T r[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) r[j] = from_f32<T>(sum[j]);
+  T* to = out + (size_t)n * width + c;
+  if (V * sizeof(T) == 16) *reinterpret_cast<uint4*>(to) = *reinterpret_cast<const uint4*>(r);
+  else to[0] = r[0];
+}
+
+template <typename T>
+int combine_launch(const void* y, const float* wts, int top, int width, void* out, int n, cudaStream_t st) {
+  constexpr int V = 16 / sizeof(T);
+  const bool vec = width % V == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  const int per = COMBINE_THREADS * (vec ? V : 1), cols = (width + per - 1) / per;
+  if (cols > 65535) return DRYFT_ERR_UNSUPPORTED;
+  if (vec) moe_combine_kernel<T, V><<<dim3(n, cols), COMBINE_THREADS, 0, st>>>((const T*)y, wts, top, width, (T*)out);
+  else moe_combine_kernel<T, 1><<<dim3(n, cols), COMBINE_THREADS, 0, st>>>((const T*)y, wts, top, width, (T*)out);
+  return launch_status();
 }
 
 template <typename T>
@@ -294,11 +333,7 @@ DRYFT_API int dryft_moe_rows(int is_bf16, const void* a_in, int a_div, const voi
 
 DRYFT_API int dryft_moe_combine(int is_bf16, const void* y, const float* wts, int top, int width, void* out, int n, cudaStream_t st) {
   if (n <= 0) return 0;
-  if (is_bf16)
-    moe_combine_kernel<__nv_bfloat16><<<n, 256, 0, st>>>((const __nv_bfloat16*)y, wts, top, width, (__nv_bfloat16*)out);
-  else
-    moe_combine_kernel<float><<<n, 256, 0, st>>>((const float*)y, wts, top, width, (float*)out);
-  return launch_status();
+  return is_bf16 ? combine_launch<__nv_bfloat16>(y, wts, top, width, out, n, st) : combine_launch<float>(y, wts, top, width, out, n, st);
 }
 
 DRYFT_API int dryft_moe_route_rows(int is_bf16, const void* h, const void* w_router, const float* bias, const float* corr, int n_tokens, int K, int E,

@@ -924,14 +924,8 @@ def moe_grouped_lib() -> ctypes.CDLL:
     global _moe_grouped
     with _lock:
         if _moe_grouped is None:
-            import os
-
-            defs = {}   # measurement knobs: the ring's slice width and depth (the source's defaults otherwise)
-            for var, name in (("DRYFT_MOE_BK", "DRYFT_MOE_BK"), ("DRYFT_MOE_STAGES", "DRYFT_MOE_STAGES")):
-                if os.environ.get(var):
-                    defs[name] = int(os.environ[var])
-            lib = _load(build.build_library("moe_grouped", ("moe_grouped.cu",), defs))
-            lib.dryft_moe_grouped.argtypes = [_p, _p, _p, _p, _i, _i, _i, _i, _i, _p, _p, _p, _i, _p, _f, _f, _f, _p]
+            lib = _load(build.build_library("moe_grouped", ("moe_grouped.cu",)))
+            lib.dryft_moe_grouped.argtypes = [_p, _p, _p, _p, _i, _i, _i, _i, _i, _p, _p, _p, _i, _p, _f, _f, _f, _p, _p]
             lib.dryft_moe_grouped.restype = _i
             lib.dryft_moe_grouped_work_ints.argtypes = [_i, _i]
             lib.dryft_moe_grouped_work_ints.restype = _ll
@@ -942,7 +936,7 @@ def moe_grouped_lib() -> ctypes.CDLL:
 def moe_grouped(h, w_gate_up, w_down, idx, y, gated: bool = True, in_w=None, limit: Optional[float] = None, alpha: float = 1.0,
                 up_offset: float = 0.0) -> None:
     """``y[n*top + k] = expert idx[n, k] applied to h[n]`` (bfloat16) with the assignments sorted by expert on the device and
-    both expert products as grouped tensor-core products (``csrc/moe_grouped.cu``: three launches, no host round trip).
+    both expert products as grouped tensor-core products (``csrc/moe_grouped.cu``: three or four launches, no host round trip).
     ``gated=False``: ``w_gate_up`` is ``[E, F, W]`` (no gate rows) and the activation is ``max(., 0)^2``.  With ``in_w [n, top]``
     (float32) each assignment's weight scales its expert's input and the activation is the clamped one of ``moe_rows``'s
     ``gate_up_clamp`` mode."""
@@ -966,7 +960,8 @@ def moe_grouped(h, w_gate_up, w_down, idx, y, gated: bool = True, in_w=None, lim
         _need(in_w, "in_w", torch.float32, (n, top))
     _ok(lib.dryft_moe_grouped(_ptr(h), _ptr(w_gate_up), _ptr(w_down), _ptr(idx), n, top, e, width, f, _ptr(act), _ptr(y), _ptr(work),
                               2 if in_w is not None else int(gated), _ptr(in_w), float("inf") if limit is None else float(limit),
-                              float(alpha), float(up_offset), _stream()), f"moe_grouped ({e} experts, {width} x {f})", n_kernels=3)
+                              float(alpha), float(up_offset), _ptr(error_flag(h.device)), _stream()),
+        f"moe_grouped ({e} experts, {width} x {f})", n_kernels=4 if width % 64 == 0 and f % 64 == 0 else 3)
 
 
 # ----------------------------------------------------------------------------- matrix products

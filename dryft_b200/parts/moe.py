@@ -151,10 +151,24 @@ class MoE:
             self.w_shared_up = torch.cat([w, torch.zeros((pad, self.hidden), dtype=w.dtype, device=w.device)]) if pad else w
             self.w_shared_down = weights.load(sp + nm["down"], "matrix")
 
-    GROUPED_MIN_TOKENS = 32   # below this every assignment streams its expert's weights itself
+    # Below this many tokens every assignment streams its expert's weights itself -- unless the tokens share so many experts
+    # that reading each one's weights once, which the grouped products do, spares more than their launches cost (measured:
+    # 64 experts of 768 x 2,048, 8 a token: 94 us against 109 with 8 tokens, which spares 207 MB, 82 against 73 with 4 and
+    # 52 MB; 32 experts of 512 x 1,024, 4 a token: 36 against 46 with 16 tokens and 111 MB, 35 against 37 with 12 and 71 MB)
+    GROUPED_MIN_TOKENS = 32
+    GROUPED_SPARES_BYTES = 75e6
     ROUTE_ROWS_MAX = 16       # up to this many tokens the router's product and choice are one launch ...
     ROUTE_ROWS_MAX_WEIGHTS = 64 * 1024   # ... while one block can stream the router's weight quickly enough (measured: 32 x 1,024
                                          # gains a launch, 64 x 2,048 takes longer than the two launches it replaces)
+
+    def _grouped(self, n: int) -> bool:
+        if not self.use_grouped or n >= self.GROUPED_MIN_TOKENS:
+            return self.use_grouped
+        if self.hidden % 64 or self.inter % 64:      # the grouped products on mma.sync: for prompts only
+            return False
+        chosen = self.experts * (1.0 - (1.0 - self.top / self.experts) ** n)      # different experts, on the mean
+        each = 2 * (self.w_gate_up[0].numel() + self.w_down[0].numel())
+        return (n * self.top - chosen) * each >= self.GROUPED_SPARES_BYTES
 
     def route(self, h: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
         """Chosen experts ``[n, top]`` int32 and their weights ``[n, top]`` float32."""
@@ -220,7 +234,7 @@ class MoE:
         y = torch.empty((n * self.top, self.hidden), dtype=h.dtype, device=h.device)
         special = self.weight_input or self.clamped      # the kernel mode with a weight on the input and the clamped activation
         in_w = wts if self.weight_input else (torch.ones_like(wts) if special else None)
-        if self.use_grouped and n >= self.GROUPED_MIN_TOKENS:
+        if self._grouped(n):
             K.moe_grouped(h, self.w_gate_up, self.w_down, idx, y, gated=self.gated, in_w=in_w, limit=self.limit, alpha=self.alpha,
                           up_offset=self.up_offset)
         else:

@@ -1,0 +1,119 @@
+"""The experts' products at the edges of their kernels: experts with no rows, one row, and row counts around 16, a tile and its
+halves; inner sizes that do and do not fill a feature tile; every activation; few tokens that share experts."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _exact(h, w1, w2, idx, act, in_w, limit, alpha, off):
+    n, top = idx.shape
+    f = w2.shape[2]
+    y = torch.zeros(n, top, w2.shape[1], dtype=torch.float64, device=h.device)
+    for e in range(w1.shape[0]):
+        t, k = torch.nonzero(idx == e, as_tuple=True)
+        if not len(t):
+            continue
+        z = h[t].double() @ w1[e].double().T
+        if act == "relu2":
+            a = z.clamp(min=0.0) ** 2
+        else:
+            g, u = z[:, :f], z[:, f:]
+            if act == "clamped":
+                s = in_w[t, k].double()[:, None]
+                g, u = (g * s).clamp(max=limit), (u * s).clamp(-limit, limit)
+                a = g * torch.sigmoid(alpha * g) * (u + off)
+            else:
+                a = g * torch.sigmoid(g) * u
+        y[t, k] = a @ w2[e].double().T
+    return y.reshape(n * top, -1)
+
+
+def _case(n, top, e, width, f, act, rows=None, seed=0):
+    gen = torch.Generator(device="cuda").manual_seed(seed + 7 * n + width + f)
+    randn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    h = randn(n, width).bfloat16()
+    w1 = (randn(e, f if act == "relu2" else 2 * f, width) * width ** -0.5).bfloat16()
+    w2 = (randn(e, width, f) * f ** -0.5).bfloat16()
+    if rows is None:
+        idx = torch.argsort(torch.rand(n, e, generator=gen, device="cuda"), dim=1)[:, :top].to(torch.int32).contiguous()
+    else:      # expert i is chosen rows[i] times, in a mixed order (top == 1)
+        idx = torch.repeat_interleave(torch.arange(len(rows), device="cuda"), torch.tensor(rows, device="cuda"))
+        idx = idx[torch.randperm(len(idx), generator=gen, device="cuda")].to(torch.int32)[:, None].contiguous()
+    in_w = torch.rand(idx.shape, generator=gen, device="cuda") + 0.2
+    return h, w1, w2, idx, in_w
+
+
+def _check(y, exact):
+    # two bfloat16 roundings on the way (the activation, the result), each half a unit in 2^8 of its value
+    err = (y.double() - exact).norm() / exact.norm()
+    assert float(err) < 2.0 * 2.0 ** -8, float(err)
+    assert float((y.double() - exact).abs().max()) < 2.0 ** -5 * float(exact.abs().max())
+
+
+ROWS = [0, 1, 15, 16, 17, 0, 64, 65, 127, 128, 129, 200, 255, 256, 257, 3]
+
+
+@pytest.mark.parametrize("act", ["silu", "relu2", "clamped"])
+@pytest.mark.parametrize("width,f,rows", [
+    (128, 64, ROWS),                                   # two tiles of accumulators (128 rows a tile), less than a feature tile
+    (64, 192, ROWS),                                   # one k slice, a feature tile and a half
+    (192, 320, [r * 6 for r in ROWS]),                 # tiles of 256 rows
+    (256, 128, [700, 0, 1, 513]),
+    (48, 80, ROWS), (112, 64, [r * 2 for r in ROWS]),  # inner sizes that the mma.sync products take
+])
+def test_grouped_products(act, width, f, rows):
+    from dryft_b200.ops import kernels as K
+
+    h, w1, w2, idx, in_w = _case(sum(rows), 1, len(rows), width, f, act, rows)
+    y = torch.full((idx.numel(), width), float("nan"), dtype=torch.bfloat16, device="cuda")
+    K.moe_grouped(h, w1, w2, idx, y, gated=act != "relu2", in_w=in_w if act == "clamped" else None, limit=1.5, alpha=1.702, up_offset=1.0)
+    _check(y, _exact(h, w1, w2, idx, act, in_w, 1.5, 1.702, 1.0))
+    K.check_error_flags()
+
+
+def test_grouped_products_of_many_assignments():
+    from dryft_b200.ops import kernels as K
+
+    # more assignments than the sorting block keeps in registers, more experts than it has tables for every warp
+    h, w1, w2, idx, in_w = _case(5000, 4, 500, 64, 64, "silu")
+    y = torch.empty((idx.numel(), 64), dtype=torch.bfloat16, device="cuda")
+    K.moe_grouped(h, w1, w2, idx, y)
+    _check(y, _exact(h, w1, w2, idx, "silu", in_w, 0, 0, 0))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,top,e,width,f", [(1, 1, 1, 64, 24), (5, 3, 7, 128, 33), (16, 8, 24, 256, 72), (32, 8, 9, 64, 40), (4, 2, 64, 72, 16)])
+def test_few_tokens_that_share_experts(dtype, n, top, e, width, f):
+    """An expert's weights read once for all its assignments give the bits that one assignment alone gives."""
+    from dryft_b200.ops import kernels as K
+
+    h, w1, _, idx, in_w = _case(n, top, e, width, f, "silu")
+    h, w1 = h.to(dtype), w1.to(dtype)
+    for mode, w in (("gate_up", w1), ("down", w1), ("up_relu2", w1), ("gate_up_clamp", w1)):
+        outs = w.shape[1] // 2 if mode.startswith("gate") else w.shape[1]
+        kw = dict(in_w=in_w, limit=1.5, alpha=1.702, up_offset=1.0) if mode == "gate_up_clamp" else {}
+        x = h if mode != "down" else torch.randn(n * top, width, device="cuda").to(dtype)
+        out = torch.full((n * top, outs), float("nan"), dtype=dtype, device="cuda")
+        K.moe_rows(x, w, idx, out, mode, **kw)
+        for t in range(0, n, 3):
+            alone = torch.empty((top, outs), dtype=dtype, device="cuda")
+            if kw:
+                kw["in_w"] = in_w[t:t + 1].contiguous()
+            K.moe_rows(x[t:t + 1] if mode != "down" else x[t * top:(t + 1) * top], w, idx[t:t + 1].contiguous(), alone, mode, **kw)
+            assert torch.equal(alone, out[t * top:(t + 1) * top]), mode
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("n,top,width", [(1, 1, 1), (3, 8, 64), (7, 9, 1000), (2, 17, 2056), (5, 2, 77)])
+def test_weighted_sum(dtype, n, top, width):
+    from dryft_b200.ops import kernels as K
+
+    y, wts = torch.randn(n * top, width, device="cuda").to(dtype), torch.rand(n, top, device="cuda")
+    out = torch.empty(n, width, dtype=dtype, device="cuda")
+    K.moe_combine(y, wts, out)
+    exact = (y.double().view(n, top, width) * wts.double()[..., None]).sum(1)
+    unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23
+    bound = unit * exact.abs() + 2.0 ** -23 * top * (y.double().view(n, top, width).abs() * wts.double()[..., None]).sum(1)
+    assert bool(((out.double() - exact).abs() <= bound).all())
