@@ -3,8 +3,8 @@
 // F.linear with TF32 switched off (engine/engine.py:32-33; engine/dryft_qwen3/model.py:153),
 // and is the matrix product of the library's 32-bit path.
 //
-// One order of additions for every shape: k is cut into chunks of 64, a chunk is accumulated in order from zero by
-// one thread, and the chunks' sums are added in order.  So a row's result does not depend on how many other rows are
+// One order of additions for every inner size: up to K = 256 one chain in order; beyond it k is cut into chunks of 64, a chunk is
+// accumulated in order from zero by one thread, and the chunks' sums are added in order.  So a row's result does not depend on how many other rows are
 // in the batch or on which of the kernels below ran: in the 32-bit path the same token gives bit-identical
 // projections whether it is run alone, in a prompt or in a batch.  (The order lets few rows spread k over threads, and
 // is closer to the exact sum than one chain of K additions: 1.7e-7 against 5.6e-7 at K = 1,030, 2.8e-7 against 1.8e-6 at
@@ -14,6 +14,7 @@
 
 namespace {
 constexpr int CH = 64;        // k per chunk
+constexpr int ONE_CHAIN = 256;   // inner sizes up to this are one chunk (of the tiles)
 constexpr int CHP = CH + 4;   // a chunk of activations in shared memory: chunks start in different banks
 
 template <int VEC> __device__ __forceinline__ void copy_async(float* dst, const float* src, bool there) {
@@ -185,7 +186,8 @@ __global__ void __launch_bounds__(TILE_THREADS) gemm_f32_tile_kernel(const float
   const int tx = tid % TX, ty = tid / TX;      // rows 4 ty + i and 32 + 4 ty + i, columns 4 tx + j
   const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
   float* const ring = reinterpret_cast<float*>(smem4) + tid * 4;      // [RING][(PA + PW) / 4][threads] of 4 floats
-  const int slices = (K + BK - 1) / BK;
+  const int slices = (K + BK - 1) / BK, per_chunk = K <= ONE_CHAIN ? slices : CH / BK;
+  int to_go = per_chunk;
   auto fetch4 = [&](float* to, const float* base, int ld, int row, int rows, int k) {
     const float* p = base + (size_t)row * ld + k;
 #pragma unroll
@@ -253,11 +255,12 @@ __global__ void __launch_bounds__(TILE_THREADS) gemm_f32_tile_kernel(const float
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = fmaf(a[kk & 1][i], w[kk & 1][j], acc[i][j]);
     }
-    if ((s + 1) % (CH / BK) == 0 || !more) {   // the chunk is complete
+    if (--to_go == 0 || !more) {   // the chunk is complete
 #pragma unroll
       for (int i = 0; i < TM; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) { total[i][j] += acc[i][j]; acc[i][j] = 0.f; }
+      to_go = per_chunk;
     }
   }
 #pragma unroll
@@ -303,7 +306,7 @@ DRYFT_API int dryft_gemm_nt_f32(const float* A, int lda, const float* W, float* 
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int rows = few_rows(M, N, K, sms);
+  const int rows = K <= ONE_CHAIN ? 0 : few_rows(M, N, K, sms);
   if (rows)
     return vec ? launch_few_m<4>(A, lda, W, C, ldc, M, N, K, rows, sms, st) : launch_few_m<1>(A, lda, W, C, ldc, M, N, K, rows, sms, st);
   return vec ? launch_tile<4>(A, lda, W, C, ldc, M, N, K, st) : launch_tile<1>(A, lda, W, C, ldc, M, N, K, st);

@@ -444,21 +444,22 @@ __global__ void head_gate_rows_kernel(const T* __restrict__ o, int hd, const T* 
 //   latent_fold_q     q_lat[h, n, r] = sum_d q[n, h, d] * w_k[h, d, r]                      (32-bit result)
 //   latent_unfold_o   out[n, h*V + v] = T( sigmoid(gate[n, h]) * sum_r o_lat[h, n, r] * w_v[h, r, v] )
 // One block per (token, head, FOLD_COLS columns).  A thread takes VN neighbouring columns (16 bytes) of every FOLD_THREADS /
-// (FOLD_COLS / VN)-th matrix row, requested before the vector is read; the threads' sums are added in order.  One token and head of 512 x 128:
+// (FOLD_COLS / VN)-th matrix row (of up to 64 rows: of every row), requested before the vector is read; the threads' sums are added in order.  One token and head of 512 x 128:
 // 3 us, where a thread per column along all rows took 18 (64 trips to memory).
 constexpr int FOLD_COLS = 128, FOLD_THREADS = 512;
 
-// out(c, sum_i vin(i) * w[i, c]) for the columns c0 .. c0 + FOLD_COLS - 1 of a [rows, cols] matrix
-template <typename T, int VN, typename In, typename Out>
-__device__ __forceinline__ void fold_columns(const T* __restrict__ w, int rows, int cols, int c0, float* vin, float* red, In in, Out out) {
-  constexpr int LR = FOLD_COLS / VN, G = FOLD_THREADS / LR, AHEAD = 16;
+// out(c, sum_i vin(i) * w[i, c]) for the columns c0 .. c0 + FOLD_COLS - 1 of a [rows, cols] matrix; G threads share a column
+template <typename T, int VN, int G, typename In, typename Out>
+__device__ __forceinline__ void fold_columns_by(const T* __restrict__ w, int rows, int cols, int c0, float* vin, float* red, In in, Out out) {
+  constexpr int LR = FOLD_COLS / VN, AHEAD = 16;
   const int c = c0 + (threadIdx.x % LR) * VN, g = threadIdx.x / LR;
+  const bool on = g < G && c < cols;
   alignas(16) T wv[AHEAD][VN];
   auto request = [&](int i0) {
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u) {
       const int i = i0 + u * G;
-      if (i < rows && c < cols) {
+      if (i < rows && on) {
         if (VN > 1) *reinterpret_cast<uint4*>(wv[u]) = *reinterpret_cast<const uint4*>(w + (size_t)i * cols + c);
         else wv[u][0] = w[(size_t)i * cols + c];
       }
@@ -474,7 +475,7 @@ __device__ __forceinline__ void fold_columns(const T* __restrict__ w, int rows, 
     if (i0 != g) request(i0);
 #pragma unroll
     for (int u = 0; u < AHEAD; ++u) {
-      if (i0 + u * G >= rows || c >= cols) continue;
+      if (i0 + u * G >= rows || !on) continue;
       const float x = vin[i0 + u * G];
 #pragma unroll
       for (int j = 0; j < VN; ++j) acc[j] = fmaf(x, to_f32<T>(wv[u][j]), acc[j]);
@@ -484,11 +485,16 @@ __device__ __forceinline__ void fold_columns(const T* __restrict__ w, int rows, 
   for (int j = 0; j < VN; ++j) red[g * FOLD_COLS + (threadIdx.x % LR) * VN + j] = acc[j];
   __syncthreads();
   for (int j = threadIdx.x; j < FOLD_COLS && c0 + j < cols; j += FOLD_THREADS) {
-    float sum = 0.f;
+    float sum = red[j];
 #pragma unroll
-    for (int k = 0; k < G; ++k) sum += red[k * FOLD_COLS + j];
+    for (int k = 1; k < G; ++k) sum += red[k * FOLD_COLS + j];
     out(c0 + j, sum);
   }
+}
+template <typename T, int VN, typename In, typename Out>
+__device__ __forceinline__ void fold_columns(const T* __restrict__ w, int rows, int cols, int c0, float* vin, float* red, In in, Out out) {
+  if (rows <= 64) fold_columns_by<T, VN, 1>(w, rows, cols, c0, vin, red, in, out);      // few rows: one thread a column, in order
+  else fold_columns_by<T, VN, FOLD_THREADS / (FOLD_COLS / VN)>(w, rows, cols, c0, vin, red, in, out);
 }
 template <int VN> constexpr size_t fold_smem(int rows) { return sizeof(float) * ((size_t)rows + FOLD_THREADS * VN); }
 
