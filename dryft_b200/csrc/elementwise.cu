@@ -133,6 +133,7 @@ template <typename T> __device__ __forceinline__ void store_vec(T* p, const floa
 template <typename T>
 __global__ void rmsnorm_kernel(const T* x, const T* __restrict__ delta, const float* __restrict__ w,
                                const int* __restrict__ rows, T* x_out, T* __restrict__ h, int hidden, float eps, int aligned) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
   // x and x_out may be the same buffer (in-place residual update): no __restrict__ on them
   extern __shared__ __align__(16) float row[];  // hidden floats + 33 scratch
   float* scratch = row + ((hidden + 3) & ~3);
