@@ -68,19 +68,48 @@ DRYFT_API int dryft_tokens_from_state(const int* seq_slot, const int* last_token
   return launch_status();
 }
 
+// A decode step's beginning in one launch: every sequence's next token and position from the per-sequence state, and its
+// length with the token that the step appends (the step itself goes by tok_pos).  Three launches of 1.6 us, which took more
+// than a hundredth of a small model's step.
+__global__ void decode_begin_kernel(const int* __restrict__ seq_slot, const int* __restrict__ last_token, int* __restrict__ seq_len,
+                                    int* __restrict__ tokens, int* __restrict__ tok_slot, int* __restrict__ tok_pos, int n_seqs) {
+  const int b = blockIdx.x * blockDim.x + threadIdx.x;
+  if (b >= n_seqs) return;
+  const int slot = seq_slot[b];
+  tok_slot[b] = slot;
+  if (slot < 0) {
+    tokens[b] = 0;
+    tok_pos[b] = 0;
+    return;
+  }
+  const int pos = seq_len[slot];
+  tokens[b] = last_token[slot];
+  tok_pos[b] = pos;
+  seq_len[slot] = pos + 1;
+}
+DRYFT_API int dryft_decode_begin(const int* seq_slot, const int* last_token, int* seq_len, int* tokens, int* tok_slot, int* tok_pos, int n_seqs,
+                                 cudaStream_t st) {
+  if (n_seqs <= 0) return 0;
+  decode_begin_kernel<<<(n_seqs + 127) / 128, 128, 0, st>>>(seq_slot, last_token, seq_len, tokens, tok_slot, tok_pos, n_seqs);
+  return launch_status();
+}
+
 // ------------------------------------------------------------------------------------------
 // Embedding gather: out[n, :] = table[tokens[n], :].  A token id outside [0, vocab) yields a
-// zero row and raises *err (the host validates ids first; this is the second fence).
+// zero row and raises *err (the host validates ids first; this is the second fence).  With `ss` it also leaves each row's
+// sum of squares for the first product of a step of few rows, added in the order of row_sumsq_kernel (256 threads).
 // ------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void embed_kernel(const int* __restrict__ tokens, const T* __restrict__ table, T* __restrict__ out,
-                             int hidden, int vocab, int* __restrict__ err) {
+                             int hidden, int vocab, int* __restrict__ err, float* __restrict__ ss) {
+  __shared__ float scratch[33];
   const int n = blockIdx.x;
   const int tok = tokens[n];
   T* o = out + (size_t)n * hidden;
   if (tok < 0 || tok >= vocab) {
     for (int i = threadIdx.x; i < hidden; i += blockDim.x) o[i] = from_f32<T>(0.f);
     if (threadIdx.x == 0 && err) atomicExch(err, 1);
+    if (threadIdx.x == 0 && ss) ss[n] = 0.f;
     return;
   }
   const T* src = table + (size_t)tok * hidden;
@@ -92,18 +121,27 @@ __global__ void embed_kernel(const int* __restrict__ tokens, const T* __restrict
   } else {
     for (int i = threadIdx.x; i < hidden; i += blockDim.x) o[i] = src[i];
   }
+  if (ss) {
+    float s = 0.f;
+    for (int i = threadIdx.x; i < hidden; i += blockDim.x) {
+      const float v = to_f32<T>(src[i]);
+      s += v * v;
+    }
+    s = block_sum(s, scratch);
+    if (threadIdx.x == 0) ss[n] = s;
+  }
 }
 
 template <typename T>
-static int embed_launch(const int* tokens, const void* table, void* out, int n, int hidden, int vocab, int* err, cudaStream_t st) {
+static int embed_launch(const int* tokens, const void* table, void* out, int n, int hidden, int vocab, int* err, float* ss, cudaStream_t st) {
   if (n <= 0) return 0;
-  embed_kernel<T><<<n, 128, 0, st>>>(tokens, (const T*)table, (T*)out, hidden, vocab, err);
+  embed_kernel<T><<<n, ss ? 256 : 128, 0, st>>>(tokens, (const T*)table, (T*)out, hidden, vocab, err, ss);
   return launch_status();
 }
 DRYFT_API int dryft_embed(int is_bf16, const int* tokens, const void* table, void* out, int n, int hidden, int vocab,
-                          int* err, cudaStream_t st) {
-  return is_bf16 ? embed_launch<__nv_bfloat16>(tokens, table, out, n, hidden, vocab, err, st)
-                 : embed_launch<float>(tokens, table, out, n, hidden, vocab, err, st);
+                          int* err, float* ss, cudaStream_t st) {
+  return is_bf16 ? embed_launch<__nv_bfloat16>(tokens, table, out, n, hidden, vocab, err, ss, st)
+                 : embed_launch<float>(tokens, table, out, n, hidden, vocab, err, ss, st);
 }
 
 // ------------------------------------------------------------------------------------------

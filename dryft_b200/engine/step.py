@@ -291,14 +291,11 @@ class _DecodeGraph:
 
     def _body(self) -> torch.Tensor:
         st = self.st
-        K.tokens_from_state(self.seq_slot, st.cache.last_token, self.tokens, self.bucket)
-        K.step_meta(self.cu_q, self.seq_slot, st.cache.seq_len, self.tok_slot, self.tok_pos, self.bucket, self.bucket)
+        K.decode_begin(self.seq_slot, st.cache.last_token, st.cache.seq_len, self.tokens, self.tok_slot, self.tok_pos, self.bucket)
         ctx = StepContext(n_tokens=self.bucket, n_seqs=self.bucket, tokens=self.tokens, cu_q=self.cu_q,
                           seq_slot=self.seq_slot, tok_slot=self.tok_slot, tok_pos=self.tok_pos, decode=True,
                           max_kv=self.kv_bucket)
-        logits = st.model.forward(ctx, st.cache, self.rows, self.bucket, all_rows=True)
-        K.step_advance(self.cu_q, self.seq_slot, st.cache.seq_len, self.bucket)
-        return logits
+        return st.model.forward(ctx, st.cache, self.rows, self.bucket, all_rows=True)
 
     def run(self, slots: Sequence[int]) -> torch.Tensor:
         n = len(slots)

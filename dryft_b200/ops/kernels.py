@@ -52,7 +52,8 @@ def core() -> ctypes.CDLL:
             lib.dryft_step_meta.argtypes = [_p, _p, _p, _i, _i, _p, _p, _p]
             lib.dryft_step_advance.argtypes = [_p, _p, _p, _i, _p]
             lib.dryft_tokens_from_state.argtypes = [_p, _p, _p, _i, _p]
-            lib.dryft_embed.argtypes = [_i, _p, _p, _p, _i, _i, _i, _p, _p]
+            lib.dryft_decode_begin.argtypes = [_p, _p, _p, _p, _p, _p, _i, _p]
+            lib.dryft_embed.argtypes = [_i, _p, _p, _p, _i, _i, _i, _p, _p, _p]
             lib.dryft_rmsnorm.argtypes = [_i, _p, _p, _p, _p, _p, _p, _i, _i, _f, _p]
             lib.dryft_residual_add.argtypes = [_i, _p, _p, _ll, _p]
             lib.dryft_silu_mul.argtypes = [_i, _p, _p, _i, _i, _p]
@@ -72,7 +73,7 @@ def core() -> ctypes.CDLL:
             lib.dryft_moe_rows.argtypes = [_i, _p, _i, _p, _p, _i, _i, _i, _i, _p, _i, _p, _f, _f, _f, _p]
             lib.dryft_moe_combine.argtypes = [_i, _p, _p, _i, _i, _p, _i, _p]
             lib.dryft_moe_route_rows.argtypes = [_i, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _p, _p, _p]
-            for name in ("dryft_step_meta", "dryft_step_advance", "dryft_tokens_from_state", "dryft_embed",
+            for name in ("dryft_step_meta", "dryft_step_advance", "dryft_tokens_from_state", "dryft_decode_begin", "dryft_embed",
                          "dryft_rmsnorm", "dryft_residual_add", "dryft_silu_mul", "dryft_qk_norm_rope_store", "dryft_rope_table",
                          "dryft_gemm_nt_f32", "dryft_argmax_rows", "dryft_sample_rows", "dryft_gemm_small_m", "dryft_row_sumsq",
                          "dryft_embed_sinusoid", "dryft_stream_norm_add", "dryft_stream_norm_rows", "dryft_kv_maps_store",
@@ -378,7 +379,19 @@ def tokens_from_state(seq_slot, last_token, tokens, n_seqs: int) -> None:
 
 
 # ----------------------------------------------------------------------------- elementwise
-def embed(tokens, table, out, err=None) -> None:
+def decode_begin(seq_slot, last_token, seq_len, tokens, tok_slot, tok_pos, n_seqs: int) -> None:
+    """A decode step's tokens, slots and positions from the per-sequence state, whose lengths go up by the step's token:
+    ``tokens_from_state``, ``step_meta`` and ``step_advance`` of one token a sequence in one launch."""
+    for t, n in ((seq_slot, "seq_slot"), (last_token, "last_token"), (seq_len, "seq_len"), (tokens, "tokens"), (tok_slot, "tok_slot"), (tok_pos, "tok_pos")):
+        _need(t, n, torch.int32)
+    if min(seq_slot.numel(), tokens.numel(), tok_slot.numel(), tok_pos.numel()) < n_seqs:
+        raise KernelError("decode_begin: index arrays shorter than the batch")
+    _ok(core().dryft_decode_begin(_ptr(seq_slot), _ptr(last_token), _ptr(seq_len), _ptr(tokens), _ptr(tok_slot), _ptr(tok_pos), n_seqs, _stream()),
+        "decode_begin")
+
+
+def embed(tokens, table, out, err=None, ss=None) -> None:
+    """``out[n] = table[tokens[n]]``; ``ss`` (float32, 64 floats, up to 64 rows): the rows' sums of squares too."""
     _need(tokens, "tokens", torch.int32)
     _need(table, "embedding table")
     n = out.shape[0]
@@ -387,8 +400,12 @@ def embed(tokens, table, out, err=None) -> None:
         raise KernelError("embed: fewer tokens than output rows")
     if err is not None:
         _need(err, "err", torch.int32)
+    if ss is not None:
+        _need(ss, "ss", torch.float32)
+        if n > SS_STRIDE or ss.numel() < SS_STRIDE:
+            raise KernelError("embed: sums of squares are left for up to 64 rows, in 64 floats")
     _ok(core().dryft_embed(_act(table, "embedding table"), _ptr(tokens), _ptr(table), _ptr(out), n, table.shape[1],
-                           table.shape[0], _ptr(err), _stream()), "embed")
+                           table.shape[0], _ptr(err), _ptr(ss), _stream()), "embed")
 
 
 def rmsnorm(x, weight, eps: float, out, delta=None, rows=None, x_out=None) -> None:

@@ -38,7 +38,13 @@ class Embedding:
 
     def forward(self, tokens: torch.Tensor, n_rows: int):
         out = torch.empty((n_rows, self.hidden), dtype=self.table.dtype, device=self.table.device)
-        K.embed(tokens, self.table, out, self.err)
+        # few rows: the sums of squares for a first product that normalises its input itself come with the rows
+        few = (self.rt.is_bf16 and self.rt.fuse_decode and not self.stream32 and not self.rt.norm_ahead and n_rows <= K.SS_STRIDE
+               and out.dtype == self.rt.dtype and fusable_rows(n_rows, self.hidden, self.rt, normed=True))
+        ss = torch.empty(K.SS_STRIDE, dtype=torch.float32, device=out.device) if few else None
+        K.embed(tokens, self.table, out, self.err, ss)
+        if few:
+            return Residual(out, None, ss, 1)
         # a table the checkpoint stores in 32-bit stays 32-bit; its rows are rounded on the way out
         h = out if out.dtype == self.rt.dtype else out.to(self.rt.dtype)
         if self.stream32:

@@ -1,0 +1,41 @@
+"""A decode step's first launches: tokens, slots, positions and lengths in one, the embedding's rows with their sums of squares."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,slots", [(1, 1), (8, 9), (64, 70), (129, 300)])
+def test_decode_begin_is_the_three_launches(n, slots):
+    from dryft_b200.ops import kernels as K
+
+    gen = torch.Generator().manual_seed(n)
+    i32 = lambda t: t.to(torch.int32).cuda()
+    seq_slot = torch.randperm(slots, generator=gen)[:n]
+    seq_slot[n // 2::3] = -1                                # padding rows
+    seq_slot, last, lens = i32(seq_slot), i32(torch.randint(0, 1000, (slots,), generator=gen)), i32(torch.randint(0, 5000, (slots,), generator=gen))
+    want = [torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(3)]
+    got = [torch.full_like(t, -7) for t in want]
+    cu = torch.arange(n + 1, dtype=torch.int32, device="cuda")
+    lens_then = lens.clone()
+    K.tokens_from_state(seq_slot, last, want[0], n)
+    K.step_meta(cu, seq_slot, lens_then, want[1], want[2], n, n)
+    K.step_advance(cu, seq_slot, lens_then, n)
+    K.decode_begin(seq_slot, last, lens, got[0], got[1], got[2], n)
+    assert all(torch.equal(a, b) for a, b in zip(got, want)) and torch.equal(lens, lens_then)
+
+
+@pytest.mark.parametrize("n,hidden", [(1, 1024), (16, 2560), (64, 80), (3, 37)])
+def test_embedding_rows_with_their_sums_of_squares(n, hidden):
+    from dryft_b200.ops import kernels as K
+
+    table = torch.randn(50, hidden, device="cuda").bfloat16()
+    toks = torch.randint(0, 50, (n,), device="cuda").to(torch.int32)
+    toks[n // 2] = 50 if n > 1 else toks[0]                  # outside the table: a row of zeros
+    rows, ss, err = torch.empty(n, hidden, dtype=torch.bfloat16, device="cuda"), torch.full((64,), -1.0, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    K.embed(toks, table, rows, err, ss)
+    plain, ss2 = torch.empty_like(rows), torch.empty(64, device="cuda")
+    K.embed(toks, table, plain)
+    K.row_sumsq(plain, ss2)
+    assert torch.equal(rows, plain) and torch.equal(ss[:n], ss2[:n]) and int(err) == (1 if n > 1 else 0)
