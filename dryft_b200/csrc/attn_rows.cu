@@ -100,16 +100,27 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
     const T* kp = k_pages + ((size_t)page * nKV + kvh) * PAGE * D;
     const T* vp = v_pages + ((size_t)page * nKV + kvh) * PAGE * D;
     __syncthreads();  // previous tile fully consumed
-    for (int i = tid; i < PAGE * VPR; i += THREADS) {
-      const int r = i / VPR, c = i % VPR;
-      const int p = p0 + r;
-      uint4 kv4 = make_uint4(0, 0, 0, 0), vv4 = make_uint4(0, 0, 0, 0);
-      if (p >= kv_lo && p < kv_hi) {
-        kv4 = reinterpret_cast<const uint4*>(kp + (size_t)r * D)[c];
-        vv4 = reinterpret_cast<const uint4*>(vp + (size_t)r * D)[c];
+    // eight words of K and of V on their way at once (two at a time left a page eight trips to memory long)
+    constexpr int AHEAD = 8;
+    for (int i0 = tid; i0 < PAGE * VPR; i0 += AHEAD * THREADS) {
+      uint4 kv4[AHEAD], vv4[AHEAD];
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) {
+        const int i = i0 + u * THREADS, r = i / VPR, c = i % VPR, p = p0 + r;
+        kv4[u] = vv4[u] = make_uint4(0, 0, 0, 0);
+        if (i < PAGE * VPR && p >= kv_lo && p < kv_hi) {
+          kv4[u] = reinterpret_cast<const uint4*>(kp + (size_t)r * D)[c];
+          vv4[u] = reinterpret_cast<const uint4*>(vp + (size_t)r * D)[c];
+        }
       }
-      *reinterpret_cast<uint4*>(kt + r * L::KSTRIDE + c * L::VEC) = kv4;
-      *reinterpret_cast<uint4*>(vt + r * D + c * L::VEC) = vv4;
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u) {
+        const int i = i0 + u * THREADS, r = i / VPR, c = i % VPR;
+        if (i < PAGE * VPR) {
+          *reinterpret_cast<uint4*>(kt + r * L::KSTRIDE + c * L::VEC) = kv4[u];
+          *reinterpret_cast<uint4*>(vt + r * D + c * L::VEC) = vv4[u];
+        }
+      }
     }
     __syncthreads();
     // scores: item -> (head g, key r); consecutive threads take consecutive keys
@@ -120,15 +131,21 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
       if (p >= kv_lo && p < kv_hi) {
         const T* kr = kt + r * L::KSTRIDE;
         const float* qg = qs + g * D;
-        float dot = 0.f;
+        float dot[4] = {0.f, 0.f, 0.f, 0.f};      // four chains of D / 4: one of D waits for every addition
 #pragma unroll 4
         for (int c = 0; c < VPR; ++c) {
           uint4 raw = *reinterpret_cast<const uint4*>(kr + c * L::VEC);
           const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
-          for (int t = 0; t < L::VEC; ++t) dot = fmaf(qg[c * L::VEC + t], to_f32<T>(e[t]), dot);
+          for (int t = 0; t < L::VEC; t += 4) {
+            const float4 q4 = *reinterpret_cast<const float4*>(qg + c * L::VEC + t);
+            dot[0] = fmaf(q4.x, to_f32<T>(e[t]), dot[0]);
+            dot[1] = fmaf(q4.y, to_f32<T>(e[t + 1]), dot[1]);
+            dot[2] = fmaf(q4.z, to_f32<T>(e[t + 2]), dot[2]);
+            dot[3] = fmaf(q4.w, to_f32<T>(e[t + 3]), dot[3]);
+          }
         }
-        s = dot * scale;
+        s = ((dot[0] + dot[1]) + (dot[2] + dot[3])) * scale;
       }
       sc[item] = s;
     }
@@ -163,6 +180,7 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
       if (d < D) {
 #pragma unroll
         for (int g = 0; g < G; ++g) acc[i][g] *= a_s[g];
+#pragma unroll 8
         for (int r = 0; r < PAGE; ++r) {
           const float v = to_f32<T>(vt[r * D + d]);
 #pragma unroll
