@@ -147,36 +147,60 @@ __device__ __forceinline__ bool locate_chunk(const int* __restrict__ cu_q, int n
   return false;
 }
 
-// rows [L][ld] of shared memory <- the rotated (and scaled) head vectors of L tokens; columns dim..ld-1 are zeroed
+// (sin, cos) of every token's angles, [n_tokens][rot / 2]: worked out once a launch of the chunked form.  Every head's blocks
+// of both products evaluated them anew before, which was a third of those blocks' time.
+__global__ void retention_angles_kernel(const int* __restrict__ tok_pos, const float* __restrict__ inv_freq, const float* __restrict__ inv_freq_lo,
+                                        float2* __restrict__ angles, int n_tokens, int half) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n_tokens * half) return;
+  const int n = i / half, j = i - n * half;
+  float sn, cs;
+  sincos_split((float)tok_pos[n], inv_freq[j], inv_freq_lo ? inv_freq_lo[j] : 0.f, &sn, &cs);
+  angles[i] = make_float2(sn, cs);
+}
+
+// rows [L][ld] of shared memory <- the rotated (and scaled) head vectors of L tokens; columns dim..ld-1 are zeroed.  A warp a row, a
+// lane both halves of a rotated pair.  `last_first`: a row's further factor, last_first[L - 1 - t].
 template <typename T>
 __device__ __forceinline__ void load_rotated(float* dst, int ld, const T* __restrict__ proj, int ldp, int col0, int n_first, int L,
-                                             int dim, int rot, const float* __restrict__ inv_freq,
-                                             const float* __restrict__ inv_freq_lo, const int* __restrict__ tok_pos, float scale) {
-  const int half = rot >> 1;
-  for (int idx = threadIdx.x; idx < L * ld; idx += CK_THREADS) {
-    const int t = idx / ld, d = idx % ld;
-    float val = 0.f;
-    if (d < dim) {
-      const T* src = proj + (size_t)(n_first + t) * ldp + col0;
-      val = to_f32<T>(src[d]);
-      if (d < rot) {
-        const int j = d < half ? d : d - half;
-        const float other = to_f32<T>(src[d < half ? d + half : d - half]);
-        float sn, cs;
-        sincos_split((float)tok_pos[n_first + t], inv_freq[j], inv_freq_lo ? inv_freq_lo[j] : 0.f, &sn, &cs);
-        val = d < half ? val * cs - other * sn : val * cs + other * sn;
-      }
-      val *= scale;
+                                             int dim, int rot, const float2* __restrict__ angles, float scale, const float* last_first = nullptr) {
+  const int half = rot >> 1, lane = threadIdx.x & 31;
+  for (int t = threadIdx.x >> 5; t < L; t += CK_THREADS / 32) {
+    const T* src = proj + (size_t)(n_first + t) * ldp + col0;
+    const float2* ang = angles + (size_t)(n_first + t) * half;
+    float* to = dst + t * ld;
+    const float more = last_first ? last_first[L - 1 - t] : 1.f;
+#pragma unroll 2
+    for (int d = lane; d < half; d += 32) {
+      const float a = to_f32<T>(src[d]), b = to_f32<T>(src[d + half]);
+      const float2 sc = ang[d];
+      float u = (a * sc.y - b * sc.x) * scale, v = (b * sc.y + a * sc.x) * scale;
+      if (last_first) { u *= more; v *= more; }
+      to[d] = u;
+      to[d + half] = v;
     }
-    dst[t * ld + d] = val;
+    for (int d = rot + lane; d < ld; d += 32) {
+      float u = d < dim ? to_f32<T>(src[d]) * scale : 0.f;
+      if (last_first) u *= more;
+      to[d] = u;
+    }
+  }
+}
+template <typename T>
+__device__ __forceinline__ void load_values(float* dst, int ld, const T* __restrict__ proj, int ldp, int col0, int n_first, int L, int rows, int vdim) {
+  const int lane = threadIdx.x & 31;
+  for (int t = threadIdx.x >> 5; t < rows; t += CK_THREADS / 32) {
+    const T* src = proj + (size_t)(n_first + t) * ldp + col0;
+#pragma unroll 4
+    for (int v = lane; v < ld; v += 32) dst[t * ld + v] = t < L && v < vdim ? to_f32<T>(src[v]) : 0.f;
   }
 }
 
 template <typename T>
 __global__ void __launch_bounds__(CK_THREADS) retention_chunk_state_kernel(
     const T* __restrict__ proj, int ld, int k_off, int v_off, const int* __restrict__ cu_q, const int* __restrict__ seq_slot,
-    int n_seqs, const int* __restrict__ tok_pos, const float* __restrict__ inv_freq, const float* __restrict__ inv_freq_lo,
-    int rot, const double* __restrict__ decay, float* __restrict__ sbuf, int H, int dim, int vdim, float k_scale) {
+    int n_seqs, const float2* __restrict__ angles, int rot, const double* __restrict__ decay, float* __restrict__ sbuf, int H, int dim,
+    int vdim, float k_scale) {
   extern __shared__ __align__(16) float smem[];
   __shared__ int loc[3];
   const int g = blockIdx.x, hd = blockIdx.y;
@@ -193,13 +217,9 @@ __global__ void __launch_bounds__(CK_THREADS) retention_chunk_state_kernel(
   float* vs = ks + CH * dP;         // [CH][vP]
   float* pw = vs + CH * vP;         // [CH + 1]
   for (int i = threadIdx.x; i <= CH; i += CK_THREADS) pw[i] = (float)pow(decay[hd], (double)i);
-  load_rotated<T>(ks, dP, proj, ld, k_off + hd * dim, n_first, L, dim, rot, inv_freq, inv_freq_lo, tok_pos, k_scale);
-  for (int idx = threadIdx.x; idx < L * vP; idx += CK_THREADS) {
-    const int t = idx / vP, v = idx % vP;
-    vs[idx] = v < vdim ? to_f32<T>(proj[(size_t)(n_first + t) * ld + v_off + hd * vdim + v]) : 0.f;
-  }
   __syncthreads();
-  for (int idx = threadIdx.x; idx < L * dP; idx += CK_THREADS) ks[idx] *= pw[L - 1 - idx / dP];
+  load_rotated<T>(ks, dP, proj, ld, k_off + hd * dim, n_first, L, dim, rot, angles, k_scale, pw);
+  load_values<T>(vs, vP, proj, ld, v_off + hd * vdim, n_first, L, L, vdim);
   __syncthreads();
   float* dst = sbuf + ((size_t)g * H + hd) * dim * vdim;
   const int tv = vP / 8, n_tiles = (dP / 8) * tv;
@@ -210,6 +230,7 @@ __global__ void __launch_bounds__(CK_THREADS) retention_chunk_state_kernel(
     for (int i = 0; i < 8; ++i)
 #pragma unroll
       for (int c = 0; c < 8; ++c) acc[i][c] = 0.f;
+#pragma unroll 4
     for (int j = 0; j < L; ++j) {
       const float4 k0 = *reinterpret_cast<const float4*>(ks + j * dP + d0), k1 = *reinterpret_cast<const float4*>(ks + j * dP + d0 + 4);
       const float4 u0 = *reinterpret_cast<const float4*>(vs + j * vP + v0), u1 = *reinterpret_cast<const float4*>(vs + j * vP + v0 + 4);
@@ -262,9 +283,8 @@ __global__ void retention_chunk_prefix_kernel(const int* __restrict__ cu_q, cons
 template <typename T>
 __global__ void __launch_bounds__(CK_THREADS) retention_chunk_out_kernel(
     const T* __restrict__ proj, int ld, int q_off, int k_off, int v_off, int g_off, const int* __restrict__ cu_q,
-    const int* __restrict__ seq_slot, int n_seqs, const int* __restrict__ tok_pos, const float* __restrict__ inv_freq,
-    const float* __restrict__ inv_freq_lo, int rot, const double* __restrict__ decay, const float* __restrict__ sbuf,
-    T* __restrict__ out, int H, int dim, int vdim, float k_scale, float eps) {
+    const int* __restrict__ seq_slot, int n_seqs, const float2* __restrict__ angles, int rot, const double* __restrict__ decay,
+    const float* __restrict__ sbuf, T* __restrict__ out, int H, int dim, int vdim, float k_scale, float eps) {
   extern __shared__ __align__(16) float smem[];
   __shared__ int loc[3];
   const int g = blockIdx.x, hd = blockIdx.y;
@@ -286,12 +306,9 @@ __global__ void __launch_bounds__(CK_THREADS) retention_chunk_out_kernel(
   float* A = ks + CH * dQ;           // [CH][CH + 1]
   float* pw = A + CH * (CH + 1);     // [CH + 1]
   for (int i = threadIdx.x; i <= CH; i += CK_THREADS) pw[i] = (float)pow(decay[hd], (double)i);
-  load_rotated<T>(qs, dQ, proj, ld, q_off + hd * dim, n_first, L, dim, rot, inv_freq, inv_freq_lo, tok_pos, 1.f);
-  load_rotated<T>(ks, dQ, proj, ld, k_off + hd * dim, n_first, L, dim, rot, inv_freq, inv_freq_lo, tok_pos, k_scale);
-  for (int idx = threadIdx.x; idx < CH * vP; idx += CK_THREADS) {
-    const int t = idx / vP, v = idx % vP;
-    vs[idx] = (t < L && v < vdim) ? to_f32<T>(proj[(size_t)(n_first + t) * ld + v_off + hd * vdim + v]) : 0.f;
-  }
+  load_rotated<T>(qs, dQ, proj, ld, q_off + hd * dim, n_first, L, dim, rot, angles, 1.f);
+  load_rotated<T>(ks, dQ, proj, ld, k_off + hd * dim, n_first, L, dim, rot, angles, k_scale);
+  load_values<T>(vs, vP, proj, ld, v_off + hd * vdim, n_first, L, CH, vdim);
   for (int idx = threadIdx.x + L * dQ; idx < CH * dQ; idx += CK_THREADS) { qs[idx] = 0.f; ks[idx] = 0.f; }   // rows behind the chunk
   __syncthreads();
   // A[i][j] = w^(i-j) q_i . k_j  for j <= i, else 0: 4 x 4 outputs a thread
@@ -303,6 +320,7 @@ __global__ void __launch_bounds__(CK_THREADS) retention_chunk_out_kernel(
 #pragma unroll
       for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
     if (j0 <= i0 + 3 && i0 < L) {
+#pragma unroll 4
       for (int d = 0; d < dim; ++d) {
         float qv[4], kv[4];
 #pragma unroll
@@ -371,6 +389,7 @@ __global__ void __launch_bounds__(CK_THREADS) retention_chunk_out_kernel(
       const int i0 = (tile / tv) * 8, v0 = (tile % tv) * 4;
       if (i0 >= L) continue;
       float (*a)[4] = acc[n_mine];
+#pragma unroll 4
       for (int dd = 0; dd < d_end; ++dd) {
         const float4 sv = *reinterpret_cast<const float4*>(slab + (size_t)dd * vP + v0);
 #pragma unroll
@@ -393,6 +412,7 @@ __global__ void __launch_bounds__(CK_THREADS) retention_chunk_out_kernel(
 #pragma unroll
         for (int c = 0; c < 4; ++c) a[r][c] *= pw[i0 + r + 1];
       const int j_end = min(L, i0 + 8);
+#pragma unroll 4
       for (int j = 0; j < j_end; ++j) {
         const float4 vv = *reinterpret_cast<const float4*>(vs + (size_t)j * vP + v0);
 #pragma unroll
@@ -428,21 +448,24 @@ __global__ void __launch_bounds__(CK_THREADS) retention_chunk_out_kernel(
   }
 }
 
-constexpr int GT = 8;          // tokens per block of rglru_gates
+constexpr int GT = 8;          // tokens a thread of rglru_gates adds up
 constexpr int G_THREADS = 256;
 
+// A block takes GT * groups tokens and one gate block: a thread an output of both gates for GT tokens, `groups` threads beside one
+// another the same output for other tokens (two with gate blocks of 128, where half of the threads had nothing to do before).  The
+// inputs lie token-fast in shared memory, two 16-byte broadcasts a k; eight k's weights are requested at a time.
 template <typename T>
 __global__ void __launch_bounds__(G_THREADS) rglru_gates_kernel(
     const T* __restrict__ proj, int ld, int x_off, const float* __restrict__ x_bias, const int* __restrict__ tok_slot,
     const float* __restrict__ conv_w, const float* __restrict__ conv_b, int taps, const float* __restrict__ tail,
     const float* __restrict__ w_gates, const float* __restrict__ b_a, const float* __restrict__ b_i,
     const float* __restrict__ sp_lam, float c_mult, float* __restrict__ a_out, float* __restrict__ b_out, int n_tokens,
-    int C, int nb) {
-  extern __shared__ __align__(16) float u_s[];   // [GT][nb]
-  const int n0 = blockIdx.x * GT, blk = blockIdx.y, c0 = blk * nb;
+    int C, int nb, int groups) {
+  extern __shared__ __align__(16) float u_s[];   // [groups][nb][GT]
+  const int n0 = blockIdx.x * GT * groups, blk = blockIdx.y, c0 = blk * nb;
   const int K1 = taps - 1;
-  for (int idx = threadIdx.x; idx < GT * nb; idx += G_THREADS) {
-    const int t = idx / nb, cc = idx % nb, n = n0 + t, c = c0 + cc;
+  for (int idx = threadIdx.x; idx < GT * groups * nb; idx += G_THREADS) {
+    const int t = idx / nb, cc = idx - t * nb, n = n0 + t, c = c0 + cc;
     float u = 0.f;
     if (n < n_tokens) {
       const int slot = tok_slot[n];
@@ -459,35 +482,43 @@ __global__ void __launch_bounds__(G_THREADS) rglru_gates_kernel(
         }
       }
     }
-    u_s[t * nb + cc] = u;
+    u_s[((t / GT) * nb + cc) * GT + t % GT] = u;
   }
   __syncthreads();
   const float* wg = w_gates + (size_t)blk * nb * 2 * nb;   // [k][2][o]
-  for (int o = threadIdx.x; o < nb; o += G_THREADS) {
+  for (int i = threadIdx.x; i < nb * groups; i += G_THREADS) {
+    const int g = i / nb, o = i - g * nb;
+    const float* ug = u_s + (size_t)g * nb * GT;
     float ar[GT], ai[GT];
     const float ba = b_a[c0 + o], bi = b_i[c0 + o];
 #pragma unroll
     for (int t = 0; t < GT; ++t) { ar[t] = ba; ai[t] = bi; }
+#pragma unroll 8
     for (int k = 0; k < nb; ++k) {
       const float wr = wg[((size_t)k * 2) * nb + o], wi = wg[((size_t)k * 2 + 1) * nb + o];
+      const float4 u0 = *reinterpret_cast<const float4*>(ug + k * GT), u1 = *reinterpret_cast<const float4*>(ug + k * GT + 4);
+      const float uv[GT] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w};
 #pragma unroll
       for (int t = 0; t < GT; ++t) {
-        const float uv = u_s[t * nb + k];
-        ar[t] = fmaf(wr, uv, ar[t]);
-        ai[t] = fmaf(wi, uv, ai[t]);
+        ar[t] = fmaf(wr, uv[t], ar[t]);
+        ai[t] = fmaf(wi, uv[t], ai[t]);
       }
     }
     const float sp = sp_lam[c0 + o];
 #pragma unroll
     for (int t = 0; t < GT; ++t) {
-      const int n = n0 + t;
+      const int n = n0 + g * GT + t;
       if (n >= n_tokens) break;
       const float r = 1.f / (1.f + expf(-ar[t])), ig = 1.f / (1.f + expf(-ai[t]));
       const float log_a = -c_mult * r * sp;
       a_out[(size_t)n * C + c0 + o] = expm1f(log_a);   // a - 1: a decay close to one keeps its distance from one
-      b_out[(size_t)n * C + c0 + o] = sqrtf(-expm1f(2.f * log_a)) * ig * u_s[t * nb + o];
+      b_out[(size_t)n * C + c0 + o] = sqrtf(-expm1f(2.f * log_a)) * ig * ug[o * GT + t];
     }
   }
+}
+
+__device__ __forceinline__ float gelu_tanh_f(float z) {
+  return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
 }
 
 // The same for steps of few tokens.  There a block per gate block leaves a thread 2 nb dependent trips long (22 us for one
@@ -589,12 +620,9 @@ __global__ void __launch_bounds__(G_THREADS) rglru_gates_few_kernel(
     b_out[(size_t)n * C + c0 + c] = sqrtf(-expm1f(2.f * log_a)) * ig * u_s[t * nb + c];
   }
 }
-// Steps of up to this many tokens (a decode step's rows): beyond it the prompt form's blocks fill the SMs.
+// Steps of up to this many tokens (a decode step's rows): beyond it the prompt form's blocks fill the SMs, and read the weights half
+// as often (1,300 tokens: 277 us this way).
 constexpr int FEW_TOKENS = 64;
-
-__device__ __forceinline__ float gelu_tanh_f(float z) {
-  return 0.5f * z * (1.f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
-}
 
 // A block takes 32 channels (a lane each) of one sequence and walks time in pieces of SCAN_WARPS * SCAN_SEG steps: every
 // warp folds its own SCAN_SEG steps into one (E, B) pair  S_out = S_in + (E * S_in + B),  the pairs of the warps before it give its
@@ -694,7 +722,8 @@ DRYFT_API int dryft_retention_scan(int is_bf16, const void* proj, int ld, int q_
   return launch_status();
 }
 
-// The chunked form: `sbuf` holds (n_tokens / CH + n_seqs) * H * dim * vdim floats.  Three launches.
+// The chunked form: `sbuf` holds (n_tokens / CH + n_seqs) * H * dim * vdim floats, then n_tokens * rot (on an 8-byte boundary:
+// one float more).  Four launches.
 DRYFT_API int dryft_retention_chunked(int is_bf16, const void* proj, int ld, int q_off, int k_off, int v_off, int g_off,
                                       const int* cu_q, const int* seq_slot, const int* tok_pos, const float* inv_freq,
                                       const float* inv_freq_lo, int rot, const double* decay, float* state, float* sbuf,
@@ -714,13 +743,19 @@ DRYFT_API int dryft_retention_chunked(int is_bf16, const void* proj, int ld, int
   if (rc) return rc;
   rc = is_bf16 ? opt_in_smem(retention_chunk_out_kernel<bf>, smem_c) : opt_in_smem(retention_chunk_out_kernel<float>, smem_c);
   if (rc) return rc;
+  size_t states = (size_t)n_chunks * H * dim * vdim;
+  states += states & 1;
+  float2* const angles = reinterpret_cast<float2*>(sbuf + states);
+  if (rot > 0) {
+    retention_angles_kernel<<<(unsigned)(((size_t)n_tokens * (rot / 2) + 255) / 256), 256, 0, st>>>(tok_pos, inv_freq, inv_freq_lo, angles, n_tokens, rot / 2);
+    rc = launch_status();
+    if (rc) return rc;
+  }
   dim3 grid(n_chunks, H);
   if (is_bf16)
-    retention_chunk_state_kernel<bf><<<grid, CK_THREADS, smem_a, st>>>((const bf*)proj, ld, k_off, v_off, cu_q, seq_slot, n_seqs, tok_pos,
-                                                                       inv_freq, inv_freq_lo, rot, decay, sbuf, H, dim, vdim, k_scale);
+    retention_chunk_state_kernel<bf><<<grid, CK_THREADS, smem_a, st>>>((const bf*)proj, ld, k_off, v_off, cu_q, seq_slot, n_seqs, angles, rot, decay, sbuf, H, dim, vdim, k_scale);
   else
-    retention_chunk_state_kernel<float><<<grid, CK_THREADS, smem_a, st>>>((const float*)proj, ld, k_off, v_off, cu_q, seq_slot, n_seqs,
-                                                                          tok_pos, inv_freq, inv_freq_lo, rot, decay, sbuf, H, dim, vdim,
+    retention_chunk_state_kernel<float><<<grid, CK_THREADS, smem_a, st>>>((const float*)proj, ld, k_off, v_off, cu_q, seq_slot, n_seqs, angles, rot, decay, sbuf, H, dim, vdim,
                                                                           k_scale);
   int e = launch_status();
   if (e) return e;
@@ -730,12 +765,11 @@ DRYFT_API int dryft_retention_chunked(int is_bf16, const void* proj, int ld, int
   e = launch_status();
   if (e) return e;
   if (is_bf16)
-    retention_chunk_out_kernel<bf><<<grid, CK_THREADS, smem_c, st>>>((const bf*)proj, ld, q_off, k_off, v_off, g_off, cu_q, seq_slot, n_seqs,
-                                                                     tok_pos, inv_freq, inv_freq_lo, rot, decay, sbuf, (bf*)out, H, dim,
+    retention_chunk_out_kernel<bf><<<grid, CK_THREADS, smem_c, st>>>((const bf*)proj, ld, q_off, k_off, v_off, g_off, cu_q, seq_slot, n_seqs, angles, rot, decay, sbuf, (bf*)out, H, dim,
                                                                      vdim, k_scale, eps);
   else
     retention_chunk_out_kernel<float><<<grid, CK_THREADS, smem_c, st>>>((const float*)proj, ld, q_off, k_off, v_off, g_off, cu_q, seq_slot,
-                                                                        n_seqs, tok_pos, inv_freq, inv_freq_lo, rot, decay, sbuf,
+                                                                        n_seqs, angles, rot, decay, sbuf,
                                                                         (float*)out, H, dim, vdim, k_scale, eps);
   return launch_status();
 }
@@ -761,15 +795,17 @@ DRYFT_API int dryft_rglru_gates(int is_bf16, const void* proj, int ld, int x_off
                                                                   tail, w_gates, b_a, b_i, sp_lam, c_mult, a_out, b_out, n_tokens, C, nb);
     return launch_status();
   }
-  int rc = is_bf16 ? opt_in_smem(rglru_gates_kernel<bf>, smem) : opt_in_smem(rglru_gates_kernel<float>, smem);
+  const int groups = nb >= G_THREADS ? 1 : G_THREADS / nb < 4 ? G_THREADS / nb : 4;
+  const size_t many = smem * groups;
+  int rc = is_bf16 ? opt_in_smem(rglru_gates_kernel<bf>, many) : opt_in_smem(rglru_gates_kernel<float>, many);
   if (rc) return rc;
-  dim3 grid((n_tokens + GT - 1) / GT, n_blocks);
+  dim3 grid((n_tokens + GT * groups - 1) / (GT * groups), n_blocks);
   if (is_bf16)
-    rglru_gates_kernel<bf><<<grid, G_THREADS, smem, st>>>((const bf*)proj, ld, x_off, x_bias, tok_slot, conv_w, conv_b, taps, tail,
-                                                          w_gates, b_a, b_i, sp_lam, c_mult, a_out, b_out, n_tokens, C, nb);
+    rglru_gates_kernel<bf><<<grid, G_THREADS, many, st>>>((const bf*)proj, ld, x_off, x_bias, tok_slot, conv_w, conv_b, taps, tail,
+                                                          w_gates, b_a, b_i, sp_lam, c_mult, a_out, b_out, n_tokens, C, nb, groups);
   else
-    rglru_gates_kernel<float><<<grid, G_THREADS, smem, st>>>((const float*)proj, ld, x_off, x_bias, tok_slot, conv_w, conv_b, taps,
-                                                             tail, w_gates, b_a, b_i, sp_lam, c_mult, a_out, b_out, n_tokens, C, nb);
+    rglru_gates_kernel<float><<<grid, G_THREADS, many, st>>>((const float*)proj, ld, x_off, x_bias, tok_slot, conv_w, conv_b, taps,
+                                                             tail, w_gates, b_a, b_i, sp_lam, c_mult, a_out, b_out, n_tokens, C, nb, groups);
   return launch_status();
 }
 

@@ -1442,15 +1442,15 @@ def retention_scan(proj, offsets, cu_q, seq_slot, tok_pos, inv_freq, rot: int, d
     _need(state, "state", torch.float32, (None, heads, dim, vdim))
     _need(out, "out", proj.dtype, (n, heads * vdim))
     if chunked and vdim <= RETENTION_CHUNKED_MAX_VDIM:
-        # steps of many tokens: chunk states, their prefix, chunk outputs (three launches, the work spread over chunks)
+        # steps of many tokens: angles, chunk states, their prefix, chunk outputs (the work spread over chunks)
         lib = recurrent_lib()
         ch = int(lib.dryft_retention_chunk_tokens())
-        sbuf = torch.empty((n // ch + n_seqs) * heads * dim * vdim, dtype=torch.float32, device=proj.device)
+        sbuf = torch.empty((n // ch + n_seqs) * heads * dim * vdim + 1 + n * rot, dtype=torch.float32, device=proj.device)
         rc = lib.dryft_retention_chunked(_act(proj, "proj"), _ptr(proj), ld, q_off, k_off, v_off, g_off, _ptr(cu_q), _ptr(seq_slot),
                                          _ptr(tok_pos), _ptr(inv_freq), _ptr(_freq_lo(inv_freq_lo, rot)), int(rot), _ptr(decay), _ptr(state),
                                          _ptr(sbuf), _ptr(out), n, n_seqs, heads, dim, vdim, float(k_scale), float(eps), _stream())
         if rc != UNSUPPORTED:   # sizes whose chunk does not fit its shared memory are walked token by token below
-            _ok(rc, f"retention_chunked ({heads} heads of {dim} x {vdim})", n_kernels=3)
+            _ok(rc, f"retention_chunked ({heads} heads of {dim} x {vdim})", n_kernels=4 if rot else 3)
             return
     _ok(recurrent_lib().dryft_retention_scan(_act(proj, "proj"), _ptr(proj), ld, q_off, k_off, v_off, g_off, _ptr(cu_q), _ptr(seq_slot),
                                              _ptr(tok_pos), _ptr(inv_freq), _ptr(_freq_lo(inv_freq_lo, rot)), int(rot), _ptr(decay), _ptr(state), _ptr(out), n_seqs,
