@@ -325,6 +325,7 @@ DRYFT_API int dryft_residual_add(int is_bf16, void* x, const void* d, long long 
 // ------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ y, int inter, size_t total) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   size_t r = i / inter;
@@ -342,6 +343,7 @@ template <> __device__ __forceinline__ float silu_f32<__nv_bfloat16>(float g) { 
 // 16 bytes of gate and of up per thread (inter a multiple of the vector width)
 template <typename T>
 __global__ void silu_mul_vec_kernel(const T* __restrict__ gu, T* __restrict__ y, int inter, size_t total_vecs) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
   constexpr int V = Vec16<T>::N;
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total_vecs) return;

@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(128) gemm_f32_few_kernel(const float* __restri
       copy_async<VEC>(to + ((size_t)m * x_chunks + c / CH) * CHP + c % CH, there ? A + (size_t)m * lda + k : A, there);
     }
   };
-  auto load = [&](int step) {
+  auto load_w = [&](int step) {
     if (step < steps) {
       const int n0 = ((int)blockIdx.x + (step / pieces) * (int)gridDim.x) * R, k0 = (step % pieces) * KP;
       float* const to = wst + (step % STAGES) * R * KP;
@@ -69,13 +69,21 @@ __global__ void __launch_bounds__(128) gemm_f32_few_kernel(const float* __restri
         const bool there = n0 + row < N && k0 + c < K;
         copy_async<VEC>(to + row * KP + (c ^ (swz * 4)), there ? W + (size_t)(n0 + row) * K + k0 + c : W, there);
       }
-      if (!XRES) load_x(xs + (size_t)(step % STAGES) * MT * x_chunks * CHP, k0, Q);
     }
-    copies_commit();
   };
+  auto load_own_x = [&](int step) {
+    if (!XRES && step < steps) load_x(xs + (size_t)(step % STAGES) * MT * x_chunks * CHP, (step % pieces) * KP, Q);
+  };
+  // the first weights depend on nothing; the activations are the launch before's (a programmatic dependent: 16-byte copies only,
+  // which go past L1)
+#pragma unroll
+  for (int s = 0; s < STAGES; ++s) load_w(s);
+  asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory");
   if (XRES) load_x(xs, 0, x_chunks);
 #pragma unroll
-  for (int s = 0; s < STAGES; ++s) load(s);
+  for (int s = 0; s < STAGES; ++s) load_own_x(s);
+#pragma unroll
+  for (int s = 0; s < STAGES; ++s) copies_commit();      // everything so far is the first group's
   float total[OUTS];
   for (int s = 0; s < steps; ++s) {
     const int p = s % pieces;
@@ -106,7 +114,9 @@ __global__ void __launch_bounds__(128) gemm_f32_few_kernel(const float* __restri
       part[(m * Q + q) * R + H + r] = acc[1][m];
     }
     __syncthreads();
-    load(s + STAGES);      // into the stage that every thread has just left
+    load_w(s + STAGES);    // into the stage that every thread has just left
+    load_own_x(s + STAGES);
+    copies_commit();
     const int n0 = ((int)blockIdx.x + (s / pieces) * (int)gridDim.x) * R;
 #pragma unroll
     for (int o = 0; o < OUTS; ++o) {
@@ -124,44 +134,54 @@ __global__ void __launch_bounds__(128) gemm_f32_few_kernel(const float* __restri
 }
 
 template <int MT, int R, int VEC, bool XRES, int STAGES>
-int launch_few(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, int x_chunks, size_t smem, int sms, cudaStream_t st) {
+int launch_few(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, int x_chunks, size_t smem, int sms, int pdl, cudaStream_t st) {
   auto kern = gemm_f32_few_kernel<MT, R, VEC, XRES, STAGES>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
   const int tiles = (N + R - 1) / R;
-  kern<<<dim3(tiles < sms ? tiles : sms, (M + MT - 1) / MT), 128, smem, st>>>(A, lda, W, C, ldc, M, N, K, x_chunks);
-  return launch_status();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tiles < sms ? tiles : sms, (M + MT - 1) / MT);
+  cfg.blockDim = dim3(128);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl && VEC == 4 ? 1 : 0;
+  e = cudaLaunchKernelEx(&cfg, kern, A, lda, W, C, ldc, M, N, K, x_chunks);
+  return e != cudaSuccess ? (int)e : launch_status();
 }
 
 template <int MT, int R, int VEC>
-int launch_few_x(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, int sms, cudaStream_t st) {
+int launch_few_x(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, int sms, int pdl, cudaStream_t st) {
   constexpr int Q = 256 / R;
   constexpr size_t most = 227 * 1024, stage = 64 * 1024, part = (size_t)4 * MT * 256;
   static_assert(2 * (stage + (size_t)4 * MT * Q * CHP) + part <= most, "two stages with their own columns of A fit a block");
   const int all = (K + CH - 1) / CH;
   const size_t x = (size_t)4 * MT * all * CHP;
-  if (3 * stage + part + x <= most) return launch_few<MT, R, VEC, true, 3>(A, lda, W, C, ldc, M, N, K, all, 3 * stage + part + x, sms, st);
-  if (2 * stage + part + x <= most) return launch_few<MT, R, VEC, true, 2>(A, lda, W, C, ldc, M, N, K, all, 2 * stage + part + x, sms, st);
-  return launch_few<MT, R, VEC, false, 2>(A, lda, W, C, ldc, M, N, K, Q, 2 * (stage + (size_t)4 * MT * Q * CHP) + part, sms, st);
+  if (3 * stage + part + x <= most) return launch_few<MT, R, VEC, true, 3>(A, lda, W, C, ldc, M, N, K, all, 3 * stage + part + x, sms, pdl, st);
+  if (2 * stage + part + x <= most) return launch_few<MT, R, VEC, true, 2>(A, lda, W, C, ldc, M, N, K, all, 2 * stage + part + x, sms, pdl, st);
+  return launch_few<MT, R, VEC, false, 2>(A, lda, W, C, ldc, M, N, K, Q, 2 * (stage + (size_t)4 * MT * Q * CHP) + part, sms, pdl, st);
 }
 
 template <int MT, int VEC>
-int launch_few_r(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, int sms, cudaStream_t st) {
+int launch_few_r(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, int sms, int pdl, cudaStream_t st) {
   // the more rows of A, the fewer columns of them fit beside a piece of W
   if constexpr (MT <= 4)
-    if (K > 1024) return launch_few_x<MT, 8, VEC>(A, lda, W, C, ldc, M, N, K, sms, st);
+    if (K > 1024) return launch_few_x<MT, 8, VEC>(A, lda, W, C, ldc, M, N, K, sms, pdl, st);
   if constexpr (MT <= 8)
-    if (K > 512) return launch_few_x<MT, 16, VEC>(A, lda, W, C, ldc, M, N, K, sms, st);
-  return launch_few_x<MT, 32, VEC>(A, lda, W, C, ldc, M, N, K, sms, st);
+    if (K > 512) return launch_few_x<MT, 16, VEC>(A, lda, W, C, ldc, M, N, K, sms, pdl, st);
+  return launch_few_x<MT, 32, VEC>(A, lda, W, C, ldc, M, N, K, sms, pdl, st);
 }
 
 template <int VEC>
-int launch_few_m(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, int rows, int sms, cudaStream_t st) {
-  if (M == 1) return launch_few_r<1, VEC>(A, lda, W, C, ldc, M, N, K, sms, st);
-  if (M == 2) return launch_few_r<2, VEC>(A, lda, W, C, ldc, M, N, K, sms, st);
-  if (M <= 4) return launch_few_r<4, VEC>(A, lda, W, C, ldc, M, N, K, sms, st);
-  if (rows == 8) return launch_few_r<8, VEC>(A, lda, W, C, ldc, M, N, K, sms, st);
-  return launch_few_r<16, VEC>(A, lda, W, C, ldc, M, N, K, sms, st);
+int launch_few_m(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, int rows, int sms, int pdl, cudaStream_t st) {
+  if (M == 1) return launch_few_r<1, VEC>(A, lda, W, C, ldc, M, N, K, sms, pdl, st);
+  if (M == 2) return launch_few_r<2, VEC>(A, lda, W, C, ldc, M, N, K, sms, pdl, st);
+  if (M <= 4) return launch_few_r<4, VEC>(A, lda, W, C, ldc, M, N, K, sms, pdl, st);
+  if (rows == 8) return launch_few_r<8, VEC>(A, lda, W, C, ldc, M, N, K, sms, pdl, st);
+  return launch_few_r<16, VEC>(A, lda, W, C, ldc, M, N, K, sms, pdl, st);
 }
 
 // ---------------------------------------------------------------------------- many rows
@@ -298,7 +318,7 @@ int few_rows(int M, int N, int K, int sms) {
 }  // namespace
 
 DRYFT_API int dryft_gemm_nt_f32(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K,
-                                cudaStream_t st) {
+                                int pdl, cudaStream_t st) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0) return DRYFT_ERR_UNSUPPORTED;
   // 16-byte accesses where every row of both operands starts on one
@@ -308,6 +328,6 @@ DRYFT_API int dryft_gemm_nt_f32(const float* A, int lda, const float* W, float* 
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int rows = K <= ONE_CHAIN ? 0 : few_rows(M, N, K, sms);
   if (rows)
-    return vec ? launch_few_m<4>(A, lda, W, C, ldc, M, N, K, rows, sms, st) : launch_few_m<1>(A, lda, W, C, ldc, M, N, K, rows, sms, st);
+    return vec ? launch_few_m<4>(A, lda, W, C, ldc, M, N, K, rows, sms, pdl, st) : launch_few_m<1>(A, lda, W, C, ldc, M, N, K, rows, sms, pdl, st);
   return vec ? launch_tile<4>(A, lda, W, C, ldc, M, N, K, st) : launch_tile<1>(A, lda, W, C, ldc, M, N, K, st);
 }

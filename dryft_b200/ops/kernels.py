@@ -60,7 +60,7 @@ def core() -> ctypes.CDLL:
             lib.dryft_qk_norm_rope_store.argtypes = [_i, _p, _i, _p, _p, _p, _p, _p, _p, _p, _p, _p, _p, _i, _i, _i, _i, _i,
                                                      _i, _i, _f, _i, _i, _i, _p]
             lib.dryft_rope_table.argtypes = [_i, _p, _p, _p, _i, _i, _p]
-            lib.dryft_gemm_nt_f32.argtypes = [_p, _i, _p, _p, _i, _i, _i, _i, _p]
+            lib.dryft_gemm_nt_f32.argtypes = [_p, _i, _p, _p, _i, _i, _i, _i, _i, _p]
             lib.dryft_argmax_rows.argtypes = [_p, _i, _i, _ll, _p, _p, _p, _p]
             lib.dryft_sample_rows.argtypes = [_p, _i, _i, _ll, _f, _i, _ull, _p, _p, _i, _p, _p, _p, _p]
             lib.dryft_gemm_small_m.argtypes = [_p, _i, _p, _p, _i, _i, _i, _i, _i, _p, _p, _i, _f, _p, _i, _p]
@@ -982,14 +982,15 @@ def moe_grouped(h, w_gate_up, w_down, idx, y, gated: bool = True, in_w=None, lim
 
 
 # ----------------------------------------------------------------------------- matrix products
-def gemm_nt_f32(a, w, out) -> None:
-    """``out[M,N] = a[M,K] @ w[N,K].T`` in true 32-bit."""
+def gemm_nt_f32(a, w, out, pdl: bool = False) -> None:
+    """``out[M,N] = a[M,K] @ w[N,K].T`` in true 32-bit.  ``pdl``: few rows are launched as a programmatic dependent of the launch
+    before, whose tail their first weight requests overlap."""
     m, k = a.shape
     n = w.shape[0]
     _need(a, "a", torch.float32)
     _need(w, "w", torch.float32, (n, k))
     _need(out, "out", torch.float32, (m, n))
-    _ok(core().dryft_gemm_nt_f32(_ptr(a), k, _ptr(w), _ptr(out), n, m, n, k, _stream()), "gemm_nt_f32")
+    _ok(core().dryft_gemm_nt_f32(_ptr(a), k, _ptr(w), _ptr(out), n, m, n, k, int(pdl), _stream()), "gemm_nt_f32")
 
 
 SMALL_M_LIMIT = 16  # rows the weight-streaming product takes

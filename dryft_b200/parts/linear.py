@@ -31,7 +31,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, rt: Runtime, out_dtype: Optional[to
         if w.dtype != torch.float32:
             raise ValueError(f"linear: 32-bit activations need a 32-bit weight, got {w.dtype}")
         out = torch.empty((m, n), dtype=torch.float32, device=x.device)
-        K.gemm_nt_f32(x, w, out)
+        K.gemm_nt_f32(x, w, out, pdl=rt.pdl)
         return out if out_dtype == torch.float32 else out.to(out_dtype)
     if x.dtype != torch.bfloat16:
         raise ValueError(f"linear: activations are float32 or bfloat16, got {x.dtype}")
