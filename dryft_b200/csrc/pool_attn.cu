@@ -384,11 +384,12 @@ __global__ void __launch_bounds__(BLOCKS_THREADS) pool_attn_blocks_kernel(
   }
 }
 
-template <typename T> __device__ __forceinline__ void dot_row(const T* __restrict__ kr, const float (*qs)[D], float* dots) {
+// a key row against the queries, or lane `sub`'s part of it
+template <typename T, int LPK> __device__ __forceinline__ void dot_row(const T* __restrict__ kr, const float (*qs)[D], float* dots, int sub) {
   constexpr int V = 16 / sizeof(T);
   if (D % V == 0) {
-#pragma unroll 2
-    for (int c = 0; c < D; c += V) {
+#pragma unroll (LPK > 1 ? 8 : 2)
+    for (int c = sub * V; c < D; c += V * LPK) {
       const uint4 kv = *reinterpret_cast<const uint4*>(kr + c);
       const T* ke = reinterpret_cast<const T*>(&kv);
 #pragma unroll
@@ -399,13 +400,35 @@ template <typename T> __device__ __forceinline__ void dot_row(const T* __restric
       }
     }
   } else {
-    for (int c = 0; c < D; ++c) {
+    for (int c = sub; c < D; c += LPK) {
       const float kf = to_f32<T>(kr[c]);
 #pragma unroll
       for (int h = 0; h < REP; ++h) dots[h] = fmaf(kf, qs[h][c], dots[h]);
     }
   }
 }
+
+// A lane's columns of one value row: side by side in one access where a row is whole lanes of 4, 8 or 16 bytes, else every 32nd.
+template <typename T> struct Lanes {
+  static constexpr int BYTES = DVR * (int)sizeof(T);
+  static constexpr bool WIDE = DV % 32 == 0 && (BYTES == 4 || BYTES == 8 || BYTES == 16);
+  __align__(WIDE ? BYTES : (int)sizeof(T)) T v[DVR];
+  static __device__ __forceinline__ int column(int lane, int r) { return WIDE ? lane * DVR + r : lane + 32 * r; }
+  // the row of key j of `cnt`, whose address lane j * lpk holds; zeros behind the last key
+  __device__ __forceinline__ void load(unsigned long long addr, int j, int lpk, int cnt, int lane) {
+    const T* row = reinterpret_cast<const T*>(__shfl_sync(0xffffffffu, addr, j * lpk & 31));
+    if (WIDE) {
+      if (BYTES == 16) *reinterpret_cast<uint4*>(v) = j < cnt ? *reinterpret_cast<const uint4*>(row + lane * DVR) : make_uint4(0, 0, 0, 0);
+      else if (BYTES == 8) *reinterpret_cast<uint2*>(v) = j < cnt ? *reinterpret_cast<const uint2*>(row + lane * DVR) : make_uint2(0, 0);
+      else *reinterpret_cast<unsigned*>(v) = j < cnt ? *reinterpret_cast<const unsigned*>(row + lane * DVR) : 0u;
+    } else {
+#pragma unroll
+      for (int r = 0; r < DVR; ++r) v[r] = j < cnt && lane + 32 * r < DV ? row[lane + 32 * r] : from_f32<T>(0.f);
+    }
+  }
+};
+// value rows on their way at a time: all 16 of a tile, or what fits 64 registers
+template <typename T> constexpr int V_AHEAD = DVR * (int)sizeof(T) <= 16 ? 16 : DVR * (int)sizeof(T) <= 32 ? 8 : 4;
 
 // the factor of output value c of a token's head: the sigmoid of its logit in [n, H * DV] (no gate: one)
 template <typename T> __device__ __forceinline__ float gate_at(const T* __restrict__ gate, int gate_ld, int t, int head, int c) {
@@ -425,7 +448,12 @@ template <typename T> __device__ __forceinline__ float mod_score(float s, float 
   return s - r1 * __logf(fmaf(r2, dist, 1.f));
 }
 
-template <typename T, bool MODS>
+// LPK lanes share a key.  One lane a key (a warp's tile is 32 keys) has the fewest instructions a key: many rows.  A decode step's few rows
+// are bound by the chain of one warp instead -- position, page, key row, value rows -- and a block's share is often no more than 64 keys,
+// two warps' tiles: two lanes a key spread them over all four warps, with a key's words and the first value rows on their way together.
+// Measured with L2 flushed and the combining launch, bfloat16 / 32-bit, sizes 192 and 128, 8 heads: 4 rows of 400 keys 45.8 -> 36.3 / 65.1 ->
+// 34.8 us; 24 rows of 600 keys (384 blocks, the most measured) 89 -> 76 / 151 -> 77 us; nothing slower at 1 to 24 rows of 64 to 8,000 keys.
+template <typename T, bool MODS, int LPK>
 __global__ void __launch_bounds__(ROWS_WARPS * 32) pool_attn_rows_kernel(
     const T* __restrict__ q, const T* __restrict__ k_pages, const T* __restrict__ v_pages, const int* __restrict__ page_table,
     int max_pages, int page_size, const T* __restrict__ pk_pages, const T* __restrict__ pv_pages, const int* __restrict__ pool_table,
@@ -436,6 +464,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) pool_attn_rows_kernel(
   __shared__ float qs[REP][D];
   __shared__ float wo[ROWS_WARPS][REP][DV];
   __shared__ float wml[ROWS_WARPS][REP][2];
+  constexpr int KPT = 32 / LPK;                   // keys of a warp's tile
   const int t = blockIdx.x, g = blockIdx.y, sp = blockIdx.z;
   const int slot = tok_slot[t];
   if (slot < 0) return;
@@ -465,8 +494,8 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) pool_attn_rows_kernel(
 #pragma unroll
     for (int r = 0; r < DVR; ++r) o[h][r] = 0.f;
   }
-  for (int tile = u0 + warp * 32; tile < u1; tile += ROWS_WARPS * 32) {
-    const int u = tile + lane;
+  for (int tile = u0 + warp * KPT; tile < u1; tile += ROWS_WARPS * KPT) {
+    const int u = tile + lane / LPK;
     const bool valid = u < u1;
     const T* kr = k_pages;
     const T* vr = v_pages;
@@ -486,10 +515,21 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) pool_attn_rows_kernel(
         vr = v_pages + r * DV;
       }
     }
+    const unsigned long long vaddr = reinterpret_cast<unsigned long long>(vr);
+    const int cnt = min(KPT, u1 - tile);
     float dots[REP];
 #pragma unroll
     for (int h = 0; h < REP; ++h) dots[h] = 0.f;
-    if (valid) dot_row<T>(kr, qs, dots);
+    Lanes<T> vv[LPK > 1 ? V_AHEAD<T> : 1];
+    if constexpr (LPK > 1) {
+#pragma unroll
+      for (int jj = 0; jj < V_AHEAD<T>; ++jj) vv[jj].load(vaddr, jj, LPK, cnt, lane);
+    }
+    if (valid) dot_row<T, LPK>(kr, qs, dots, lane % LPK);
+#pragma unroll
+    for (int d = 1; d < LPK; d *= 2)
+#pragma unroll
+      for (int h = 0; h < REP; ++h) dots[h] += __shfl_xor_sync(0xffffffffu, dots[h], d);
     float pr[REP];
 #pragma unroll
     for (int h = 0; h < REP; ++h) {
@@ -498,27 +538,44 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) pool_attn_rows_kernel(
       const float mn = fmaxf(m[h], warp_max(sc));          // finite: the tile holds at least one key
       const float corr = expf(m[h] - mn);                  // exp(-inf) = 0 for the first tile
       const float pv = valid ? expf(sc - mn) : 0.f;
-      l[h] = fmaf(l[h], corr, warp_sum(pv));
+      l[h] = fmaf(l[h], corr, warp_sum(lane % LPK == 0 ? pv : 0.f));
       m[h] = mn;
       pr[h] = pv;
 #pragma unroll
       for (int r = 0; r < DVR; ++r) o[h][r] *= corr;
     }
-    const int cnt = min(32, u1 - tile);
-    const unsigned long long vaddr = reinterpret_cast<unsigned long long>(vr);
-    for (int jj = 0; jj < cnt; ++jj) {
-      const T* vj = reinterpret_cast<const T*>(__shfl_sync(0xffffffffu, vaddr, jj));
-      float vv[DVR];
+    if constexpr (LPK > 1) {
+      for (int j0 = 0; j0 < KPT; j0 += V_AHEAD<T>) {
+        if (j0 >= cnt) break;
+        if (j0 > 0) {
 #pragma unroll
-      for (int r = 0; r < DVR; ++r) {
-        const int c = lane + 32 * r;
-        vv[r] = c < DV ? to_f32<T>(vj[c]) : 0.f;
+          for (int jj = 0; jj < V_AHEAD<T>; ++jj) vv[jj].load(vaddr, j0 + jj, LPK, cnt, lane);
+        }
+#pragma unroll
+        for (int jj = 0; jj < V_AHEAD<T>; ++jj) {
+#pragma unroll
+          for (int h = 0; h < REP; ++h) {
+            const float pj = __shfl_sync(0xffffffffu, pr[h], (j0 + jj) * LPK & 31);   // zero behind the last key
+#pragma unroll
+            for (int r = 0; r < DVR; ++r) o[h][r] = fmaf(pj, to_f32<T>(vv[jj].v[r]), o[h][r]);
+          }
+        }
       }
+    } else {
+      for (int jj = 0; jj < cnt; ++jj) {
+        const T* vj = reinterpret_cast<const T*>(__shfl_sync(0xffffffffu, vaddr, jj));
+        float vv[DVR];
 #pragma unroll
-      for (int h = 0; h < REP; ++h) {
-        const float pj = __shfl_sync(0xffffffffu, pr[h], jj);
+        for (int r = 0; r < DVR; ++r) {
+          const int c = lane + 32 * r;
+          vv[r] = c < DV ? to_f32<T>(vj[c]) : 0.f;
+        }
 #pragma unroll
-        for (int r = 0; r < DVR; ++r) o[h][r] = fmaf(pj, vv[r], o[h][r]);
+        for (int h = 0; h < REP; ++h) {
+          const float pj = __shfl_sync(0xffffffffu, pr[h], jj);
+#pragma unroll
+          for (int r = 0; r < DVR; ++r) o[h][r] = fmaf(pj, vv[r], o[h][r]);
+        }
       }
     }
   }
@@ -528,7 +585,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) pool_attn_rows_kernel(
     if (lane == 0) { wml[warp][h][0] = m[h]; wml[warp][h][1] = l[h]; }
 #pragma unroll
     for (int r = 0; r < DVR; ++r) {
-      const int c = lane + 32 * r;
+      const int c = LPK > 1 ? Lanes<T>::column(lane, r) : lane + 32 * r;
       if (c < DV) wo[warp][h][c] = o[h][r];
     }
   }
@@ -609,7 +666,12 @@ int rows_launch(const void* q, const void* k_pages, const void* v_pages, const i
                 const int* tok_pos, void* out, float* part_o, float* part_ml, int n, int G, int n_splits, float scale, int size, int P,
                 int keep, const void* gate, int gate_ld, ScoreMods mods, cudaStream_t st) {
   dim3 grid(n, G, n_splits);
-  auto kernel = mods.cap > 0.f || mods.r1 != nullptr ? pool_attn_rows_kernel<T, true> : pool_attn_rows_kernel<T, false>;
+  // two lanes a key while all blocks run at once (three a multiprocessor: faster at every size measured up to there, see the kernel), with value
+  // rows in whole lanes, which wants aligned pages; beyond that other blocks hide a warp's chain and the fewer instructions count
+  const bool few = (long long)n * G * n_splits <= 148 * 3 && (((uintptr_t)v_pages | (uintptr_t)pv) & 15) == 0;
+  const bool m = mods.cap > 0.f || mods.r1 != nullptr;
+  auto kernel = few ? (m ? pool_attn_rows_kernel<T, true, 2> : pool_attn_rows_kernel<T, false, 2>)
+                    : (m ? pool_attn_rows_kernel<T, true, 1> : pool_attn_rows_kernel<T, false, 1>);
   kernel<<<grid, ROWS_WARPS * 32, 0, st>>>((const T*)q, (const T*)k_pages, (const T*)v_pages, page_table, max_pages, page_size, (const T*)pk,
                                            (const T*)pv, pool_table, pool_max_pages, sink, tok_slot, tok_pos, (T*)out, part_o, part_ml, G,
                                            n_splits, scale, size, P, keep, (const T*)gate, gate_ld, mods);
