@@ -154,9 +154,10 @@ class MoE:
     # Below this many tokens every assignment streams its expert's weights itself -- unless the tokens share so many experts
     # that reading each one's weights once, which the grouped products do, spares more than their launches cost (measured:
     # 64 experts of 768 x 2,048, 8 a token: 94 us against 109 with 8 tokens, which spares 207 MB, 82 against 73 with 4 and
-    # 52 MB; 32 experts of 512 x 1,024, 4 a token: 36 against 46 with 16 tokens and 111 MB, 35 against 37 with 12 and 71 MB)
+    # 52 MB; whole calls of such a layer: 91 against 106 with 6 and 120 MB, while assignment by assignment 5 tokens, 83 MB, take 83;
+    # 32 experts of 512 x 1,024, 4 a token: 36 against 46 with 16 tokens and 111 MB, 35 against 37 with 12 and 71 MB)
     GROUPED_MIN_TOKENS = 32
-    GROUPED_SPARES_BYTES = 75e6
+    GROUPED_SPARES_BYTES = 100e6
     ROUTE_ROWS_MAX = 16       # up to this many tokens the router's product and choice are one launch ...
     ROUTE_ROWS_MAX_WEIGHTS = 64 * 1024   # ... while one block can stream the router's weight quickly enough (measured: 32 x 1,024
                                          # gains a launch, 64 x 2,048 takes longer than the two launches it replaces)
