@@ -68,11 +68,12 @@ DRYFT_API int dryft_tokens_from_state(const int* seq_slot, const int* last_token
   return launch_status();
 }
 
-// A decode step's beginning in one launch: every sequence's next token and position from the per-sequence state, and its
-// length with the token that the step appends (the step itself goes by tok_pos).  Three launches of 1.6 us, which took more
-// than a hundredth of a small model's step.
+// A decode step's beginning in one launch: every sequence's next token and position from the per-sequence state, and, with
+// `advance`, its length with the token that the step appends (the step itself goes by tok_pos).  Three launches of 1.6 us, which
+// took more than a hundredth of a small model's step.  A captured step runs as a whole and counts here; a step that is launched
+// piece by piece may end in an error between them, and counts behind its last launch (step_advance).
 __global__ void decode_begin_kernel(const int* __restrict__ seq_slot, const int* __restrict__ last_token, int* __restrict__ seq_len,
-                                    int* __restrict__ tokens, int* __restrict__ tok_slot, int* __restrict__ tok_pos, int n_seqs) {
+                                    int* __restrict__ tokens, int* __restrict__ tok_slot, int* __restrict__ tok_pos, int n_seqs, int advance) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= n_seqs) return;
   const int slot = seq_slot[b];
@@ -85,12 +86,12 @@ __global__ void decode_begin_kernel(const int* __restrict__ seq_slot, const int*
   const int pos = seq_len[slot];
   tokens[b] = last_token[slot];
   tok_pos[b] = pos;
-  seq_len[slot] = pos + 1;
+  if (advance) seq_len[slot] = pos + 1;
 }
 DRYFT_API int dryft_decode_begin(const int* seq_slot, const int* last_token, int* seq_len, int* tokens, int* tok_slot, int* tok_pos, int n_seqs,
-                                 cudaStream_t st) {
+                                 int advance, cudaStream_t st) {
   if (n_seqs <= 0) return 0;
-  decode_begin_kernel<<<(n_seqs + 127) / 128, 128, 0, st>>>(seq_slot, last_token, seq_len, tokens, tok_slot, tok_pos, n_seqs);
+  decode_begin_kernel<<<(n_seqs + 127) / 128, 128, 0, st>>>(seq_slot, last_token, seq_len, tokens, tok_slot, tok_pos, n_seqs, advance);
   return launch_status();
 }
 

@@ -291,11 +291,17 @@ class _DecodeGraph:
 
     def _body(self) -> torch.Tensor:
         st = self.st
-        K.decode_begin(self.seq_slot, st.cache.last_token, st.cache.seq_len, self.tokens, self.tok_slot, self.tok_pos, self.bucket)
+        # A captured step's lengths go up in its first launch; an eager step that raises half-way must leave them alone, so they
+        # go up in its last.
+        K.decode_begin(self.seq_slot, st.cache.last_token, st.cache.seq_len, self.tokens, self.tok_slot, self.tok_pos, self.bucket,
+                       advance=st.cuda_graphs)
         ctx = StepContext(n_tokens=self.bucket, n_seqs=self.bucket, tokens=self.tokens, cu_q=self.cu_q,
                           seq_slot=self.seq_slot, tok_slot=self.tok_slot, tok_pos=self.tok_pos, decode=True,
                           max_kv=self.kv_bucket)
-        return st.model.forward(ctx, st.cache, self.rows, self.bucket, all_rows=True)
+        logits = st.model.forward(ctx, st.cache, self.rows, self.bucket, all_rows=True)
+        if not st.cuda_graphs:
+            K.step_advance(self.cu_q, self.seq_slot, st.cache.seq_len, self.bucket)
+        return logits
 
     def run(self, slots: Sequence[int]) -> torch.Tensor:
         n = len(slots)

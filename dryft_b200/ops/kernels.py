@@ -52,7 +52,7 @@ def core() -> ctypes.CDLL:
             lib.dryft_step_meta.argtypes = [_p, _p, _p, _i, _i, _p, _p, _p]
             lib.dryft_step_advance.argtypes = [_p, _p, _p, _i, _p]
             lib.dryft_tokens_from_state.argtypes = [_p, _p, _p, _i, _p]
-            lib.dryft_decode_begin.argtypes = [_p, _p, _p, _p, _p, _p, _i, _p]
+            lib.dryft_decode_begin.argtypes = [_p, _p, _p, _p, _p, _p, _i, _i, _p]
             lib.dryft_embed.argtypes = [_i, _p, _p, _p, _i, _i, _i, _p, _p, _p]
             lib.dryft_rmsnorm.argtypes = [_i, _p, _p, _p, _p, _p, _p, _i, _i, _f, _p]
             lib.dryft_residual_add.argtypes = [_i, _p, _p, _ll, _p]
@@ -379,15 +379,16 @@ def tokens_from_state(seq_slot, last_token, tokens, n_seqs: int) -> None:
 
 
 # ----------------------------------------------------------------------------- elementwise
-def decode_begin(seq_slot, last_token, seq_len, tokens, tok_slot, tok_pos, n_seqs: int) -> None:
+def decode_begin(seq_slot, last_token, seq_len, tokens, tok_slot, tok_pos, n_seqs: int, advance: bool = True) -> None:
     """A decode step's tokens, slots and positions from the per-sequence state, whose lengths go up by the step's token:
-    ``tokens_from_state``, ``step_meta`` and ``step_advance`` of one token a sequence in one launch."""
+    ``tokens_from_state``, ``step_meta`` and ``step_advance`` of one token a sequence in one launch.  ``advance=False`` leaves
+    the lengths to a ``step_advance`` behind the step."""
     for t, n in ((seq_slot, "seq_slot"), (last_token, "last_token"), (seq_len, "seq_len"), (tokens, "tokens"), (tok_slot, "tok_slot"), (tok_pos, "tok_pos")):
         _need(t, n, torch.int32)
     if min(seq_slot.numel(), tokens.numel(), tok_slot.numel(), tok_pos.numel()) < n_seqs:
         raise KernelError("decode_begin: index arrays shorter than the batch")
-    _ok(core().dryft_decode_begin(_ptr(seq_slot), _ptr(last_token), _ptr(seq_len), _ptr(tokens), _ptr(tok_slot), _ptr(tok_pos), n_seqs, _stream()),
-        "decode_begin")
+    _ok(core().dryft_decode_begin(_ptr(seq_slot), _ptr(last_token), _ptr(seq_len), _ptr(tokens), _ptr(tok_slot), _ptr(tok_pos), n_seqs, int(advance),
+                                  _stream()), "decode_begin")
 
 
 def embed(tokens, table, out, err=None, ss=None) -> None:

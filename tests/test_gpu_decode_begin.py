@@ -39,3 +39,35 @@ def test_embedding_rows_with_their_sums_of_squares(n, hidden):
     K.embed(toks, table, plain)
     K.row_sumsq(plain, ss2)
     assert torch.equal(rows, plain) and torch.equal(ss[:n], ss2[:n]) and int(err) == (1 if n > 1 else 0)
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_a_step_that_raises_leaves_the_lengths_as_they_were(model_dirs, graphs):
+    """An eager decode step that ends in an error half-way has appended nothing: device and host agree on the lengths, and the
+    step done again gives the logits of one that was never disturbed.  (A captured step is replayed whole or not at all.)"""
+    from dryft_b200.engine.api import Engine
+
+    def run(disturb):
+        eng = Engine(model_dirs["a"], dtype="bfloat16", max_batch=4, max_seq_len=256, max_tokens=1024, cuda_graphs=graphs)
+        out = []
+        with torch.inference_mode():
+            slots = eng.cache.open_sequences(3)
+            eng.stepper.step(slots, [[1, 2, 3], [4] * 20, [5]], [[], [], []])
+            at = torch.tensor(slots, device="cuda")
+            for t in range(4):
+                eng.cache.last_token.index_copy_(0, at, torch.tensor([t + 1, 2 * t, 3], dtype=torch.int32, device="cuda"))
+                if disturb and t in (0, 2):
+                    forward = eng.model.forward
+                    if graphs and t == 2:
+                        eng.stepper._graphs.clear()          # another capture, which fails
+                    eng.model.forward = lambda *a, **k: (forward(*a, **k), 1 / 0)
+                    with pytest.raises(ZeroDivisionError):
+                        eng.stepper.decode_from_state(slots)
+                    del eng.model.forward
+                    torch.cuda.synchronize()
+                    assert [int(n) for n in eng.cache.seq_len[at]] == [eng.cache.len_host[s] for s in slots]
+                out.append(eng.stepper.decode_from_state(slots)[:3].clone())
+            assert [int(n) for n in eng.cache.seq_len[at]] == [eng.cache.len_host[s] for s in slots]
+        return torch.stack(out)
+
+    assert torch.equal(run(True), run(False))
