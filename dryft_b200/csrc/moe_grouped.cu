@@ -371,6 +371,19 @@ __device__ __forceinline__ void tmem_ld16(unsigned taddr, unsigned (&r)[16]) {
                : "r"(taddr));
 }
 
+// n / d for d >= 1: the quotient by an approximate reciprocal, and one of Newton's corrections of it by what is left of n.  Without a
+// branch, so that a thread's sixteen quotients overlap: with the compiler's division, which branches for extreme exponents, a layer of
+// 64 experts of 768 x 2,048 takes 280 us for 2,048 tokens x 8, with this one 266.  For silu of every gate between -88.7 and 200 the two
+// give the same 32-bit values, 4.2 x 2^-24 off at most; a fast exponential and division (258 us) are 18 x 2^-24 off and give zero
+// below -87.3.
+__device__ __forceinline__ float over(float n, float d) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = n * r;
+  const float better = fmaf(fmaf(-q, d, n), r, q);
+  return d <= 1.f ? n : d <= 3.402823466e38f ? better : n * 0.f;      // (infinite n and d: the products above are no numbers)
+}
+
 // The product is computed transposed: two tiles of 128 weight rows (gate and up rows of the same 128 features, or 256
 // features) are the 128-row operands, up to NMAX sorted rows of one expert the columns, so that an expert's last tile is
 // padded to 16 rows and not to 128.  What bounds it: operands on their way from L2 (a k slice of 64 is 32 KB of weights and
@@ -521,11 +534,11 @@ __global__ void __launch_bounds__(TC_THREADS) moe_grouped_tc_kernel(
 #pragma unroll
         for (int c = 0; c < 16; ++c) {
           float x = __uint_as_float(r0[c]), y = __uint_as_float(r1[c]);
-          if (MODE == 0) x = __fdividef(x, 1.f + __expf(-x)) * y;     // (rounded to bfloat16 right away)
+          if (MODE == 0) x = over(x, 1.f + expf(-x)) * y;
           if (MODE == 3) {
             const float sc = __shfl_sync(0xffffffffu, my_w, c);
             const float g = fminf(x * sc, limit), up = fminf(fmaxf(y * sc, -limit), limit);
-            x = __fdividef(g, 1.f + __expf(-alpha * g)) * (up + up_off);
+            x = over(g, 1.f + expf(-alpha * g)) * (up + up_off);
           }
           if (MODE == 2) {
             x = fmaxf(x, 0.f); x *= x;

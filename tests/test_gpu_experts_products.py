@@ -117,3 +117,26 @@ def test_weighted_sum(dtype, n, top, width):
     unit = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -23
     bound = unit * exact.abs() + 2.0 ** -23 * top * (y.double().view(n, top, width).abs() * wts.double()[..., None]).sum(1)
     assert bool(((out.double() - exact).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("act", ["silu", "clamped"])
+@pytest.mark.parametrize("n", [8, 300])
+def test_activation_of_gates_far_below_zero(act, n):
+    """Gates of -86 to -88.5: one plus the exponential is beyond 2^126, where a fast division gives zero.  With an up value of
+    2^100 the activation is an ordinary bfloat16 number."""
+    from dryft_b200.ops import kernels as K
+
+    f = width = 64
+    gates = torch.linspace(-88.5, -86.0, 6, device="cuda").repeat(11)[:f]          # steps of a half: exact in bfloat16
+    w1 = torch.zeros(1, 2 * f, width, device="cuda")
+    w1[0, :f, 0], w1[0, f:, 0] = gates, 2.0 ** 100
+    w1, w2 = w1.bfloat16(), torch.eye(f, device="cuda")[None].bfloat16().contiguous()
+    h = torch.zeros(n, width, dtype=torch.bfloat16, device="cuda")
+    h[:, 0] = 1.0
+    idx, in_w = torch.zeros(n, 1, dtype=torch.int32, device="cuda"), torch.ones(n, 1, device="cuda")
+    y = torch.empty(n, width, dtype=torch.bfloat16, device="cuda")
+    K.moe_grouped(h, w1, w2, idx, y, in_w=in_w if act == "clamped" else None, limit=2.0 ** 120, alpha=1.0)
+    exact = _exact(h, w1, w2, idx, act, in_w, 2.0 ** 120, 1.0, 0.0)
+    assert float(exact.abs().min()) > 1e-8
+    # two roundings to bfloat16 (the second of a value that has been rounded); the 32-bit evaluation is exact to 2^-20
+    assert bool(((y.double() - exact).abs() <= 2.0 ** -8 * exact.abs()).all())
