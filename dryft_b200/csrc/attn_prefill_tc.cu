@@ -25,6 +25,7 @@
 // every role leaves its loop; the block then gives its own copies a bounded time to land, frees its
 // tensor memory and returns.  No block waits on another block.  No TMA load uses cluster multicast.
 #include "common.cuh"
+#include "drain.h"
 #include <cuda.h>
 #include <math.h>
 
@@ -175,7 +176,8 @@ __global__ void __launch_bounds__(THREADS, 2) attn_prefill_tc_kernel(
   unsigned long long* p_ready = s_full + 2;             // [2] softmax warps (128 arrivals) -> MMA
   unsigned long long* o_done = p_ready + 2;             // P V product done -> softmax warps
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(o_done + 1);
-  __shared__ int failed_s;
+  __shared__ int failed_s, k_issued_s, v_issued_s;    // copies of K and of V that the copying thread has issued
+  __shared__ unsigned long long drained_s;            // after a failure: the products issued so far are done
   volatile int* failed = &failed_s;
 
   // Heads run fastest: the host lists the tiles with the most keys first, so all heads of the longest
@@ -193,7 +195,8 @@ __global__ void __launch_bounds__(THREADS, 2) attn_prefill_tc_kernel(
   const int* pt = page_table + (size_t)slot * max_pages;
 
   if (threadIdx.x == 0) {
-    failed_s = 0;
+    failed_s = k_issued_s = v_issued_s = 0;
+    mbar_init(&drained_s, 1);
     mbar_init(q_full, 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&k_full[s], 1); mbar_init(&k_free[s], 1); mbar_init(&v_full[s], 1); mbar_init(&v_free[s], 1);
@@ -234,17 +237,22 @@ __global__ void __launch_bounds__(THREADS, 2) attn_prefill_tc_kernel(
 #pragma unroll
       for (int a = 0; a < DA; ++a) tma_load_3d(q_s + a * Q_ATOM, &map_q, a * 64, h, tok0, q_full);
       load_k(0);
+      int k_issued = 1, v_issued = 0;
       bool ok = true;
       for (int j = 0; j < n_tiles && ok; ++j) {
         if (j + 1 < n_tiles) {
           if (j + 1 >= STAGES) ok = mbar_wait(&k_free[(j + 1) % STAGES], (unsigned)((((j + 1) / STAGES) - 1) & 1), err, failed, 2);
           if (!ok) break;
           load_k(j + 1);
+          ++k_issued;
         }
         if (j >= STAGES) ok = mbar_wait(&v_free[j % STAGES], (unsigned)(((j / STAGES) - 1) & 1), err, failed, 3);
         if (!ok) break;
         load_v(j);
+        ++v_issued;
       }
+      k_issued_s = k_issued;
+      v_issued_s = v_issued;
     }
   } else if (warp == 5) {
     if (lane == 0) {
@@ -413,13 +421,17 @@ __global__ void __launch_bounds__(THREADS, 2) attn_prefill_tc_kernel(
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (*failed) {
-    // a wait ran out: give copies that may still be in flight a bounded time to land
-    if (threadIdx.x == 0) {
-      const long long t0 = clock64();
-      for (int s = 0; s < STAGES; ++s) {
-        while (!mbar_try_wait(&k_full[s], 0) && !mbar_try_wait(&k_full[s], 1) && clock64() - t0 < WAIT_CYCLES) {}
-        while (!mbar_try_wait(&v_full[s], 0) && !mbar_try_wait(&v_full[s], 1) && clock64() - t0 < WAIT_CYCLES) {}
-      }
+    // a wait ran out: give copies and products that may still be in flight a bounded time to end
+    const long long t0 = clock64();
+    auto expired = [&] { return clock64() - t0 > WAIT_CYCLES; };
+    if (threadIdx.x == 128) {     // the thread that issued the copies
+      while (!mbar_try_wait(q_full, 0) && !expired()) {}
+      ring_drain(k_issued_s, STAGES, [&](int s, unsigned parity) { return mbar_try_wait(&k_full[s], parity); }, expired);
+      ring_drain(v_issued_s, STAGES, [&](int s, unsigned parity) { return mbar_try_wait(&v_full[s], parity); }, expired);
+    }
+    if (threadIdx.x == 160) {     // the thread that issued the products
+      umma_commit(&drained_s);
+      while (!mbar_try_wait(&drained_s, 0) && !expired()) {}
     }
     __syncthreads();
   }

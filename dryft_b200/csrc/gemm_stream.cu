@@ -32,6 +32,7 @@
 //
 // Requires K % 64 == 0 and 16-byte aligned rows; N and M are arbitrary (M <= 64).
 #include "common.cuh"
+#include "drain.h"
 #include <cuda.h>
 #include <math.h>
 
@@ -154,7 +155,8 @@ __global__ void __launch_bounds__(NORM ? 320 : 192) gemm_stream_kernel(const __g
   float* ssw_s = inv_s + 64;                                // [4][64] sums of squares per finishing warp
   unsigned* tmem_slot = reinterpret_cast<unsigned*>(ssw_s + 4 * 64);
   int* last_s = reinterpret_cast<int*>(tmem_slot + 1);
-  __shared__ int failed_s;
+  __shared__ int failed_s, issued_s;                  // issued_s: stages that the copying thread has filled
+  __shared__ unsigned long long drained_s;            // after a failure: the products issued so far are done
   volatile int* failed = &failed_s;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -165,7 +167,8 @@ __global__ void __launch_bounds__(NORM ? 320 : 192) gemm_stream_kernel(const __g
   const int n_units = (int)(u1 - u0);
 
   if (threadIdx.x == 0) {
-    failed_s = 0;
+    failed_s = issued_s = 0;
+    mbar_init(&drained_s, 1);
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&w_full[s], 1); mbar_init(&x_full[s], 1); mbar_init(&x_ready[s], 128); mbar_init(&empty[s], 1);
     }
@@ -209,11 +212,13 @@ __global__ void __launch_bounds__(NORM ? 320 : 192) gemm_stream_kernel(const __g
       for (int i = 0; i < pre; ++i) load_w(i);
       pdl_wait();
       for (int i = 0; i < pre; ++i) load_x(i);
-      for (int i = pre; i < n_units; ++i) {
+      int i = pre;
+      for (; i < n_units; ++i) {
         if (!mbar_wait(&empty[i % STAGES], (unsigned)(((i / STAGES) - 1) & 1), p.err, failed, 1)) break;
         load_w(i);
         load_x(i);
       }
+      issued_s = i;
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -436,13 +441,16 @@ __global__ void __launch_bounds__(NORM ? 320 : 192) gemm_stream_kernel(const __g
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (*failed) {
-    // a wait ran out: give copies that may still be in flight a bounded time to land
+    // a wait ran out: give copies and products that may still be in flight a bounded time to end
+    const long long t0 = clock64();
+    auto expired = [&] { return clock64() - t0 > WAIT_CYCLES; };
     if (threadIdx.x == 0) {
-      const long long t0 = clock64();
-      for (int s = 0; s < STAGES; ++s) {
-        while (!mbar_try_wait(&w_full[s], 0) && !mbar_try_wait(&w_full[s], 1) && clock64() - t0 < WAIT_CYCLES) {}
-        while (!mbar_try_wait(&x_full[s], 0) && !mbar_try_wait(&x_full[s], 1) && clock64() - t0 < WAIT_CYCLES) {}
-      }
+      ring_drain(issued_s, STAGES, [&](int s, unsigned parity) { return mbar_try_wait(&w_full[s], parity); }, expired);
+      ring_drain(issued_s, STAGES, [&](int s, unsigned parity) { return mbar_try_wait(&x_full[s], parity); }, expired);
+    }
+    if (threadIdx.x == 32) {      // the thread that issued the products
+      umma_commit(&drained_s);
+      while (!mbar_try_wait(&drained_s, 0) && !expired()) {}
     }
     __syncthreads();
   }

@@ -16,6 +16,7 @@
 //
 // No block waits on another block.
 #include "common.cuh"
+#include "drain.h"
 #include <cuda.h>
 #include <math.h>
 #include <type_traits>
@@ -424,13 +425,15 @@ __global__ void __launch_bounds__(TC_THREADS) moe_grouped_tc_kernel(
   unsigned long long* const acc_empty = acc_full + L::BUFS;
   unsigned* const tmem_slot = reinterpret_cast<unsigned*>(acc_empty + L::BUFS);
   volatile int* const ring = reinterpret_cast<volatile int*>(tmem_slot + 4);
-  __shared__ int failed_s;
+  __shared__ int failed_s, issued_s;                  // issued_s: stages that the copying thread has filled or closed
+  __shared__ unsigned long long drained_s;            // after a failure: the products issued so far are done
   volatile int* failed = &failed_s;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rows_per_expert = L::GATED ? 2 * n_out : n_out;
 
   if (threadIdx.x == 0) {
-    failed_s = 0;
+    failed_s = issued_s = 0;
+    mbar_init(&drained_s, 1);
     for (int s = 0; s < L::STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
     for (int b = 0; b < L::BUFS; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 256); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -472,8 +475,10 @@ __global__ void __launch_bounds__(TC_THREADS) moe_grouped_tc_kernel(
       }
       if (ok && stage_free(i % L::STAGES)) {
         ring[drawn % L::RING] = -1;
+        ++i;
         mbar_arrive(&full[i % L::STAGES]);
       }
+      issued_s = i;
     }
   } else if (warp == 1) {
     if (lane == 0) {
@@ -573,11 +578,13 @@ __global__ void __launch_bounds__(TC_THREADS) moe_grouped_tc_kernel(
 
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (*failed) {   // a wait ran out: give copies that may still be in flight a bounded time to land
-    if (threadIdx.x == 0) {
-      const long long t0 = clock64();
-      for (int s = 0; s < L::STAGES; ++s)
-        while (!mbar_try_wait(&full[s], 0) && !mbar_try_wait(&full[s], 1) && clock64() - t0 < WAIT_CYCLES) {}
+  if (*failed) {   // a wait ran out: give copies and products that may still be in flight a bounded time to end
+    const long long t0 = clock64();
+    auto expired = [&] { return clock64() - t0 > WAIT_CYCLES; };
+    if (threadIdx.x == 0) ring_drain(issued_s, L::STAGES, [&](int s, unsigned parity) { return mbar_try_wait(&full[s], parity); }, expired);
+    if (threadIdx.x == 32) {      // the thread that issued the products
+      umma_commit(&drained_s);
+      while (!mbar_try_wait(&drained_s, 0) && !expired()) {}
     }
     __syncthreads();
   }
