@@ -475,8 +475,8 @@ __global__ void __launch_bounds__(TC_THREADS) moe_grouped_tc_kernel(
       }
       if (ok && stage_free(i % L::STAGES)) {
         ring[drawn % L::RING] = -1;
-        ++i;
         mbar_arrive(&full[i % L::STAGES]);
+        ++i;
       }
       issued_s = i;
     }
