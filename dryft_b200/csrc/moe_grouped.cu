@@ -623,7 +623,7 @@ struct Sorted { const int *perm, *tile_expert, *tile_row0, *tile_rows, *n_tiles;
 
 template <int MODE, int NMAX>
 int tc_launch(const void* x, long long x_rows, const void* w, int E, const Sorted& t, int K, int n_out, void* out, int sms,
-              const float* in_w, float limit, float alpha, float up_off, int* err, cudaStream_t st) {
+              const float* in_w, float limit, float alpha, float up_off, int* err, int pdl, cudaStream_t st) {
   typedef Tc<MODE, NMAX> L;
   CUtensorMap map_w, map_x;
   if (!encode(&map_w, w, (long long)E * (L::GATED ? 2 : 1) * n_out, K, 128) || !encode(&map_x, x, x_rows, K, 64)) return DRYFT_ERR_UNSUPPORTED;
@@ -640,7 +640,7 @@ int tc_launch(const void* x, long long x_rows, const void* w, int E, const Sorte
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = pdl ? 1 : 0;
   const cudaError_t rc = cudaLaunchKernelEx(&cfg, moe_grouped_tc_kernel<MODE, NMAX>, map_w, map_x, t.perm, t.tile_expert, t.tile_row0, t.tile_rows,
                                             t.n_tiles, t.next + (MODE == 1), K / 64, n_out, f_tiles, (bf16*)out, in_w, limit, alpha, up_off, err);
   if (rc != cudaSuccess) return (int)rc;
@@ -673,9 +673,10 @@ DRYFT_API long long dryft_moe_grouped_work_ints(int n_assign, int E) {
 // y[n*top, C] = experts of idx[n, top] applied to h[n, W]; act [n*top, F] is scratch (sorted order), as y is before its values
 // `gated`: 1 = w_gate_up is [E, 2F, W] and the activation is silu(gate) * up; 0 = it is [E, F, W] and the activation is max(., 0)^2;
 // 2 = [E, 2F, W] with the clamped activation of MODE 3 (in_w [n*top]: each assignment's weight on the expert's input)
+// `pdl`: the tcgen05 products are programmatic dependents of the launches before them; `tcgen05` 0: the mma.sync products at any size
 DRYFT_API int dryft_moe_grouped(const void* h, const void* w_gate_up, const void* w_down, const int* idx, int n_tokens, int top,
                                 int E, int W, int F, void* act, void* y, int* work, int gated, const float* in_w, float limit,
-                                float alpha, float up_off, int* err, cudaStream_t st) {
+                                float alpha, float up_off, int* err, int pdl, int tcgen05, cudaStream_t st) {
   if (n_tokens <= 0) return 0;
   if (top < 1 || E < 1 || W % 16 || F % 16 || W < 16 || F < 16 || gated < 0 || gated > 2 || (gated == 2 && !in_w)) return DRYFT_ERR_UNSUPPORTED;
   const long long n_assign_ll = (long long)n_tokens * top;
@@ -683,7 +684,7 @@ DRYFT_API int dryft_moe_grouped(const void* h, const void* w_gate_up, const void
       (long long)E * W > (1LL << 31) - 1)
     return DRYFT_ERR_UNSUPPORTED;
   const int n_assign = (int)n_assign_ll;
-  const bool tc = tc_takes(W, F, h, w_gate_up, w_down, act, y);
+  const bool tc = tcgen05 && tc_takes(W, F, h, w_gate_up, w_down, act, y);
   const int bm = tile_rows_for(n_assign, E, tc), max_tiles = max_tiles_for(n_assign, E, tc);
   int* const perm = work;
   int* const place = perm + n_assign;
@@ -707,10 +708,10 @@ DRYFT_API int dryft_moe_grouped(const void* h, const void* w_gate_up, const void
     if (rc) return rc;
     auto both = [&](auto nmax) {
       constexpr int N = decltype(nmax)::value;
-      int r = gated == 2 ? tc_launch<3, N>(y, n_assign, w_gate_up, E, t, W, F, act, sms, in_w, limit, alpha, up_off, err, st)
-              : gated    ? tc_launch<0, N>(y, n_assign, w_gate_up, E, t, W, F, act, sms, nullptr, 0.f, 1.f, 0.f, err, st)
-                         : tc_launch<2, N>(y, n_assign, w_gate_up, E, t, W, F, act, sms, nullptr, 0.f, 1.f, 0.f, err, st);
-      return r ? r : tc_launch<1, N>(act, n_assign, w_down, E, t, F, W, y, sms, nullptr, 0.f, 1.f, 0.f, err, st);
+      int r = gated == 2 ? tc_launch<3, N>(y, n_assign, w_gate_up, E, t, W, F, act, sms, in_w, limit, alpha, up_off, err, pdl, st)
+              : gated    ? tc_launch<0, N>(y, n_assign, w_gate_up, E, t, W, F, act, sms, nullptr, 0.f, 1.f, 0.f, err, pdl, st)
+                         : tc_launch<2, N>(y, n_assign, w_gate_up, E, t, W, F, act, sms, nullptr, 0.f, 1.f, 0.f, err, pdl, st);
+      return r ? r : tc_launch<1, N>(act, n_assign, w_down, E, t, F, W, y, sms, nullptr, 0.f, 1.f, 0.f, err, pdl, st);
     };
     return bm == 256 ? both(std::integral_constant<int, 256>()) : both(std::integral_constant<int, 128>());
   }

@@ -24,7 +24,7 @@ namespace {
 constexpr int THREADS = 256, WIDE_THREADS = 512;
 constexpr int MAX_STREAMS = 8;
 
-// A launch of up to FEW_ROWS rows is a programmatic dependent: its blocks come in, and fetch the layer's own numbers, while the
+// A launch of up to FEW_ROWS rows is (where the caller's `pdl` asks for it) a programmatic dependent: its blocks come in, and fetch the layer's own numbers, while the
 // launch before it drains; the kernel waits before it reads or writes what other launches touch, and reads that past L1 (ld_prev).
 // The rows are those up to which the products on both sides overlap their launches too.
 constexpr int FEW_ROWS = 16;
@@ -309,7 +309,7 @@ DRYFT_API int dryft_seq_last_token(const int* tokens, const int* tok_slot, int n
 
 DRYFT_API int dryft_hc_step(int is_bf16, const float* x_in, int s_in, float* x_out, int n_streams, const void* y, const float* mix,
                             const float* outw, float mult, const float* inw, const float* norm_w, float eps, const int* rows,
-                            void* h, int n_rows, int width, cudaStream_t st) {
+                            void* h, int n_rows, int width, int pdl, cudaStream_t st) {
   if (n_rows <= 0) return 0;
   if (n_streams < 1 || n_streams > MAX_STREAMS || (s_in != 1 && s_in != n_streams)) return DRYFT_ERR_UNSUPPORTED;
   if (y && (!mix || !outw)) return DRYFT_ERR_UNSUPPORTED;
@@ -320,7 +320,7 @@ DRYFT_API int dryft_hc_step(int is_bf16, const float* x_in, int s_in, float* x_o
   do {                                                                                                                          \
     int rc = row_smem(hc_step_kernel<TT, MS>, width);                                                                           \
     if (rc) return rc;                                                                                                          \
-    return launch_rows(hc_step_kernel<TT, MS>, dim3(n_rows), width > 1024 ? WIDE_THREADS : THREADS, smem, n_rows <= FEW_ROWS, st, x_in, s_in, x_out, \
+    return launch_rows(hc_step_kernel<TT, MS>, dim3(n_rows), width > 1024 ? WIDE_THREADS : THREADS, smem, pdl && n_rows <= FEW_ROWS, st, x_in, s_in, x_out, \
                        n_streams, (const TT*)y, mix, outw, mult, inw, norm_w, eps, rows, (TT*)h, width);                        \
   } while (0)
 #define DRYFT_HC_BY_STREAMS(TT)                                                                                                  \
@@ -337,12 +337,12 @@ DRYFT_API int dryft_hc_step(int is_bf16, const float* x_in, int s_in, float* x_o
 }
 
 DRYFT_API int dryft_glu_clamp(int is_bf16, const void* gate_up, void* out, int rows, int inter, float limit, int has_limit,
-                              float alpha, float up_offset, cudaStream_t st) {
+                              float alpha, float up_offset, int pdl, cudaStream_t st) {
   if (rows <= 0 || inter <= 0) return 0;
   typedef __nv_bfloat16 bf;
   const int vec = (inter & 3) == 0 ? 4 : 1;
   const unsigned blocks = (unsigned)(((size_t)rows * inter / vec + 255) / 256);
-  const bool behind = rows <= FEW_ROWS;
+  const bool behind = pdl && rows <= FEW_ROWS;
 #define DRYFT_GLU(TT, VEC) \
   launch_rows(glu_clamp_kernel<TT, VEC>, dim3(blocks), 256, 0, behind, st, (const TT*)gate_up, (TT*)out, rows, inter, limit, has_limit, alpha, up_offset)
   if (is_bf16) return vec == 4 ? DRYFT_GLU(bf, 4) : DRYFT_GLU(bf, 1);

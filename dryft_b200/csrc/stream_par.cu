@@ -25,7 +25,7 @@
 namespace {
 constexpr int THREADS = 256, WIDE_THREADS = 512;
 
-// A launch of up to FEW_ROWS rows is a programmatic dependent: its blocks come in, and fetch the layer's own numbers, while the
+// A launch of up to FEW_ROWS rows is (where the caller's `pdl` asks for it) a programmatic dependent: its blocks come in, and fetch the layer's own numbers, while the
 // launch before it drains; the kernel waits before it reads or writes what other launches touch, and reads that past L1 (ld_prev).
 // The rows are those up to which the products on both sides overlap their launches too.
 constexpr int FEW_ROWS = 16;
@@ -185,15 +185,16 @@ __global__ void __launch_bounds__(WIDE_THREADS) stream_sum_ln_kernel(
 
 template <typename T, int VEC>
 int sum_ln_launch(float* x32, const int* rows, const void* y0, float s0, const void* y1, float s1, const void* y2, float s2, const float* w0,
-                  const float* b0, void* h0, const float* w1, const float* b1, void* h1, float eps, int n, int width, cudaStream_t st) {
+                  const float* b0, void* h0, const float* w1, const float* b1, void* h1, float eps, int n, int width, int pdl,
+                  cudaStream_t st) {
   const size_t smem = sizeof(float) * (size_t)width;
   if (smem > 200 * 1024) return DRYFT_ERR_UNSUPPORTED;
   if (smem > 48 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(stream_sum_ln_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
   }
-  return launch_rows(stream_sum_ln_kernel<T, VEC>, dim3(n), width > 1024 ? WIDE_THREADS : THREADS, smem, n <= FEW_ROWS, st, x32, rows, (const T*)y0, s0,
-                     (const T*)y1, s1, (const T*)y2, s2, w0, b0, (T*)h0, w1, b1, (T*)h1, eps, width);
+  return launch_rows(stream_sum_ln_kernel<T, VEC>, dim3(n), width > 1024 ? WIDE_THREADS : THREADS, smem, pdl && n <= FEW_ROWS, st, x32, rows,
+                     (const T*)y0, s0, (const T*)y1, s1, (const T*)y2, s2, w0, b0, (T*)h0, w1, b1, (T*)h1, eps, width);
 }
 
 template <typename T, int VEC>
@@ -378,17 +379,17 @@ DRYFT_API int dryft_stream_sum(int is_bf16, float* x32, const float* src, const 
 
 DRYFT_API int dryft_stream_sum_ln(int is_bf16, float* x32, const int* rows, const void* y0, float s0, const void* y1, float s1, const void* y2,
                                   float s2, const float* w0, const float* b0, void* h0, const float* w1, const float* b1, void* h1, float eps,
-                                  int n, int width, cudaStream_t st) {
+                                  int n, int width, int pdl, cudaStream_t st) {
   if (n <= 0) return 0;
   if (width <= 0 || (rows != nullptr && (y0 != nullptr || y1 != nullptr || y2 != nullptr)) || (h0 != nullptr && (w0 == nullptr || b0 == nullptr)) ||
       (h1 != nullptr && (w1 == nullptr || b1 == nullptr)))
     return DRYFT_ERR_UNSUPPORTED;
   const bool vec = width % 4 == 0;
   if (is_bf16)
-    return vec ? sum_ln_launch<__nv_bfloat16, 4>(x32, rows, y0, s0, y1, s1, y2, s2, w0, b0, h0, w1, b1, h1, eps, n, width, st)
-               : sum_ln_launch<__nv_bfloat16, 1>(x32, rows, y0, s0, y1, s1, y2, s2, w0, b0, h0, w1, b1, h1, eps, n, width, st);
-  return vec ? sum_ln_launch<float, 4>(x32, rows, y0, s0, y1, s1, y2, s2, w0, b0, h0, w1, b1, h1, eps, n, width, st)
-             : sum_ln_launch<float, 1>(x32, rows, y0, s0, y1, s1, y2, s2, w0, b0, h0, w1, b1, h1, eps, n, width, st);
+    return vec ? sum_ln_launch<__nv_bfloat16, 4>(x32, rows, y0, s0, y1, s1, y2, s2, w0, b0, h0, w1, b1, h1, eps, n, width, pdl, st)
+               : sum_ln_launch<__nv_bfloat16, 1>(x32, rows, y0, s0, y1, s1, y2, s2, w0, b0, h0, w1, b1, h1, eps, n, width, pdl, st);
+  return vec ? sum_ln_launch<float, 4>(x32, rows, y0, s0, y1, s1, y2, s2, w0, b0, h0, w1, b1, h1, eps, n, width, pdl, st)
+             : sum_ln_launch<float, 1>(x32, rows, y0, s0, y1, s1, y2, s2, w0, b0, h0, w1, b1, h1, eps, n, width, pdl, st);
 }
 
 DRYFT_API int dryft_stream_norm_join(int is_bf16, float* x32, const void* y0, float s0, const void* y1, float s1, const void* y2, float s2,

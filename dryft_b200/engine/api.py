@@ -49,13 +49,13 @@ class EngineOptions:
     stream_m_max: int = 0                  # rows up to which they stream them by TMA into tcgen05.mma above that (0: cuBLAS,
                                            # which is faster today: profiles/gemm_stream_microbench.md)
     fuse_decode: bool = True               # fold norms, adds and SiLU*mul into the decode products
-    pdl: bool = True                       # programmatic dependent launch between the decode products
+    pdl: bool = True                       # programmatic dependent launches: the decode products and what stands between them
     # fused decode: the next norm's weight is applied by the product before it and the norm's factor by the product
     # behind it.  3 % faster at batch 1 to 8, but the activations are then rounded once where the reference rounds twice
     # (engine/dryft_qwen3/model.py:28-32): as close to 32-bit as the default, 1.3 times further from a plain bfloat16
     # evaluation.  Off by default: the default path keeps the reference's rounding points.
     norm_ahead: bool = False
-    tcgen05: bool = True                   # prefill attention on tcgen05 / TMEM / TMA where the head size allows
+    tcgen05: bool = True                   # prefill attention and experts' products on tcgen05 / TMEM / TMA where the sizes allow
     # steps of up to this many rows run sublayers that read the same input (a mixer beside a feed-forward, two mixers side
     # by side) on streams of their own, joined before their results are summed: in a captured step they are parallel
     # branches of the graph.  0: one after another.  The results are the same bits either way.

@@ -943,7 +943,7 @@ def moe_grouped_lib() -> ctypes.CDLL:
     with _lock:
         if _moe_grouped is None:
             lib = _load(build.build_library("moe_grouped", ("moe_grouped.cu",)))
-            lib.dryft_moe_grouped.argtypes = [_p, _p, _p, _p, _i, _i, _i, _i, _i, _p, _p, _p, _i, _p, _f, _f, _f, _p, _p]
+            lib.dryft_moe_grouped.argtypes = [_p, _p, _p, _p, _i, _i, _i, _i, _i, _p, _p, _p, _i, _p, _f, _f, _f, _p, _i, _i, _p]
             lib.dryft_moe_grouped.restype = _i
             lib.dryft_moe_grouped_work_ints.argtypes = [_i, _i]
             lib.dryft_moe_grouped_work_ints.restype = _ll
@@ -952,12 +952,12 @@ def moe_grouped_lib() -> ctypes.CDLL:
 
 
 def moe_grouped(h, w_gate_up, w_down, idx, y, gated: bool = True, in_w=None, limit: Optional[float] = None, alpha: float = 1.0,
-                up_offset: float = 0.0) -> None:
+                up_offset: float = 0.0, pdl: bool = True, tcgen05: bool = True) -> None:
     """``y[n*top + k] = expert idx[n, k] applied to h[n]`` (bfloat16) with the assignments sorted by expert on the device and
     both expert products as grouped tensor-core products (``csrc/moe_grouped.cu``: three or four launches, no host round trip).
     ``gated=False``: ``w_gate_up`` is ``[E, F, W]`` (no gate rows) and the activation is ``max(., 0)^2``.  With ``in_w [n, top]``
     (float32) each assignment's weight scales its expert's input and the activation is the clamped one of ``moe_rows``'s
-    ``gate_up_clamp`` mode."""
+    ``gate_up_clamp`` mode.  ``pdl``: the tcgen05 products are programmatic dependents; ``tcgen05=False``: ``mma.sync`` at any size."""
     n, width = h.shape
     top = idx.shape[1]
     e, two_f, _ = w_gate_up.shape
@@ -978,8 +978,8 @@ def moe_grouped(h, w_gate_up, w_down, idx, y, gated: bool = True, in_w=None, lim
         _need(in_w, "in_w", torch.float32, (n, top))
     _ok(lib.dryft_moe_grouped(_ptr(h), _ptr(w_gate_up), _ptr(w_down), _ptr(idx), n, top, e, width, f, _ptr(act), _ptr(y), _ptr(work),
                               2 if in_w is not None else int(gated), _ptr(in_w), float("inf") if limit is None else float(limit),
-                              float(alpha), float(up_offset), _ptr(error_flag(h.device)), _stream()),
-        f"moe_grouped ({e} experts, {width} x {f})", n_kernels=4 if width % 64 == 0 and f % 64 == 0 else 3)
+                              float(alpha), float(up_offset), _ptr(error_flag(h.device)), int(pdl), int(tcgen05), _stream()),
+        f"moe_grouped ({e} experts, {width} x {f})", n_kernels=4 if tcgen05 and width % 64 == 0 and f % 64 == 0 else 3)
 
 
 # ----------------------------------------------------------------------------- matrix products
@@ -1286,8 +1286,8 @@ def stream_hc_lib() -> ctypes.CDLL:
     return _single_lib("stream_hc", {
         "dryft_embed_pair_norm": [_i, _p, _p, _p, _p, _p, _p, _i, _ll, _ll, _f, _p, _f, _p, _i, _i, _i, _p, _p],
         "dryft_seq_last_token": [_p, _p, _i, _p, _p],
-        "dryft_hc_step": [_i, _p, _i, _p, _i, _p, _p, _p, _f, _p, _p, _f, _p, _p, _i, _i, _p],
-        "dryft_glu_clamp": [_i, _p, _p, _i, _i, _f, _i, _f, _f, _p],
+        "dryft_hc_step": [_i, _p, _i, _p, _i, _p, _p, _p, _f, _p, _p, _f, _p, _p, _i, _i, _i, _p],
+        "dryft_glu_clamp": [_i, _p, _p, _i, _i, _f, _i, _f, _f, _i, _p],
     })
 
 
@@ -1353,11 +1353,12 @@ def seq_last_token(tokens, tok_slot, n: int, prev_state) -> None:
 
 
 def hc_step(x_in, n_streams: int, *, x_out=None, y=None, mix=None, outw=None, mult: float = 1.0, inw=None, norm_w=None,
-            eps: float = 0.0, rows=None, h=None) -> None:
+            eps: float = 0.0, rows=None, h=None, pdl: bool = True) -> None:
     """One joint of a residual stream held as ``n_streams`` 32-bit copies.  ``x_in`` is ``[n, n_streams, W]`` or ``[n, W]``
     (one copy standing for all).  With ``y [n, W]``: ``x'_t = sum_s mix[s, t] x_s + mult * outw[t] * y``; written to
     ``x_out [n, n_streams, W]`` if given (may be ``x_in``).  With ``inw``: ``h = T(rmsnorm(sum_t inw[t] x'_t) * norm_w)``;
-    with ``rows`` (int32) ``h[r]`` is made from row ``rows[r]`` (``x_out`` must then be left out)."""
+    with ``rows`` (int32) ``h[r]`` is made from row ``rows[r]`` (``x_out`` must then be left out).  ``pdl``: up to 16 rows are
+    launched as a programmatic dependent of the launch before."""
     _need(x_in, "streams", torch.float32)
     if x_in.dim() == 3:
         n, s_in, width = x_in.shape
@@ -1395,13 +1396,15 @@ def hc_step(x_in, n_streams: int, *, x_out=None, y=None, mix=None, outw=None, mu
     if act is None:
         raise KernelError("hc_step: nothing to do (neither y nor inw)")
     _ok(stream_hc_lib().dryft_hc_step(_act(act, "activations"), _ptr(x_in), s_in, _ptr(x_out), n_streams, _ptr(y), _ptr(mix), _ptr(outw),
-                                      float(mult), _ptr(inw), _ptr(norm_w), float(eps), _ptr(rows), _ptr(h), n_rows, width, _stream()),
+                                      float(mult), _ptr(inw), _ptr(norm_w), float(eps), _ptr(rows), _ptr(h), n_rows, width,
+                                      int(pdl), _stream()),
         f"hc_step ({n_streams} streams, width {width})")
 
 
-def glu_clamp(gate_up, out, limit: Optional[float], alpha: float, up_offset: float) -> None:
+def glu_clamp(gate_up, out, limit: Optional[float], alpha: float, up_offset: float, pdl: bool = True) -> None:
     """``out = g * sigmoid(alpha * g) * (u + up_offset)`` with ``g = min(gate, limit)``, ``u = clamp(up, -limit, limit)``
-    (no clamping when ``limit`` is None); ``gate_up [rows, 2F]`` holds the gate columns first."""
+    (no clamping when ``limit`` is None); ``gate_up [rows, 2F]`` holds the gate columns first.  ``pdl``: up to 16 rows are
+    launched as a programmatic dependent of the launch before."""
     rows, two_f = gate_up.shape
     _need(gate_up, "gate_up")
     if two_f % 2:
@@ -1409,7 +1412,7 @@ def glu_clamp(gate_up, out, limit: Optional[float], alpha: float, up_offset: flo
     _need(out, "glu_clamp output", gate_up.dtype, (rows, two_f // 2))
     _ok(stream_hc_lib().dryft_glu_clamp(_act(gate_up, "gate_up"), _ptr(gate_up), _ptr(out), rows, two_f // 2,
                                         float(limit if limit is not None else 0.0), int(limit is not None), float(alpha),
-                                        float(up_offset), _stream()), "glu_clamp")
+                                        float(up_offset), int(pdl), _stream()), "glu_clamp")
 
 
 # ----------------------------------------------------------------------------- recurrent mixers
@@ -2057,7 +2060,7 @@ def pool_attn_rows(q, k_pages, v_pages, page_table, pooled, sink, tok_slot, tok_
 def stream_par_lib() -> ctypes.CDLL:
     return _single_lib("stream_par", {
         "dryft_stream_sum": [_i, _p, _p, _p, _f, _p, _f, _p, _f, _p, _i, _f, _p, _p, _f, _p, _i, _i, _p],
-        "dryft_stream_sum_ln": [_i, _p, _p, _p, _f, _p, _f, _p, _f, _p, _p, _p, _p, _p, _p, _f, _i, _i, _p],
+        "dryft_stream_sum_ln": [_i, _p, _p, _p, _f, _p, _f, _p, _f, _p, _p, _p, _p, _p, _p, _f, _i, _i, _i, _p],
         "dryft_stream_norm_join": [_i, _p, _p, _f, _p, _f, _p, _f, _p, _p, _i, _p, _f, _p, _f, _p, _i, _i, _p],
         "dryft_pack_pair": [_i, _p, _p, _p, _i, _i, _p],
         "dryft_softcap": [_p, _ll, _f, _p],
@@ -2106,10 +2109,11 @@ def stream_sum(x32, terms=(), *, rows=None, top: int = 0, rows_scale: float = 1.
                                           n, width, _stream()), "stream_sum")
 
 
-def stream_sum_ln(x32, terms=(), *, norms=(), eps: float = 0.0, rows=None, n_rows: Optional[int] = None) -> None:
+def stream_sum_ln(x32, terms=(), *, norms=(), eps: float = 0.0, rows=None, n_rows: Optional[int] = None, pdl: bool = True) -> None:
     """``x32[n] += sum_i scale_i * y_i[n]`` in 32-bit for up to three ``terms`` ``(y_i, scale_i)`` of the activation type, and up to two
     layer norms of the new rows: ``norms`` lists ``(weight, bias, out)`` (``out [n, width]`` of the activation type).  ``rows``
-    (int32): output row ``r`` reads stream row ``rows[r]``; there are no terms then and the stream stays as it is."""
+    (int32): output row ``r`` reads stream row ``rows[r]``; there are no terms then and the stream stays as it is.  ``pdl``: up to
+    16 rows are launched as a programmatic dependent of the launch before."""
     width = x32.shape[1]
     n = x32.shape[0] if rows is None else (n_rows if n_rows is not None else rows.numel())
     _need(x32, "x32", torch.float32)
@@ -2136,7 +2140,7 @@ def stream_sum_ln(x32, terms=(), *, norms=(), eps: float = 0.0, rows=None, n_row
     (w0, b0, h0), (w1, b1, h1) = (list(norms) + [(None, None, None)] * 2)[:2]
     _ok(stream_par_lib().dryft_stream_sum_ln(int(act == torch.bfloat16), _ptr(x32), _ptr(rows), _ptr(terms[0][0]), terms[0][1], _ptr(terms[1][0]),
                                              terms[1][1], _ptr(terms[2][0]), terms[2][1], _ptr(w0), _ptr(b0), _ptr(h0), _ptr(w1), _ptr(b1), _ptr(h1),
-                                             float(eps), n, width, _stream()), "stream_sum_ln")
+                                             float(eps), n, width, int(pdl), _stream()), "stream_sum_ln")
 
 
 def stream_norm_join(x32, terms=(), *, factor, eps: float, rows=None, wts=None, norm_w=None, norm_eps: float = 0.0, h=None) -> None:

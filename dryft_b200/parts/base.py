@@ -63,9 +63,9 @@ class Runtime:
     stream_m_max: int = 0        # decode rows up to which the tcgen05 weight-streaming product runs above that (0: the library's)
     ffn_chunk_rows: int = 16384  # rows of the feed-forward processed at once (bounds [rows, 2I])
     fuse_decode: bool = True     # few rows: fold norms, residual adds and SiLU*mul into the products
-    pdl: bool = True             # launch the fused decode products as programmatic dependents
+    pdl: bool = True             # launch decode products, joins and experts' products as programmatic dependents
     norm_ahead: bool = False     # fused decode: a residual product leaves the stream weighted for the next norm (one rounding fewer than the reference)
-    tcgen05: bool = True         # prompts: attention on tcgen05.mma / tensor memory / TMA where sizes allow
+    tcgen05: bool = True         # attention of prompts and experts' products on tcgen05.mma / tensor memory / TMA where sizes allow
     branch_rows: int = 0         # steps of up to this many rows run independent sublayers on streams of their own (0: in turn)
     side_streams: list = field(default_factory=list, repr=False, compare=False)
 

@@ -320,12 +320,12 @@ class ParallelNormsBlock:
         K.stream_par_lib()
 
     @staticmethod
-    def _sum_and_norms(x: torch.Tensor, terms, norms, dtype) -> list:
+    def _sum_and_norms(x: torch.Tensor, terms, norms, rt) -> list:
         """``x`` plus the terms, in place, and the norms of the result (None for a norm that is None or of another kind)."""
         params = [nm.layer_params() if nm is not None and hasattr(nm, "layer_params") else None for nm in norms]
         eps = next((p[2] for p in params if p is not None), 0.0)
-        outs = [torch.empty(x.shape, dtype=dtype, device=x.device) if p is not None and p[2] == eps else None for p in params]
-        K.stream_sum_ln(x, terms, norms=[(p[0], p[1], o) for p, o in zip(params, outs) if o is not None], eps=eps)
+        outs = [torch.empty(x.shape, dtype=rt.dtype, device=x.device) if p is not None and p[2] == eps else None for p in params]
+        K.stream_sum_ln(x, terms, norms=[(p[0], p[1], o) for p, o in zip(params, outs) if o is not None], eps=eps, pdl=rt.pdl)
         return outs
 
     def forward(self, res: Residual, ctx: StepContext, cache, state, owns_cache: bool = True, next_norms=(None, None)) -> Residual:
@@ -337,7 +337,7 @@ class ParallelNormsBlock:
         hm = res.hn if (res.hn is not None and res.hn_norm is self.norm_mixer) else None
         hf = res.hn2 if (res.hn2 is not None and res.hn2_norm is self.norm_ffn) else None
         if hm is None or (self.ffn is not None and hf is None):
-            hm, hf = self._sum_and_norms(x, (), (self.norm_mixer, self.norm_ffn), rt.dtype)
+            hm, hf = self._sum_and_norms(x, (), (self.norm_mixer, self.norm_ffn), rt)
             if self.ffn is not None and hf is None:      # another eps than the mixer's norm: a launch of its own
                 hf = self.norm_ffn.forward(x)
 
@@ -353,7 +353,7 @@ class ParallelNormsBlock:
         else:
             a, f = rt.run_branches([mix, feed], first_stream=0) if rt.branches(x.shape[0]) else (mix(), feed())
             terms = a + f
-        outs = self._sum_and_norms(x, [(y, s * self.mult) for y, s in terms], next_norms, rt.dtype)
+        outs = self._sum_and_norms(x, [(y, s * self.mult) for y, s in terms], next_norms, rt)
         return Residual(x, hn=outs[0], hn_norm=next_norms[0] if outs[0] is not None else None,
                         hn2=outs[1], hn2_norm=next_norms[1] if outs[1] is not None else None)
 

@@ -114,7 +114,7 @@ class ClampedGLU:
     def _rows(self, h: torch.Tensor) -> torch.Tensor:
         gu = linear(h, self.w_gate_up, self.rt)
         act = torch.empty((h.shape[0], self.inter), dtype=h.dtype, device=h.device)
-        K.glu_clamp(gu, act, self.limit, self.alpha, self.up_offset)
+        K.glu_clamp(gu, act, self.limit, self.alpha, self.up_offset, pdl=self.rt.pdl)
         return linear(act, self.w_down, self.rt)
 
     def forward(self, h: torch.Tensor, ctx: StepContext) -> torch.Tensor:

@@ -90,7 +90,7 @@ class HyperBlock:
         write = res.delta is not None or out.data_ptr() != x.data_ptr()
         K.hc_step(x, self.streams, x_out=out if write else None, y=res.delta, mix=pend.mix if pend is not None else None,
                   outw=pend.outw if pend is not None else None, mult=pend.mult if pend is not None else 1.0, inw=conn.inw,
-                  norm_w=w, eps=eps, h=h)
+                  norm_w=w, eps=eps, h=h, pdl=self.mixer.rt.pdl)
         return out, h
 
     def forward(self, res: Residual, ctx: StepContext, cache, state, owns_cache: bool = True) -> Residual:
@@ -115,7 +115,7 @@ class HyperBlock:
         pend = res.conn
         K.hc_step(x, self.streams, y=res.delta, mix=pend.mix if pend is not None else None,
                   outw=pend.outw if pend is not None else None, mult=pend.mult if pend is not None else 1.0, inw=self._ones,
-                  norm_w=rms[0], eps=rms[1], rows=rows, h=h)
+                  norm_w=rms[0], eps=rms[1], rows=rows, h=h, pdl=self.mixer.rt.pdl)
         return h
 
     def stream_sum(self, res: Residual) -> torch.Tensor:

@@ -165,7 +165,7 @@ class MoE:
     def _grouped(self, n: int) -> bool:
         if not self.use_grouped or n >= self.GROUPED_MIN_TOKENS:
             return self.use_grouped
-        if self.hidden % 64 or self.inter % 64:      # the grouped products on mma.sync: for prompts only
+        if not self.rt.tcgen05 or self.hidden % 64 or self.inter % 64:      # the grouped products on mma.sync: for prompts only
             return False
         chosen = self.experts * (1.0 - (1.0 - self.top / self.experts) ** n)      # different experts, on the mean
         each = 2 * (self.w_gate_up[0].numel() + self.w_down[0].numel())
@@ -208,7 +208,8 @@ class MoE:
             self.side_out = z[:, self.side[0]:self.side[0] + self.side[1]]
         act = torch.empty((h.shape[0], self.shared_inter), dtype=h.dtype, device=h.device)
         if self.gated:
-            K.glu_clamp(z if z.shape[1] == self.shared_cols else z[:, :self.shared_cols].contiguous(), act, None, 1.0, 0.0)
+            K.glu_clamp(z if z.shape[1] == self.shared_cols else z[:, :self.shared_cols].contiguous(), act, None, 1.0, 0.0,
+                        pdl=self.rt.pdl)
         else:
             K.relu2(z[:, :self.shared_inter], act)
         ys = linear(act, self.w_shared_down, self.rt)
@@ -237,7 +238,7 @@ class MoE:
         in_w = wts if self.weight_input else (torch.ones_like(wts) if special else None)
         if self._grouped(n):
             K.moe_grouped(h, self.w_gate_up, self.w_down, idx, y, gated=self.gated, in_w=in_w, limit=self.limit, alpha=self.alpha,
-                          up_offset=self.up_offset)
+                          up_offset=self.up_offset, pdl=self.rt.pdl, tcgen05=self.rt.tcgen05)
         else:
             act = torch.empty((n * self.top, self.inter), dtype=h.dtype, device=h.device)
             if special:

@@ -143,7 +143,7 @@ class LayerNorm:
         n = n_rows if n_rows is not None else (rows.numel() if rows is not None else x.shape[0])
         out = torch.empty((n, self.size), dtype=self.rt.dtype, device=x.device)
         K.stream_sum_ln(x if x.dtype == torch.float32 else x.to(torch.float32), norms=[(self.weight, self.bias, out)], eps=self.eps, rows=rows,
-                        n_rows=n)
+                        n_rows=n, pdl=self.rt.pdl)
         return out
 
     def add_forward(self, x: torch.Tensor, delta: torch.Tensor, rows: Optional[torch.Tensor] = None,
