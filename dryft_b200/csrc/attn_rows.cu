@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
     T* __restrict__ out,                                       // [N, nH*D]
     float* __restrict__ part_o, float* __restrict__ part_ml,   // [N, nH, S, D], [N, nH, S, 2]
     int nKV, int n_splits, float scale, int window) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   using L = Smem<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* kt = reinterpret_cast<T*>(smem_raw);                 // [PAGE][KSTRIDE]
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
 template <typename T>
 __global__ void attn_rows_reduce_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                         T* __restrict__ out, int n_splits) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   const size_t rh = blockIdx.x;  // row * nH + head
   const float* ml = part_ml + rh * n_splits * 2;
   float mx = -INFINITY;

@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(DEC_THREADS) delta_decode_kernel(
     int gate_ld, const float* __restrict__ conv_w, int taps, T* __restrict__ ring, const float* __restrict__ a_log,
     const float* __restrict__ dt_bias, const float* __restrict__ norm_w, float eps, int sigmoid_gate, const int* __restrict__ tok_slot,
     const int* __restrict__ tok_pos, int H, int G, int d, int dv, int dp, float* __restrict__ state, T* __restrict__ out) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float sm[];
   __shared__ float scratch[33];
   const int h = blockIdx.x, t = blockIdx.y;

@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(THREADS) diff_attn_rows_kernel(
     const T* __restrict__ proj, int proj_stride, const float* __restrict__ q_w, const float* __restrict__ k_w, float qk_eps,
     int fuse, T* __restrict__ k_pages_w, T* __restrict__ v_pages_w,
     int nKV, int n_splits, float scale, int window, int chunk, float lambda, float sub_eps, float out_scale) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   using L = Smem<T>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* kt = reinterpret_cast<T*>(smem_raw);                 // [PAGE][KSTRIDE]

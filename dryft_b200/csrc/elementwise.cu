@@ -172,7 +172,7 @@ template <typename T> __device__ __forceinline__ void store_vec(T* p, const floa
 template <typename T>
 __global__ void rmsnorm_kernel(const T* x, const T* __restrict__ delta, const float* __restrict__ w,
                                const int* __restrict__ rows, T* x_out, T* __restrict__ h, int hidden, float eps, int aligned) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   // x and x_out may be the same buffer (in-place residual update): no __restrict__ on them
   extern __shared__ __align__(16) float row[];  // hidden floats + 33 scratch
   float* scratch = row + ((hidden + 3) & ~3);
@@ -326,7 +326,7 @@ DRYFT_API int dryft_residual_add(int is_bf16, void* x, const void* d, long long 
 // ------------------------------------------------------------------------------------------
 template <typename T>
 __global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ y, int inter, size_t total) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   size_t r = i / inter;
@@ -344,7 +344,7 @@ template <> __device__ __forceinline__ float silu_f32<__nv_bfloat16>(float g) { 
 // 16 bytes of gate and of up per thread (inter a multiple of the vector width)
 template <typename T>
 __global__ void silu_mul_vec_kernel(const T* __restrict__ gu, T* __restrict__ y, int inter, size_t total_vecs) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   constexpr int V = Vec16<T>::N;
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total_vecs) return;

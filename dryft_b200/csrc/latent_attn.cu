@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(PREP_THREADS) latent_prep_kernel(
     const float* __restrict__ inv_freq_lo, int interleaved, const int* __restrict__ tok_slot,
     const int* __restrict__ tok_pos, T* __restrict__ cq, T* __restrict__ k_pages,
     const int* __restrict__ page_table, int max_pages, int page_size, T* __restrict__ c_out) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float buf[];   // [rot]
   __shared__ float scratch[33];
   const int n = blockIdx.x;
@@ -353,7 +353,7 @@ __global__ void latent_combine_kernel(const float* __restrict__ part, const int*
 template <typename T>
 __global__ void head_gate_kernel(const float* __restrict__ o, const T* __restrict__ gate, int gate_ld, T* __restrict__ out,
                                  int n_tokens, int H, int vdim, int per_value) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)n_tokens * H * vdim) return;
   const int v = (int)(i % vdim);
@@ -515,7 +515,7 @@ template <typename T, int VN>
 __global__ void __launch_bounds__(FOLD_THREADS) latent_unfold_o_kernel(const T* __restrict__ o_lat, const T* __restrict__ w,
                                                                        const T* __restrict__ gate, int gate_ld, T* __restrict__ out,
                                                                        int n_tokens, int H, int kv_rank, int vdim, int per_value) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float sm_fold[];
   const int n = blockIdx.x, h = blockIdx.y;
   const T* from = o_lat + ((size_t)h * n_tokens + n) * kv_rank;

@@ -251,7 +251,7 @@ constexpr int COMBINE_THREADS = 128;
 template <typename T, int V>
 __global__ void __launch_bounds__(COMBINE_THREADS) moe_combine_kernel(const T* __restrict__ y, const float* __restrict__ wts, int top, int width,
                                                                       T* __restrict__ out) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   const int n = blockIdx.x, c = (blockIdx.y * COMBINE_THREADS + threadIdx.x) * V;
   if (c >= width) return;
   const T* from = y + (size_t)n * top * width + c;

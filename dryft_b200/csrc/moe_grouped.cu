@@ -308,7 +308,7 @@ int gemm_launch(const void* a_in, const void* w, const int* perm, const int* til
 // 128 bytes is bound by the engine's request rate).  A warp a row; it leaves perm[place[a]] = a beside it.
 __global__ void __launch_bounds__(256) moe_gather_kernel(const uint4* __restrict__ h, const int* __restrict__ place, int n_assign, int top,
                                                          int per_row, uint4* __restrict__ xs, int* __restrict__ perm) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  let_next_launch_in();
   const int a = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (a >= n_assign) return;
   const int p = place[a];

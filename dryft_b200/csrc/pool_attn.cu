@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) pool_attn_rows_kernel(
     int pool_max_pages, const float* __restrict__ sink, const int* __restrict__ tok_slot, const int* __restrict__ tok_pos,
     T* __restrict__ out, float* __restrict__ part_o, float* __restrict__ part_ml, int G, int n_splits, float scale, int size, int P, int keep, const T* __restrict__ gate,
     int gate_ld, ScoreMods mods) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   __shared__ float qs[REP][D];
   __shared__ float wo[ROWS_WARPS][REP][DV];
   __shared__ float wml[ROWS_WARPS][REP][2];
@@ -622,7 +622,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) pool_attn_combine_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                                 const float* __restrict__ sink, const int* __restrict__ tok_slot,
                                                                 T* __restrict__ out, int H, int n_splits, const T* __restrict__ gate, int gate_ld) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   const int t = blockIdx.x, head = blockIdx.y;
   if (tok_slot[t] < 0) return;
   const size_t base = ((size_t)t * H + head) * n_splits;

@@ -50,7 +50,7 @@ __global__ void __launch_bounds__(RT_THREADS) retention_scan_kernel(
     const int* __restrict__ seq_slot, const int* __restrict__ tok_pos, const float* __restrict__ inv_freq,
     const float* __restrict__ inv_freq_lo, int rot, const double* __restrict__ decay, float* __restrict__ state,
     T* __restrict__ out, int H, int dim, int vdim, float k_scale, float eps) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float smem[];
   const int b = blockIdx.x, hd = blockIdx.y;
   const int slot = seq_slot[b];
@@ -636,7 +636,7 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32) rglru_scan_kernel(
     const float* __restrict__ x_bias, const int* __restrict__ cu_q, const int* __restrict__ seq_slot,
     const float* __restrict__ a_in, const float* __restrict__ b_in, float* __restrict__ state, float* __restrict__ tail,
     int taps, T* __restrict__ out, int C) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   __shared__ float As[SCAN_WARPS][32], Bs[SCAN_WARPS][32], carry[32];
   const int b = blockIdx.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(ROW_THREADS) gated_postnorm_kernel(
     const T* __restrict__ y, const float* __restrict__ wts, int top, const T* __restrict__ ys, const T* __restrict__ sgl,
     int sgl_ld, const T* __restrict__ gl, int gl_ld, const float* __restrict__ gb, const float* __restrict__ w, float alpha,
     float eps, float* __restrict__ x32, T* __restrict__ h, int W) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ float row[];     // [W] the row before the norm
   __shared__ float scratch[33];
   const int n = blockIdx.x;
@@ -60,7 +60,7 @@ __global__ void __launch_bounds__(ROW_THREADS) gated_postnorm_kernel(
 template <typename T>
 __global__ void __launch_bounds__(ROW_THREADS) polynorm_kernel(const T* __restrict__ z, int ldz, const float* __restrict__ coef,
                                                                float eps, T* __restrict__ out, int F) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   __shared__ float scratch[33];
   const int n = blockIdx.x;
   const T* zr = z + (size_t)n * ldz;
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(ROW_THREADS) polynorm_kernel(const T* __restri
 
 template <typename T>
 __global__ void relu2_kernel(const T* __restrict__ z, int ldz, T* __restrict__ out, int n, int F) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   const long long total = (long long)n * F;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
     const int r = (int)(i / F), c = (int)(i % F);
@@ -96,7 +96,7 @@ __global__ void relu2_kernel(const T* __restrict__ z, int ldz, T* __restrict__ o
 // rows of whole 16-byte vectors: a thread a vector of one row
 template <typename T>
 __global__ void relu2_vec_kernel(const T* __restrict__ z, int ldz, T* __restrict__ out, int F) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   constexpr int V = 16 / (int)sizeof(T);
   const size_t r = blockIdx.x;
   const int c = ((int)blockIdx.y * blockDim.x + (int)threadIdx.x) * V;
@@ -126,7 +126,7 @@ template <typename T>
 __global__ void __launch_bounds__(ROW_THREADS) gated_group_norm_kernel(const float* __restrict__ y, const float* __restrict__ z,
                                                                        int ldz, const float* __restrict__ w, int part, float eps,
                                                                        T* __restrict__ out, int inner) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   __shared__ float scratch[33];
   const int n = blockIdx.x, c0 = blockIdx.y * part;
   float ss = 0.f;

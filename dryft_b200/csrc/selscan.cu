@@ -63,7 +63,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) selscan_kernel(
     const float* __restrict__ dt_bias, const float* __restrict__ a_log, const float* __restrict__ Dp, const float* __restrict__ zrows,
     int z_ld, int z_off, const int* __restrict__ cu_q, const int* __restrict__ seq_slot, int n_seqs, int cht, int inner, int N,
     int lpc, float* __restrict__ state, float* __restrict__ cstate, float* __restrict__ cdt, T* __restrict__ out) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float sm[];
   const int NP = NR * lpc;
   float* bc = sm;                               // [TILE][2][NP]: B and C of the tile's tokens, read by every channel

@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32) ssm_scan_kernel(
     const float* __restrict__ a_log, const float* __restrict__ Dp, const int* __restrict__ cu_q, const int* __restrict__ seq_slot,
     int n_seqs, int cht, int heads, int groups, int N, int dv, float* __restrict__ state, float* __restrict__ cstate,
     float* __restrict__ cdec, float* __restrict__ y) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   const int hd = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int p0 = (blockIdx.z * SCAN_WARPS + warp) * COLS;

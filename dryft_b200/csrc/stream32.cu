@@ -22,7 +22,7 @@ __global__ void __launch_bounds__(THREADS) embed_sinusoid_kernel(
     const int* __restrict__ tokens, const int* __restrict__ tok_pos, const TT* __restrict__ table,
     const float* __restrict__ freq, float scale, float* __restrict__ x32, T* __restrict__ h, int width, int vocab,
     int* __restrict__ err) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   const int n = blockIdx.x;
   const int tok = tokens[n];
   const bool bad = tok < 0 || tok >= vocab;
@@ -62,7 +62,7 @@ template <typename T>
 __global__ void __launch_bounds__(THREADS) stream_norm_add_kernel(
     const T* __restrict__ y, const float* __restrict__ wts, int top, const float* __restrict__ w, float offset, float eps,
     float* __restrict__ x32, T* __restrict__ h, int width) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float row[];
   __shared__ float scratch[33];
   const int n = blockIdx.x;
@@ -120,7 +120,7 @@ template <typename TI, typename T>
 __global__ void __launch_bounds__(THREADS) stream_norm_rows_kernel(
     const TI* __restrict__ x, const int* __restrict__ rows, const float* __restrict__ w, float offset, float eps,
     T* __restrict__ out, int width) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float row[];
   __shared__ float scratch[33];
   const int r = blockIdx.x;

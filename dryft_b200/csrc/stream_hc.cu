@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(THREADS) embed_pair_norm_kernel(
     const int* __restrict__ prev_state, const TT* __restrict__ table, const TT* __restrict__ pair_table, int buckets,
     long long mul_prev, long long mul_cur, float scale, const float* __restrict__ norm_w, float eps,
     float* __restrict__ x32, int width, int vocab, int* __restrict__ err) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float row[];
   __shared__ float scratch[33];
   const int n = blockIdx.x;
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(WIDE_THREADS) hc_step_kernel(
     const float* __restrict__ x_in, int s_in, float* __restrict__ x_out, int S, const T* __restrict__ y,
     const float* __restrict__ mix, const float* __restrict__ outw, float mult, const float* __restrict__ inw,
     const float* __restrict__ norm_w, float eps, const int* __restrict__ rows, T* __restrict__ h, int width) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float row[];
   __shared__ float scratch[33];
   __shared__ float c_mix[MS * MS], c_out[MS], c_in[MS];
@@ -255,7 +255,7 @@ __device__ __forceinline__ float glu_one(float g, float u, float limit, int has_
 template <typename T, int VEC>
 __global__ void glu_clamp_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int rows, int inter, float limit,
                                  int has_limit, float alpha, float up_offset) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   wait_for_earlier_launches();
   const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   if (i >= (size_t)rows * inter) return;

@@ -51,7 +51,7 @@ __global__ void __launch_bounds__(THREADS) stream_sum_kernel(
     float* __restrict__ x32, const float* __restrict__ src, const T* __restrict__ y0, float s0, const T* __restrict__ y1, float s1,
     const T* __restrict__ y2, float s2, const T* __restrict__ yr, int top, float sr, const float* __restrict__ vec,
     const float* __restrict__ norm_w, float eps, T* __restrict__ h, int width) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   __shared__ float scratch[33];
   const size_t n = blockIdx.x;
   float* x = x32 + n * width;
@@ -108,7 +108,7 @@ __global__ void __launch_bounds__(WIDE_THREADS) stream_sum_ln_kernel(
     float* __restrict__ x32, const int* __restrict__ rows, const T* __restrict__ y0, float s0, const T* __restrict__ y1, float s1,
     const T* __restrict__ y2, float s2, const float* __restrict__ w0, const float* __restrict__ b0, T* __restrict__ h0,
     const float* __restrict__ w1, const float* __restrict__ b1, T* __restrict__ h1, float eps, int width) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float row[];
   __shared__ float scratch[33];
   const size_t n = blockIdx.x;
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(THREADS) stream_norm_join_kernel(
     float* __restrict__ x32, const T* __restrict__ y0, float s0, const T* __restrict__ y1, float s1, const T* __restrict__ y2, float s2,
     const T* __restrict__ yr, const float* __restrict__ wts, int top, const float* __restrict__ factor, float eps,
     const float* __restrict__ norm_w, float norm_eps, T* __restrict__ h, int width) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float row[];
   __shared__ float scratch[33];
   const size_t n = blockIdx.x;
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(THREADS) stream_norm_join_regs_kernel(
     float* __restrict__ x32, const T* __restrict__ y0, float s0, const T* __restrict__ y1, float s1, const T* __restrict__ y2, float s2,
     const T* __restrict__ yr, const float* __restrict__ wts, int top, const float* __restrict__ factor, float eps,
     const float* __restrict__ norm_w, float norm_eps, T* __restrict__ h, int width) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   __shared__ float scratch[33];
   const size_t n = blockIdx.x;
   float* x = x32 + n * width;

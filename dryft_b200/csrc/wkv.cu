@@ -87,7 +87,7 @@ constexpr int MIX_THREADS = 256;
 template <typename T, int V>
 __global__ void __launch_bounds__(MIX_THREADS) wkv_mix_kernel(const T* __restrict__ h, const T* __restrict__ last, const float* __restrict__ mu,
                                                             const int* __restrict__ tok_slot, T* __restrict__ out, int n, int width) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   const int t = blockIdx.x;
   const int c = ((int)blockIdx.y * MIX_THREADS + (int)threadIdx.x) * V;
   if (c >= width) return;
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(MIX_THREADS) wkv_mix_kernel(const T* __restric
 }
 
 template <typename T> __global__ void wkv_tanh_kernel(const float* __restrict__ low, T* __restrict__ out, size_t count) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < count) out[i] = from_f32<T>(tanhf(low[i]));
 }
@@ -469,7 +469,7 @@ __global__ void __launch_bounds__(NORM_WARPS * 32) wkv_norm_kernel(const float* 
                                                                 const float* __restrict__ norm_w, float eps, const T* __restrict__ h, int width,
                                                                 T* __restrict__ last, const int* __restrict__ tok_slot, int n, int H, int dv,
                                                                 T* __restrict__ out) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   const int t = blockIdx.x, slot = tok_slot[t];
   if (slot < 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(DEC_THREADS) wkv_decode_kernel(
     const float* __restrict__ low, int low_ld, int R, const T* __restrict__ w2, const float* __restrict__ w0, const float* __restrict__ u,
     const float* __restrict__ norm_w, float eps, const T* __restrict__ h, int width, T* __restrict__ last, const int* __restrict__ tok_slot, int H,
     int d, int dv, float* __restrict__ state, T* __restrict__ out) {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // a product behind this launch may start on its weights
+  let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float sm[];      // r, k, w [d each], v [dv], tanh(low) [R], partial read-outs [row groups][dv]
   __shared__ float scratch[33];
   const int t = blockIdx.x, hd = blockIdx.y, tid = threadIdx.x;
