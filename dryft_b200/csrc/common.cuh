@@ -40,11 +40,11 @@ __device__ __forceinline__ float ld_prev_bf16(const __nv_bfloat16* p) {
 }
 
 // Lets the launch behind this one, where it was launched as a programmatic dependent, come in and start on what this one has no part
-// in.  Only launches of about one wave of blocks say so: every block pays for it (the squares of relu, 2,048 rows of 9,728 columns, 10,240
-// blocks: 22.6 us with it and 12.6 without; 300 blocks: no difference), and larger launches have no such dependent.
-__device__ __forceinline__ void let_next_launch_in() {
-  if (gridDim.x * gridDim.y * gridDim.z <= 592u) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
+// in.  Every block pays for saying so: nothing that shows where a block has work to do, but launches of many short blocks, which have
+// no such dependent, must not (the squares of relu, 2,048 rows of 9,728 columns in 10,240 blocks: 22.6 us with it and 12.6 without); their
+// kernels say so up to about a wave of blocks, or the rows that such a dependent takes.
+__device__ __forceinline__ void let_next_launch_in() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+constexpr unsigned SIGNAL_BLOCKS = 592, SIGNAL_ROWS = 64;
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll

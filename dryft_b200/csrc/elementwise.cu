@@ -324,9 +324,9 @@ DRYFT_API int dryft_residual_add(int is_bf16, void* x, const void* d, long long 
 // SiLU*mul over the fused gate|up product [rows, 2*inter] (gate columns first):
 //   y = T( T(g / (1 + exp(-g))) * u )            (silu_mul.py:29-32; model.py:44-46)
 // ------------------------------------------------------------------------------------------
-template <typename T>
+template <typename T, bool SIGNAL>
 __global__ void silu_mul_kernel(const T* __restrict__ gu, T* __restrict__ y, int inter, size_t total) {
-  let_next_launch_in();   // a product behind this launch may start on its weights
+  if (SIGNAL) let_next_launch_in();   // a product behind this launch may start on its weights
   size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= total) return;
   size_t r = i / inter;
@@ -367,7 +367,8 @@ static int silu_launch(const void* gu, void* y, int rows, int inter, cudaStream_
     silu_mul_vec_kernel<T><<<(unsigned)((total + 255) / 256), 256, 0, st>>>((const T*)gu, (T*)y, inter, total);
   } else {
     size_t total = (size_t)rows * inter;
-    silu_mul_kernel<T><<<(unsigned)((total + 255) / 256), 256, 0, st>>>((const T*)gu, (T*)y, inter, total);
+    const unsigned blocks = (unsigned)((total + 255) / 256);
+    (blocks <= SIGNAL_BLOCKS ? silu_mul_kernel<T, true> : silu_mul_kernel<T, false>)<<<blocks, 256, 0, st>>>((const T*)gu, (T*)y, inter, total);
   }
   return launch_status();
 }

@@ -350,10 +350,10 @@ __global__ void latent_combine_kernel(const float* __restrict__ part, const int*
   }
 }
 
-template <typename T>
+template <typename T, bool SIGNAL>
 __global__ void head_gate_kernel(const float* __restrict__ o, const T* __restrict__ gate, int gate_ld, T* __restrict__ out,
                                  int n_tokens, int H, int vdim, int per_value) {
-  let_next_launch_in();   // a product behind this launch may start on its weights
+  if (SIGNAL) let_next_launch_in();   // a product behind this launch may start on its weights
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (size_t)n_tokens * H * vdim) return;
   const int v = (int)(i % vdim);
@@ -694,7 +694,8 @@ DRYFT_API int dryft_head_gate(int is_bf16, const float* o, const void* gate, int
   typedef __nv_bfloat16 bf;
   const size_t total = (size_t)n_tokens * H * vdim;
   const unsigned blocks = (unsigned)((total + 255) / 256);
-  if (is_bf16) head_gate_kernel<bf><<<blocks, 256, 0, st>>>(o, (const bf*)gate, gate_ld, (bf*)out, n_tokens, H, vdim, per_value);
-  else head_gate_kernel<float><<<blocks, 256, 0, st>>>(o, (const float*)gate, gate_ld, (float*)out, n_tokens, H, vdim, per_value);
+  const bool signal = blocks <= SIGNAL_BLOCKS;
+  if (is_bf16) (signal ? head_gate_kernel<bf, true> : head_gate_kernel<bf, false>)<<<blocks, 256, 0, st>>>(o, (const bf*)gate, gate_ld, (bf*)out, n_tokens, H, vdim, per_value);
+  else (signal ? head_gate_kernel<float, true> : head_gate_kernel<float, false>)<<<blocks, 256, 0, st>>>(o, (const float*)gate, gate_ld, (float*)out, n_tokens, H, vdim, per_value);
   return launch_status();
 }

@@ -248,10 +248,10 @@ __global__ void __launch_bounds__(ROWS_THREADS) moe_rows_kernel(
 // rows' words are requested together, eight at a time, and added in the order of k.  2,048 tokens x 8 rows of 2,048: 12 us
 // for 75 MB, 31 with one column a thread; 8 tokens: 2 us against 13.
 constexpr int COMBINE_THREADS = 128;
-template <typename T, int V>
+template <typename T, int V, bool SIGNAL>
 __global__ void __launch_bounds__(COMBINE_THREADS) moe_combine_kernel(const T* __restrict__ y, const float* __restrict__ wts, int top, int width,
                                                                       T* __restrict__ out) {
-  let_next_launch_in();   // a product behind this launch may start on its weights
+  if (SIGNAL) let_next_launch_in();   // a product behind this launch may start on its weights
   const int n = blockIdx.x, c = (blockIdx.y * COMBINE_THREADS + threadIdx.x) * V;
   if (c >= width) return;
   const T* from = y + (size_t)n * top * width + c;
@@ -289,8 +289,9 @@ int combine_launch(const void* y, const float* wts, int top, int width, void* ou
   const bool vec = width % V == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   const int per = COMBINE_THREADS * (vec ? V : 1), cols = (width + per - 1) / per;
   if (cols > 65535) return DRYFT_ERR_UNSUPPORTED;
-  if (vec) moe_combine_kernel<T, V><<<dim3(n, cols), COMBINE_THREADS, 0, st>>>((const T*)y, wts, top, width, (T*)out);
-  else moe_combine_kernel<T, 1><<<dim3(n, cols), COMBINE_THREADS, 0, st>>>((const T*)y, wts, top, width, (T*)out);
+  auto kern = n <= SIGNAL_ROWS ? (vec ? moe_combine_kernel<T, V, true> : moe_combine_kernel<T, 1, true>)
+                               : (vec ? moe_combine_kernel<T, V, false> : moe_combine_kernel<T, 1, false>);
+  kern<<<dim3(n, cols), COMBINE_THREADS, 0, st>>>((const T*)y, wts, top, width, (T*)out);
   return launch_status();
 }
 

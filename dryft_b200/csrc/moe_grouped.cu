@@ -306,9 +306,10 @@ int gemm_launch(const void* a_in, const void* w, const int* perm, const int* til
 // ---------------------------------------------------------------------------- tcgen05
 // xs[place[a]] = h[a / top]: the sorted rows as one matrix that the copy engine takes in boxes (a copy of its own for each row's
 // 128 bytes is bound by the engine's request rate).  A warp a row; it leaves perm[place[a]] = a beside it.
+template <bool SIGNAL>
 __global__ void __launch_bounds__(256) moe_gather_kernel(const uint4* __restrict__ h, const int* __restrict__ place, int n_assign, int top,
                                                          int per_row, uint4* __restrict__ xs, int* __restrict__ perm) {
-  let_next_launch_in();
+  if (SIGNAL) let_next_launch_in();
   const int a = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (a >= n_assign) return;
   const int p = place[a];
@@ -703,7 +704,9 @@ DRYFT_API int dryft_moe_grouped(const void* h, const void* w_gate_up, const void
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const Sorted t = {perm, tile_expert, tile_row0, tile_rows, n_tiles, n_tiles + 1, max_tiles};
-    moe_gather_kernel<<<(n_assign + 7) / 8, 256, 0, st>>>((const uint4*)h, place, n_assign, top, W / 8, (uint4*)y, perm);
+    const int gather_blocks = (n_assign + 7) / 8;
+    (gather_blocks <= SIGNAL_BLOCKS ? moe_gather_kernel<true> : moe_gather_kernel<false>)<<<gather_blocks, 256, 0, st>>>(
+        (const uint4*)h, place, n_assign, top, W / 8, (uint4*)y, perm);
     rc = launch_status();
     if (rc) return rc;
     auto both = [&](auto nmax) {

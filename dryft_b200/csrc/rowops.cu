@@ -94,9 +94,9 @@ __global__ void relu2_kernel(const T* __restrict__ z, int ldz, T* __restrict__ o
 }
 
 // rows of whole 16-byte vectors: a thread a vector of one row
-template <typename T>
+template <typename T, bool SIGNAL>
 __global__ void relu2_vec_kernel(const T* __restrict__ z, int ldz, T* __restrict__ out, int F) {
-  let_next_launch_in();   // a product behind this launch may start on its weights
+  if (SIGNAL) let_next_launch_in();   // a product behind this launch may start on its weights
   constexpr int V = 16 / (int)sizeof(T);
   const size_t r = blockIdx.x;
   const int c = ((int)blockIdx.y * blockDim.x + (int)threadIdx.x) * V;
@@ -113,7 +113,7 @@ template <typename T>
 int relu2_launch(const T* z, int ldz, T* out, int n, int F, cudaStream_t st) {
   constexpr int V = 16 / (int)sizeof(T);
   if (F % V == 0 && ldz % V == 0 && (((uintptr_t)z | (uintptr_t)out) & 15) == 0 && F / V <= 65535 * 128) {
-    relu2_vec_kernel<T><<<dim3(n, (F / V + 127) / 128), 128, 0, st>>>(z, ldz, out, F);
+    (n <= SIGNAL_ROWS ? relu2_vec_kernel<T, true> : relu2_vec_kernel<T, false>)<<<dim3(n, (F / V + 127) / 128), 128, 0, st>>>(z, ldz, out, F);
     return launch_status();
   }
   const long long total = (long long)n * F;

@@ -255,7 +255,7 @@ __device__ __forceinline__ float glu_one(float g, float u, float limit, int has_
 template <typename T, int VEC>
 __global__ void glu_clamp_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int rows, int inter, float limit,
                                  int has_limit, float alpha, float up_offset) {
-  let_next_launch_in();   // a product behind this launch may start on its weights
+  if (VEC > 1) let_next_launch_in();   // a product behind this launch may start on its weights
   wait_for_earlier_launches();
   const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   if (i >= (size_t)rows * inter) return;
