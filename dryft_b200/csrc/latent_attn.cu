@@ -445,23 +445,26 @@ __global__ void head_gate_rows_kernel(const T* __restrict__ o, int hd, const T* 
 // path (sums in a fixed order, so a row's result does not depend on its company):
 //   latent_fold_q     q_lat[h, n, r] = sum_d q[n, h, d] * w_k[h, d, r]                      (32-bit result)
 //   latent_unfold_o   out[n, h*V + v] = T( sigmoid(gate[n, h]) * sum_r o_lat[h, n, r] * w_v[h, r, v] )
-// One block per (token, head, FOLD_COLS columns).  A thread takes VN neighbouring columns (16 bytes) of every FOLD_THREADS /
-// (FOLD_COLS / VN)-th matrix row (of up to 64 rows: of every row), requested before the vector is read; the threads' sums are added in order.  One token and head of 512 x 128:
-// 3 us, where a thread per column along all rows took 18 (64 trips to memory).
-constexpr int FOLD_COLS = 128, FOLD_THREADS = 512;
+// One order of additions in both kernels below: up to FOLD_ONE_CHAIN matrix rows are one chain; more are cut into pieces of FOLD_PIECE rows, a
+// piece is accumulated in order from zero, and the pieces' sums are added in order.
+constexpr int FOLD_COLS = 128, FOLD_THREADS = 512, FOLD_ONE_CHAIN = 64, FOLD_PIECE = 16, FOLD_FEW_ROWS = 1024;
 
-// out(c, sum_i vin(i) * w[i, c]) for the columns c0 .. c0 + FOLD_COLS - 1 of a [rows, cols] matrix; G threads share a column
-template <typename T, int VN, int G, typename In, typename Out>
-__device__ __forceinline__ void fold_columns_by(const T* __restrict__ w, int rows, int cols, int c0, float* vin, float* red, In in, Out out) {
-  constexpr int LR = FOLD_COLS / VN, AHEAD = 16;
+// out(c, sum_i vin(i) * w[i, c]) for the columns c0 .. c0 + FOLD_COLS - 1 of a [rows, cols] matrix.  One block per (token, head,
+// FOLD_COLS columns): a thread takes VN neighbouring columns (16 bytes) of a piece at a time, its rows' words requested together and the
+// first before the vector is read.  For few blocks, where a thread per column along all rows waits for one trip to memory after the
+// other: one token and 16 heads, 128 x 512 and 512 x 128, 32-bit: 3 and 4 us against 8 and 28.
+template <typename T, int VN, typename In, typename Out>
+__device__ __forceinline__ void fold_columns(const T* __restrict__ w, int rows, int cols, int c0, float* vin, float* red, In in, Out out) {
+  constexpr int LR = FOLD_COLS / VN, G = FOLD_THREADS / LR;
+  const int pieces = (rows + FOLD_PIECE - 1) / FOLD_PIECE;
   const int c = c0 + (threadIdx.x % LR) * VN, g = threadIdx.x / LR;
-  const bool on = g < G && c < cols;
-  alignas(16) T wv[AHEAD][VN];
-  auto request = [&](int i0) {
+  const bool on = c < cols;
+  alignas(16) T wv[FOLD_PIECE][VN];
+  auto request = [&](int piece) {
 #pragma unroll
-    for (int u = 0; u < AHEAD; ++u) {
-      const int i = i0 + u * G;
-      if (i < rows && on) {
+    for (int u = 0; u < FOLD_PIECE; ++u) {
+      const int i = piece * FOLD_PIECE + u;
+      if (on && i < rows) {
         if (VN > 1) *reinterpret_cast<uint4*>(wv[u]) = *reinterpret_cast<const uint4*>(w + (size_t)i * cols + c);
         else wv[u][0] = w[(size_t)i * cols + c];
       }
@@ -470,59 +473,97 @@ __device__ __forceinline__ void fold_columns_by(const T* __restrict__ w, int row
   request(g);
   for (int i = threadIdx.x; i < rows; i += FOLD_THREADS) vin[i] = in(i);
   __syncthreads();
-  float acc[VN];
+  for (int piece = g; piece < pieces; piece += G) {
+    if (piece != g) request(piece);
+    float acc[VN];
 #pragma unroll
-  for (int j = 0; j < VN; ++j) acc[j] = 0.f;
-  for (int i0 = g; i0 < rows; i0 += AHEAD * G) {
-    if (i0 != g) request(i0);
+    for (int j = 0; j < VN; ++j) acc[j] = 0.f;
 #pragma unroll
-    for (int u = 0; u < AHEAD; ++u) {
-      if (i0 + u * G >= rows || !on) continue;
-      const float x = vin[i0 + u * G];
+    for (int u = 0; u < FOLD_PIECE; ++u) {
+      const int i = piece * FOLD_PIECE + u;
+      if (!on || i >= rows) continue;
+      const float x = vin[i];
 #pragma unroll
       for (int j = 0; j < VN; ++j) acc[j] = fmaf(x, to_f32<T>(wv[u][j]), acc[j]);
     }
-  }
 #pragma unroll
-  for (int j = 0; j < VN; ++j) red[g * FOLD_COLS + (threadIdx.x % LR) * VN + j] = acc[j];
+    for (int j = 0; j < VN; ++j) red[piece * FOLD_COLS + (threadIdx.x % LR) * VN + j] = acc[j];
+  }
   __syncthreads();
   for (int j = threadIdx.x; j < FOLD_COLS && c0 + j < cols; j += FOLD_THREADS) {
     float sum = red[j];
-#pragma unroll
-    for (int k = 1; k < G; ++k) sum += red[k * FOLD_COLS + j];
+#pragma unroll 8
+    for (int k = 1; k < pieces; ++k) sum += red[k * FOLD_COLS + j];
     out(c0 + j, sum);
   }
 }
-template <typename T, int VN, typename In, typename Out>
-__device__ __forceinline__ void fold_columns(const T* __restrict__ w, int rows, int cols, int c0, float* vin, float* red, In in, Out out) {
-  if (rows <= 64) fold_columns_by<T, VN, 1>(w, rows, cols, c0, vin, red, in, out);      // few rows: one thread a column, in order
-  else fold_columns_by<T, VN, FOLD_THREADS / (FOLD_COLS / VN)>(w, rows, cols, c0, vin, red, in, out);
-}
-template <int VN> constexpr size_t fold_smem(int rows) { return sizeof(float) * ((size_t)rows + FOLD_THREADS * VN); }
+constexpr size_t fold_smem(int rows) { return sizeof(float) * ((size_t)rows + (size_t)(rows + FOLD_PIECE - 1) / FOLD_PIECE * FOLD_COLS); }
 
-template <typename T, int VN>
-__global__ void __launch_bounds__(FOLD_THREADS) latent_fold_q_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ w,
-                                                                     float* __restrict__ q_lat, int n_tokens, int H, int dim, int kv_rank) {
+// The same for many blocks: one per (token, head), a thread a column along all rows, half a piece's words on their way at a time.  1,024
+// tokens of 16 heads, 128 x 512 and 512 x 128, 32-bit: 192 and 196 us (one chain in a loop that the compiler unrolls by eight: 203 and
+// 201; the kernel for few blocks: 895 and 488).
+template <typename T, typename In, typename Out>
+__device__ __forceinline__ void fold_rows(const T* __restrict__ w, int rows, int cols, float* vin, In in, Out out) {
+  for (int i = threadIdx.x; i < rows; i += blockDim.x) vin[i] = in(i);
+  __syncthreads();
+  for (int c = threadIdx.x; c < cols; c += blockDim.x) {
+    const T* p = w + c;
+    float sum = 0.f;
+    int i = 0;
+    if (rows > FOLD_ONE_CHAIN) {
+      for (; i + FOLD_PIECE <= rows; i += FOLD_PIECE) {
+        float acc = 0.f;
+#pragma unroll
+        for (int half = 0; half < FOLD_PIECE; half += 8) {
+          T v[8];
+#pragma unroll
+          for (int u = 0; u < 8; ++u) { v[u] = *p; p += cols; }
+#pragma unroll
+          for (int u = 0; u < 8; ++u) acc = fmaf(vin[i + half + u], to_f32<T>(v[u]), acc);
+        }
+        sum = i == 0 ? acc : sum + acc;
+      }
+    }
+    if (i < rows) {      // all of few rows, or the rest of many: one chain
+      float acc = 0.f;
+#pragma unroll 8
+      for (int k = i; k < rows; ++k) { acc = fmaf(vin[k], to_f32<T>(*p), acc); p += cols; }
+      sum = i == 0 ? acc : sum + acc;
+    }
+    out(c, sum);
+  }
+}
+
+template <typename T, int VN, bool FEW>
+__global__ void __launch_bounds__(FEW ? FOLD_THREADS : 256) latent_fold_q_kernel(const T* __restrict__ q, int q_stride, const T* __restrict__ w,
+                                                                                 float* __restrict__ q_lat, int n_tokens, int H, int dim,
+                                                                                 int kv_rank) {
   extern __shared__ __align__(16) float sm_fold[];
   const int n = blockIdx.x, h = blockIdx.y;
   const T* qr = q + ((size_t)n * H + h) * q_stride;
+  const T* wh = w + (size_t)h * dim * kv_rank;
   float* to = q_lat + ((size_t)h * n_tokens + n) * kv_rank;
-  fold_columns<T, VN>(w + (size_t)h * dim * kv_rank, dim, kv_rank, blockIdx.z * FOLD_COLS, sm_fold, sm_fold + dim,
-                      [&](int d) { return to_f32<T>(qr[d]); }, [&](int r, float v) { to[r] = v; });
+  auto in = [&](int d) { return to_f32<T>(qr[d]); };
+  auto out = [&](int r, float v) { to[r] = v; };
+  if constexpr (FEW) fold_columns<T, VN>(wh, dim, kv_rank, blockIdx.z * FOLD_COLS, sm_fold, sm_fold + dim, in, out);
+  else fold_rows<T>(wh, dim, kv_rank, sm_fold, in, out);
 }
 
-template <typename T, int VN>
-__global__ void __launch_bounds__(FOLD_THREADS) latent_unfold_o_kernel(const T* __restrict__ o_lat, const T* __restrict__ w,
-                                                                       const T* __restrict__ gate, int gate_ld, T* __restrict__ out,
-                                                                       int n_tokens, int H, int kv_rank, int vdim, int per_value) {
+template <typename T, int VN, bool FEW>
+__global__ void __launch_bounds__(FEW ? FOLD_THREADS : 256) latent_unfold_o_kernel(const T* __restrict__ o_lat, const T* __restrict__ w,
+                                                                                   const T* __restrict__ gate, int gate_ld,
+                                                                                   T* __restrict__ out_rows, int n_tokens, int H, int kv_rank,
+                                                                                   int vdim, int per_value) {
   let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float sm_fold[];
   const int n = blockIdx.x, h = blockIdx.y;
   const T* from = o_lat + ((size_t)h * n_tokens + n) * kv_rank;
+  const T* wh = w + (size_t)h * kv_rank * vdim;
   auto gate_of = [&](int v) { return gate ? 1.f / (1.f + expf(-to_f32<T>(gate[(size_t)n * gate_ld + (per_value ? h * vdim + v : h)]))) : 1.f; };
-  fold_columns<T, VN>(w + (size_t)h * kv_rank * vdim, kv_rank, vdim, blockIdx.z * FOLD_COLS, sm_fold, sm_fold + kv_rank,
-                      [&](int r) { return to_f32<T>(from[r]); },
-                      [&](int v, float x) { out[((size_t)n * H + h) * vdim + v] = from_f32<T>(x * gate_of(v)); });
+  auto in = [&](int r) { return to_f32<T>(from[r]); };
+  auto out = [&](int v, float x) { out_rows[((size_t)n * H + h) * vdim + v] = from_f32<T>(x * gate_of(v)); };
+  if constexpr (FEW) fold_columns<T, VN>(wh, kv_rank, vdim, blockIdx.z * FOLD_COLS, sm_fold, sm_fold + kv_rank, in, out);
+  else fold_rows<T>(wh, kv_rank, vdim, sm_fold, in, out);
 }
 
 template <typename K> int opt_in(K kernel, size_t bytes) {
@@ -601,23 +642,46 @@ DRYFT_API int dryft_latent_attn_rows(int is_bf16, const float* q_lat, const void
 }
 
 namespace {
+// The kernel for few blocks: up to two a multiprocessor, where its pieces' sums fit a block (16 heads, 32-bit: 128 x 512, 4 tokens 4.5 us
+// against 8.5, 8 tokens 8.3 against 8.7; 512 x 128, 16 tokens 8.9 against 14.6, 32 tokens 16.4 against 16; 256 x 64, 16 tokens 5.7
+// against 8.5, 32 tokens 10.1 against 8.9).
+bool fold_few(int n_tokens, int H, int rows, int cols) {
+  if (rows <= FOLD_ONE_CHAIN || rows > FOLD_FEW_ROWS) return false;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return (long long)n_tokens * H * ((cols + FOLD_COLS - 1) / FOLD_COLS) <= 2LL * sms;
+}
 template <typename T, int VN>
 int launch_fold(const void* q, int q_stride, const void* w, float* q_lat, int n_tokens, int H, int dim, int kv_rank, cudaStream_t st) {
-  const size_t smem = fold_smem<VN>(dim);
-  const int rc = opt_in(latent_fold_q_kernel<T, VN>, smem);
+  if (!fold_few(n_tokens, H, dim, kv_rank)) {
+    const int threads = kv_rank >= 256 ? 256 : (kv_rank >= 128 ? 128 : 64);
+    latent_fold_q_kernel<T, VN, false><<<dim3(n_tokens, H), threads, sizeof(float) * (size_t)dim, st>>>((const T*)q, q_stride, (const T*)w, q_lat,
+                                                                                                        n_tokens, H, dim, kv_rank);
+    return launch_status();
+  }
+  const size_t smem = fold_smem(dim);
+  const int rc = opt_in(latent_fold_q_kernel<T, VN, true>, smem);
   if (rc) return rc;
-  latent_fold_q_kernel<T, VN><<<dim3(n_tokens, H, (kv_rank + FOLD_COLS - 1) / FOLD_COLS), FOLD_THREADS, smem, st>>>((const T*)q, q_stride, (const T*)w,
-                                                                                                                  q_lat, n_tokens, H, dim, kv_rank);
+  const dim3 grid(n_tokens, H, (kv_rank + FOLD_COLS - 1) / FOLD_COLS);
+  latent_fold_q_kernel<T, VN, true><<<grid, FOLD_THREADS, smem, st>>>((const T*)q, q_stride, (const T*)w, q_lat, n_tokens, H, dim, kv_rank);
   return launch_status();
 }
 template <typename T, int VN>
 int launch_unfold(const void* o_lat, const void* w, const void* gate, int gate_ld, void* out, int n_tokens, int H, int kv_rank, int vdim,
                   int per_value, cudaStream_t st) {
-  const size_t smem = fold_smem<VN>(kv_rank);
-  const int rc = opt_in(latent_unfold_o_kernel<T, VN>, smem);
+  if (!fold_few(n_tokens, H, kv_rank, vdim)) {
+    const int threads = vdim >= 256 ? 256 : (vdim >= 128 ? 128 : 64);
+    latent_unfold_o_kernel<T, VN, false><<<dim3(n_tokens, H), threads, sizeof(float) * (size_t)kv_rank, st>>>(
+        (const T*)o_lat, (const T*)w, (const T*)gate, gate_ld, (T*)out, n_tokens, H, kv_rank, vdim, per_value);
+    return launch_status();
+  }
+  const size_t smem = fold_smem(kv_rank);
+  const int rc = opt_in(latent_unfold_o_kernel<T, VN, true>, smem);
   if (rc) return rc;
-  latent_unfold_o_kernel<T, VN><<<dim3(n_tokens, H, (vdim + FOLD_COLS - 1) / FOLD_COLS), FOLD_THREADS, smem, st>>>(
-      (const T*)o_lat, (const T*)w, (const T*)gate, gate_ld, (T*)out, n_tokens, H, kv_rank, vdim, per_value);
+  const dim3 grid(n_tokens, H, (vdim + FOLD_COLS - 1) / FOLD_COLS);
+  latent_unfold_o_kernel<T, VN, true><<<grid, FOLD_THREADS, smem, st>>>((const T*)o_lat, (const T*)w, (const T*)gate, gate_ld, (T*)out, n_tokens, H,
+                                                                       kv_rank, vdim, per_value);
   return launch_status();
 }
 // 16-byte reads of the matrix: every row of every head starts on a 16-byte boundary

@@ -62,3 +62,28 @@ def test_recurrence_gates_of_few_and_many_tokens(blocks, nb):
         parts, s1 = run(cuts)
         torch.testing.assert_close(parts, whole, rtol=2e-5, atol=2e-5)      # sums of up to 132 products in two orders, carried over 35 steps
         torch.testing.assert_close(s1, s0, rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("heads,rows,cols", [(2, 64, 256), (4, 65, 132), (3, 128, 512), (2, 513, 77), (16, 512, 128), (1, 300, 40), (5, 1030, 24)])
+def test_folded_matrices_do_not_depend_on_company(dtype, heads, rows, cols):
+    """A token's fold has the same bits alone, where threads share a column, and among so many that a thread takes whole columns."""
+    from dryft_b200.ops import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(rows + cols)
+    randn = lambda *s: torch.randn(*s, generator=gen, device="cuda").to(dtype)
+    n = 700
+    w, q, o_lat, gate = randn(heads, rows, cols), randn(n, heads, rows + 5), randn(heads, n, rows), randn(n, heads)
+
+    def run(who):
+        lat, out = torch.empty(heads, len(who), cols, device="cuda"), torch.empty(len(who), heads * cols, dtype=dtype, device="cuda")
+        K.latent_fold_q(q[who].contiguous(), w, lat, rows)
+        K.latent_unfold_o(o_lat[:, who].contiguous(), w, gate[who].contiguous(), 0, out)
+        return lat, out
+
+    lat, out = run(list(range(n)))
+    exact, scale = (torch.einsum("nhd,hdr->hnr", a[:, :, :rows].double(), b.double()) for a, b in ((q, w), (q.abs(), w.abs())))
+    assert bool(((lat.double() - exact).abs() <= (rows + 1) * 2.0 ** -24 * scale).all())
+    for who in ([0], [699], [5, 600], list(range(40, 49)), list(range(100, 164))):
+        a, b = run(who)
+        assert torch.equal(a, lat[:, who]) and torch.equal(b, out[who]), len(who)
