@@ -64,6 +64,33 @@ def test_recurrence_gates_of_few_and_many_tokens(blocks, nb):
         torch.testing.assert_close(s1, s0, rtol=2e-5, atol=2e-5)
 
 
+@pytest.mark.parametrize("blocks,nb", [(2, 128), (3, 20), (1, 132), (4, 4), (2, 7), (1, 300)])
+def test_recurrence_gates_do_not_depend_on_company(blocks, nb):
+    """A sequence's token gives the same bits alone, in the form for few tokens and among so many that the prompt form takes it."""
+    from dryft_b200.ops import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(nb)
+    c, taps, seqs = blocks * nb, 4, 90
+    randn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    proj, yb, xb, conv, cb = randn(seqs, 2 * c), randn(c) * 0.1, randn(c) * 0.1, randn(c, taps) * 0.5, randn(c) * 0.1
+    wg, ba, bi, lam = randn(blocks, nb, 2, nb) * nb ** -0.5, randn(c), randn(c), torch.rand(c, generator=gen, device="cuda")
+    state0, tail0 = randn(seqs, c), randn(seqs, taps - 1, c)
+
+    def run(who):
+        n = len(who)
+        at = torch.tensor(who, dtype=torch.int32, device="cuda")
+        state, tail, out = state0.clone(), tail0.clone(), torch.empty(n, c, device="cuda")
+        cu = torch.arange(n + 1, dtype=torch.int32, device="cuda")
+        K.rglru(proj[who].contiguous(), 0, c, yb, xb, cu, at, at, conv, cb, wg, ba, bi, lam, 8.0, state, tail, out, n, blocks)
+        return out, state[who]
+
+    everyone = list(range(seqs))
+    out, state = run(everyone)
+    for who in ([0], [7, 3], everyone[10:19], everyone[20:84], everyone[25:90]):
+        o, s = run(who)
+        assert torch.equal(o, out[who]) and torch.equal(s, state[who]), len(who)
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("heads,rows,cols", [(2, 64, 256), (4, 65, 132), (3, 128, 512), (2, 513, 77), (16, 512, 128), (1, 300, 40), (5, 1030, 24)])
 def test_folded_matrices_do_not_depend_on_company(dtype, heads, rows, cols):
