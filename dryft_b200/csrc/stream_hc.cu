@@ -17,33 +17,12 @@
 //
 // Sums, norms and the streams are 32-bit whatever the activation type T.  One block per row; widths are runtime
 // arguments of any size.  No block waits on another.
-#include "common.cuh"
+#include "few_rows.cuh"
 #include <math.h>
 
 namespace {
-constexpr int THREADS = 256, WIDE_THREADS = 512;
+constexpr int THREADS = 256;
 constexpr int MAX_STREAMS = 8;
-
-// A launch of up to FEW_ROWS rows is (where the caller's `pdl` asks for it) a programmatic dependent: its blocks come in, and fetch the layer's own numbers, while the
-// launch before it drains; the kernel waits before it reads or writes what other launches touch, and reads that past L1 (ld_prev).
-// The rows are those up to which the products on both sides overlap their launches too.
-constexpr int FEW_ROWS = 16;
-template <typename... P, typename... A>
-int launch_rows(void (*kern)(P...), dim3 grid, int threads, size_t smem, bool behind, cudaStream_t st, A... a) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = behind ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, (P)a...);
-  return e != cudaSuccess ? (int)e : launch_status();
-}
-__device__ __forceinline__ void wait_for_earlier_launches() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename TT>
 __global__ void __launch_bounds__(THREADS) embed_pair_norm_kernel(
@@ -100,33 +79,11 @@ __global__ void seq_last_token_kernel(const int* __restrict__ tokens, const int*
   if (n + 1 == n_tokens || tok_slot[n + 1] != slot) prev_state[slot] = tokens[n];
 }
 
-// four consecutive elements of an earlier launch's result at once (8 or 16 bytes)
-template <typename T> __device__ __forceinline__ float4 load4(const T* p);
-template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return ld_prev(reinterpret_cast<const float4*>(p)); }
-template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
-  const uint2 raw = ld_prev(reinterpret_cast<const uint2*>(p));
-  const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), b = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
-  return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
-}
-template <typename T> __device__ __forceinline__ float load1(const T* p);
-template <> __device__ __forceinline__ float load1<float>(const float* p) { return ld_prev(p); }
-template <> __device__ __forceinline__ float load1<__nv_bfloat16>(const __nv_bfloat16* p) { return ld_prev_bf16(p); }
-template <typename T> __device__ __forceinline__ void store4(T* p, float4 v);
-template <> __device__ __forceinline__ void store4<float>(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, float4 v) {
-  __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-  uint2 raw;
-  raw.x = *reinterpret_cast<unsigned*>(&a);
-  raw.y = *reinterpret_cast<unsigned*>(&b);
-  *reinterpret_cast<uint2*>(p) = raw;
-}
-
 // MS: the most streams this instantiation holds in registers (1, 2, 4 or MAX_STREAMS); fewer registers, more blocks an SM.
-// A row is one block, so few rows are bound by the block's chain: launch, matrices, streams, block-wide sum, norm weight.  Rows wider
-// than 1,024 have 512 threads (2,048 columns: one trip to the streams instead of two).
-// With overlapped launches (and the activation's) a request of 1,300 tokens and 16 steps, four streams of 2,048: 15.6 -> 15.1 ms.
-template <typename T, int MS>
-__global__ void __launch_bounds__(WIDE_THREADS) hc_step_kernel(
+// A row is one block.  FEW: a programmatic dependent that is bound by the block's chain: launch, matrices, streams, block-wide sum, norm
+// weight.  With overlapped launches (and the activation's) a request of 1,300 tokens and 16 steps, four streams of 2,048: 15.6 -> 15.1 ms.
+template <typename T, int MS, bool FEW, int THR>
+__global__ void __launch_bounds__(THR) hc_step_kernel(
     const float* __restrict__ x_in, int s_in, float* __restrict__ x_out, int S, const T* __restrict__ y,
     const float* __restrict__ mix, const float* __restrict__ outw, float mult, const float* __restrict__ inw,
     const float* __restrict__ norm_w, float eps, const int* __restrict__ rows, T* __restrict__ h, int width) {
@@ -134,27 +91,29 @@ __global__ void __launch_bounds__(WIDE_THREADS) hc_step_kernel(
   extern __shared__ __align__(16) float row[];
   __shared__ float scratch[33];
   __shared__ float c_mix[MS * MS], c_out[MS], c_in[MS];
-  const int r = blockIdx.x, nthr = blockDim.x;
+  const int r = blockIdx.x;
   if (threadIdx.x < S * S) c_mix[threadIdx.x] = y ? mix[threadIdx.x] : 0.f;
   if (threadIdx.x < S) {
     c_out[threadIdx.x] = y ? mult * outw[threadIdx.x] : 0.f;
     c_in[threadIdx.x] = inw ? inw[threadIdx.x] : 0.f;
   }
   float4 w_first = make_float4(0.f, 0.f, 0.f, 0.f);      // the norm weight of the thread's first columns
-  if (inw && (width & 3) == 0 && threadIdx.x * 4 < width) w_first = *reinterpret_cast<const float4*>(norm_w + threadIdx.x * 4);
+  if (FEW && inw && (width & 3) == 0 && threadIdx.x * 4 < width) w_first = *reinterpret_cast<const float4*>(norm_w + threadIdx.x * 4);
   __syncthreads();
-  wait_for_earlier_launches();
-  const size_t src = rows ? (size_t)ld_prev(rows + r) : (size_t)r;
+  if (FEW) wait_for_earlier_launches();
+  const size_t src = rows ? (size_t)load_word<FEW>(rows + r) : (size_t)r;
+  constexpr bool LATER = THR > ROW_THREADS;      // the sum is formed from shared memory, by the first ROW_THREADS threads
   float ss = 0.f;
   if ((width & 3) == 0) {
     // four columns a thread, 16-byte accesses to the streams: the pass is bound by bytes in flight
-    for (int c = threadIdx.x * 4; c < width; c += nthr * 4) {
+    auto add = [&](const float4& u) { ss = fmaf(u.x, u.x, fmaf(u.y, u.y, fmaf(u.z, u.z, fmaf(u.w, u.w, ss)))); };
+    for (int c = threadIdx.x * 4; c < width; c += THR * 4) {
       float4 x[MS];
 #pragma unroll
       for (int s = 0; s < MS; ++s)
-        if (s < S) x[s] = load4<float>(x_in + (src * s_in + (s_in == 1 ? 0 : s)) * width + c);
+        if (s < S) x[s] = load4<FEW>(x_in + (src * s_in + (s_in == 1 ? 0 : s)) * width + c);
       if (y) {
-        const float4 yv = load4<T>(y + src * width + c);
+        const float4 yv = load4<FEW>(y + src * width + c);
         float4 xn[MS];
 #pragma unroll
         for (int t = 0; t < MS; ++t) {
@@ -188,26 +147,31 @@ __global__ void __launch_bounds__(WIDE_THREADS) hc_step_kernel(
             u.x = fmaf(w, x[t].x, u.x); u.y = fmaf(w, x[t].y, u.y); u.z = fmaf(w, x[t].z, u.z); u.w = fmaf(w, x[t].w, u.w);
           }
         *reinterpret_cast<float4*>(row + c) = u;
-        ss = fmaf(u.x, u.x, fmaf(u.y, u.y, fmaf(u.z, u.z, fmaf(u.w, u.w, ss))));
+        if (!LATER) add(u);
       }
     }
     if (!inw) return;
+    if (LATER) {
+      __syncthreads();
+      if (threadIdx.x < ROW_THREADS)
+        for (int c = threadIdx.x * 4; c < width; c += ROW_THREADS * 4) add(*reinterpret_cast<const float4*>(row + c));
+    }
     ss = block_sum(ss, scratch);
     const float inv = 1.f / sqrtf(ss / (float)width + eps);
-    for (int c = threadIdx.x * 4; c < width; c += nthr * 4) {
+    for (int c = threadIdx.x * 4; c < width; c += THR * 4) {
       const float4 u = *reinterpret_cast<const float4*>(row + c);
-      const float4 w = c == threadIdx.x * 4 ? w_first : *reinterpret_cast<const float4*>(norm_w + c);
-      store4<T>(h + (size_t)r * width + c, make_float4(u.x * inv * w.x, u.y * inv * w.y, u.z * inv * w.z, u.w * inv * w.w));
+      const float4 w = FEW && c == threadIdx.x * 4 ? w_first : *reinterpret_cast<const float4*>(norm_w + c);
+      store4(h + (size_t)r * width + c, make_float4(u.x * inv * w.x, u.y * inv * w.y, u.z * inv * w.z, u.w * inv * w.w));
     }
     return;
   }
-  for (int c = threadIdx.x; c < width; c += nthr) {
+  for (int c = threadIdx.x; c < width; c += THR) {
     float x[MS];
 #pragma unroll
     for (int s = 0; s < MS; ++s)
-      if (s < S) x[s] = ld_prev(x_in + (src * s_in + (s_in == 1 ? 0 : s)) * width + c);
+      if (s < S) x[s] = load1<FEW>(x_in + (src * s_in + (s_in == 1 ? 0 : s)) * width + c);
     if (y) {
-      const float yv = load1<T>(y + src * width + c);
+      const float yv = load1<FEW>(y + src * width + c);
       float xn[MS];
 #pragma unroll
       for (int t = 0; t < MS; ++t) {
@@ -234,13 +198,18 @@ __global__ void __launch_bounds__(WIDE_THREADS) hc_step_kernel(
       for (int t = 0; t < MS; ++t)
         if (t < S) u = fmaf(c_in[t], x[t], u);
       row[c] = u;
-      ss = fmaf(u, u, ss);
+      if (!LATER) ss = fmaf(u, u, ss);
     }
   }
   if (!inw) return;
+  if (LATER) {
+    __syncthreads();
+    if (threadIdx.x < ROW_THREADS)
+      for (int c = threadIdx.x; c < width; c += ROW_THREADS) ss = fmaf(row[c], row[c], ss);
+  }
   ss = block_sum(ss, scratch);
   const float inv = 1.f / sqrtf(ss / (float)width + eps);
-  for (int c = threadIdx.x; c < width; c += nthr) h[(size_t)r * width + c] = from_f32<T>(row[c] * inv * norm_w[c]);
+  for (int c = threadIdx.x; c < width; c += THR) h[(size_t)r * width + c] = from_f32<T>(row[c] * inv * norm_w[c]);
 }
 
 __device__ __forceinline__ float glu_one(float g, float u, float limit, int has_limit, float alpha, float up_offset) {
@@ -252,21 +221,21 @@ __device__ __forceinline__ float glu_one(float g, float u, float limit, int has_
 }
 
 // VEC = 4: four columns a thread (8- or 16-byte accesses; the width is then a multiple of four), VEC = 1: any width
-template <typename T, int VEC>
+template <typename T, int VEC, bool FEW>
 __global__ void glu_clamp_kernel(const T* __restrict__ gate_up, T* __restrict__ out, int rows, int inter, float limit,
                                  int has_limit, float alpha, float up_offset) {
-  if (VEC > 1) let_next_launch_in();   // a product behind this launch may start on its weights
-  wait_for_earlier_launches();
+  if (FEW || VEC > 1) let_next_launch_in();   // a product behind this launch may start on its weights
+  if (FEW) wait_for_earlier_launches();
   const size_t i = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   if (i >= (size_t)rows * inter) return;
   const size_t r = i / inter, f = i % inter;
   const T* g = gate_up + r * 2 * inter + f;
   if (VEC == 4) {
-    const float4 gv = load4<T>(g), uv = load4<T>(g + inter);
-    store4<T>(out + i, make_float4(glu_one(gv.x, uv.x, limit, has_limit, alpha, up_offset), glu_one(gv.y, uv.y, limit, has_limit, alpha, up_offset),
+    const float4 gv = load4<FEW>(g), uv = load4<FEW>(g + inter);
+    store4(out + i, make_float4(glu_one(gv.x, uv.x, limit, has_limit, alpha, up_offset), glu_one(gv.y, uv.y, limit, has_limit, alpha, up_offset),
                                    glu_one(gv.z, uv.z, limit, has_limit, alpha, up_offset), glu_one(gv.w, uv.w, limit, has_limit, alpha, up_offset)));
   } else {
-    out[i] = from_f32<T>(glu_one(load1<T>(g), load1<T>(g + inter), limit, has_limit, alpha, up_offset));
+    out[i] = from_f32<T>(glu_one(load1<FEW>(g), load1<FEW>(g + inter), limit, has_limit, alpha, up_offset));
   }
 }
 
@@ -316,12 +285,18 @@ DRYFT_API int dryft_hc_step(int is_bf16, const float* x_in, int s_in, float* x_o
   if (inw && (!norm_w || !h)) return DRYFT_ERR_UNSUPPORTED;
   typedef __nv_bfloat16 bf;
   const size_t smem = sizeof(float) * (size_t)width;
+#define DRYFT_HC_FORM(TT, MS, FEW, THR)                                                                                          \
+  do {                                                                                                                          \
+    const int rc = row_smem(hc_step_kernel<TT, MS, FEW, THR>, width);                                                           \
+    if (rc) return rc;                                                                                                          \
+    return launch_rows(hc_step_kernel<TT, MS, FEW, THR>, dim3(n_rows), THR, smem, pdl && n_rows <= FEW_ROWS, st, x_in, s_in, x_out, n_streams, \
+                       (const TT*)y, mix, outw, mult, inw, norm_w, eps, rows, (TT*)h, width);                                   \
+  } while (0)
 #define DRYFT_HC_LAUNCH(TT, MS)                                                                                                  \
   do {                                                                                                                          \
-    int rc = row_smem(hc_step_kernel<TT, MS>, width);                                                                           \
-    if (rc) return rc;                                                                                                          \
-    return launch_rows(hc_step_kernel<TT, MS>, dim3(n_rows), width > 1024 ? WIDE_THREADS : THREADS, smem, pdl && n_rows <= FEW_ROWS, st, x_in, s_in, x_out, \
-                       n_streams, (const TT*)y, mix, outw, mult, inw, norm_w, eps, rows, (TT*)h, width);                        \
+    if (n_rows > (n_streams == 1 && width % 4 != 0 ? FEW_ROWS : FORM_ROWS)) DRYFT_HC_FORM(TT, MS, false, ROW_THREADS);                                                           \
+    else if (width > WIDE_ROW) DRYFT_HC_FORM(TT, MS, true, 2 * ROW_THREADS);                                                    \
+    else DRYFT_HC_FORM(TT, MS, true, ROW_THREADS);                                                                              \
   } while (0)
 #define DRYFT_HC_BY_STREAMS(TT)                                                                                                  \
   do {                                                                                                                          \
@@ -334,6 +309,7 @@ DRYFT_API int dryft_hc_step(int is_bf16, const float* x_in, int s_in, float* x_o
   else DRYFT_HC_BY_STREAMS(float);
 #undef DRYFT_HC_BY_STREAMS
 #undef DRYFT_HC_LAUNCH
+#undef DRYFT_HC_FORM
 }
 
 DRYFT_API int dryft_glu_clamp(int is_bf16, const void* gate_up, void* out, int rows, int inter, float limit, int has_limit,
@@ -342,10 +318,13 @@ DRYFT_API int dryft_glu_clamp(int is_bf16, const void* gate_up, void* out, int r
   typedef __nv_bfloat16 bf;
   const int vec = (inter & 3) == 0 ? 4 : 1;
   const unsigned blocks = (unsigned)(((size_t)rows * inter / vec + 255) / 256);
-  const bool behind = pdl && rows <= FEW_ROWS;
-#define DRYFT_GLU(TT, VEC) \
-  launch_rows(glu_clamp_kernel<TT, VEC>, dim3(blocks), 256, 0, behind, st, (const TT*)gate_up, (TT*)out, rows, inter, limit, has_limit, alpha, up_offset)
+  const bool few = rows <= FEW_ROWS;
+#define DRYFT_GLU_FORM(TT, VEC, FEW)                                                                                                  \
+  launch_rows(glu_clamp_kernel<TT, VEC, FEW>, dim3(blocks), 256, 0, FEW && pdl, st, (const TT*)gate_up, (TT*)out, rows, inter, limit, \
+              has_limit, alpha, up_offset)
+#define DRYFT_GLU(TT, VEC) (few ? DRYFT_GLU_FORM(TT, VEC, true) : DRYFT_GLU_FORM(TT, VEC, false))
   if (is_bf16) return vec == 4 ? DRYFT_GLU(bf, 4) : DRYFT_GLU(bf, 1);
   return vec == 4 ? DRYFT_GLU(float, 4) : DRYFT_GLU(float, 1);
 #undef DRYFT_GLU
+#undef DRYFT_GLU_FORM
 }

@@ -19,32 +19,11 @@
 //
 // One block per row; widths are runtime arguments of any size.  Rows whose slot is -1 (padding) are computed like any
 // other: they read and write only their own row.  No block waits on another.
-#include "common.cuh"
+#include "few_rows.cuh"
 #include <math.h>
 
 namespace {
-constexpr int THREADS = 256, WIDE_THREADS = 512;
-
-// A launch of up to FEW_ROWS rows is (where the caller's `pdl` asks for it) a programmatic dependent: its blocks come in, and fetch the layer's own numbers, while the
-// launch before it drains; the kernel waits before it reads or writes what other launches touch, and reads that past L1 (ld_prev).
-// The rows are those up to which the products on both sides overlap their launches too.
-constexpr int FEW_ROWS = 16;
-template <typename... P, typename... A>
-int launch_rows(void (*kern)(P...), dim3 grid, int threads, size_t smem, bool behind, cudaStream_t st, A... a) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = behind ? 1 : 0;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, (P)a...);
-  return e != cudaSuccess ? (int)e : launch_status();
-}
-__device__ __forceinline__ void wait_for_earlier_launches() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+constexpr int THREADS = 256;
 
 template <typename T>
 __global__ void __launch_bounds__(THREADS) stream_sum_kernel(
@@ -79,32 +58,12 @@ __global__ void __launch_bounds__(THREADS) stream_sum_kernel(
   for (int c = threadIdx.x; c < width; c += THREADS) h[n * width + c] = from_f32<T>(x[c] * rinv * norm_w[c]);   // the thread's own writes
 }
 
-// four consecutive elements of an earlier launch's result at once (8 or 16 bytes)
-template <typename T> __device__ __forceinline__ float4 load4(const T* p);
-template <> __device__ __forceinline__ float4 load4<float>(const float* p) { return ld_prev(reinterpret_cast<const float4*>(p)); }
-template <> __device__ __forceinline__ float4 load4<__nv_bfloat16>(const __nv_bfloat16* p) {
-  const uint2 raw = ld_prev(reinterpret_cast<const uint2*>(p));
-  const __nv_bfloat162 a = *reinterpret_cast<const __nv_bfloat162*>(&raw.x), b = *reinterpret_cast<const __nv_bfloat162*>(&raw.y);
-  return make_float4(__low2float(a), __high2float(a), __low2float(b), __high2float(b));
-}
-template <typename T> __device__ __forceinline__ float load1(const T* p);
-template <> __device__ __forceinline__ float load1<float>(const float* p) { return ld_prev(p); }
-template <> __device__ __forceinline__ float load1<__nv_bfloat16>(const __nv_bfloat16* p) { return ld_prev_bf16(p); }
-template <typename T> __device__ __forceinline__ void store4(T* p, float4 v);
-template <> __device__ __forceinline__ void store4<float>(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-template <> __device__ __forceinline__ void store4<__nv_bfloat16>(__nv_bfloat16* p, float4 v) {
-  __nv_bfloat162 a = __floats2bfloat162_rn(v.x, v.y), b = __floats2bfloat162_rn(v.z, v.w);
-  uint2 raw;
-  raw.x = *reinterpret_cast<unsigned*>(&a);
-  raw.y = *reinterpret_cast<unsigned*>(&b);
-  *reinterpret_cast<uint2*>(p) = raw;
-}
-
-// VEC 4 (widths that are a multiple of four) or 1.  Few rows are bound by a block's chain (launch, row and terms, two block-wide sums,
-// weights): rows wider than 1,024 have 512 threads, and the norms' numbers for a thread's first columns are fetched before the wait.
-// A request of four prompts and 12 steps of a 2,048-wide model with 13 such launches a step: 12.3 -> 12.1 ms (with the activation's launch).
-template <typename T, int VEC>
-__global__ void __launch_bounds__(WIDE_THREADS) stream_sum_ln_kernel(
+// VEC 4 (widths that are a multiple of four) or 1.  FEW: a programmatic dependent that is bound by a block's chain (launch, row and terms,
+// two block-wide sums, weights); the norms' numbers for a thread's first columns are fetched before the wait, and all of a row's words
+// are on their way before the first sum.  A request of four prompts and 12 steps of a 2,048-wide model with 13 such launches a step: 12.3 ->
+// 12.1 ms (with the activation's launch).
+template <typename T, int VEC, bool FEW, int THR>
+__global__ void __launch_bounds__(THR) stream_sum_ln_kernel(
     float* __restrict__ x32, const int* __restrict__ rows, const T* __restrict__ y0, float s0, const T* __restrict__ y1, float s1,
     const T* __restrict__ y2, float s2, const float* __restrict__ w0, const float* __restrict__ b0, T* __restrict__ h0,
     const float* __restrict__ w1, const float* __restrict__ b1, T* __restrict__ h1, float eps, int width) {
@@ -112,70 +71,90 @@ __global__ void __launch_bounds__(WIDE_THREADS) stream_sum_ln_kernel(
   extern __shared__ __align__(16) float row[];
   __shared__ float scratch[33];
   const size_t n = blockIdx.x;
-  const int nthr = blockDim.x, c_first = threadIdx.x * 4;
+  const int c_first = threadIdx.x * 4;
   float4 wf[2], bf[2];
-  if (VEC == 4 && c_first < width) {
+  if (FEW && VEC == 4 && c_first < width) {
     if (h0 != nullptr) { wf[0] = *reinterpret_cast<const float4*>(w0 + c_first); bf[0] = *reinterpret_cast<const float4*>(b0 + c_first); }
     if (h1 != nullptr) { wf[1] = *reinterpret_cast<const float4*>(w1 + c_first); bf[1] = *reinterpret_cast<const float4*>(b1 + c_first); }
   }
-  wait_for_earlier_launches();
-  float* x = x32 + (rows != nullptr ? (size_t)ld_prev(rows + n) : n) * width;
+  if (FEW) wait_for_earlier_launches();
+  float* x = x32 + (rows != nullptr ? (size_t)load_word<FEW>(rows + n) : n) * width;
   const bool adds = y0 != nullptr || y1 != nullptr || y2 != nullptr;
+  constexpr bool LATER = THR > ROW_THREADS;      // sums are formed from shared memory, by the first ROW_THREADS threads
   float sum = 0.f;
   if (VEC == 4) {
-    for (int c = threadIdx.x * 4; c < width; c += nthr * 4) {
-      float4 v = load4<float>(x + c), t0, t1, t2;                    // all on their way before the first sum
-      if (y0 != nullptr) t0 = load4<T>(y0 + n * width + c);
-      if (y1 != nullptr) t1 = load4<T>(y1 + n * width + c);
-      if (y2 != nullptr) t2 = load4<T>(y2 + n * width + c);
+    auto add = [&](const float4& v) { sum += (v.x + v.y) + (v.z + v.w); };
+    for (int c = threadIdx.x * 4; c < width; c += THR * 4) {
+      float4 v = load4<FEW>(x + c), t0, t1, t2;
       auto term = [&](const float4& t, float s) {
         v.x = fmaf(s, t.x, v.x); v.y = fmaf(s, t.y, v.y); v.z = fmaf(s, t.z, v.z); v.w = fmaf(s, t.w, v.w);
       };
-      if (y0 != nullptr) term(t0, s0);
-      if (y1 != nullptr) term(t1, s1);
-      if (y2 != nullptr) term(t2, s2);
+      if (FEW) {
+        if (y0 != nullptr) t0 = load4<FEW>(y0 + n * width + c);
+        if (y1 != nullptr) t1 = load4<FEW>(y1 + n * width + c);
+        if (y2 != nullptr) t2 = load4<FEW>(y2 + n * width + c);
+        if (y0 != nullptr) term(t0, s0);
+        if (y1 != nullptr) term(t1, s1);
+        if (y2 != nullptr) term(t2, s2);
+      } else {
+        if (y0 != nullptr) term(load4<FEW>(y0 + n * width + c), s0);
+        if (y1 != nullptr) term(load4<FEW>(y1 + n * width + c), s1);
+        if (y2 != nullptr) term(load4<FEW>(y2 + n * width + c), s2);
+      }
       if (adds) *reinterpret_cast<float4*>(x + c) = v;
       *reinterpret_cast<float4*>(row + c) = v;
-      sum += (v.x + v.y) + (v.z + v.w);
+      if (!LATER) add(v);
+    }
+    if (LATER) {
+      __syncthreads();
+      if (threadIdx.x < ROW_THREADS)
+        for (int c = threadIdx.x * 4; c < width; c += ROW_THREADS * 4) add(*reinterpret_cast<const float4*>(row + c));
     }
   } else {
-    for (int c = threadIdx.x; c < width; c += nthr) {
-      float v = ld_prev(x + c);
-      if (y0 != nullptr) v = fmaf(s0, load1<T>(y0 + n * width + c), v);
-      if (y1 != nullptr) v = fmaf(s1, load1<T>(y1 + n * width + c), v);
-      if (y2 != nullptr) v = fmaf(s2, load1<T>(y2 + n * width + c), v);
+    for (int c = threadIdx.x; c < width; c += THR) {
+      float v = load1<FEW>(x + c);
+      if (y0 != nullptr) v = fmaf(s0, load1<FEW>(y0 + n * width + c), v);
+      if (y1 != nullptr) v = fmaf(s1, load1<FEW>(y1 + n * width + c), v);
+      if (y2 != nullptr) v = fmaf(s2, load1<FEW>(y2 + n * width + c), v);
       if (adds) x[c] = v;
       row[c] = v;
-      sum += v;
+      if (!LATER) sum += v;
+    }
+    if (LATER) {
+      __syncthreads();
+      if (threadIdx.x < ROW_THREADS)
+        for (int c = threadIdx.x; c < width; c += ROW_THREADS) sum += row[c];
     }
   }
   if (h0 == nullptr && h1 == nullptr) return;
   const float mean = block_sum(sum, scratch) / (float)width;
-  float ss = 0.f;      // every thread reads the entries it wrote itself
-  if (VEC == 4) {
-    for (int c = threadIdx.x * 4; c < width; c += nthr * 4) {
-      const float4 v = *reinterpret_cast<const float4*>(row + c);
-      const float a = v.x - mean, b = v.y - mean, d = v.z - mean, e = v.w - mean;
-      ss = fmaf(a, a, fmaf(b, b, fmaf(d, d, fmaf(e, e, ss))));
+  float ss = 0.f;      // (in the form of ROW_THREADS threads every thread reads the entries it wrote itself)
+  if (threadIdx.x < ROW_THREADS) {
+    if (VEC == 4) {
+      for (int c = threadIdx.x * 4; c < width; c += ROW_THREADS * 4) {
+        const float4 v = *reinterpret_cast<const float4*>(row + c);
+        const float a = v.x - mean, b = v.y - mean, d = v.z - mean, e = v.w - mean;
+        ss = fmaf(a, a, fmaf(b, b, fmaf(d, d, fmaf(e, e, ss))));
+      }
+    } else {
+      for (int c = threadIdx.x; c < width; c += ROW_THREADS) { const float d = row[c] - mean; ss = fmaf(d, d, ss); }
     }
-  } else {
-    for (int c = threadIdx.x; c < width; c += nthr) { const float d = row[c] - mean; ss = fmaf(d, d, ss); }
   }
   const float rinv = 1.f / sqrtf(block_sum(ss, scratch) / (float)width + eps);
   if (VEC == 4) {
-    for (int c = threadIdx.x * 4; c < width; c += nthr * 4) {
+    for (int c = threadIdx.x * 4; c < width; c += THR * 4) {
       float4 v = *reinterpret_cast<const float4*>(row + c);
       v.x = (v.x - mean) * rinv; v.y = (v.y - mean) * rinv; v.z = (v.z - mean) * rinv; v.w = (v.w - mean) * rinv;
       auto out = [&](const float* w, const float* b, T* h, int k) {
-        const bool first = c == c_first;
+        const bool first = FEW && c == c_first;
         const float4 ww = first ? wf[k] : *reinterpret_cast<const float4*>(w + c), bb = first ? bf[k] : *reinterpret_cast<const float4*>(b + c);
-        store4<T>(h + n * width + c, make_float4(fmaf(v.x, ww.x, bb.x), fmaf(v.y, ww.y, bb.y), fmaf(v.z, ww.z, bb.z), fmaf(v.w, ww.w, bb.w)));
+        store4(h + n * width + c, make_float4(fmaf(v.x, ww.x, bb.x), fmaf(v.y, ww.y, bb.y), fmaf(v.z, ww.z, bb.z), fmaf(v.w, ww.w, bb.w)));
       };
       if (h0 != nullptr) out(w0, b0, h0, 0);
       if (h1 != nullptr) out(w1, b1, h1, 1);
     }
   } else {
-    for (int c = threadIdx.x; c < width; c += nthr) {
+    for (int c = threadIdx.x; c < width; c += THR) {
       const float v = (row[c] - mean) * rinv;
       if (h0 != nullptr) h0[n * width + c] = from_f32<T>(fmaf(v, w0[c], b0[c]));
       if (h1 != nullptr) h1[n * width + c] = from_f32<T>(fmaf(v, w1[c], b1[c]));
@@ -183,18 +162,25 @@ __global__ void __launch_bounds__(WIDE_THREADS) stream_sum_ln_kernel(
   }
 }
 
+template <typename T, int VEC, bool FEW, int THR>
+int sum_ln_form(float* x32, const int* rows, const void* y0, float s0, const void* y1, float s1, const void* y2, float s2, const float* w0,
+                const float* b0, void* h0, const float* w1, const float* b1, void* h1, float eps, int n, int width, int pdl, cudaStream_t st) {
+  const size_t smem = sizeof(float) * (size_t)width;
+  if (smem > 200 * 1024) return DRYFT_ERR_UNSUPPORTED;
+  if (smem > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(stream_sum_ln_kernel<T, VEC, FEW, THR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+  }
+  return launch_rows(stream_sum_ln_kernel<T, VEC, FEW, THR>, dim3(n), THR, smem, pdl && n <= FEW_ROWS, st, x32, rows, (const T*)y0, s0,
+                     (const T*)y1, s1, (const T*)y2, s2, w0, b0, (T*)h0, w1, b1, (T*)h1, eps, width);
+}
 template <typename T, int VEC>
 int sum_ln_launch(float* x32, const int* rows, const void* y0, float s0, const void* y1, float s1, const void* y2, float s2, const float* w0,
                   const float* b0, void* h0, const float* w1, const float* b1, void* h1, float eps, int n, int width, int pdl,
                   cudaStream_t st) {
-  const size_t smem = sizeof(float) * (size_t)width;
-  if (smem > 200 * 1024) return DRYFT_ERR_UNSUPPORTED;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(stream_sum_ln_kernel<T, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-  }
-  return launch_rows(stream_sum_ln_kernel<T, VEC>, dim3(n), width > 1024 ? WIDE_THREADS : THREADS, smem, pdl && n <= FEW_ROWS, st, x32, rows,
-                     (const T*)y0, s0, (const T*)y1, s1, (const T*)y2, s2, w0, b0, (T*)h0, w1, b1, (T*)h1, eps, width);
+  auto form = n > (VEC == 4 ? FORM_ROWS : FEW_ROWS) ? sum_ln_form<T, VEC, false, ROW_THREADS>
+              : width > WIDE_ROW ? sum_ln_form<T, VEC, true, 2 * ROW_THREADS> : sum_ln_form<T, VEC, true, ROW_THREADS>;
+  return form(x32, rows, y0, s0, y1, s1, y2, s2, w0, b0, h0, w1, b1, h1, eps, n, width, pdl, st);
 }
 
 template <typename T, int VEC>
@@ -214,7 +200,7 @@ __global__ void __launch_bounds__(THREADS) stream_norm_join_kernel(
     for (int c = threadIdx.x * 4; c < width; c += THREADS * 4) {
       float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
       auto term = [&](const T* y, float s) {
-        const float4 t = load4<T>(y + c);
+        const float4 t = load4<false>(y + c);
         v.x = fmaf(s, t.x, v.x); v.y = fmaf(s, t.y, v.y); v.z = fmaf(s, t.z, v.z); v.w = fmaf(s, t.w, v.w);
       };
       if (y0 != nullptr) term(y0 + n * width, s0);
@@ -263,7 +249,7 @@ __global__ void __launch_bounds__(THREADS) stream_norm_join_kernel(
   if (VEC == 4) {
     for (int c = threadIdx.x * 4; c < width; c += THREADS * 4) {
       const float4 v = *reinterpret_cast<const float4*>(row + c), w = *reinterpret_cast<const float4*>(norm_w + c);
-      store4<T>(h + n * width + c, make_float4(v.x * rinv * w.x, v.y * rinv * w.y, v.z * rinv * w.z, v.w * rinv * w.w));
+      store4(h + n * width + c, make_float4(v.x * rinv * w.x, v.y * rinv * w.y, v.z * rinv * w.z, v.w * rinv * w.w));
     }
   } else {
     for (int c = threadIdx.x; c < width; c += THREADS) h[n * width + c] = from_f32<T>(row[c] * rinv * norm_w[c]);
@@ -292,7 +278,7 @@ __global__ void __launch_bounds__(THREADS) stream_norm_join_regs_kernel(
       f[i] = *reinterpret_cast<const float4*>(factor + c);
       if (norm_w != nullptr) w[i] = *reinterpret_cast<const float4*>(norm_w + c);
       auto term = [&](const T* p, float s) {
-        const float4 t = load4<T>(p + c);
+        const float4 t = load4<false>(p + c);
         y[i].x = fmaf(s, t.x, y[i].x); y[i].y = fmaf(s, t.y, y[i].y); y[i].z = fmaf(s, t.z, y[i].z); y[i].w = fmaf(s, t.w, y[i].w);
       };
       if (y0 != nullptr) term(y0 + n * width, s0);
@@ -324,7 +310,7 @@ __global__ void __launch_bounds__(THREADS) stream_norm_join_regs_kernel(
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int c = (i * THREADS + (int)threadIdx.x) * 4;
-    if (c < width) store4<T>(h + n * width + c, make_float4(y[i].x * rinv * w[i].x, y[i].y * rinv * w[i].y, y[i].z * rinv * w[i].z, y[i].w * rinv * w[i].w));
+    if (c < width) store4(h + n * width + c, make_float4(y[i].x * rinv * w[i].x, y[i].y * rinv * w[i].y, y[i].z * rinv * w[i].z, y[i].w * rinv * w[i].w));
   }
 }
 
