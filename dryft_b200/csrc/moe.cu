@@ -244,9 +244,8 @@ __global__ void __launch_bounds__(ROWS_THREADS) moe_rows_kernel(
   }
 }
 
-// A thread sums 16 bytes of columns (one column where the width or the addresses are no multiple of 16 bytes): its `top`
-// rows' words are requested together, eight at a time, and added in the order of k.  2,048 tokens x 8 rows of 2,048: 12 us
-// for 75 MB, 31 with one column a thread; 8 tokens: 2 us against 13.
+// A thread sums V columns, 16 bytes or one: its `top` rows' words are requested together, eight at a time, and added in the order of k.
+// 2,048 tokens x 8 rows of 2,048: 12 us for 75 MB, 31 with one column a thread; 8 tokens: 2 us against 13.
 constexpr int COMBINE_THREADS = 128;
 template <typename T, int V, bool SIGNAL>
 __global__ void __launch_bounds__(COMBINE_THREADS) moe_combine_kernel(const T* __restrict__ y, const float* __restrict__ wts, int top, int width,
@@ -283,11 +282,34 @@ __global__ void __launch_bounds__(COMBINE_THREADS) moe_combine_kernel(const T* _
   else to[0] = r[0];
 }
 
+// The same where the width or an address is no multiple of 16 bytes and the rows are many: a block a token, a column a thread at a time, in
+// the same order.
+template <typename T>
+__global__ void __launch_bounds__(256) moe_combine_rows_kernel(const T* __restrict__ y, const float* __restrict__ wts, int top, int width,
+                                                               T* __restrict__ out) {
+  let_next_launch_in();   // a product behind this launch may start on its weights
+  const int n = blockIdx.x;
+  for (int c = threadIdx.x; c < width; c += blockDim.x) {
+    float v = 0.f;
+    for (int k = 0; k < top; ++k) v = fmaf(wts[(size_t)n * top + k], to_f32<T>(y[((size_t)n * top + k) * width + c]), v);
+    out[(size_t)n * width + c] = from_f32<T>(v);
+  }
+}
+
 template <typename T>
 int combine_launch(const void* y, const float* wts, int top, int width, void* out, int n, cudaStream_t st) {
   constexpr int V = 16 / sizeof(T);
   const bool vec = width % V == 0 && ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
   const int per = COMBINE_THREADS * (vec ? V : 1), cols = (width + per - 1) / per;
+  // one column a thread pays while the blocks are few (2 rows of 2,050, 32-bit: 64 tokens 2.7 us against 4.1, 300 tokens 6.4 against 4.3,
+  // 2,048 tokens 37 against 11)
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (!vec && (long long)n * cols > 8LL * sms) {
+    moe_combine_rows_kernel<T><<<n, 256, 0, st>>>((const T*)y, wts, top, width, (T*)out);
+    return launch_status();
+  }
   if (cols > 65535) return DRYFT_ERR_UNSUPPORTED;
   auto kern = n <= SIGNAL_ROWS ? (vec ? moe_combine_kernel<T, V, true> : moe_combine_kernel<T, 1, true>)
                                : (vec ? moe_combine_kernel<T, V, false> : moe_combine_kernel<T, 1, false>);
