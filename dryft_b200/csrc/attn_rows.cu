@@ -181,7 +181,6 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
       if (d < D) {
 #pragma unroll
         for (int g = 0; g < G; ++g) acc[i][g] *= a_s[g];
-#pragma unroll 8
         for (int r = 0; r < PAGE; ++r) {
           const float v = to_f32<T>(vt[r * D + d]);
 #pragma unroll
