@@ -668,7 +668,10 @@ int rows_launch(const void* q, const void* k_pages, const void* v_pages, const i
   dim3 grid(n, G, n_splits);
   // two lanes a key while all blocks run at once (three a multiprocessor: faster at every size measured up to there, see the kernel), with value
   // rows in whole lanes, which wants aligned pages; beyond that other blocks hide a warp's chain and the fewer instructions count
-  const bool few = (long long)n * G * n_splits <= 148 * 3 && (((uintptr_t)v_pages | (uintptr_t)pv) & 15) == 0;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const bool few = (long long)n * G * n_splits <= 3LL * sms && (((uintptr_t)v_pages | (uintptr_t)pv) & 15) == 0;
   const bool m = mods.cap > 0.f || mods.r1 != nullptr;
   auto kernel = few ? (m ? pool_attn_rows_kernel<T, true, 2> : pool_attn_rows_kernel<T, false, 2>)
                     : (m ? pool_attn_rows_kernel<T, true, 1> : pool_attn_rows_kernel<T, false, 1>);
