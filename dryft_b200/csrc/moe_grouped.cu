@@ -373,17 +373,17 @@ __device__ __forceinline__ void tmem_ld16(unsigned taddr, unsigned (&r)[16]) {
                : "r"(taddr));
 }
 
-// n / d for d >= 1: the quotient by an approximate reciprocal, and one of Newton's corrections of it by what is left of n.  Without a
-// branch, so that a thread's sixteen quotients overlap: with the compiler's division, which branches for extreme exponents, a layer of
-// 64 experts of 768 x 2,048 takes 280 us for 2,048 tokens x 8, with this one 266.  For silu of every gate between -88.7 and 200 the two
-// give the same 32-bit values, 4.2 x 2^-24 off at most; a fast exponential and division (258 us) are 18 x 2^-24 off and give zero
-// below -87.3.
-__device__ __forceinline__ float over(float n, float d) {
+// n / (1 + e) for e >= 0: the quotient by an approximate reciprocal, and one of Newton's corrections of it by what is left of n; quarters of
+// both, so that the reciprocal of a sum beyond 2^126 is still a normal number.  Without a branch, so that a thread's sixteen quotients
+// overlap: with the compiler's division, which branches for extreme exponents, a layer of 64 experts of 768 x 2,048 takes 280 us for
+// 2,048 tokens x 8, with this one 262.  For silu of every gate between -88.7 and 200 the two give the same 32-bit values, 4.2 x 2^-24 off at
+// most; a fast exponential and division (258 us) are 18 x 2^-24 off and give zero below -87.3.
+__device__ __forceinline__ float over_one_plus(float n, float e) {
+  const float d = fmaf(e, 0.25f, 0.25f), m = 0.25f * n;
   float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(d));
-  const float q = n * r;
-  const float better = fmaf(fmaf(-q, d, n), r, q);
-  return d <= 1.f ? n : d <= 3.402823466e38f ? better : n * 0.f;      // (infinite n and d: the products above are no numbers)
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = m * r, better = fmaf(fmaf(-q, d, m), r, q);
+  return better == better ? better : q;      // infinite n or e: nothing to correct
 }
 
 // The product is computed transposed: two tiles of 128 weight rows (gate and up rows of the same 128 features, or 256
@@ -540,11 +540,11 @@ __global__ void __launch_bounds__(TC_THREADS) moe_grouped_tc_kernel(
 #pragma unroll
         for (int c = 0; c < 16; ++c) {
           float x = __uint_as_float(r0[c]), y = __uint_as_float(r1[c]);
-          if (MODE == 0) x = over(x, 1.f + expf(-x)) * y;
+          if (MODE == 0) x = over_one_plus(x, expf(-x)) * y;
           if (MODE == 3) {
             const float sc = __shfl_sync(0xffffffffu, my_w, c);
             const float g = fminf(x * sc, limit), up = fminf(fmaxf(y * sc, -limit), limit);
-            x = over(g, 1.f + expf(-alpha * g)) * (up + up_off);
+            x = over_one_plus(g, expf(-alpha * g)) * (up + up_off);
           }
           if (MODE == 2) {
             x = fmaxf(x, 0.f); x *= x;
