@@ -131,6 +131,7 @@ class MoE:
                             and K.moe_grouped_supported(self.hidden, self.inter))
         if self.use_grouped:
             K.moe_grouped_lib()
+        self._plan_grouped()
         # the always-on expert: its first product also yields the per-token gate logit (one more row of the weight, padded)
         self.shared_inter = 0
         self.side, self.side_out = None, None      # (first column, columns) of rows that ride with the always-on expert's product
@@ -162,14 +163,20 @@ class MoE:
     ROUTE_ROWS_MAX_WEIGHTS = 64 * 1024   # ... while one block can stream the router's weight quickly enough (measured: 32 x 1,024
                                          # gains a launch, 64 x 2,048 takes longer than the two launches it replaces)
 
+    def _plan_grouped(self) -> None:
+        """The fewest tokens whose products run grouped."""
+        self.grouped_from = self.GROUPED_MIN_TOKENS
+        # (on mma.sync: for prompts only; the sorting block's counters take 6,144 experts)
+        if self.rt.tcgen05 and self.hidden % 64 == 0 and self.inter % 64 == 0 and self.experts <= 6144:
+            each = 2 * (self.w_gate_up[0].numel() + self.w_down[0].numel())
+            for n in range(1, self.GROUPED_MIN_TOKENS):
+                chosen = self.experts * (1.0 - (1.0 - self.top / self.experts) ** n)      # different experts, on the mean
+                if (n * self.top - chosen) * each >= self.GROUPED_SPARES_BYTES:
+                    self.grouped_from = n
+                    break
+
     def _grouped(self, n: int) -> bool:
-        if not self.use_grouped or n >= self.GROUPED_MIN_TOKENS:
-            return self.use_grouped
-        if not self.rt.tcgen05 or self.hidden % 64 or self.inter % 64:      # the grouped products on mma.sync: for prompts only
-            return False
-        chosen = self.experts * (1.0 - (1.0 - self.top / self.experts) ** n)      # different experts, on the mean
-        each = 2 * (self.w_gate_up[0].numel() + self.w_down[0].numel())
-        return (n * self.top - chosen) * each >= self.GROUPED_SPARES_BYTES
+        return self.use_grouped and n >= self.grouped_from
 
     def route(self, h: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
         """Chosen experts ``[n, top]`` int32 and their weights ``[n, top]`` float32."""

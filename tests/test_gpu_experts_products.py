@@ -86,7 +86,7 @@ def test_grouped_products_of_many_assignments():
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("n,top,e,width,f", [(1, 1, 1, 64, 24), (5, 3, 7, 128, 33), (16, 8, 24, 256, 72), (32, 8, 9, 64, 40), (4, 2, 64, 72, 16)])
 def test_few_tokens_that_share_experts(dtype, n, top, e, width, f):
-    """An expert's weights read once for all its assignments give the bits that one assignment alone gives."""
+    """Assignment by assignment: an assignment among others has the bits that it has alone, whoever shares its expert."""
     from dryft_b200.ops import kernels as K
 
     h, w1, _, idx, in_w = _case(n, top, e, width, f, "silu")
@@ -140,3 +140,81 @@ def test_activation_of_gates_far_below_zero(act, n):
     assert float(exact.abs().min()) > 1e-8
     # two roundings to bfloat16 (the second of a value that has been rounded); the 32-bit evaluation is exact to 2^-20
     assert bool(((y.double() - exact).abs() <= 2.0 ** -8 * exact.abs()).all())
+
+
+@pytest.mark.parametrize("params", [dict(activation="swiglu"), dict(activation="relu2"), dict(activation="clamped", limit=1.5, alpha=1.702, up_offset=1.0),
+                                    dict(activation="swiglu", weight_input=True)])
+def test_few_tokens_of_a_layer_grouped_and_one_by_one(monkeypatch, params):
+    """Below 32 tokens a layer multiplies its experts grouped where that spares enough bytes: with the threshold at zero and out of
+    reach, the same outputs up to their roundings."""
+    from dryft_b200.ops import kernels as K
+    from dryft_b200.parts.base import FFNS, Runtime, StepContext
+    from dryft_b200.parts.moe import MoE
+    from dryft_b200.weights import RandomSource
+
+    params = dict(params, hidden_size=128, intermediate_size=64, experts=8, top=3)
+    cls = FFNS.get("moe")
+    dev = torch.device("cuda:0")
+
+    def layer(threshold):
+        monkeypatch.setattr(MoE, "GROUPED_SPARES_BYTES", threshold)
+        rt = Runtime(dtype=torch.bfloat16, device=dev)
+        return cls(params, "f.", RandomSource(cls.tensors(params, "f."), 5, torch.bfloat16, dev, std=0.1), rt)
+
+    grouped, single = layer(0.0), layer(1e18)
+    calls = []
+    real = K.moe_grouped
+    monkeypatch.setattr(K, "moe_grouped", lambda *a, **k: (calls.append(a[0].shape[0]), real(*a, **k)))
+    for n in (1, 2, 5, 16, 17, 31, 32):
+        h = torch.randn(n, 128, device="cuda").bfloat16()
+        ints = torch.zeros(n + 1, dtype=torch.int32, device="cuda")
+        ctx = StepContext(n_tokens=n, n_seqs=1, tokens=ints[:n], cu_q=ints[:2], seq_slot=ints[:1], tok_slot=ints[:n], tok_pos=ints[:n], decode=False)
+        with torch.inference_mode():
+            del calls[:]
+            a = grouped.forward(h, ctx)
+            assert calls == [n]
+            b = single.forward(h, ctx)
+            assert calls == [n] + [n] * (n >= 32)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph):
+                c = grouped.forward(h, ctx)
+            graph.replay()
+        assert torch.isfinite(a).all() and torch.equal(a, c)
+        # activation, expert's row and weighted sum are rounded to bfloat16 on either side, each half a unit in 2^8
+        assert float((a.double() - b.double()).norm() / b.double().norm()) < 6.0 * 2.0 ** -9, n
+    K.check_error_flags()
+
+
+def test_few_tokens_grouped_in_decode_steps(monkeypatch):
+    """The same inside a model's decode steps: captured and eager give the same bits, and stay within bfloat16 of the other form."""
+    import copy
+
+    from dryft_b200.config import preset
+    from dryft_b200.engine.api import Engine
+    from dryft_b200.ops import kernels as K
+    from dryft_b200.parts.moe import MoE
+
+    cfg = copy.deepcopy(preset("tevovik-tiny"))
+    for one in cfg["layers"]:
+        one["mlp"]["expert"]["ff"] = 64
+    logits = {}
+    for threshold in (0.0, 1e18):
+        monkeypatch.setattr(MoE, "GROUPED_SPARES_BYTES", threshold)
+        for graphs in (True, False):
+            eng = Engine.from_config(cfg, seed=3, dtype="bfloat16", max_batch=8, max_seq_len=256, max_tokens=1024, cuda_graphs=graphs)
+            with torch.inference_mode():
+                slots = eng.cache.open_sequences(5)
+                eng.stepper.step(slots, [[1, 2, 3], [4] * 9, [5], [6, 7], [8] * 40], [[]] * 5)
+                out = []
+                for t in range(8):
+                    at = torch.tensor(slots, device="cuda")
+                    eng.cache.last_token.index_copy_(0, at, torch.tensor([t + 1, 2 * t, 3, 9, t], dtype=torch.int32, device="cuda"))
+                    out.append(eng.stepper.decode_from_state(slots)[:5].clone())
+            logits[threshold, graphs] = torch.stack(out)
+    assert torch.isfinite(logits[0.0, True]).all()
+    assert torch.equal(logits[0.0, True], logits[0.0, False]) and torch.equal(logits[1e18, True], logits[1e18, False])
+    a, b = logits[0.0, True].double(), logits[1e18, True].double()
+    # roundings of three layers of experts, some of which decide a router's close call the other way: most logits agree closely
+    err = (a - b).norm(dim=-1) / b.norm(dim=-1)
+    assert float(err.median()) < 3e-2, err
+    K.check_error_flags()
