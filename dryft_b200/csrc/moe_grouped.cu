@@ -18,6 +18,7 @@
 #include "common.cuh"
 #include "drain.h"
 #include <cuda.h>
+#include <atomic>
 #include <math.h>
 #include <type_traits>
 
@@ -628,8 +629,14 @@ int tc_launch(const void* x, long long x_rows, const void* w, int E, const Sorte
   typedef Tc<MODE, NMAX> L;
   CUtensorMap map_w, map_x;
   if (!encode(&map_w, w, (long long)E * (L::GATED ? 2 : 1) * n_out, K, 128) || !encode(&map_x, x, x_rows, K, 64)) return DRYFT_ERR_UNSUPPORTED;
-  const cudaError_t e = cudaFuncSetAttribute(moe_grouped_tc_kernel<MODE, NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
-  if (e != cudaSuccess) return (int)e;
+  static std::atomic<unsigned long long> set{0};      // a bit a device (setting the attribute twice does no harm)
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev >= 64 || !(set.load(std::memory_order_relaxed) >> dev & 1)) {
+    const cudaError_t e = cudaFuncSetAttribute(moe_grouped_tc_kernel<MODE, NMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 64) set.fetch_or(1ull << dev, std::memory_order_relaxed);
+  }
   const int f_tiles = (n_out + L::FEATURES - 1) / L::FEATURES;
   const long long most = (long long)t.max_tiles * f_tiles;
   cudaLaunchConfig_t cfg = {};
@@ -648,9 +655,12 @@ int tc_launch(const void* x, long long x_rows, const void* w, int E, const Sorte
   return launch_status();
 }
 
-bool tc_takes(int W, int F, const void* h, const void* w_gate_up, const void* w_down, const void* act, const void* y) {
+// What runs on tcgen05: inner sizes that fill its k slices, and addresses that the copy engine takes.  Many rows of a few very small
+// experts are the exception (up to 32 of 128 x 64, more than 1,024 rows: 31 us against 28 on mma.sync, whose small tiles spread over more
+// blocks; fewer rows 22 against 27, 64 experts 35 against 38, 256 x 64 as fast).
+bool tc_takes(int E, int n_assign, int W, int F, const void* h, const void* w_gate_up, const void* w_down, const void* act, const void* y) {
   const uintptr_t all = (uintptr_t)h | (uintptr_t)w_gate_up | (uintptr_t)w_down | (uintptr_t)act | (uintptr_t)y;
-  return W % 64 == 0 && F % 64 == 0 && (all & 15) == 0;
+  return W % 64 == 0 && F % 64 == 0 && (all & 15) == 0 && !(E <= 32 && n_assign > 1024 && (long long)W * F <= 128 * 64);
 }
 
 // rows per tile: tcgen05: 256 once experts get about that many rows on average (the weights are read half as often), 128 below
@@ -685,7 +695,7 @@ DRYFT_API int dryft_moe_grouped(const void* h, const void* w_gate_up, const void
       (long long)E * W > (1LL << 31) - 1)
     return DRYFT_ERR_UNSUPPORTED;
   const int n_assign = (int)n_assign_ll;
-  const bool tc = tcgen05 && tc_takes(W, F, h, w_gate_up, w_down, act, y);
+  const bool tc = tcgen05 && tc_takes(E, n_assign, W, F, h, w_gate_up, w_down, act, y);
   const int bm = tile_rows_for(n_assign, E, tc), max_tiles = max_tiles_for(n_assign, E, tc);
   int* const perm = work;
   int* const place = perm + n_assign;
@@ -694,7 +704,9 @@ DRYFT_API int dryft_moe_grouped(const void* h, const void* w_gate_up, const void
   int* const tile_rows = tile_row0 + max_tiles;
   int* const n_tiles = tile_rows + max_tiles;
   int hists = SORT_INTS / E - 1;
-  hists = hists < 1 ? 1 : hists > SORT_THREADS / 32 ? SORT_THREADS / 32 : hists;
+  hists = hists > SORT_THREADS / 32 ? SORT_THREADS / 32 : hists;
+  if (hists > n_assign / 256) hists = n_assign / 256;      // few assignments hardly collide: less to clear and to add up
+  if (hists < 1) hists = 1;
   moe_sort_kernel<<<1, SORT_THREADS, sizeof(int) * (hists + 1) * E, st>>>(idx, n_assign, E, bm, hists, perm, tc ? place : nullptr,
                                                                                   tile_expert, tile_row0, tile_rows, n_tiles, n_tiles + 1);
   int rc = launch_status();

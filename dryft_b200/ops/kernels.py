@@ -976,10 +976,11 @@ def moe_grouped(h, w_gate_up, w_down, idx, y, gated: bool = True, in_w=None, lim
         if not gated:
             raise KernelError("moe_grouped: weights on the experts' input go with gated experts")
         _need(in_w, "in_w", torch.float32, (n, top))
+    on_tensor_memory = tcgen05 and width % 64 == 0 and f % 64 == 0 and not (e <= 32 and n * top > 1024 and width * f <= 128 * 64)
     _ok(lib.dryft_moe_grouped(_ptr(h), _ptr(w_gate_up), _ptr(w_down), _ptr(idx), n, top, e, width, f, _ptr(act), _ptr(y), _ptr(work),
                               2 if in_w is not None else int(gated), _ptr(in_w), float("inf") if limit is None else float(limit),
                               float(alpha), float(up_offset), _ptr(error_flag(h.device)), int(pdl), int(tcgen05), _stream()),
-        f"moe_grouped ({e} experts, {width} x {f})", n_kernels=4 if tcgen05 and width % 64 == 0 and f % 64 == 0 else 3)
+        f"moe_grouped ({e} experts, {width} x {f})", n_kernels=4 if on_tensor_memory else 3)
 
 
 # ----------------------------------------------------------------------------- matrix products

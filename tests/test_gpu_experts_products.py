@@ -57,10 +57,11 @@ ROWS = [0, 1, 15, 16, 17, 0, 64, 65, 127, 128, 129, 200, 255, 256, 257, 3]
 
 @pytest.mark.parametrize("act", ["silu", "relu2", "clamped"])
 @pytest.mark.parametrize("width,f,rows", [
-    (128, 64, ROWS),                                   # two tiles of accumulators (128 rows a tile), less than a feature tile
+    (128, 64, ROWS),                                   # many rows of a few small experts: mma.sync
     (64, 192, ROWS),                                   # one k slice, a feature tile and a half
     (192, 320, [r * 6 for r in ROWS]),                 # tiles of 256 rows
     (256, 128, [700, 0, 1, 513]),
+    (256, 64, ROWS), (128, 64, [128, 0, 1, 129, 255, 64]),   # less than a feature tile on tcgen05: not all too small, not too many rows
     (48, 80, ROWS), (112, 64, [r * 2 for r in ROWS]),  # inner sizes that the mma.sync products take
 ])
 def test_grouped_products(act, width, f, rows):
@@ -218,3 +219,18 @@ def test_few_tokens_grouped_in_decode_steps(monkeypatch):
     err = (a - b).norm(dim=-1) / b.norm(dim=-1)
     assert float(err.median()) < 3e-2, err
     K.check_error_flags()
+
+
+@pytest.mark.parametrize("e,rows,width,f,launches", [(32, 1025, 128, 64, 3), (32, 1024, 128, 64, 4), (33, 1025, 128, 64, 4), (32, 1025, 192, 64, 4),
+                                                     (8, 2048, 64, 128, 3)])
+def test_many_rows_of_a_few_small_experts_run_on_mma_sync(e, rows, width, f, launches):
+    from dryft_b200.ops import kernels as K
+
+    h, w1, w2, idx, in_w = _case(rows, 1, e, width, f, "silu")
+    y, plain = (torch.empty(rows, width, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    before = K.launch_count
+    K.moe_grouped(h, w1, w2, idx, y)
+    assert K.launch_count - before == launches
+    K.moe_grouped(h, w1, w2, idx, plain, tcgen05=False)
+    _check(y, _exact(h, w1, w2, idx, "silu", in_w, 0, 0, 0))
+    assert launches != 3 or torch.equal(y, plain)
