@@ -54,22 +54,8 @@ DRYFT_API int dryft_step_advance(const int* cu_q, const int* seq_slot, int* seq_
   return launch_status();
 }
 
-// Decode input from the per-sequence state: tokens[b] = last_token[slot[b]] (0 for padding).
-__global__ void tokens_from_state_kernel(const int* __restrict__ seq_slot, const int* __restrict__ last_token,
-                                         int* __restrict__ tokens, int n_seqs) {
-  int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= n_seqs) return;
-  int slot = seq_slot[b];
-  tokens[b] = slot < 0 ? 0 : last_token[slot];
-}
-DRYFT_API int dryft_tokens_from_state(const int* seq_slot, const int* last_token, int* tokens, int n_seqs, cudaStream_t st) {
-  if (n_seqs <= 0) return 0;
-  tokens_from_state_kernel<<<(n_seqs + 127) / 128, 128, 0, st>>>(seq_slot, last_token, tokens, n_seqs);
-  return launch_status();
-}
-
 // A decode step's beginning in one launch: every sequence's next token and position from the per-sequence state, and, with
-// `advance`, its length with the token that the step appends (the step itself goes by tok_pos).  Three launches of 1.6 us, which
+// `advance`, its length with the token that the step appends (the step itself goes by tok_pos).  Three launches of 1.6 us
 // took more than a hundredth of a small model's step.  A captured step runs as a whole and counts here; a step that is launched
 // piece by piece may end in an error between them, and counts behind its last launch (step_advance).
 __global__ void decode_begin_kernel(const int* __restrict__ seq_slot, const int* __restrict__ last_token, int* __restrict__ seq_len,

@@ -165,7 +165,6 @@ __global__ void __launch_bounds__(128) moe_grouped_kernel(
   if (tile >= *n_tiles) return;
   const int e = tile_expert[tile], p0 = tile_row0[tile];
   const int rows = tile_rows[tile];
-  if (rows <= 0) return;
   const int n0 = blockIdx.y * BN;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int wm = warp >> 1, wn = warp & 1;

@@ -51,7 +51,6 @@ def core() -> ctypes.CDLL:
             lib = _load(build.build_library("core", CORE_SOURCES))
             lib.dryft_step_meta.argtypes = [_p, _p, _p, _i, _i, _p, _p, _p]
             lib.dryft_step_advance.argtypes = [_p, _p, _p, _i, _p]
-            lib.dryft_tokens_from_state.argtypes = [_p, _p, _p, _i, _p]
             lib.dryft_decode_begin.argtypes = [_p, _p, _p, _p, _p, _p, _i, _i, _p]
             lib.dryft_embed.argtypes = [_i, _p, _p, _p, _i, _i, _i, _p, _p, _p]
             lib.dryft_rmsnorm.argtypes = [_i, _p, _p, _p, _p, _p, _p, _i, _i, _f, _p]
@@ -73,7 +72,7 @@ def core() -> ctypes.CDLL:
             lib.dryft_moe_rows.argtypes = [_i, _p, _i, _p, _p, _i, _i, _i, _i, _p, _i, _p, _f, _f, _f, _p]
             lib.dryft_moe_combine.argtypes = [_i, _p, _p, _i, _i, _p, _i, _p]
             lib.dryft_moe_route_rows.argtypes = [_i, _p, _p, _p, _p, _i, _i, _i, _i, _i, _i, _i, _f, _p, _p, _p]
-            for name in ("dryft_step_meta", "dryft_step_advance", "dryft_tokens_from_state", "dryft_decode_begin", "dryft_embed",
+            for name in ("dryft_step_meta", "dryft_step_advance", "dryft_decode_begin", "dryft_embed",
                          "dryft_rmsnorm", "dryft_residual_add", "dryft_silu_mul", "dryft_qk_norm_rope_store", "dryft_rope_table",
                          "dryft_gemm_nt_f32", "dryft_argmax_rows", "dryft_sample_rows", "dryft_gemm_small_m", "dryft_row_sumsq",
                          "dryft_embed_sinusoid", "dryft_stream_norm_add", "dryft_stream_norm_rows", "dryft_kv_maps_store",
@@ -372,17 +371,9 @@ def step_advance(cu_q, seq_slot, seq_len, n_seqs: int) -> None:
     _ok(core().dryft_step_advance(_ptr(cu_q), _ptr(seq_slot), _ptr(seq_len), n_seqs, _stream()), "step_advance")
 
 
-def tokens_from_state(seq_slot, last_token, tokens, n_seqs: int) -> None:
-    for t, n in ((seq_slot, "seq_slot"), (last_token, "last_token"), (tokens, "tokens")):
-        _need(t, n, torch.int32)
-    _ok(core().dryft_tokens_from_state(_ptr(seq_slot), _ptr(last_token), _ptr(tokens), n_seqs, _stream()), "tokens_from_state")
-
-
-# ----------------------------------------------------------------------------- elementwise
 def decode_begin(seq_slot, last_token, seq_len, tokens, tok_slot, tok_pos, n_seqs: int, advance: bool = True) -> None:
-    """A decode step's tokens, slots and positions from the per-sequence state, whose lengths go up by the step's token:
-    ``tokens_from_state``, ``step_meta`` and ``step_advance`` of one token a sequence in one launch.  ``advance=False`` leaves
-    the lengths to a ``step_advance`` behind the step."""
+    """A decode step's tokens (0 for padding), slots and positions from the per-sequence state, whose lengths go up by the step's token.
+    ``advance=False`` leaves the lengths to a ``step_advance`` behind the step."""
     for t, n in ((seq_slot, "seq_slot"), (last_token, "last_token"), (seq_len, "seq_len"), (tokens, "tokens"), (tok_slot, "tok_slot"), (tok_pos, "tok_pos")):
         _need(t, n, torch.int32)
     if min(seq_slot.numel(), tokens.numel(), tok_slot.numel(), tok_pos.numel()) < n_seqs:
@@ -391,6 +382,7 @@ def decode_begin(seq_slot, last_token, seq_len, tokens, tok_slot, tok_pos, n_seq
                                   _stream()), "decode_begin")
 
 
+# ----------------------------------------------------------------------------- elementwise
 def embed(tokens, table, out, err=None, ss=None) -> None:
     """``out[n] = table[tokens[n]]``; ``ss`` (float32, 64 floats, up to 64 rows): the rows' sums of squares too."""
     _need(tokens, "tokens", torch.int32)

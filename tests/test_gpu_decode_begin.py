@@ -6,24 +6,29 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("advance", [True, False])
 @pytest.mark.parametrize("n,slots", [(1, 1), (8, 9), (64, 70), (129, 300)])
-def test_decode_begin_is_the_three_launches(n, slots):
+def test_decode_begin(n, slots, advance):
+    """Every sequence's token, slot and position; its length goes up by one, or stays for the launch behind the step."""
     from dryft_b200.ops import kernels as K
 
     gen = torch.Generator().manual_seed(n)
-    i32 = lambda t: t.to(torch.int32).cuda()
     seq_slot = torch.randperm(slots, generator=gen)[:n]
     seq_slot[n // 2::3] = -1                                # padding rows
-    seq_slot, last, lens = i32(seq_slot), i32(torch.randint(0, 1000, (slots,), generator=gen)), i32(torch.randint(0, 5000, (slots,), generator=gen))
-    want = [torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(3)]
-    got = [torch.full_like(t, -7) for t in want]
-    cu = torch.arange(n + 1, dtype=torch.int32, device="cuda")
-    lens_then = lens.clone()
-    K.tokens_from_state(seq_slot, last, want[0], n)
-    K.step_meta(cu, seq_slot, lens_then, want[1], want[2], n, n)
-    K.step_advance(cu, seq_slot, lens_then, n)
-    K.decode_begin(seq_slot, last, lens, got[0], got[1], got[2], n)
-    assert all(torch.equal(a, b) for a, b in zip(got, want)) and torch.equal(lens, lens_then)
+    last, lens = torch.randint(0, 1000, (slots,), generator=gen), torch.randint(0, 5000, (slots,), generator=gen)
+    live = seq_slot >= 0
+    want = [torch.where(live, last[seq_slot], 0), seq_slot, torch.where(live, lens[seq_slot], 0)]
+    after = lens.clone()
+    after[seq_slot[live]] += 1
+    i32 = lambda t: t.to(torch.int32).cuda()
+    d_slot, d_lens = i32(seq_slot), i32(lens)
+    got = [torch.full((n,), -7, dtype=torch.int32, device="cuda") for _ in range(3)]
+    K.decode_begin(d_slot, i32(last), d_lens, got[0], got[1], got[2], n, advance=advance)
+    assert all(torch.equal(a, i32(b)) for a, b in zip(got, want))
+    if not advance:
+        assert torch.equal(d_lens, i32(lens))
+        K.step_advance(torch.arange(n + 1, dtype=torch.int32, device="cuda"), d_slot, d_lens, n)
+    assert torch.equal(d_lens, i32(after))
 
 
 @pytest.mark.parametrize("n,hidden", [(1, 1024), (16, 2560), (64, 80), (3, 37)])
