@@ -4,8 +4,8 @@
 // and is the matrix product of the library's 32-bit path.
 //
 // One order of additions for every inner size: up to K = 256 one chain in order; beyond it k is cut into chunks of 64, a chunk is
-// accumulated in order from zero by one thread, and the chunks' sums are added in order.  So a row's result does not depend on how many other rows are
-// in the batch or on which of the kernels below ran: in the 32-bit path the same token gives bit-identical
+// accumulated in order from zero by one thread, and the chunks' sums are added in order.  So a row's result does not depend on
+// how many other rows are in the batch or on which of the kernels below ran: in the 32-bit path the same token gives bit-identical
 // projections whether it is run alone, in a prompt or in a batch.  (The order lets few rows spread k over threads, and
 // is closer to the exact sum than one chain of K additions: 1.7e-7 against 5.6e-7 at K = 1,030, 2.8e-7 against 1.8e-6 at
 // K = 9,728.)
@@ -14,7 +14,10 @@
 
 namespace {
 constexpr int CH = 64;        // k per chunk
-constexpr int ONE_CHAIN = 256;   // inner sizes up to this are one chunk (of the tiles)
+// Inner sizes up to this are one chunk, of the tiles: they keep the order of one chain, the only one that small models' sums have had.
+// That costs them closeness (K = 256: 2.9e-7 off 64 bits; chunks 1.5e-7, at every size) and few rows the kernel that streams (1 row
+// and 1,024 outputs over 64 / 128 / 256: 3.9 / 6.5 / 11.6 us; streamed 1.7 / 1.9 / 1.9; 64 rows and 4,096 outputs alike).
+constexpr int ONE_CHAIN = 256;
 constexpr int CHP = CH + 4;   // a chunk of activations in shared memory: chunks start in different banks
 
 template <int VEC> __device__ __forceinline__ void copy_async(float* dst, const float* src, bool there) {
@@ -134,7 +137,8 @@ __global__ void __launch_bounds__(128) gemm_f32_few_kernel(const float* __restri
 }
 
 template <int MT, int R, int VEC, bool XRES, int STAGES>
-int launch_few(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, int x_chunks, size_t smem, int sms, int pdl, cudaStream_t st) {
+int launch_few(const float* A, int lda, const float* W, float* C, int ldc, int M, int N, int K, int x_chunks, size_t smem, int sms, int pdl,
+               cudaStream_t st) {
   auto kern = gemm_f32_few_kernel<MT, R, VEC, XRES, STAGES>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return (int)e;
@@ -328,6 +332,7 @@ DRYFT_API int dryft_gemm_nt_f32(const float* A, int lda, const float* W, float* 
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int rows = K <= ONE_CHAIN ? 0 : few_rows(M, N, K, sms);
   if (rows)
-    return vec ? launch_few_m<4>(A, lda, W, C, ldc, M, N, K, rows, sms, pdl, st) : launch_few_m<1>(A, lda, W, C, ldc, M, N, K, rows, sms, pdl, st);
+    return vec ? launch_few_m<4>(A, lda, W, C, ldc, M, N, K, rows, sms, pdl, st)
+               : launch_few_m<1>(A, lda, W, C, ldc, M, N, K, rows, sms, pdl, st);
   return vec ? launch_tile<4>(A, lda, W, C, ldc, M, N, K, st) : launch_tile<1>(A, lda, W, C, ldc, M, N, K, st);
 }
