@@ -12,9 +12,9 @@
 //                    position-window+1 .. position (all keys from 0 if window is 0) are staged 32 at a time in shared memory
 //                    as floats (16-byte loads, several in flight per thread); a lane takes a key for the scores (softmax
 //                    running maximum and sum in 32-bit) and a slice of the latent for the weighted sum.  A step of few
-//                    tokens splits each token's keys over several blocks, joined by latent_combine.  The query's rotated part is rotated here.  Heads-major input and output:
-//                    q_lat [H, N, kv_rank] (32-bit), q [N, H, q_stride] with the rotated part at q_rot_off,
-//                    o_lat [H, N, kv_rank].
+//                    tokens splits each token's keys over several blocks, joined by latent_combine.  The query's rotated
+//                    part is rotated here.  Heads-major input and output: q_lat [H, N, kv_rank] (32-bit), q [N, H, q_stride]
+//                    with the rotated part at q_rot_off, o_lat [H, N, kv_rank].
 // head_gate          out[n, h, :] = T( o[h, n, :] * sigmoid(gate_logit[n, h]) )      (`per_value`: gate_logit[n, h * V + v], here and below)
 //
 // Rotation: pairs (2i, 2i+1) when `interleaved`, else (i, i + R/2); angle = position * inv_freq[i] (sincos_split below).
@@ -759,7 +759,11 @@ DRYFT_API int dryft_head_gate(int is_bf16, const float* o, const void* gate, int
   const size_t total = (size_t)n_tokens * H * vdim;
   const unsigned blocks = (unsigned)((total + 255) / 256);
   const bool signal = blocks <= SIGNAL_BLOCKS;
-  if (is_bf16) (signal ? head_gate_kernel<bf, true> : head_gate_kernel<bf, false>)<<<blocks, 256, 0, st>>>(o, (const bf*)gate, gate_ld, (bf*)out, n_tokens, H, vdim, per_value);
-  else (signal ? head_gate_kernel<float, true> : head_gate_kernel<float, false>)<<<blocks, 256, 0, st>>>(o, (const float*)gate, gate_ld, (float*)out, n_tokens, H, vdim, per_value);
+  if (is_bf16)
+    (signal ? head_gate_kernel<bf, true> : head_gate_kernel<bf, false>)<<<blocks, 256, 0, st>>>(o, (const bf*)gate, gate_ld, (bf*)out, n_tokens,
+                                                                                               H, vdim, per_value);
+  else
+    (signal ? head_gate_kernel<float, true> : head_gate_kernel<float, false>)<<<blocks, 256, 0, st>>>(o, (const float*)gate, gate_ld, (float*)out,
+                                                                                                     n_tokens, H, vdim, per_value);
   return launch_status();
 }

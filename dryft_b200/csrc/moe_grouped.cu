@@ -52,8 +52,9 @@ constexpr int SORT_THREADS = 1024, SORT_INTS = 12 * 1024 /* 48 KB of counters */
 
 // Warps count into `hists` tables of their own (32 while E <= 372), so that atomics on a popular expert's counter collide
 // inside a warp only, and scatter through the same tables: 16,384 assignments to 64 experts take 7.7 us where one table took 19.
-// What leaves is `place[assignment]` or, where that is null, `perm[place]`.  Rows of an expert are cut into equal tiles of up to `BM`, rounded up to 16; tiles of more than BM / 2 rows come first in the
-// list (blocks that draw their work draw the long pieces first).  `next`: the products' counters of work drawn, set to zero.
+// What leaves is `place[assignment]` or, where that is null, `perm[place]`.  Rows of an expert are cut into equal tiles of up to `BM`,
+// rounded up to 16; tiles of more than BM / 2 rows come first in the list (blocks that draw their work draw the long pieces first).
+// `next`: the products' counters of work drawn, set to zero.
 __global__ void __launch_bounds__(SORT_THREADS) moe_sort_kernel(
     const int* __restrict__ idx, int n_assign, int E, int BM, int hists, int* __restrict__ perm, int* __restrict__ place,
     int* __restrict__ tile_expert, int* __restrict__ tile_row0, int* __restrict__ tile_rows, int* __restrict__ n_tiles,

@@ -778,16 +778,18 @@ DRYFT_API int dryft_retention_chunked(int is_bf16, const void* proj, int ld, int
   states += states & 1;
   float2* const angles = reinterpret_cast<float2*>(sbuf + states);
   if (rot > 0) {
-    retention_angles_kernel<<<(unsigned)(((size_t)n_tokens * (rot / 2) + 255) / 256), 256, 0, st>>>(tok_pos, inv_freq, inv_freq_lo, angles, n_tokens, rot / 2);
+    const unsigned blocks = (unsigned)(((size_t)n_tokens * (rot / 2) + 255) / 256);
+    retention_angles_kernel<<<blocks, 256, 0, st>>>(tok_pos, inv_freq, inv_freq_lo, angles, n_tokens, rot / 2);
     rc = launch_status();
     if (rc) return rc;
   }
   dim3 grid(n_chunks, H);
   if (is_bf16)
-    retention_chunk_state_kernel<bf><<<grid, CK_THREADS, smem_a, st>>>((const bf*)proj, ld, k_off, v_off, cu_q, seq_slot, n_seqs, angles, rot, decay, sbuf, H, dim, vdim, k_scale);
+    retention_chunk_state_kernel<bf><<<grid, CK_THREADS, smem_a, st>>>((const bf*)proj, ld, k_off, v_off, cu_q, seq_slot, n_seqs, angles,
+                                                                       rot, decay, sbuf, H, dim, vdim, k_scale);
   else
-    retention_chunk_state_kernel<float><<<grid, CK_THREADS, smem_a, st>>>((const float*)proj, ld, k_off, v_off, cu_q, seq_slot, n_seqs, angles, rot, decay, sbuf, H, dim, vdim,
-                                                                          k_scale);
+    retention_chunk_state_kernel<float><<<grid, CK_THREADS, smem_a, st>>>((const float*)proj, ld, k_off, v_off, cu_q, seq_slot, n_seqs, angles,
+                                                                          rot, decay, sbuf, H, dim, vdim, k_scale);
   int e = launch_status();
   if (e) return e;
   const int per_head = dim * vdim;
@@ -796,8 +798,8 @@ DRYFT_API int dryft_retention_chunked(int is_bf16, const void* proj, int ld, int
   e = launch_status();
   if (e) return e;
   if (is_bf16)
-    retention_chunk_out_kernel<bf><<<grid, CK_THREADS, smem_c, st>>>((const bf*)proj, ld, q_off, k_off, v_off, g_off, cu_q, seq_slot, n_seqs, angles, rot, decay, sbuf, (bf*)out, H, dim,
-                                                                     vdim, k_scale, eps);
+    retention_chunk_out_kernel<bf><<<grid, CK_THREADS, smem_c, st>>>((const bf*)proj, ld, q_off, k_off, v_off, g_off, cu_q, seq_slot, n_seqs,
+                                                                     angles, rot, decay, sbuf, (bf*)out, H, dim, vdim, k_scale, eps);
   else
     retention_chunk_out_kernel<float><<<grid, CK_THREADS, smem_c, st>>>((const float*)proj, ld, q_off, k_off, v_off, g_off, cu_q, seq_slot,
                                                                         n_seqs, angles, rot, decay, sbuf,
