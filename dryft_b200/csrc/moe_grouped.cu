@@ -397,8 +397,8 @@ __device__ __forceinline__ float over_one_plus(float n, float e) {
 //   warp 1 (one thread)  tcgen05.mma, accumulators 512 columns of tensor memory: with NMAX = 128 two units' worth
 //   warps 2-9            read a unit's sums (lane = feature, column = sorted row), activation, store; neighbouring lanes swap
 //                        so that a lane stores two features of one row
-// MODE as in moe_grouped_kernel.  2,048 tokens x 8 of 64 experts of 768 x 2,048: 129 us for the first product (0.80 PFLOP/s), 79 for the
-// second, where mma.sync takes 447 and 207.
+// MODE as in moe_grouped_kernel.  2,048 tokens x 8 of 64 experts of 768 x 2,048, each alone and cold: 132 us for the first product (0.78
+// PFLOP/s), 86 for the second, where mma.sync takes 447 and 207.
 template <int MODE, int NMAX> struct Tc {
   static constexpr bool GATED = MODE == 0 || MODE == 3;
   static constexpr int FEATURES = GATED ? 128 : 256;          // output features of a unit
@@ -663,8 +663,12 @@ bool tc_takes(int E, int n_assign, int W, int F, const void* h, const void* w_ga
   return W % 64 == 0 && F % 64 == 0 && (all & 15) == 0 && !(E <= 32 && n_assign > 1024 && (long long)W * F <= 128 * 64);
 }
 
-// rows per tile: tcgen05: 256 once experts get about that many rows on average (the weights are read half as often), 128 below
-// (accumulators for two units: one is finished while the next is multiplied); mma.sync: 128 once an expert gets about a hundred
+// rows per tile: tcgen05: 128 for few rows an expert (accumulators for two units: one is finished while the next is multiplied), 256
+// once tiles of 128 would read an expert's weights twice.  Sort, gather and both products, tiles of 128 / 256, 64 experts of 768 x 2,048:
+// 112 rows an expert 136 / 152 us, 144 172 / 165, 160 183 / 172, 256 228 / 226, 512 428 / 365; 32 of 512 x 1,024: 112 rows 44 / 45,
+// 144 53 / 48, 160 53 / 50, 256 (some experts get more) 70 / 84, 512 90 / 113; 8 of 1,024 x 2,048, one wave of units either way:
+// 160 rows 48 / 56, 256 72 / 64, 384 76 / 61, 512 82 / 102.  mma.sync (535, 144 and 127 us of the three at 160
+// rows): 128 once an expert gets about a hundred
 int tile_rows_for(int n_assign, int E, bool tc) {
   if (tc) return n_assign / E >= 160 ? 256 : 128;
   return n_assign / E >= 96 ? 128 : 64;

@@ -156,7 +156,12 @@ class MoE:
     # that reading each one's weights once, which the grouped products do, spares more than their launches cost (measured:
     # 64 experts of 768 x 2,048, 8 a token: 94 us against 109 with 8 tokens, which spares 207 MB, 82 against 73 with 4 and
     # 52 MB; whole calls of such a layer: 91 against 106 with 6 and 120 MB, while assignment by assignment 5 tokens, 83 MB, take 83;
-    # 32 experts of 512 x 1,024, 4 a token: 36 against 46 with 16 tokens and 111 MB, 35 against 37 with 12 and 71 MB)
+    # 32 experts of 512 x 1,024, 4 a token: 36 against 46 with 16 tokens and 111 MB, 35 against 37 with 12 and 71 MB).  Products alone,
+    # sort and gather included, assignment by assignment / grouped: 64 experts of 768 x 2,048: 4 tokens 58 / 71 us, 6 77 / 74, 8 96 / 83,
+    # 31 297 / 112; 128 of 512 x 2,048, 8 a token: 6 tokens 58 / 71, 8 74 / 74, 12 102 / 87; 32 of 512 x 1,024: 8 tokens 25 / 32, 12
+    # 31 / 32, 16 39 / 34; 16 of 512 x 1,024, 2 a token: 16 tokens 23 / 30, 24 30 / 30, 32 37 / 30.  From 32 tokens on every size is
+    # grouped, as it was on mma.sync: experts too small to fill the launches wait for those (8 of 256 x 512, 2 a token: 32 tokens 16 / 22,
+    # on mma.sync 30; 64 tokens 27 / 22)
     GROUPED_MIN_TOKENS = 32
     GROUPED_SPARES_BYTES = 100e6
     ROUTE_ROWS_MAX = 16       # up to this many tokens the router's product and choice are one launch ...
