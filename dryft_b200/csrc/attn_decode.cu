@@ -24,6 +24,15 @@
 // (row, kv head) combines all partials in split order, so the result does not depend on arrival
 // order, and puts the ticket counter back to zero.  No block waits for another: there is no spin.
 //
+// Code.  A decode step runs five kernels in turn on every SM, whose instruction cache holds 32 KB: what a launch executes is fetched
+// anew, at about 0.05 us a kilobyte (straight-line code of 16 KB: 2,700 cycles the first time, 1,040 the second).  So loops that run once
+// or twice a launch are not unrolled, and one piece of code serves queries, keys and values: 59 KB became 40.
+//
+// A token with 40 keys, two kv heads, behind its projection's end: 7.1 us until the output product begins before, 4.4 now (one block
+// instead of a cluster of six, accumulators handed over without bank conflicts, less code); 540 keys, eight kv heads, clusters of six:
+// 8.4 us before, 6.6 now (partial sums are sent, not fetched: the loads went one after the other, 1.7 us behind the barrier, and
+// a second barrier kept the blocks from leaving).
+//
 // Formulas and rounding points are those of csrc/rope_kv.cu and csrc/attn_prefill.cu.
 #include "common.cuh"
 #include <math.h>
@@ -48,18 +57,23 @@ static_assert(G >= 1 && G <= 16, "1..16 query heads per kv head");
 static_assert(PAGE % SLICE == 0, "page size must be a multiple of 16");
 // shared memory: Q [8 or 16][KS] bf16 (rows from GROUP on zero) and the new token's K and V rows, then per warp STAGES stages of
 // (K slice, V slice) [16][KS] bf16 each.
-// The combine buffers (m, l: [NWARP][16]; acc: [NWARP][G][D] floats) overlay the stages at the end.
+// The combine buffers (m, l: [NWARP][16]; the warps' accumulators as they lie in registers, [NWARP][W][32] floats) overlay the stages at
+// the end.  Blocks of a cluster send one another partial sums into a part of their own behind the stages.
 // The block's shape is a template: NWARP warps with STAGES slices staged per warp (STAGES - 1 in flight
 // while one is used).  Few (row, kv head) pairs: wide blocks, one per SM, so that one sequence's keys
 // are walked by many warps.  Many pairs: narrow blocks with deeper rings, several per SM, so that no SM
 // waits on the one block it holds and the grid is not cut into a few coarse waves.
+constexpr int ALONE_PAGES = 256 / PAGE;      // a sequence of up to 256 keys: two slices a warp
 constexpr int PT_CACHE = 64;                // page numbers of a block kept in shared memory (more are read from global)
 constexpr int Q_ROWS = (G + 7) / 8 * 8;                     // the query heads, padded with zero rows to whole column tiles
 constexpr size_t Q_BYTES = (size_t)(Q_ROWS + 2) * KS * 2;  // then the new key and the new value
+constexpr int W = NT * MT * 4;              // accumulators of a thread
+// what a block of a cluster receives: maximum and sum of every split and head, and of every split the accumulators that it adds up
+constexpr size_t RECEIVED_BYTES = 8 * 16 * 2 * 4 + (size_t)(W + 8) * 32 * 4;
 template <int NWARP, int STAGES> struct Shape {
   static constexpr int THREADS = NWARP * 32;
   static constexpr size_t WARP_STAGE_BYTES = (size_t)STAGES * 2 * SLICE * KS * 2;
-  static constexpr size_t COMBINE_BYTES = (size_t)NWARP * 16 * 2 * 4 + (size_t)NWARP * G * D * 4 + (size_t)G * D * 4 + (size_t)G * 2 * 4;
+  static constexpr size_t COMBINE_BYTES = (size_t)NWARP * 16 * 2 * 4 + (size_t)NWARP * W * 32 * 4;
   static constexpr size_t PIPE_BYTES = NWARP * WARP_STAGE_BYTES;
   static constexpr size_t SMEM_BYTES = Q_BYTES + (PIPE_BYTES > COMBINE_BYTES ? PIPE_BYTES : COMBINE_BYTES);
 };
@@ -98,16 +112,13 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
   return *reinterpret_cast<unsigned*>(&v);
 }
 __device__ __forceinline__ float bfr(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// a float of block `rank`'s shared memory at the same offset as `local` (between two cluster barriers)
-__device__ __forceinline__ float ld_remote(const float* local, unsigned rank) {
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// a float into block `rank`'s shared memory at the same offset as `local`
+__device__ __forceinline__ void st_remote(const float* local, unsigned rank, float v) {
   unsigned raddr;
-  float v;
   asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(raddr) : "r"((unsigned)__cvta_generic_to_shared(local)), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(raddr));
-  return v;
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(raddr), "f"(v) : "memory");
 }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
@@ -138,9 +149,12 @@ __device__ __forceinline__ void rope_consts(RopeConsts& c, const float* __restri
 }
 // One warp: RMSNorm (optional) + RoPE of one head `src` [D] -> dst (bf16), with the token's constants
 // already in registers: one read of the head, one reduction, one write.  Same arithmetic as
-// qk_norm_rope_store_kernel.  `w` is only read for dims beyond the rotary part.
+// qk_norm_rope_store_kernel.  `w` is only read for dims beyond the rotary part.  The new value goes through here as it is: a copy of this
+// code for each kind of head would be fetched anew by every launch (see "Code" at the top).
+enum Kind { QUERY = 0, KEY = 1, VALUE = 2 };
 __device__ __forceinline__ void norm_rope_head(const bf16* __restrict__ src, const float* __restrict__ w, const RopeConsts& c,
-                                               bool is_q, int R, float eps, int has_norm, bf16* dst, bf16* dst2, int lane) {
+                                               int kind, int R, float eps, int has_norm, bf16* dst, bf16* dst2, int lane) {
+  if (kind == VALUE) { R = D; has_norm = 0; }
   const int half = R >> 1;
   float a[MAXJ], b[MAXJ];
   float ss = 0.f;
@@ -156,6 +170,7 @@ __device__ __forceinline__ void norm_rope_head(const bf16* __restrict__ src, con
   }
   float inv = 1.f;
   if (has_norm) {
+#pragma unroll 1
     for (int i = R + lane; i < D; i += 32) {
       const float v = ld_prev_bf16(src + i);
       ss += v * v;
@@ -169,16 +184,21 @@ __device__ __forceinline__ void norm_rope_head(const bf16* __restrict__ src, con
     if (j < half) {
       float x = a[jj], y = b[jj];
       if (has_norm) {
-        x = bfr(bfr(x * inv) * (is_q ? c.wq_a[jj] : c.wk_a[jj]));
-        y = bfr(bfr(y * inv) * (is_q ? c.wq_b[jj] : c.wk_b[jj]));
+        x = bfr(bfr(x * inv) * (kind == QUERY ? c.wq_a[jj] : c.wk_a[jj]));
+        y = bfr(bfr(y * inv) * (kind == QUERY ? c.wq_b[jj] : c.wk_b[jj]));
       }
-      const bf16 o1 = __float2bfloat16_rn(__fadd_rn(bfr(__fmul_rn(x, c.cs[jj])), -bfr(__fmul_rn(y, c.sn[jj]))));
-      const bf16 o2 = __float2bfloat16_rn(__fadd_rn(bfr(__fmul_rn(y, c.cs[jj])), bfr(__fmul_rn(x, c.sn[jj]))));
+      if (kind != VALUE) {
+        const float u = __fadd_rn(bfr(__fmul_rn(x, c.cs[jj])), -bfr(__fmul_rn(y, c.sn[jj])));
+        y = __fadd_rn(bfr(__fmul_rn(y, c.cs[jj])), bfr(__fmul_rn(x, c.sn[jj])));
+        x = u;
+      }
+      const bf16 o1 = __float2bfloat16_rn(x), o2 = __float2bfloat16_rn(y);
       dst[j] = o1;
       dst[j + half] = o2;
       if (dst2) { dst2[j] = o1; dst2[j + half] = o2; }
     }
   }
+#pragma unroll 1
   for (int i = R + lane; i < D; i += 32) {
     float x = ld_prev_bf16(src + i);
     if (has_norm) x = bfr(bfr(x * inv) * w[i]);
@@ -223,12 +243,17 @@ __global__ void __launch_bounds__(NWARP * 32) attn_decode_kernel(const Params p)
   const int kv_lo = p.window > 0 ? max(0, kv_hi - p.window) : 0;
   const int first_page = kv_lo / PAGE, last_page = pos / PAGE;
   const int n_pages = last_page - first_page + 1;
-  const int per_split = (n_pages + p.n_splits - 1) / p.n_splits;
+  // A cluster's first block takes a short sequence alone: a few more slices a warp cost less than partial sums sent around.
+  const bool alone = p.cluster && n_pages <= ALONE_PAGES;
+  const int per_split = alone ? n_pages : (n_pages + p.n_splits - 1) / p.n_splits;
   const int pg_begin = first_page + split * per_split;
   const int pg_end = min(pg_begin + per_split, last_page + 1);
   const int* pt = p.page_table + (size_t)(slot < 0 ? 0 : slot) * p.max_pages;
+  if (alone && split > 0) return;      // (every block of the cluster knows, and none waits for another then)
+  if (p.cluster && !alone) cluster_arrive();      // shared memory may be written from outside once every block has begun
   __shared__ int pt_s[PT_CACHE];
   if (slot >= 0)
+#pragma unroll 1
     for (int i = tid; i < min(pg_end - pg_begin, PT_CACHE); i += THREADS) pt_s[i] = pt[pg_begin + i];
   RopeConsts rc;
   if (slot >= 0) rope_consts(rc, p.wq, p.wk, p.inv_freq, pos, p.R, p.has_norm, lane);
@@ -267,47 +292,37 @@ __global__ void __launch_bounds__(NWARP * 32) attn_decode_kernel(const Params p)
   };
   // a layer that reads another layer's cache must see that layer's write of this step's token first
   const bool early = slot >= 0 && p.write_kv;
-  if (early) {
-#pragma unroll
+  if (!early) pdl_wait();
+  if (slot >= 0) {
+#pragma unroll 1
     for (int i = 0; i < STAGES - 1; ++i) request(sl_begin + warp + i * NWARP, i);
   }
-
-  pdl_wait();  // the projection that made qkv is complete
+  if (early) pdl_wait();  // the projection that made qkv is complete
   if (slot < 0) {  // padding row: defined zeros (written by split 0), no cache access, no ticket
+    if (p.cluster && !alone) cluster_wait();
     if (split == 0)
+#pragma unroll 1
       for (int i = tid; i < G * D; i += THREADS) p.out[(size_t)n * nH * D + (size_t)kvh * G * D + i] = __float2bfloat16_rn(0.f);
     return;
   }
   const bf16* row = p.qkv + (size_t)n * p.qkv_stride;
 
-  if (!early) {
-#pragma unroll
-    for (int i = 0; i < STAGES - 1; ++i) request(sl_begin + warp + i * NWARP, i);
-  }
-
   // ---- the row's queries; and, in the block that owns the last page, the new key and value ----
   bf16* new_k = qs + Q_ROWS * KS;
   bf16* new_v = new_k + KS;
+#pragma unroll 1
   for (int i = tid; i < (Q_ROWS - G) * (D / 8); i += THREADS)  // zero the padding rows of Q
     *reinterpret_cast<uint4*>(qs + (G + i / (D / 8)) * KS + (i % (D / 8)) * 8) = make_uint4(0, 0, 0, 0);
   const bool owns_new = p.write_kv && last_page >= pg_begin && last_page < pg_end;
   const int n_items = G + (owns_new ? 2 : 0);
+#pragma unroll 1
   for (int item = warp; item < n_items; item += NWARP) {
-    if (item < G) {
-      norm_rope_head(row + (size_t)(kvh * G + item) * D, p.wq, rc, true, p.R, p.eps, p.has_norm, qs + item * KS, nullptr, lane);
-    } else {
-      const size_t off = (((size_t)page_of(last_page) * p.nKV + kvh) * PAGE + (pos % PAGE)) * D;
-      if (item == G) {
-        norm_rope_head(row + (size_t)(nH + kvh) * D, p.wk, rc, false, p.R, p.eps, p.has_norm, p.k_pages + off, new_k, lane);
-      } else {
-        const bf16* vsrc = row + (size_t)(nH + p.nKV + kvh) * D;
-        for (int i = lane; i < D; i += 32) {
-          const bf16 v = __ushort_as_bfloat16(ld_prev(reinterpret_cast<const unsigned short*>(vsrc) + i));   // written by the projection before this launch
-          p.v_pages[off + i] = v;
-          new_v[i] = v;
-        }
-      }
-    }
+    const int kind = item < G ? QUERY : item == G ? KEY : VALUE;
+    const int head = kind == QUERY ? kvh * G + item : kind == KEY ? nH + kvh : nH + p.nKV + kvh;
+    bf16* cached = nullptr;
+    if (kind != QUERY) cached = (kind == KEY ? p.k_pages : p.v_pages) + (((size_t)page_of(last_page) * p.nKV + kvh) * PAGE + (pos % PAGE)) * D;
+    norm_rope_head(row + (size_t)head * D, kind == QUERY ? p.wq : p.wk, rc, kind, p.R, p.eps, p.has_norm,
+                   kind == QUERY ? qs + item * KS : kind == KEY ? new_k : new_v, cached, lane);
   }
   __syncthreads();  // queries (and the new key and value) are in shared memory
 
@@ -349,6 +364,7 @@ __global__ void __launch_bounds__(NWARP * 32) attn_decode_kernel(const Params p)
     if (sl == pos / SLICE) {
       const int r = pos % SLICE;
       if (owns_new) {  // the staged copy of the token's own row may predate its write
+#pragma unroll 1
         for (int i = lane; i < CPR; i += 32) {
           *reinterpret_cast<uint4*>(kst + r * KS + i * 8) = *reinterpret_cast<const uint4*>(new_k + i * 8);
           *reinterpret_cast<uint4*>(vst + r * KS + i * 8) = *reinterpret_cast<const uint4*>(new_v + i * 8);
@@ -357,6 +373,7 @@ __global__ void __launch_bounds__(NWARP * 32) attn_decode_kernel(const Params p)
       // The rows behind the token's own hold what the page's last holder left.  Their keys are masked below
       // (probability exactly zero), but 0 * v is only 0 for a finite v: the staged values are zeroed
       // (the reference zeroes its whole cache once for the same reason, engine/dryft_qwen3/cache.py:43-47).
+#pragma unroll 1
       for (int i = lane; i < (SLICE - 1 - r) * CPR; i += 32)
         *reinterpret_cast<uint4*>(vst + (r + 1 + i / CPR) * KS + (i % CPR) * 8) = make_uint4(0, 0, 0, 0);
       __syncwarp();
@@ -440,79 +457,123 @@ __global__ void __launch_bounds__(NWARP * 32) attn_decode_kernel(const Params p)
   __syncthreads();  // every warp is done with its stages: they become the combine buffers
 
   // ---- combine the warps of this block ----
+  // Only the first `busy` warps had slices.  Accumulators are handed over as they lie in registers: word i of a thread is, of column tile
+  // i / (4 MT), dim tile i / 4 mod MT, head 2t + (i & 1) and dim g + 8 (i / 2 & 1).
   float* wm = reinterpret_cast<float*>(pipe);          // [NWARP][16]
   float* wl = wm + NWARP * 16;                         // [NWARP][16]
-  float* wacc = wl + NWARP * 16;                       // [NWARP][G][D]
+  float* wacc = wl + NWARP * 16;                       // [NWARP][W][32]
+  const int busy = max(0, min(NWARP, sl_end - sl_begin));
+  if (warp < busy) {
 #pragma unroll
-  for (int nt = 0; nt < NT; ++nt) {
-    float l0 = l_run[nt][0], l1 = l_run[nt][1];
+    for (int nt = 0; nt < NT; ++nt) {
+      float l0 = l_run[nt][0], l1 = l_run[nt][1];
 #pragma unroll
-    for (int o = 4; o < 32; o <<= 1) {
-      l0 += __shfl_xor_sync(0xffffffffu, l0, o);
-      l1 += __shfl_xor_sync(0xffffffffu, l1, o);
-    }
-    const int h0 = nt * 8 + 2 * t;
-    if (g == 0) {
-      wm[warp * 16 + h0] = m_run[nt][0]; wl[warp * 16 + h0] = l0;
-      wm[warp * 16 + h0 + 1] = m_run[nt][1]; wl[warp * 16 + h0 + 1] = l1;
-    }
+      for (int o = 4; o < 32; o <<= 1) {
+        l0 += __shfl_xor_sync(0xffffffffu, l0, o);
+        l1 += __shfl_xor_sync(0xffffffffu, l1, o);
+      }
+      const int h0 = nt * 8 + 2 * t;
+      if (g == 0) {
+        *reinterpret_cast<float2*>(wm + warp * 16 + h0) = make_float2(m_run[nt][0], m_run[nt][1]);
+        *reinterpret_cast<float2*>(wl + warp * 16 + h0) = make_float2(l0, l1);
+      }
+      if (h0 < G) {
 #pragma unroll
-    for (int j = 0; j < MT; ++j) {
-      const int d = j * 16 + g;
-      if (h0 < G) { wacc[(warp * G + h0) * D + d] = o_acc[nt][j][0]; wacc[(warp * G + h0) * D + d + 8] = o_acc[nt][j][2]; }
-      if (h0 + 1 < G) { wacc[(warp * G + h0 + 1) * D + d] = o_acc[nt][j][1]; wacc[(warp * G + h0 + 1) * D + d + 8] = o_acc[nt][j][3]; }
+        for (int j = 0; j < MT; ++j)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) wacc[(warp * W + (nt * MT + j) * 4 + i) * 32 + lane] = o_acc[nt][j][i];
+      }
     }
   }
   __syncthreads();
-  float* bp_num = wacc + NWARP * G * D;   // [G][D] this block's partial (cluster mode)
-  float* bp_ml = bp_num + G * D;          // [G][2] its maximum and sum
-  const size_t pidx = ((size_t)n * p.nKV + kvh) * p.n_splits + split;
-  for (int i = tid; i < G * D; i += THREADS) {
-    const int h = i / D, d = i % D;
-    float mx = -INFINITY;
+  // a warp adds pairs of words (two heads) of one column tile: pair `first`, and each TEAM-th behind it
+  constexpr int TEAM = NWARP / NT, PER = 2 * ((2 * MT + TEAM - 1) / TEAM);
+  static_assert(NWARP % NT == 0, "as many warps for every column tile");
+  const int tile = warp / TEAM, first = warp % TEAM, h0 = tile * 8 + 2 * t;
+  auto word = [&](int i) { return (tile * MT * 2 + first + (i >> 1) * TEAM) * 2 + (i & 1); };
+  auto mine = [&](int i) { return first + (i >> 1) * TEAM < 2 * MT && h0 + (i & 1) < G; };
+  float num[PER], mx[2] = {-INFINITY, -INFINITY}, den[2] = {0.f, 0.f};
 #pragma unroll
-    for (int w = 0; w < NWARP; ++w) mx = fmaxf(mx, wm[w * 16 + h]);
-    float num = 0.f, den = 0.f;
-#pragma unroll
-    for (int w = 0; w < NWARP; ++w) {
-      const float m = wm[w * 16 + h];
-      if (m == -INFINITY) continue;
-      const float sc = exp2f(m - mx);
-      num += sc * wacc[(w * G + h) * D + d];
-      den += sc * wl[w * 16 + h];
+  for (int i = 0; i < PER; ++i) num[i] = 0.f;
+  if (h0 < G) {
+#pragma unroll 1
+    for (int w = 0; w < busy; ++w) {
+      const float2 m = *reinterpret_cast<const float2*>(wm + w * 16 + h0);
+      mx[0] = fmaxf(mx[0], m.x);
+      mx[1] = fmaxf(mx[1], m.y);
     }
-    if (p.n_splits == 1) {
-      p.out[((size_t)n * nH + kvh * G + h) * D + d] = __float2bfloat16_rn(den > 0.f ? num / den : 0.f);
-    } else if (p.cluster) {
-      bp_num[i] = num;  // relative to mx
-      if (d == 0) { bp_ml[h * 2] = mx; bp_ml[h * 2 + 1] = den; }
-    } else {
-      p.part_o[(pidx * G + h) * D + d] = num;  // relative to mx
-      if (d == 0) { p.part_ml[(pidx * G + h) * 2] = mx; p.part_ml[(pidx * G + h) * 2 + 1] = den; }
+#pragma unroll 2
+    for (int w = 0; w < busy; ++w) {
+      const float2 m = *reinterpret_cast<const float2*>(wm + w * 16 + h0), l = *reinterpret_cast<const float2*>(wl + w * 16 + h0);
+      const float s0 = m.x == -INFINITY ? 0.f : exp2f(m.x - mx[0]), s1 = m.y == -INFINITY ? 0.f : exp2f(m.y - mx[1]);
+      den[0] += s0 * l.x;
+      den[1] += s1 * l.y;
+#pragma unroll
+      for (int i = 0; i < PER; ++i)
+        if (first + (i >> 1) * TEAM < 2 * MT) num[i] += (i & 1 ? s1 : s0) * wacc[(w * W + word(i)) * 32 + lane];
     }
   }
-  if (p.n_splits == 1) return;
-  if (p.cluster) {
-    // ---- the splits are the blocks of one cluster: every block combines a slice of the outputs over
-    // all blocks' partials, in split order, reading them through distributed shared memory ----
-    cluster_sync_all();
-    const int per = (G * D + p.n_splits - 1) / p.n_splits;
-    for (int i = split * per + tid; i < min((split + 1) * per, G * D); i += THREADS) {
-      const int h = i / D, d = i % D;
-      float mx = -INFINITY;
-      for (int s2 = 0; s2 < p.n_splits; ++s2) mx = fmaxf(mx, ld_remote(bp_ml + h * 2, (unsigned)s2));
-      float num = 0.f, den = 0.f;
-      for (int s2 = 0; s2 < p.n_splits; ++s2) {
-        const float m = ld_remote(bp_ml + h * 2, (unsigned)s2);
-        if (m == -INFINITY) continue;
-        const float sc = exp2f(m - mx);
-        num += sc * ld_remote(bp_num + i, (unsigned)s2);
-        den += sc * ld_remote(bp_ml + h * 2 + 1, (unsigned)s2);
-      }
-      p.out[((size_t)n * nH + kvh * G + h) * D + d] = __float2bfloat16_rn(den > 0.f ? num / den : 0.f);
-    }
-    cluster_sync_all();   // nobody leaves while another block may still read its partial
+  auto place = [&](int i) {   // where word i of the row goes, from the start of this kv head's heads
+    return (i / (MT * 4) * 8 + 2 * t + (i & 1)) * D + (i / 4 % MT) * 16 + g + (i >> 1 & 1) * 8;
+  };
+  bf16* out_row = p.out + ((size_t)n * nH + (size_t)kvh * G) * D;
+  if (p.n_splits == 1 || alone) {
+#pragma unroll
+    for (int i = 0; i < PER; ++i)
+      if (mine(i)) out_row[place(word(i))] = __float2bfloat16_rn(den[i & 1] > 0.f ? num[i] / den[i & 1] : 0.f);
     return;
+  }
+  if (p.cluster) {
+    // ---- the splits are the blocks of one cluster: block r adds up words r * share and on over all splits, in split order.  Every block
+    // sends each other block its words and its maxima and sums; one barrier behind the sending, none behind the reading. ----
+    float* got_ml = reinterpret_cast<float*>(smem + Shape<NWARP, STAGES>::SMEM_BYTES);   // [split][16 heads][2]
+    float* got = got_ml + 8 * 16 * 2;                                                    // [split][share][32]
+    const int share = (W + p.n_splits - 1) / p.n_splits;
+    cluster_wait();      // every block has begun
+    if (h0 < G) {
+#pragma unroll
+      for (int i = 0; i < PER; ++i)
+        if (mine(i)) {
+          const int to = word(i) / share;
+          st_remote(got + (split * share + word(i) - to * share) * 32 + lane, (unsigned)to, num[i]);
+        }
+      if (first == 0 && g < p.n_splits) {      // one warp a column tile; thread g of a head pair tells block g
+        st_remote(got_ml + (split * 16 + h0) * 2, (unsigned)g, mx[0]);
+        st_remote(got_ml + (split * 16 + h0) * 2 + 1, (unsigned)g, den[0]);
+        st_remote(got_ml + (split * 16 + h0 + 1) * 2, (unsigned)g, mx[1]);
+        st_remote(got_ml + (split * 16 + h0 + 1) * 2 + 1, (unsigned)g, den[1]);
+      }
+    }
+    cluster_arrive();
+    cluster_wait();
+#pragma unroll 1
+    for (int i = split * share + warp; i < min((split + 1) * share, W); i += NWARP) {
+      const int h = i / (MT * 4) * 8 + 2 * t + (i & 1);
+      if (h >= G) continue;
+      float top = -INFINITY, sum = 0.f, all = 0.f;
+#pragma unroll 2
+      for (int s2 = 0; s2 < p.n_splits; ++s2) top = fmaxf(top, got_ml[(s2 * 16 + h) * 2]);
+#pragma unroll 2
+      for (int s2 = 0; s2 < p.n_splits; ++s2) {
+        const float m = got_ml[(s2 * 16 + h) * 2], sc = m == -INFINITY ? 0.f : exp2f(m - top);
+        sum += sc * got[(s2 * share + i - split * share) * 32 + lane];
+        all += sc * got_ml[(s2 * 16 + h) * 2 + 1];
+      }
+      out_row[place(i)] = __float2bfloat16_rn(all > 0.f ? sum / all : 0.f);
+    }
+    return;
+  }
+  const size_t pidx = ((size_t)n * p.nKV + kvh) * p.n_splits + split;
+#pragma unroll
+  for (int i = 0; i < PER; ++i)
+    if (mine(i)) p.part_o[pidx * G * D + place(word(i))] = num[i];      // relative to mx
+  if (first == 0 && g == 0) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      if (h0 + i < G) {
+        p.part_ml[(pidx * G + h0 + i) * 2] = mx[i];
+        p.part_ml[(pidx * G + h0 + i) * 2 + 1] = den[i];
+      }
   }
 
   // ---- the block that draws the last ticket combines all splits, in split order ----
@@ -532,6 +593,7 @@ __global__ void __launch_bounds__(NWARP * 32) attn_decode_kernel(const Params p)
   float* cl = cm + p.n_splits * G;                   // [S][G] sums
   float* cw = cl + p.n_splits * G;                   // [S][G] weights exp2(m - max) / total
   __syncthreads();
+#pragma unroll 2
   for (int i = tid; i < p.n_splits * G; i += THREADS) {
     cm[i] = __ldcg(&p.part_ml[(pbase * G + i) * 2]);
     cl[i] = __ldcg(&p.part_ml[(pbase * G + i) * 2 + 1]);
@@ -539,8 +601,10 @@ __global__ void __launch_bounds__(NWARP * 32) attn_decode_kernel(const Params p)
   __syncthreads();
   if (tid < G) {
     float mx = -INFINITY;
+#pragma unroll 1
     for (int s2 = 0; s2 < p.n_splits; ++s2) mx = fmaxf(mx, cm[s2 * G + tid]);
     float den = 0.f;
+#pragma unroll 1
     for (int s2 = 0; s2 < p.n_splits; ++s2) {
       const float m = cm[s2 * G + tid];
       const float sc = m == -INFINITY ? 0.f : exp2f(m - mx);  // maxima are kept in log2 units
@@ -548,9 +612,11 @@ __global__ void __launch_bounds__(NWARP * 32) attn_decode_kernel(const Params p)
       den += sc * cl[s2 * G + tid];
     }
     const float inv = den > 0.f ? 1.f / den : 0.f;
+#pragma unroll 1
     for (int s2 = 0; s2 < p.n_splits; ++s2) cw[s2 * G + tid] *= inv;
   }
   __syncthreads();
+#pragma unroll 1
   for (int i = tid; i < G * D; i += THREADS) {
     const int h = i / D, d = i % D;
     float num = 0.f;
@@ -563,17 +629,17 @@ __global__ void __launch_bounds__(NWARP * 32) attn_decode_kernel(const Params p)
 template <int NWARP, int STAGES>
 static int launch_shape(const Params& p, int n_rows, int nKV, int n_splits, int pdl, cudaStream_t st) {
   typedef Shape<NWARP, STAGES> S;
-  if (S::SMEM_BYTES > 227 * 1024) return DRYFT_ERR_UNSUPPORTED;
+  if (S::SMEM_BYTES + RECEIVED_BYTES > 227 * 1024) return DRYFT_ERR_UNSUPPORTED;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(n_rows, nKV, n_splits);
   cfg.blockDim = dim3(S::THREADS);
   static bool attr_set = false;  // per shape; set by the first (eager) launch, outside any stream capture
-  if (S::SMEM_BYTES > 48 * 1024 && !attr_set) {
-    cudaError_t ea = cudaFuncSetAttribute(attn_decode_kernel<NWARP, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM_BYTES);
+  if (S::SMEM_BYTES + RECEIVED_BYTES > 48 * 1024 && !attr_set) {
+    cudaError_t ea = cudaFuncSetAttribute(attn_decode_kernel<NWARP, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(S::SMEM_BYTES + RECEIVED_BYTES));
     if (ea != cudaSuccess) return (int)ea;
     attr_set = true;
   }
-  cfg.dynamicSmemBytes = S::SMEM_BYTES;
+  cfg.dynamicSmemBytes = S::SMEM_BYTES + (p.cluster ? RECEIVED_BYTES : 0);
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   int n_attr = 0;
