@@ -3,13 +3,17 @@
 // position).  Compiled per model with -DDRYFT_HEAD_DIM, -DDRYFT_GROUP, -DDRYFT_PAGE.
 //
 // Grid (rows, kv heads, splits).  One block serves the GROUP query heads that share a kv head for
-// one query row over one contiguous range of cache pages.  Row n at position p of slot s sees the
+// one query row over one contiguous range of keys.  Row n at position p of slot s sees the
 // keys j with  max(0, p+1-window) <= j <= p  (window <= 0: all keys) — the new token's own key is
 // already in the cache (hari495/dryft, engine/dryft_qwen3/model.py:235,249-257;
 // kernels/attn_decode.py:8-10,52-55).  Scores, the running maximum and the sums are 32-bit
 // (attn_decode.py:77-90).  With one split the block writes the output; otherwise it writes an
 // un-normalised partial (acc, m, l) and `attn_rows_reduce_kernel` combines them
 // (attn_decode.py:102-118).
+//
+// A split is a multiple of 16 keys, not of pages: a block takes 10 us for the 64 keys of a page (32-bit, two trips to memory, scores and
+// values of 64 keys by 128 threads), and while rows are few most blocks of a launch would have none.  Four rows of about 150 keys, two kv
+// heads, 32 splits: 11 + 5.5 us for the two launches by pages, 6.0 + 4.3 by 16 keys.
 //
 // No block waits on another block; there is no spin anywhere in this file.
 #include "common.cuh"
@@ -24,6 +28,7 @@ namespace {
 constexpr int D = DRYFT_HEAD_DIM;
 constexpr int G = DRYFT_GROUP;
 constexpr int PAGE = DRYFT_PAGE;
+constexpr int GRAIN = 16;
 constexpr int THREADS = 128;
 constexpr int NWARP = THREADS / 32;
 constexpr int DIMS_PER_THREAD = (D + THREADS - 1) / THREADS;
@@ -79,11 +84,18 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
   const int pos = tok_pos[n];
   const int kv_hi = pos + 1;                                        // exclusive
   const int kv_lo = window > 0 ? max(0, kv_hi - window) : 0;        // inclusive
-  const int first_page = kv_lo / PAGE, last_page = (kv_hi - 1) / PAGE;
-  const int n_pages = last_page - first_page + 1;
-  const int per_split = (n_pages + n_splits - 1) / n_splits;
-  const int pg_begin = first_page + split * per_split;
-  const int pg_end = min(pg_begin + per_split, last_page + 1);
+  const int base = kv_lo / GRAIN * GRAIN, grains = (kv_hi - base + GRAIN - 1) / GRAIN;
+  const int per_split = (grains + n_splits - 1) / n_splits;
+  const int k_begin = max(kv_lo, (int)min((long long)base + (long long)split * per_split * GRAIN, (long long)kv_hi));      // this block's keys
+  const int k_end = (int)min((long long)base + (long long)(split + 1) * per_split * GRAIN, (long long)kv_hi);
+  if (n_splits > 1 && k_begin >= k_end) {      // nothing to add: a maximum of -inf says so
+    if (tid < G) {
+      const size_t pi = ((size_t)n * nH + kvh * G + tid) * n_splits + split;
+      part_ml[pi * 2] = -INFINITY;
+      part_ml[pi * 2 + 1] = 0.f;
+    }
+    return;
+  }
 
   for (int i = tid; i < G * D; i += THREADS) qs[i] = to_f32<T>(q[((size_t)n * nH + (size_t)kvh * G) * D + i]);
   if (tid < G) { m_s[tid] = -INFINITY; l_s[tid] = 0.f; a_s[tid] = 1.f; }
@@ -95,21 +107,21 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
 
   const int* pt = page_table + (size_t)slot * max_pages;
   constexpr int VPR = D / L::VEC;  // 16-byte vectors per row
-  for (int pg = pg_begin; pg < pg_end; ++pg) {
+  for (int pg = k_begin / PAGE; pg * PAGE < k_end; ++pg) {
     const int page = pt[pg];
     const int p0 = pg * PAGE;
+    const int r0 = max(k_begin - p0, 0), r1 = min(k_end - p0, PAGE), rows = r1 - r0;      // of the page
     const T* kp = k_pages + ((size_t)page * nKV + kvh) * PAGE * D;
     const T* vp = v_pages + ((size_t)page * nKV + kvh) * PAGE * D;
     __syncthreads();  // previous tile fully consumed
     // eight words of K and of V on their way at once (two at a time left a page eight trips to memory long)
     constexpr int AHEAD = 8;
-    for (int i0 = tid; i0 < PAGE * VPR; i0 += AHEAD * THREADS) {
+    for (int i0 = r0 * VPR + tid; i0 < r1 * VPR; i0 += AHEAD * THREADS) {
       uint4 kv4[AHEAD], vv4[AHEAD];
 #pragma unroll
       for (int u = 0; u < AHEAD; ++u) {
-        const int i = i0 + u * THREADS, r = i / VPR, c = i % VPR, p = p0 + r;
-        kv4[u] = vv4[u] = make_uint4(0, 0, 0, 0);
-        if (i < PAGE * VPR && p >= kv_lo && p < kv_hi) {
+        const int i = i0 + u * THREADS, r = i / VPR, c = i % VPR;
+        if (i < r1 * VPR) {
           kv4[u] = reinterpret_cast<const uint4*>(kp + (size_t)r * D)[c];
           vv4[u] = reinterpret_cast<const uint4*>(vp + (size_t)r * D)[c];
         }
@@ -117,24 +129,24 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
 #pragma unroll
       for (int u = 0; u < AHEAD; ++u) {
         const int i = i0 + u * THREADS, r = i / VPR, c = i % VPR;
-        if (i < PAGE * VPR) {
+        if (i < r1 * VPR) {
           *reinterpret_cast<uint4*>(kt + r * L::KSTRIDE + c * L::VEC) = kv4[u];
           *reinterpret_cast<uint4*>(vt + r * D + c * L::VEC) = vv4[u];
         }
       }
     }
     __syncthreads();
-    // scores: item -> (head g, key r); consecutive threads take consecutive keys
-    for (int item = tid; item < G * PAGE; item += THREADS) {
-      const int g = item / PAGE, r = item % PAGE;
-      const int p = p0 + r;
-      float s = -INFINITY;
-      if (p >= kv_lo && p < kv_hi) {
+    // scores: item -> (head g, key r); consecutive threads take consecutive keys, or two or four threads one key where the items are few
+    const int items = G * rows, share = 4 * items <= THREADS ? 4 : 2 * items <= THREADS ? 2 : 1;
+    for (int i0 = 0; i0 < items * share; i0 += THREADS) {
+      const int item = (i0 + tid) / share, sub = tid % share;
+      const int g = item / rows, r = r0 + item - g * rows;
+      float dot[4] = {0.f, 0.f, 0.f, 0.f};      // four chains of D / 4: one of D waits for every addition
+      if (item < items) {
         const T* kr = kt + r * L::KSTRIDE;
         const float* qg = qs + g * D;
-        float dot[4] = {0.f, 0.f, 0.f, 0.f};      // four chains of D / 4: one of D waits for every addition
 #pragma unroll 4
-        for (int c = 0; c < VPR; ++c) {
+        for (int c = sub; c < VPR; c += share) {
           uint4 raw = *reinterpret_cast<const uint4*>(kr + c * L::VEC);
           const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
@@ -146,20 +158,21 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
             dot[3] = fmaf(q4.w, to_f32<T>(e[t + 3]), dot[3]);
           }
         }
-        s = ((dot[0] + dot[1]) + (dot[2] + dot[3])) * scale;
       }
-      sc[item] = s;
+      float s = (dot[0] + dot[1]) + (dot[2] + dot[3]);
+      for (int o = 1; o < share; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (item < items && sub == 0) sc[g * PAGE + r] = s * scale;
     }
     __syncthreads();
     // online softmax, one warp per head
     for (int g = warp; g < G; g += NWARP) {
       float mx = -INFINITY;
-      for (int r = lane; r < PAGE; r += 32) mx = fmaxf(mx, sc[g * PAGE + r]);
+      for (int r = r0 + lane; r < r1; r += 32) mx = fmaxf(mx, sc[g * PAGE + r]);
       mx = warp_max(mx);
       const float m_old = m_s[g];
       const float m_new = fmaxf(m_old, mx);
       float sum = 0.f;
-      for (int r = lane; r < PAGE; r += 32) {
+      for (int r = r0 + lane; r < r1; r += 32) {
         const float s = sc[g * PAGE + r];
         const float p = (s == -INFINITY) ? 0.f : expf(s - m_new);
         sc[g * PAGE + r] = p;
@@ -181,7 +194,8 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
       if (d < D) {
 #pragma unroll
         for (int g = 0; g < G; ++g) acc[i][g] *= a_s[g];
-        for (int r = 0; r < PAGE; ++r) {
+#pragma unroll 8
+        for (int r = r0; r < r1; ++r) {
           const float v = to_f32<T>(vt[r * D + d]);
 #pragma unroll
           for (int g = 0; g < G; ++g) acc[i][g] = fmaf(sc[g * PAGE + r], v, acc[i][g]);
@@ -212,27 +226,60 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
   }
 }
 
-// Combine the partials of one (row, head):  w_s = exp(m_s - max m);  o = sum w_s acc_s / sum w_s l_s.
+// Combine the partials of one (row, head):  w_s = exp(m_s - max m);  o = sum w_s acc_s / sum w_s l_s, in the order of the splits.  A thread
+// makes the weights of some splits, all of them share them; several splits' values are on their way together.
+constexpr int REDUCE_TILE = 128;
 template <typename T>
-__global__ void attn_rows_reduce_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                        T* __restrict__ out, int n_splits) {
+__global__ void __launch_bounds__(128) attn_rows_reduce_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+                                                               T* __restrict__ out, int n_splits) {
   let_next_launch_in();   // a product behind this launch may start on its weights
+  __shared__ float wgt[REDUCE_TILE], sum[REDUCE_TILE], top[4];
   const size_t rh = blockIdx.x;  // row * nH + head
   const float* ml = part_ml + rh * n_splits * 2;
+  const int tid = threadIdx.x;
   float mx = -INFINITY;
-  for (int s = 0; s < n_splits; ++s) mx = fmaxf(mx, ml[s * 2]);
-  float denom = 0.f;
-  for (int s = 0; s < n_splits; ++s) {
-    const float m = ml[s * 2];
-    if (m != -INFINITY) denom += expf(m - mx) * ml[s * 2 + 1];
-  }
-  for (int d = threadIdx.x; d < D; d += blockDim.x) {
-    float num = 0.f;
-    for (int s = 0; s < n_splits; ++s) {
-      const float m = ml[s * 2];
-      if (m != -INFINITY) num += expf(m - mx) * part_o[(rh * n_splits + s) * D + d];
+  for (int s = tid; s < n_splits; s += blockDim.x) mx = fmaxf(mx, ml[s * 2]);
+  mx = warp_max(mx);
+  if (tid % 32 == 0) top[tid / 32] = mx;
+  __syncthreads();
+  mx = top[0];
+  for (int w = 1; w < (int)blockDim.x / 32; ++w) mx = fmaxf(mx, top[w]);
+  constexpr int MINE = (D + 63) / 64;      // dims a thread (64 or 128 threads)
+  float num[MINE], denom = 0.f;
+#pragma unroll
+  for (int i = 0; i < MINE; ++i) num[i] = 0.f;
+  for (int s0 = 0; s0 < n_splits; s0 += REDUCE_TILE) {
+    const int n = min(REDUCE_TILE, n_splits - s0);
+    for (int s = tid; s < n; s += blockDim.x) {
+      const float m = ml[(s0 + s) * 2];
+      wgt[s] = m == -INFINITY ? -1.f : expf(m - mx);      // -1: an empty split, which wrote no values
+      sum[s] = ml[(s0 + s) * 2 + 1];
     }
-    out[rh * D + d] = from_f32<T>(denom > 0.f ? num / denom : 0.f);
+    __syncthreads();
+    constexpr int AT_ONCE = 16 / MINE;
+    for (int q = 0; q < n; q += AT_ONCE) {
+      float v[AT_ONCE][MINE];
+#pragma unroll
+      for (int u = 0; u < AT_ONCE; ++u)
+#pragma unroll
+        for (int i = 0; i < MINE; ++i) {
+          const int d = tid + i * (int)blockDim.x;
+          v[u][i] = q + u < n && d < D ? part_o[(rh * n_splits + s0 + q + u) * D + d] : 0.f;
+        }
+#pragma unroll
+      for (int u = 0; u < AT_ONCE; ++u) {
+        if (q + u >= n || wgt[q + u] == -1.f) continue;
+        denom += wgt[q + u] * sum[q + u];
+#pragma unroll
+        for (int i = 0; i < MINE; ++i) num[i] += wgt[q + u] * v[u][i];
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int i = 0; i < MINE; ++i) {
+    const int d = tid + i * (int)blockDim.x;
+    if (d < D) out[rh * D + d] = from_f32<T>(denom > 0.f ? num[i] / denom : 0.f);
   }
 }
 
@@ -321,8 +368,8 @@ DRYFT_API int dryft_attn_rows_static_scratch(int is_bf16, const void* q, const v
   }
   float* part_o = g_static_scratch_ptr[dev];
   float* part_ml = part_o + need_o;
-  // Nothing in the scratch has to start at zero: every split writes its partial of every
-  // (row, head) before the combining kernel reads any of them.
+  // Nothing in the scratch has to start at zero: every split writes its maximum and sum of every
+  // (row, head), and its values where it had keys, before the combining kernel reads any of them.
   return is_bf16 ? launch<__nv_bfloat16>(q, k_pages, v_pages, page_table, max_pages, tok_slot, tok_pos, out, part_o, part_ml,
                                          n_rows, nKV, n_splits, scale, window, st)
                  : launch<float>(q, k_pages, v_pages, page_table, max_pages, tok_slot, tok_pos, out, part_o, part_ml,
