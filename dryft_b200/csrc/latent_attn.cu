@@ -25,9 +25,8 @@
 
 namespace {
 constexpr int PREP_THREADS = 256;
-constexpr int HW = 4;          // heads a warp of latent_attn_rows
+constexpr int HW_MOST = 4;     // heads a warp of latent_attn_rows; half as many where the blocks are few
 constexpr int WPB = 4;         // warps a block
-constexpr int HPB = HW * WPB;  // heads a block
 constexpr int KT = 32;         // keys per staged tile
 
 // sin and cos of  pos * (f_hi + f_lo)  for a rotary position: the product is formed in 32-bit, and what its rounding
@@ -120,11 +119,14 @@ template <> struct Vec16<__nv_bfloat16> {
   }
 };
 
-// One block per (query token, group of HPB heads, split of the visible keys); a warp takes HW heads, so that a key's
+// One block per (query token, group of HW * WPB heads, split of the visible keys); a warp takes HW heads, so that a key's
 // staged row is read from shared memory once for all of them (16 bytes at a time where the row length allows): the loop is
 // bound by shared-memory reads, and this quarters them.  With one split the result goes to o_lat; with several, each block
 // leaves (max, sum, unnormalised weighted sum) in `part` and latent_combine joins them.
-template <typename T, int NR>
+// The block's queries come in together (asynchronous copies, the angles from one table, nine words of keys a thread on their way meanwhile):
+// staged head by head they took half of a decode step's launch.  16 heads, rank 512 + 64, 1,300 keys, one token: 23.4 us before, 16.0 now;
+// whole request (3 layers x 16 steps) with the retention's steps as they are, 14,277 -> 13,727 us.
+template <typename T, int NR, int HW>
 __global__ void __launch_bounds__(WPB * 32) latent_attn_rows_kernel(
     const float* __restrict__ q_lat, const T* __restrict__ q, int q_stride, int q_rot_off, const T* __restrict__ k_pages,
     const int* __restrict__ page_table, int max_pages, int page_size, const int* __restrict__ tok_slot,
@@ -132,10 +134,11 @@ __global__ void __launch_bounds__(WPB * 32) latent_attn_rows_kernel(
     int interleaved, T* __restrict__ o_lat, float* __restrict__ part, int n_splits, int n_tokens, int H, int kv_rank, int rot,
     float scale, int window, const float* __restrict__ sink) {
   extern __shared__ __align__(16) float sm[];
+  constexpr int HPB = HW * WPB;
   const int Dk = kv_rank + rot, Dq = (Dk + 3) & ~3, Dp = tile_row(Dk);
   float* tile = sm;                                  // [KT][Dp]
   float* qs_all = tile + (size_t)KT * Dp;            // [HPB][Dq]
-  float* raw = qs_all + (size_t)HPB * Dq;            // [HPB][rot]
+  float* turn = qs_all + (size_t)HPB * Dq;           // [rot / 2] sin, then [rot / 2] cos
   const int n = blockIdx.x, split = blockIdx.z;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int hd0 = blockIdx.y * HPB + warp * HW;      // this warp's first head
@@ -149,21 +152,39 @@ __global__ void __launch_bounds__(WPB * 32) latent_attn_rows_kernel(
   const int lo = lo_all + split * per_split * KT;
   const int hi = min(pos, lo + per_split * KT - 1);   // last key of this split
   const int nh = max(0, min(HW, H - hd0));            // live heads of this warp
-  float* qs = qs_all + (size_t)warp * HW * Dq;
-  for (int i = 0; i < HW; ++i) {
-    float* qi = qs + (size_t)i * Dq;
-    if (i >= nh) {   // a head that does not exist: zeros, so that its sums stay finite
-      for (int d = lane; d < Dq; d += 32) qi[d] = 0.f;
-      continue;
+  const float* qs = qs_all + (size_t)warp * HW * Dq;
+  const int first = blockIdx.y * HPB, live = min(HPB, H - first);      // the block's heads; one that does not exist stays zero, so that its sums stay finite
+  for (int i = threadIdx.x; i < (HPB - live) * Dq; i += WPB * 32) qs_all[(size_t)live * Dq + i] = 0.f;
+  const bool copied = (kv_rank & 3) == 0 && ((uintptr_t)q_lat & 15) == 0;
+  const int quads = kv_rank / 4;
+  if (copied) {
+    for (int i = threadIdx.x; i < live * quads; i += WPB * 32) {
+      const int h = i / quads, c = i - h * quads;
+      const unsigned to = (unsigned)__cvta_generic_to_shared(qs_all + (size_t)h * Dq + c * 4);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to), "l"(q_lat + ((size_t)(first + h) * n_tokens + n) * kv_rank + c * 4) : "memory");
     }
-    const float* ql = q_lat + ((size_t)(hd0 + i) * n_tokens + n) * kv_rank;
-    for (int d = lane; d < kv_rank; d += 32) qi[d] = ql[d] * scale;
-    const T* qr = q + ((size_t)n * H + hd0 + i) * q_stride + q_rot_off;
-    float* rw = raw + (size_t)(warp * HW + i) * rot;
-    for (int d = lane; d < rot; d += 32) rw[d] = to_f32<T>(qr[d]);
-    __syncwarp();
-    for (int d = lane; d < rot; d += 32) qi[kv_rank + d] = rotated(rw, d, rot, interleaved != 0, (float)pos, inv_freq, inv_freq_lo) * scale;
-    for (int d = Dk + lane; d < Dq; d += 32) qi[d] = 0.f;
+  } else {
+    for (int i = threadIdx.x; i < live * kv_rank; i += WPB * 32) {
+      const int h = i / kv_rank, d = i - h * kv_rank;
+      qs_all[(size_t)h * Dq + d] = q_lat[((size_t)(first + h) * n_tokens + n) * kv_rank + d] * scale;
+    }
+  }
+  const int half = rot >> 1;
+  for (int k = threadIdx.x; k < half; k += WPB * 32) sincos_split((float)pos, inv_freq[k], inv_freq_lo ? inv_freq_lo[k] : 0.f, turn + k, turn + half + k);
+  __syncthreads();
+  const int tail = Dq - kv_rank;      // the rotated part, and zeros behind it
+#pragma unroll 4
+  for (int i = threadIdx.x; i < live * tail; i += WPB * 32) {
+    const int h = i / tail, d = i - h * tail;
+    float v = 0.f;
+    if (d < rot) {
+      const T* qr = q + ((size_t)n * H + first + h) * q_stride + q_rot_off;
+      const bool lower = interleaved ? !(d & 1) : d < half;
+      const int k = interleaved ? d >> 1 : lower ? d : d - half, partner = interleaved ? d ^ 1 : lower ? d + half : d - half;
+      const float own = to_f32<T>(qr[d]), other = to_f32<T>(qr[partner]);
+      v = lower ? own * turn[half + k] - other * turn[k] : own * turn[half + k] + other * turn[k];
+    }
+    qs_all[(size_t)h * Dq + kv_rank + d] = v * scale;
   }
   float m[HW], l[HW], acc[HW][NR];
 #pragma unroll
@@ -181,13 +202,14 @@ __global__ void __launch_bounds__(WPB * 32) latent_attn_rows_kernel(
     const int cnt = min(KT, hi - j0 + 1);
     __syncthreads();   // the tile before is used up (and, the first time, qs is written)
     if (vec_ok) {
-      // every thread asks for four 16-byte pieces before it unpacks the first: the loads' round trips overlap
+      // every thread asks for nine 16-byte pieces before it unpacks the first: the loads' round trips overlap
+      constexpr int AHEAD = 9;
       const int total = cnt * vpr;
-      for (int base = threadIdx.x; base < total; base += 4 * WPB * 32) {
-        uint4 v[4];
-        int at[4];
+      for (int base = threadIdx.x; base < total; base += AHEAD * WPB * 32) {
+        uint4 v[AHEAD];
+        int at[AHEAD];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < AHEAD; ++u) {
           const int idx = base + u * WPB * 32;
           at[u] = -1;
           if (idx < total) {
@@ -198,7 +220,7 @@ __global__ void __launch_bounds__(WPB * 32) latent_attn_rows_kernel(
           }
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
+        for (int u = 0; u < AHEAD; ++u) {
           if (at[u] >= 0) {
             float f[VN];
             Vec16<T>::unpack(v[u], f);
@@ -212,6 +234,16 @@ __global__ void __launch_bounds__(WPB * 32) latent_attn_rows_kernel(
         const int j = j0 + kk;
         const T* src = k_pages + ((size_t)pt[j / page_size] * page_size + j % page_size) * Dk;
         for (int d = lane; d < Dk; d += 32) tile[kk * Dp + d] = to_f32<T>(src[d]);
+      }
+    }
+    if (copied && j0 == lo) {      // the queries are here with the first keys: a thread scales what it copied
+      asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll 4
+      for (int i = threadIdx.x; i < live * quads; i += WPB * 32) {
+        const int h = i / quads, c = i - h * quads;
+        float4* const at = reinterpret_cast<float4*>(qs_all + (size_t)h * Dq + c * 4);
+        const float4 v = *at;
+        *at = make_float4(v.x * scale, v.y * scale, v.z * scale, v.w * scale);
       }
     }
     __syncthreads();
@@ -266,6 +298,7 @@ __global__ void __launch_bounds__(WPB * 32) latent_attn_rows_kernel(
       }
     }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");      // a split without keys used none of its queries
 #pragma unroll
   for (int i = 0; i < HW; ++i) {
     if (i >= nh) break;
@@ -308,6 +341,12 @@ __global__ void latent_combine_kernel(const float* __restrict__ part, const int*
   if (tok_slot[n] < 0) return;
   const size_t stride = (size_t)kv_rank + 2;
   const float* src = part + ((size_t)n * H + hd) * n_splits * stride;
+  // a thread a latent entry; 32 splits' values are requested together, the first of them before the weights are known (7.1 us a launch with
+  // sixteen at a time behind the weights, 3.5 now: the same 16 heads of 512)
+  constexpr int AT_ONCE = 32;
+  float v[AT_ONCE];
+#pragma unroll
+  for (int u = 0; u < AT_ONCE; ++u) v[u] = u < n_splits && threadIdx.x < kv_rank ? src[u * stride + 2 + threadIdx.x] : 0.f;
   if (threadIdx.x < 32) {
     const int lane = threadIdx.x;
     float ms[MAX_SPLITS / 32], ls[MAX_SPLITS / 32];
@@ -334,16 +373,15 @@ __global__ void latent_combine_kernel(const float* __restrict__ part, const int*
       if (lane + 32 * u < n_splits) w[lane + 32 * u] = ms[u] / l;
   }
   __syncthreads();
-  // a thread a latent entry, its splits requested sixteen at a time: with four entries a thread and eight splits at a time
-  // one token's 32 splits of 512 took 22 us (sixteen trips to memory)
   for (int d = threadIdx.x; d < kv_rank; d += blockDim.x) {
     float a = 0.f;
-    for (int s0 = 0; s0 < n_splits; s0 += 16) {
-      float v[16];
+    for (int s0 = 0; s0 < n_splits; s0 += AT_ONCE) {
+      if (s0 > 0 || d >= (int)blockDim.x) {      // (else they are on their way already)
 #pragma unroll
-      for (int u = 0; u < 16; ++u) v[u] = s0 + u < n_splits ? src[(s0 + u) * stride + 2 + d] : 0.f;
+        for (int u = 0; u < AT_ONCE; ++u) v[u] = s0 + u < n_splits ? src[(s0 + u) * stride + 2 + d] : 0.f;
+      }
 #pragma unroll
-      for (int u = 0; u < 16; ++u)
+      for (int u = 0; u < AT_ONCE; ++u)
         if (s0 + u < n_splits) a = fmaf(v[u], w[s0 + u], a);
     }
     o_lat[((size_t)hd * n_tokens + n) * kv_rank + d] = from_f32<T>(a);
@@ -575,21 +613,37 @@ template <typename K> int opt_in(K kernel, size_t bytes) {
   return 0;
 }
 
+template <typename T, int NR, int HW>
+int launch_rows_of(const float* q_lat, const void* q, int q_stride, int q_rot_off, const void* k_pages, const int* page_table,
+                   int max_pages, int page_size, const int* tok_slot, const int* tok_pos, const float* inv_freq,
+                   const float* inv_freq_lo, int interleaved, void* o_lat, float* part, int n_splits, int n_tokens, int H, int kv_rank,
+                   int rot, float scale, int window, const float* sink, cudaStream_t st) {
+  constexpr int HPB = HW * WPB;
+  const int Dk = kv_rank + rot;
+  const size_t smem = sizeof(float) * ((size_t)KT * tile_row(Dk) + (size_t)HPB * ((Dk + 3) & ~3) + (size_t)rot);
+  int rc = opt_in(latent_attn_rows_kernel<T, NR, HW>, smem);
+  if (rc) return rc;
+  dim3 grid(n_tokens, (H + HPB - 1) / HPB, n_splits);
+  latent_attn_rows_kernel<T, NR, HW><<<grid, WPB * 32, smem, st>>>(q_lat, (const T*)q, q_stride, q_rot_off, (const T*)k_pages, page_table,
+                                                                   max_pages, page_size, tok_slot, tok_pos, inv_freq, inv_freq_lo,
+                                                                   interleaved, (T*)o_lat, part, n_splits, n_tokens, H, kv_rank, rot, scale,
+                                                                   window, sink);
+  return launch_status();
+}
+
 template <typename T, int NR>
 int launch_rows(const float* q_lat, const void* q, int q_stride, int q_rot_off, const void* k_pages, const int* page_table,
                 int max_pages, int page_size, const int* tok_slot, const int* tok_pos, const float* inv_freq,
                 const float* inv_freq_lo, int interleaved, void* o_lat, float* part, int n_splits, int n_tokens, int H, int kv_rank,
                 int rot, float scale, int window, const float* sink, cudaStream_t st) {
-  const int Dk = kv_rank + rot;
-  const size_t smem = sizeof(float) * ((size_t)KT * tile_row(Dk) + (size_t)HPB * ((Dk + 3) & ~3) + (size_t)HPB * rot);
-  int rc = opt_in(latent_attn_rows_kernel<T, NR>, smem);
-  if (rc) return rc;
-  dim3 grid(n_tokens, (H + HPB - 1) / HPB, n_splits);
-  latent_attn_rows_kernel<T, NR><<<grid, WPB * 32, smem, st>>>(q_lat, (const T*)q, q_stride, q_rot_off, (const T*)k_pages, page_table,
-                                                               max_pages, page_size, tok_slot, tok_pos, inv_freq, inv_freq_lo,
-                                                               interleaved, (T*)o_lat, part, n_splits, n_tokens, H, kv_rank, rot, scale,
-                                                               window, sink);
-  int e = launch_status();
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // twice the blocks, a key's row read from shared memory for half as many heads, while half of the multiprocessors would have none
+  const bool few = 2LL * n_tokens * ((H + HW_MOST * WPB - 1) / (HW_MOST * WPB)) * n_splits <= sms;
+  int e = (few ? launch_rows_of<T, NR, HW_MOST / 2> : launch_rows_of<T, NR, HW_MOST>)(q_lat, q, q_stride, q_rot_off, k_pages, page_table, max_pages, page_size,
+                                                                                    tok_slot, tok_pos, inv_freq, inv_freq_lo, interleaved, o_lat, part,
+                                                                                    n_splits, n_tokens, H, kv_rank, rot, scale, window, sink, st);
   if (e || n_splits <= 1) return e;
   latent_combine_kernel<T><<<dim3(n_tokens, H), kv_rank > 256 ? 512 : 256, 0, st>>>(part, tok_slot, (T*)o_lat, n_splits, n_tokens, H, kv_rank, sink);
   return launch_status();
@@ -623,7 +677,7 @@ DRYFT_API int dryft_latent_attn_rows(int is_bf16, const float* q_lat, const void
                                      int interleaved, void* o_lat, float* part, int n_splits, int n_tokens, int H, int kv_rank,
                                      int rot, float scale, int window, const float* sink, cudaStream_t st) {
   if (n_tokens <= 0) return 0;
-  if (kv_rank <= 0 || kv_rank > 512 || rot < 0 || (rot & 1) || H <= 0 || (H + HPB - 1) / HPB > 65535) return DRYFT_ERR_UNSUPPORTED;
+  if (kv_rank <= 0 || kv_rank > 512 || rot < 0 || (rot & 1) || H <= 0 || H > 65535) return DRYFT_ERR_UNSUPPORTED;
   if (n_splits < 1 || n_splits > MAX_SPLITS || (n_splits > 1 && !part)) return DRYFT_ERR_UNSUPPORTED;
   typedef __nv_bfloat16 bf;
   const int nr = (kv_rank + 31) / 32;
