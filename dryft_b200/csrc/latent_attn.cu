@@ -125,7 +125,7 @@ template <> struct Vec16<__nv_bfloat16> {
 // leaves (max, sum, unnormalised weighted sum) in `part` and latent_combine joins them.
 // The block's queries come in together (asynchronous copies, the angles from one table, nine words of keys a thread on their way meanwhile):
 // staged head by head they took half of a decode step's launch.  16 heads, rank 512 + 64, 1,300 keys, one token: 23.4 us before, 16.0 now;
-// whole request (3 layers x 16 steps) with the retention's steps as they are, 14,277 -> 13,727 us.
+// whole request (3 layers x 16 steps) with the retention's steps as they are, 14,263 -> 13,785 us.
 template <typename T, int NR, int HW>
 __global__ void __launch_bounds__(WPB * 32) latent_attn_rows_kernel(
     const float* __restrict__ q_lat, const T* __restrict__ q, int q_stride, int q_rot_off, const T* __restrict__ k_pages,
@@ -639,7 +639,8 @@ int launch_rows(const float* q_lat, const void* q, int q_stride, int q_rot_off, 
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // twice the blocks, a key's row read from shared memory for half as many heads, while half of the multiprocessors would have none
+  // twice the blocks, a key's row read from shared memory for half as many heads, while half of the multiprocessors would have none (the figures at the
+  // row kernel are with both: the line itself is where the second half still runs in the same wave)
   const bool few = 2LL * n_tokens * ((H + HW_MOST * WPB - 1) / (HW_MOST * WPB)) * n_splits <= sms;
   int e = (few ? launch_rows_of<T, NR, HW_MOST / 2> : launch_rows_of<T, NR, HW_MOST>)(q_lat, q, q_stride, q_rot_off, k_pages, page_table, max_pages, page_size,
                                                                                     tok_slot, tok_pos, inv_freq, inv_freq_lo, interleaved, o_lat, part,
