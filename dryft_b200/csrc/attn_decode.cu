@@ -70,12 +70,15 @@ constexpr size_t Q_BYTES = (size_t)(Q_ROWS + 2) * KS * 2;  // then the new key a
 constexpr int W = NT * MT * 4;              // accumulators of a thread
 // what a block of a cluster receives: maximum and sum of every split and head, and of every split the accumulators that it adds up
 constexpr size_t RECEIVED_BYTES = 8 * 16 * 2 * 4 + (size_t)(W + 8) * 32 * 4;
+constexpr size_t SMEM_MOST = 227 * 1024;    // of a block
 template <int NWARP, int STAGES> struct Shape {
   static constexpr int THREADS = NWARP * 32;
   static constexpr size_t WARP_STAGE_BYTES = (size_t)STAGES * 2 * SLICE * KS * 2;
   static constexpr size_t COMBINE_BYTES = (size_t)NWARP * 16 * 2 * 4 + (size_t)NWARP * W * 32 * 4;
   static constexpr size_t PIPE_BYTES = NWARP * WARP_STAGE_BYTES;
   static constexpr size_t SMEM_BYTES = Q_BYTES + (PIPE_BYTES > COMBINE_BYTES ? PIPE_BYTES : COMBINE_BYTES);
+  static constexpr size_t bytes(bool cluster) { return SMEM_BYTES + (cluster ? RECEIVED_BYTES : 0); }      // of a launch
+  static constexpr bool fits(bool cluster) { return bytes(cluster) <= SMEM_MOST; }
 };
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -629,17 +632,18 @@ __global__ void __launch_bounds__(NWARP * 32) attn_decode_kernel(const Params p)
 template <int NWARP, int STAGES>
 static int launch_shape(const Params& p, int n_rows, int nKV, int n_splits, int pdl, cudaStream_t st) {
   typedef Shape<NWARP, STAGES> S;
-  if (S::SMEM_BYTES + RECEIVED_BYTES > 227 * 1024) return DRYFT_ERR_UNSUPPORTED;
+  if (!S::fits(p.cluster)) return DRYFT_ERR_UNSUPPORTED;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(n_rows, nKV, n_splits);
   cfg.blockDim = dim3(S::THREADS);
   static bool attr_set = false;  // per shape; set by the first (eager) launch, outside any stream capture
-  if (S::SMEM_BYTES + RECEIVED_BYTES > 48 * 1024 && !attr_set) {
-    cudaError_t ea = cudaFuncSetAttribute(attn_decode_kernel<NWARP, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(S::SMEM_BYTES + RECEIVED_BYTES));
+  constexpr size_t most = S::bytes(S::fits(true));      // of any launch of this shape
+  if (most > 48 * 1024 && !attr_set) {
+    cudaError_t ea = cudaFuncSetAttribute(attn_decode_kernel<NWARP, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (ea != cudaSuccess) return (int)ea;
     attr_set = true;
   }
-  cfg.dynamicSmemBytes = S::SMEM_BYTES + (p.cluster ? RECEIVED_BYTES : 0);
+  cfg.dynamicSmemBytes = S::bytes(p.cluster);
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   int n_attr = 0;
@@ -690,11 +694,13 @@ DRYFT_API int dryft_attn_decode(const void* qkv, int qkv_stride, const float* wq
         sms = 1;
     }
     const long long blocks = (long long)n_rows * nKV * n_splits;
-    const long long usable = 227 * 1024;
-    const long long per_sm_8 = usable / (long long)(Shape<8, 2>::SMEM_BYTES + 1024);   // 0: does not fit at all
-    const long long per_sm_4 = usable / (long long)(Shape<4, 2>::SMEM_BYTES + 1024);
+    const long long usable = SMEM_MOST;
+    const long long per_sm_8 = usable / (long long)(Shape<8, 2>::bytes(cluster) + 1024);   // 0: does not fit at all
+    const long long per_sm_4 = usable / (long long)(Shape<4, 2>::bytes(cluster) + 1024);
     shape = (per_sm_8 >= 1 && blocks <= sms * per_sm_8) ? 0 : ((per_sm_4 >= 1 && blocks <= sms * per_sm_4) ? 1 : 2);
-    if (shape == 2 && (long long)(Shape<2, 2>::SMEM_BYTES + 1024) > usable) shape = per_sm_4 >= 1 ? 1 : 0;
+    if (shape == 2 && (long long)(Shape<2, 2>::bytes(cluster) + 1024) > usable) shape = per_sm_4 >= 1 ? 1 : 0;
+  } else if (shape != 1 && shape != 2 && cluster && Shape<8, 2>::fits(false) && !Shape<8, 2>::fits(true)) {
+    shape = 1;      // eight warps' rings fit, but not beside what a block of a cluster receives (head size 208): four warps
   }
   return shape == 1 ? launch_shape<4, 2>(p, n_rows, nKV, n_splits, pdl, st)
        : shape == 2 ? launch_shape<2, 2>(p, n_rows, nKV, n_splits, pdl, st)
