@@ -129,8 +129,11 @@ __global__ void __launch_bounds__(RT_THREADS) retention_scan_kernel(
 }
 
 // The same for steps in which every sequence brings one token (token b is sequence b's): bound by one trip to memory for a head's state.
-// A thread holds up to STEP_ROWS rows' 16-byte words of it in registers, all requested before the launch before this one is waited for (a
-// state depends on the step before only), and works the angles out meanwhile; rows are summed in order by each thread, threads in order.
+// A thread holds up to STEP_ROWS rows' 16-byte words of it in registers, all requested at once, and works the angles out meanwhile; rows are
+// summed in order by each thread, threads in order.  `early`: the words are requested before the launch before this one is waited for.  That
+// is right only where whatever wrote the state last was complete before this step's first overlapped launch: a run step's own state, which
+// the step before wrote.  A state that an earlier run step of the same step wrote (or two direct calls in a row) is read behind the wait:
+// every launch in between may have signalled at its start, and then nothing else orders that write before this read.
 // 16 heads of 128 x 128, one token: 11.1 us a launch with the walk above, 9.7 here, of which half runs beside the product before it (5.2 us of
 // its own): a 1,300-token prompt + 16 steps, 6 such launches a step, 14,709 -> 14,266 us.  Sizes it does not take (rows that are no 16-byte words, more
 // than STEP_ROWS rows a thread, angles or partial sums beyond 48 KB of shared memory) are walked as longer steps are.
@@ -143,12 +146,15 @@ template <typename T>
 __global__ void __launch_bounds__(RT_THREADS) retention_step_kernel(
     const T* __restrict__ proj, int ld, int q_off, int k_off, int v_off, int g_off, const int* __restrict__ seq_slot, const int* __restrict__ tok_pos,
     const float* __restrict__ inv_freq, const float* __restrict__ inv_freq_lo, int rot, const double* __restrict__ decay, float* __restrict__ state,
-    T* __restrict__ out, int H, int dim, int vdim, float k_scale, float eps) {
+    T* __restrict__ out, int H, int dim, int vdim, float k_scale, float eps, int early) {
   let_next_launch_in();   // a product behind this launch may start on its weights
   extern __shared__ __align__(16) float smem[];
   const int b = blockIdx.x, hd = blockIdx.y, tid = threadIdx.x;
   const int slot = seq_slot[b];
-  if (slot < 0) return;
+  if (slot < 0) {      // (waits too: a launch of padding alone must not be complete before the launch before it)
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    return;
+  }
   const int words = vdim / 4, groups = RT_THREADS / words, cv = tid % words, rg = tid / words, half = rot >> 1;
   float4* const red = reinterpret_cast<float4*>(smem);      // [groups][words]
   float* const qs = smem + (size_t)groups * vdim;           // [dim]
@@ -158,11 +164,14 @@ __global__ void __launch_bounds__(RT_THREADS) retention_step_kernel(
   __shared__ float scratch[33];
   float4* const Sg = reinterpret_cast<float4*>(state + ((size_t)slot * H + hd) * dim * vdim);
   float4 old[STEP_ROWS];
+  auto request = [&]() {      // (through L2: a state written while this launch was resident is no read-only data)
 #pragma unroll
-  for (int i = 0; i < STEP_ROWS; ++i) {
-    const int d = rg + i * groups;
-    old[i] = rg < groups && d < dim ? Sg[(size_t)d * words + cv] : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+    for (int i = 0; i < STEP_ROWS; ++i) {
+      const int d = rg + i * groups;
+      old[i] = rg < groups && d < dim ? __ldcg(Sg + (size_t)d * words + cv) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  if (early) request();
   // the decay as a 32-bit value and what that drops, as above
   const float dec = (float)decay[hd], dec_lo = (float)(decay[hd] - (double)dec);
   const float pos = (float)tok_pos[b];
@@ -174,6 +183,7 @@ __global__ void __launch_bounds__(RT_THREADS) retention_step_kernel(
   }
   __syncthreads();
   asm volatile("griddepcontrol.wait;" ::: "memory");      // the projection; what it wrote is read through L2
+  if (!early) request();
   const T* const row = proj + (size_t)b * ld;
 #pragma unroll 1
   for (int i = tid; i < 2 * dim; i += RT_THREADS) {
@@ -843,7 +853,7 @@ template <typename K> int opt_in_smem(K kernel, size_t bytes) {
 DRYFT_API int dryft_retention_scan(int is_bf16, const void* proj, int ld, int q_off, int k_off, int v_off, int g_off,
                                    const int* cu_q, const int* seq_slot, const int* tok_pos, const float* inv_freq,
                                    const float* inv_freq_lo, int rot, const double* decay, float* state, void* out, int n_seqs, int H, int dim, int vdim,
-                                   float k_scale, float eps, int one_token, int pdl, cudaStream_t st) {
+                                   float k_scale, float eps, int one_token, int pdl, int early_state, cudaStream_t st) {
   if (n_seqs <= 0) return 0;
   if (H <= 0 || dim <= 0 || vdim <= 0 || rot < 0 || rot > dim || (rot & 1) || H > 65535) return DRYFT_ERR_UNSUPPORTED;
   typedef __nv_bfloat16 bf;
@@ -862,9 +872,9 @@ DRYFT_API int dryft_retention_scan(int is_bf16, const void* proj, int ld, int q_
     if (cfg.dynamicSmemBytes <= 48 * 1024) {
       const cudaError_t e =
           is_bf16 ? cudaLaunchKernelEx(&cfg, retention_step_kernel<bf>, (const bf*)proj, ld, q_off, k_off, v_off, g_off, seq_slot, tok_pos, inv_freq,
-                                       inv_freq_lo, rot, decay, state, (bf*)out, H, dim, vdim, k_scale, eps)
+                                       inv_freq_lo, rot, decay, state, (bf*)out, H, dim, vdim, k_scale, eps, early_state || !pdl)
                   : cudaLaunchKernelEx(&cfg, retention_step_kernel<float>, (const float*)proj, ld, q_off, k_off, v_off, g_off, seq_slot, tok_pos,
-                                       inv_freq, inv_freq_lo, rot, decay, state, (float*)out, H, dim, vdim, k_scale, eps);
+                                       inv_freq, inv_freq_lo, rot, decay, state, (float*)out, H, dim, vdim, k_scale, eps, early_state || !pdl);
       return e != cudaSuccess ? (int)e : launch_status();
     }
   }

@@ -1289,7 +1289,7 @@ def recurrent_lib() -> ctypes.CDLL:
     return _single_lib("recurrent", {
         "dryft_retention_chunked": [_i, _p, _i, _i, _i, _i, _i, _p, _p, _p, _p, _p, _i, _p, _p, _p, _p, _i, _i, _i, _i, _i, _f, _f, _p],
         "dryft_retention_chunk_tokens": [],
-        "dryft_retention_scan": [_i, _p, _i, _i, _i, _i, _i, _p, _p, _p, _p, _p, _i, _p, _p, _p, _i, _i, _i, _i, _f, _f, _i, _i, _p],
+        "dryft_retention_scan": [_i, _p, _i, _i, _i, _i, _i, _p, _p, _p, _p, _p, _i, _p, _p, _p, _i, _i, _i, _i, _f, _f, _i, _i, _i, _p],
         "dryft_rglru_gates": [_i, _p, _i, _i, _p, _p, _p, _p, _i, _p, _p, _p, _p, _p, _f, _p, _p, _i, _i, _i, _p],
         "dryft_rglru_scan": [_i, _p, _i, _i, _p, _i, _p, _p, _p, _p, _p, _p, _p, _i, _p, _i, _i, _p],
     })
@@ -1421,14 +1421,16 @@ RETENTION_CHUNKED_MAX_VDIM = 512   # value sizes the chunked form holds in a thr
 
 def retention_scan(proj, offsets, cu_q, seq_slot, tok_pos, inv_freq, rot: int, decay, state, out, n_seqs: int, heads: int,
                    dim: int, vdim: int, k_scale: float, eps: float, inv_freq_lo=None, chunked: bool = False,
-                   one_token: bool = False, pdl: bool = False) -> None:
+                   one_token: bool = False, pdl: bool = False, early_state: bool = False) -> None:
     """``inv_freq_lo`` (optional, here and in the latent attention wrappers): the part of each frequency that its 32-bit
     value drops; with it the angles are as exact as the pair.
 
     Retention over the step's tokens from and to ``state [slots, heads, dim, vdim]`` (float32).  ``proj [n, ld]`` holds
     q | k | v | g at the column ``offsets`` (4 ints); ``out [n, heads * vdim]``; ``decay [heads]`` float64.  ``chunked``:
     the form for steps of many tokens (the same result up to rounding; token by token otherwise).  ``one_token``: every
-    sequence brings one token (a kernel of its own, with ``pdl`` a programmatic dependent of the launch before it)."""
+    sequence brings one token (a kernel of its own, with ``pdl`` a programmatic dependent of the launch before it, and of
+    those that this one overlaps in turn: they must not write ``seq_slot`` or ``tok_pos``).  ``early_state``: with ``pdl``
+    the state is read before the launch before is waited for; only for a state that none of those launches writes."""
     n, ld = proj.shape
     _need(proj, "proj")
     q_off, k_off, v_off, g_off = (int(o) for o in offsets)
@@ -1456,7 +1458,7 @@ def retention_scan(proj, offsets, cu_q, seq_slot, tok_pos, inv_freq, rot: int, d
             return
     _ok(recurrent_lib().dryft_retention_scan(_act(proj, "proj"), _ptr(proj), ld, q_off, k_off, v_off, g_off, _ptr(cu_q), _ptr(seq_slot),
                                              _ptr(tok_pos), _ptr(inv_freq), _ptr(_freq_lo(inv_freq_lo, rot)), int(rot), _ptr(decay), _ptr(state), _ptr(out), n_seqs,
-                                             heads, dim, vdim, float(k_scale), float(eps), int(one_token), int(pdl), _stream()),
+                                             heads, dim, vdim, float(k_scale), float(eps), int(one_token), int(pdl), int(early_state), _stream()),
         f"retention_scan ({heads} heads of {dim} x {vdim})")
 
 

@@ -75,5 +75,6 @@ class Retention:
         o = torch.empty((h.shape[0], self.n_heads * self.v_dim), dtype=h.dtype, device=h.device)
         K.retention_scan(proj, self.offsets, ctx.cu_q, ctx.seq_slot, ctx.tok_pos, self.position.inv_freq, self.position.rotary_dim,
                          self.decay, state, o, ctx.n_seqs, self.n_heads, self.qk_dim, self.v_dim, self.k_scale, self.eps,
-                         inv_freq_lo=getattr(self.position, "inv_freq_lo", None), chunked=not ctx.decode, one_token=ctx.decode, pdl=self.rt.pdl)
+                         inv_freq_lo=getattr(self.position, "inv_freq_lo", None), chunked=not ctx.decode, one_token=ctx.decode, pdl=self.rt.pdl,
+                         early_state=owns_cache)      # (the step it borrows from has just written a borrowed state)
         return linear(o, self.w_o, self.rt)
