@@ -227,30 +227,32 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
 }
 
 // Combine the partials of one (row, head):  w_s = exp(m_s - max m);  o = sum w_s acc_s / sum w_s l_s, in the order of the splits.  A thread
-// makes the weights of some splits, all of them share them; several splits' values are on their way together.
+// makes the weights of some splits, all of them share them; sixteen splits' values are on their way together at up to 128 dims,
+// eight above.
 constexpr int REDUCE_TILE = 128;
+constexpr int REDUCE_THREADS = D < 128 ? 64 : 128;
 template <typename T>
-__global__ void __launch_bounds__(128) attn_rows_reduce_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
+__global__ void __launch_bounds__(REDUCE_THREADS) attn_rows_reduce_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
                                                                T* __restrict__ out, int n_splits) {
   let_next_launch_in();   // a product behind this launch may start on its weights
-  __shared__ float wgt[REDUCE_TILE], sum[REDUCE_TILE], top[4];
+  __shared__ float wgt[REDUCE_TILE], sum[REDUCE_TILE], top[REDUCE_THREADS / 32];
   const size_t rh = blockIdx.x;  // row * nH + head
   const float* ml = part_ml + rh * n_splits * 2;
   const int tid = threadIdx.x;
   float mx = -INFINITY;
-  for (int s = tid; s < n_splits; s += blockDim.x) mx = fmaxf(mx, ml[s * 2]);
+  for (int s = tid; s < n_splits; s += REDUCE_THREADS) mx = fmaxf(mx, ml[s * 2]);
   mx = warp_max(mx);
   if (tid % 32 == 0) top[tid / 32] = mx;
   __syncthreads();
   mx = top[0];
-  for (int w = 1; w < (int)blockDim.x / 32; ++w) mx = fmaxf(mx, top[w]);
-  constexpr int MINE = (D + 63) / 64;      // dims a thread (64 or 128 threads)
+  for (int w = 1; w < REDUCE_THREADS / 32; ++w) mx = fmaxf(mx, top[w]);
+  constexpr int MINE = (D + REDUCE_THREADS - 1) / REDUCE_THREADS;      // dims a thread
   float num[MINE], denom = 0.f;
 #pragma unroll
   for (int i = 0; i < MINE; ++i) num[i] = 0.f;
   for (int s0 = 0; s0 < n_splits; s0 += REDUCE_TILE) {
     const int n = min(REDUCE_TILE, n_splits - s0);
-    for (int s = tid; s < n; s += blockDim.x) {
+    for (int s = tid; s < n; s += REDUCE_THREADS) {
       const float m = ml[(s0 + s) * 2];
       wgt[s] = m == -INFINITY ? -1.f : expf(m - mx);      // -1: an empty split, which wrote no values
       sum[s] = ml[(s0 + s) * 2 + 1];
@@ -263,7 +265,7 @@ __global__ void __launch_bounds__(128) attn_rows_reduce_kernel(const float* __re
       for (int u = 0; u < AT_ONCE; ++u)
 #pragma unroll
         for (int i = 0; i < MINE; ++i) {
-          const int d = tid + i * (int)blockDim.x;
+          const int d = tid + i * REDUCE_THREADS;
           v[u][i] = q + u < n && d < D ? part_o[(rh * n_splits + s0 + q + u) * D + d] : 0.f;
         }
 #pragma unroll
@@ -278,7 +280,7 @@ __global__ void __launch_bounds__(128) attn_rows_reduce_kernel(const float* __re
   }
 #pragma unroll
   for (int i = 0; i < MINE; ++i) {
-    const int d = tid + i * (int)blockDim.x;
+    const int d = tid + i * REDUCE_THREADS;
     if (d < D) out[rh * D + d] = from_f32<T>(denom > 0.f ? num[i] / denom : 0.f);
   }
 }
@@ -312,7 +314,7 @@ int launch(const void* q, const void* k_pages, const void* v_pages, const int* p
                                                   n_splits, scale, window);
   int rc = launch_status();
   if (rc || n_splits == 1) return rc;
-  attn_rows_reduce_kernel<T><<<(unsigned)((size_t)n_rows * nKV * G), D < 128 ? 64 : 128, 0, st>>>(part_o, part_ml, (T*)out, n_splits);
+  attn_rows_reduce_kernel<T><<<(unsigned)((size_t)n_rows * nKV * G), REDUCE_THREADS, 0, st>>>(part_o, part_ml, (T*)out, n_splits);
   return launch_status();
 }
 }  // namespace
