@@ -11,7 +11,7 @@
 // un-normalised partial (acc, m, l) and `attn_rows_reduce_kernel` combines them
 // (attn_decode.py:102-118).
 //
-// A split is a multiple of 16 keys, not of pages: a block takes 10 us for the 64 keys of a page (32-bit, two trips to memory, scores and
+// A split is 16 keys, half a page or whole pages: a block takes 10 us for the 64 keys of a page (32-bit, two trips to memory, scores and
 // values of 64 keys by 128 threads), and while rows are few most blocks of a launch would have none.  Four rows of about 150 keys, two kv
 // heads, 32 splits: 11 + 5.5 us for the two launches by pages, 6.0 + 4.3 by 16 keys.
 //
@@ -19,6 +19,7 @@
 #include "common.cuh"
 #include "attn_rows_static.h"
 #include <math.h>
+#include <type_traits>
 
 #if !defined(DRYFT_HEAD_DIM) || !defined(DRYFT_GROUP) || !defined(DRYFT_PAGE)
 #error "compile with -DDRYFT_HEAD_DIM=.. -DDRYFT_GROUP=.. -DDRYFT_PAGE=.."
@@ -41,10 +42,15 @@ template <typename T> struct Smem {
   static constexpr size_t bytes() {
     return sizeof(float) * (G * D + G * PAGE + 3 * G) + sizeof(T) * (size_t)(PAGE * KSTRIDE + PAGE * D) + 32;
   }
+  // blocks a multiprocessor that the registers have to leave room for: as many as shared memory does, up to what costs few spills
+  static constexpr int blocks() {
+    const size_t n = 227 * 1024 / (bytes() + 1024), most = G > 8 ? 5 : G > 2 ? 8 : 10;
+    return n < 1 ? 1 : (int)(n > most ? most : n);
+  }
 };
 
 template <typename T>
-__global__ void __launch_bounds__(THREADS) attn_rows_kernel(
+__global__ void __launch_bounds__(THREADS, Smem<T>::blocks()) attn_rows_kernel(
     const T* __restrict__ q,                                   // [N, nH, D]
     const T* __restrict__ k_pages, const T* __restrict__ v_pages,  // [pages, nKV, PAGE, D]
     const int* __restrict__ page_table, int max_pages,
@@ -84,8 +90,10 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
   const int pos = tok_pos[n];
   const int kv_hi = pos + 1;                                        // exclusive
   const int kv_lo = window > 0 ? max(0, kv_hi - window) : 0;        // inclusive
-  const int base = kv_lo / GRAIN * GRAIN, grains = (kv_hi - base + GRAIN - 1) / GRAIN;
-  const int per_split = (grains + n_splits - 1) / n_splits;
+  constexpr int PAGE_GRAINS = PAGE / GRAIN;
+  const int base = kv_lo / PAGE * PAGE, grains = (kv_hi - base + GRAIN - 1) / GRAIN;
+  int per_split = (grains + n_splits - 1) / n_splits;
+  if (per_split > PAGE_GRAINS / 2) per_split = (per_split + PAGE_GRAINS - 1) / PAGE_GRAINS * PAGE_GRAINS;      // no page in more parts than needed
   const int k_begin = max(kv_lo, (int)min((long long)base + (long long)split * per_split * GRAIN, (long long)kv_hi));      // this block's keys
   const int k_end = (int)min((long long)base + (long long)(split + 1) * per_split * GRAIN, (long long)kv_hi);
   if (n_splits > 1 && k_begin >= k_end) {      // nothing to add: a maximum of -inf says so
@@ -107,21 +115,28 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
 
   const int* pt = page_table + (size_t)slot * max_pages;
   constexpr int VPR = D / L::VEC;  // 16-byte vectors per row
-  for (int pg = k_begin / PAGE; pg * PAGE < k_end; ++pg) {
+  // One page.  `whole`: all its keys are this block's, and every bound is a constant; else rows [r0, r1) are.  With bounds that only the launch
+  // knows, launches of many rows, which walk whole pages mostly, were up to 1.37 times as long: probabilities read one by one instead of four
+  // at a time, a division an item, registers for loads that no thread makes.  A part of a page is widened to groups of eight rows, zeros and
+  // probabilities of zero beside the block's own.
+  auto walk = [&](auto whole, int pg) {
+    constexpr bool WHOLE = decltype(whole)::value;
     const int page = pt[pg];
     const int p0 = pg * PAGE;
-    const int r0 = max(k_begin - p0, 0), r1 = min(k_end - p0, PAGE), rows = r1 - r0;      // of the page
+    const int r0 = WHOLE ? 0 : max(k_begin - p0, 0), r1 = WHOLE ? PAGE : min(k_end - p0, PAGE);
+    const int ra = WHOLE ? 0 : r0 & ~7, rb = WHOLE ? PAGE : (r1 + 7) & ~7, rows = rb - ra;
     const T* kp = k_pages + ((size_t)page * nKV + kvh) * PAGE * D;
     const T* vp = v_pages + ((size_t)page * nKV + kvh) * PAGE * D;
     __syncthreads();  // previous tile fully consumed
-    // eight words of K and of V on their way at once (two at a time left a page eight trips to memory long)
-    constexpr int AHEAD = 8;
-    for (int i0 = r0 * VPR + tid; i0 < r1 * VPR; i0 += AHEAD * THREADS) {
+    // words of K and of V on their way at once: eight of a whole page (two at a time left it eight trips to memory long), else two grains'
+    constexpr int GRAINS = 2 * GRAIN * VPR / THREADS, AHEAD = WHOLE || GRAINS > 8 ? 8 : GRAINS < 2 ? 2 : GRAINS;
+    for (int i0 = ra * VPR + tid; i0 < rb * VPR; i0 += AHEAD * THREADS) {
       uint4 kv4[AHEAD], vv4[AHEAD];
 #pragma unroll
       for (int u = 0; u < AHEAD; ++u) {
         const int i = i0 + u * THREADS, r = i / VPR, c = i % VPR;
-        if (i < r1 * VPR) {
+        kv4[u] = vv4[u] = make_uint4(0, 0, 0, 0);
+        if (WHOLE ? i < PAGE * VPR : r >= r0 && r < r1) {
           kv4[u] = reinterpret_cast<const uint4*>(kp + (size_t)r * D)[c];
           vv4[u] = reinterpret_cast<const uint4*>(vp + (size_t)r * D)[c];
         }
@@ -129,20 +144,22 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
 #pragma unroll
       for (int u = 0; u < AHEAD; ++u) {
         const int i = i0 + u * THREADS, r = i / VPR, c = i % VPR;
-        if (i < r1 * VPR) {
+        if (i < rb * VPR) {
           *reinterpret_cast<uint4*>(kt + r * L::KSTRIDE + c * L::VEC) = kv4[u];
           *reinterpret_cast<uint4*>(vt + r * D + c * L::VEC) = vv4[u];
         }
       }
     }
     __syncthreads();
-    // scores: item -> (head g, key r); consecutive threads take consecutive keys, or two or four threads one key where the items are few
-    const int items = G * rows, share = 4 * items <= THREADS ? 4 : 2 * items <= THREADS ? 2 : 1;
+    // scores: item -> (head g, key r); consecutive threads take consecutive keys, or two or four threads one key where the items are few (not
+    // of a whole page: the threads of a key read the same banks)
+    const int items = G * rows, share = WHOLE || 2 * items > THREADS ? 1 : 4 * items > THREADS ? 2 : 4;
     for (int i0 = 0; i0 < items * share; i0 += THREADS) {
       const int item = (i0 + tid) / share, sub = tid % share;
-      const int g = item / rows, r = r0 + item - g * rows;
+      const int g = item / rows, r = ra + item - g * rows;
+      const bool seen = item < items && r >= r0 && r < r1;
       float dot[4] = {0.f, 0.f, 0.f, 0.f};      // four chains of D / 4: one of D waits for every addition
-      if (item < items) {
+      if (seen) {
         const T* kr = kt + r * L::KSTRIDE;
         const float* qg = qs + g * D;
 #pragma unroll 4
@@ -161,18 +178,18 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
       }
       float s = (dot[0] + dot[1]) + (dot[2] + dot[3]);
       for (int o = 1; o < share; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-      if (item < items && sub == 0) sc[g * PAGE + r] = s * scale;
+      if (item < items && sub == 0) sc[g * PAGE + r] = seen ? s * scale : -INFINITY;
     }
     __syncthreads();
     // online softmax, one warp per head
     for (int g = warp; g < G; g += NWARP) {
       float mx = -INFINITY;
-      for (int r = r0 + lane; r < r1; r += 32) mx = fmaxf(mx, sc[g * PAGE + r]);
+      for (int r = ra + lane; r < rb; r += 32) mx = fmaxf(mx, sc[g * PAGE + r]);
       mx = warp_max(mx);
       const float m_old = m_s[g];
       const float m_new = fmaxf(m_old, mx);
       float sum = 0.f;
-      for (int r = r0 + lane; r < r1; r += 32) {
+      for (int r = ra + lane; r < rb; r += 32) {
         const float s = sc[g * PAGE + r];
         const float p = (s == -INFINITY) ? 0.f : expf(s - m_new);
         sc[g * PAGE + r] = p;
@@ -194,14 +211,27 @@ __global__ void __launch_bounds__(THREADS) attn_rows_kernel(
       if (d < D) {
 #pragma unroll
         for (int g = 0; g < G; ++g) acc[i][g] *= a_s[g];
-#pragma unroll 8
-        for (int r = r0; r < r1; ++r) {
-          const float v = to_f32<T>(vt[r * D + d]);
+        for (int r = ra; r < rb; r += 8) {
+          float v[8];
 #pragma unroll
-          for (int g = 0; g < G; ++g) acc[i][g] = fmaf(sc[g * PAGE + r], v, acc[i][g]);
+          for (int u = 0; u < 8; ++u) v[u] = to_f32<T>(vt[(r + u) * D + d]);
+#pragma unroll
+          for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int u = 0; u < 8; u += 4) {
+              const float4 p = *reinterpret_cast<const float4*>(sc + g * PAGE + r + u);
+              acc[i][g] = fmaf(p.x, v[u], acc[i][g]);
+              acc[i][g] = fmaf(p.y, v[u + 1], acc[i][g]);
+              acc[i][g] = fmaf(p.z, v[u + 2], acc[i][g]);
+              acc[i][g] = fmaf(p.w, v[u + 3], acc[i][g]);
+            }
         }
       }
     }
+  };
+  for (int pg = k_begin / PAGE; pg * PAGE < k_end; ++pg) {
+    if (k_begin <= pg * PAGE && k_end >= (pg + 1) * PAGE) walk(std::true_type{}, pg);
+    else walk(std::false_type{}, pg);
   }
   __syncthreads();
 #pragma unroll
