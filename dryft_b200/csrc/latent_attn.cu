@@ -202,8 +202,11 @@ __global__ void __launch_bounds__(WPB * 32) latent_attn_rows_kernel(
     const int cnt = min(KT, hi - j0 + 1);
     __syncthreads();   // the tile before is used up (and, the first time, qs is written)
     if (vec_ok) {
-      // every thread asks for nine 16-byte pieces before it unpacks the first: the loads' round trips overlap
-      constexpr int AHEAD = 9;
+      // Every thread asks for some 16-byte pieces before it unpacks the first: the loads' round trips overlap.  Four where the blocks are many:
+      // with nine the registers take a block or two off a multiprocessor (1,300 tokens of 700 keys, 16 heads of 256 + 32: 555 us with four, 655
+      // with nine).  Nine where they are few; one token of 1,300 keys, bfloat16, with five / nine / fourteen: 512 + 64 31.1 / 31.9 / 32.1 us,
+      // 256 + 32 22.1 / 19.8 / 20.8, 96 + 32 15.0 / 14.0 / 14.6, 48 + 16 11.3 / 12.3 / 12.0.
+      constexpr int AHEAD = HW == HW_MOST ? 4 : 9;
       const int total = cnt * vpr;
       for (int base = threadIdx.x; base < total; base += AHEAD * WPB * 32) {
         uint4 v[AHEAD];
@@ -333,7 +336,7 @@ __global__ void __launch_bounds__(WPB * 32) latent_attn_rows_kernel(
 // maxima and sums into one weight per split (up to MAX_SPLITS of them); every thread then sums its latent entries.
 constexpr int MAX_SPLITS = 64;
 
-template <typename T>
+template <typename T, int AT_ONCE>
 __global__ void latent_combine_kernel(const float* __restrict__ part, const int* __restrict__ tok_slot, T* __restrict__ o_lat,
                                       int n_splits, int n_tokens, int H, int kv_rank, const float* __restrict__ sink) {
   __shared__ float w[MAX_SPLITS];
@@ -341,9 +344,9 @@ __global__ void latent_combine_kernel(const float* __restrict__ part, const int*
   if (tok_slot[n] < 0) return;
   const size_t stride = (size_t)kv_rank + 2;
   const float* src = part + ((size_t)n * H + hd) * n_splits * stride;
-  // a thread a latent entry; 32 splits' values are requested together, the first of them before the weights are known (7.1 us a launch with
-  // sixteen at a time behind the weights, 3.5 now: the same 16 heads of 512)
-  constexpr int AT_ONCE = 32;
+  // A thread a latent entry; 32 splits' values are requested together, the first of them before the weights are known (7.1 us a launch with
+  // sixteen at a time behind the weights, 3.5 now: the same 16 heads of 512).  Up to eight splits have a kernel with registers for eight: their
+  // launches have many blocks (64 tokens of 500 keys, both launches: 97.3 us with 32, 89.9 with eight).
   float v[AT_ONCE];
 #pragma unroll
   for (int u = 0; u < AT_ONCE; ++u) v[u] = u < n_splits && threadIdx.x < kv_rank ? src[u * stride + 2 + threadIdx.x] : 0.f;
@@ -646,7 +649,8 @@ int launch_rows(const float* q_lat, const void* q, int q_stride, int q_rot_off, 
                                                                                     tok_slot, tok_pos, inv_freq, inv_freq_lo, interleaved, o_lat, part,
                                                                                     n_splits, n_tokens, H, kv_rank, rot, scale, window, sink, st);
   if (e || n_splits <= 1) return e;
-  latent_combine_kernel<T><<<dim3(n_tokens, H), kv_rank > 256 ? 512 : 256, 0, st>>>(part, tok_slot, (T*)o_lat, n_splits, n_tokens, H, kv_rank, sink);
+  (n_splits <= 8 ? latent_combine_kernel<T, 8> : latent_combine_kernel<T, 32>)<<<dim3(n_tokens, H), kv_rank > 256 ? 512 : 256, 0, st>>>(
+      part, tok_slot, (T*)o_lat, n_splits, n_tokens, H, kv_rank, sink);
   return launch_status();
 }
 }  // namespace
