@@ -63,7 +63,11 @@ static_assert(PAGE % SLICE == 0, "page size must be a multiple of 16");
 // while one is used).  Few (row, kv head) pairs: wide blocks, one per SM, so that one sequence's keys
 // are walked by many warps.  Many pairs: narrow blocks with deeper rings, several per SM, so that no SM
 // waits on the one block it holds and the grid is not cut into a few coarse waves.
-constexpr int ALONE_PAGES = 256 / PAGE;      // a sequence of up to 256 keys: two slices a warp
+// Up to so many keys a cluster's first block takes a sequence alone: two slices for each of eight warps, three for each of fewer.  Steps of
+// engines of eight layers, batch 8, alone / as a cluster: eight warps, 32 heads of 128 on eight, 175 keys 186.5 / 196.9 us, 240 keys 190 / 198,
+// beyond the line 300 keys 199 / 208; 8 heads on two, 240 keys 145.6 / 139.8, 300 keys 150 / 142, batch 1 136.6 / 130.  Four warps, 16 heads of
+// 240 on four: 175 keys 217 / 228; 240 keys 228 / 231, batch 1 206 / 194.
+template <int NWARP> constexpr int ALONE_KEYS = NWARP >= 8 ? 256 : 3 * 16 * NWARP;
 constexpr int PT_CACHE = 64;                // page numbers of a block kept in shared memory (more are read from global)
 constexpr int Q_ROWS = (G + 7) / 8 * 8;                     // the query heads, padded with zero rows to whole column tiles
 constexpr size_t Q_BYTES = (size_t)(Q_ROWS + 2) * KS * 2;  // then the new key and the new value
@@ -248,7 +252,7 @@ __global__ void __launch_bounds__(NWARP * 32) attn_decode_kernel(const Params p)
   const int first_page = kv_lo / PAGE, last_page = pos / PAGE;
   const int n_pages = last_page - first_page + 1;
   // A cluster's first block takes a short sequence alone: a few more slices a warp cost less than partial sums sent around.
-  const bool alone = p.cluster && n_pages <= ALONE_PAGES;
+  const bool alone = p.cluster && n_pages <= ALONE_KEYS<NWARP> / PAGE;
   const int per_split = alone ? n_pages : (n_pages + p.n_splits - 1) / p.n_splits;
   const int pg_begin = first_page + split * per_split;
   const int pg_end = min(pg_begin + per_split, last_page + 1);
