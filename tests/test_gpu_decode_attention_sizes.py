@@ -61,3 +61,12 @@ def test_head_sizes_whose_widest_block_is_near_the_shared_memory_limit(n_heads, 
     """A block of eight warps takes 220 KB at 208 dims: what blocks of a cluster receive does not fit beside it, everything else does."""
     ways = [w for w in WAYS if d < 224 or w[1] != 0]      # (eight warps of 224 dims fit no launch)
     _check(n_heads, n_kv, d, 64, None, [0, 63, 200, 300, 513], ways, 0)
+
+
+@pytest.mark.parametrize("n_heads,n_kv,d,rot", [(8, 2, 128, 128), (4, 4, 64, 32), (12, 4, 96, 96), (16, 1, 32, 16), (4, 1, 256, 128)])
+@pytest.mark.parametrize("window", [None, 300])
+def test_rows_beyond_the_length_of_one_block(n_heads, n_kv, d, rot, window):
+    """Rows on both sides of the lengths up to which a cluster's first block works alone (256 keys with eight warps, 192 and 96 with four and
+    two), the new token in the last split's page and in the first, and padding whose position is far beyond them."""
+    ways = [w for w in WAYS if d < 224 or w[1] != 0]
+    _check(n_heads, n_kv, d, rot, window, [0, 40, 127, 190, 191, 192, 255, 256, 320, 513, 700], ways, 700)
