@@ -19,14 +19,17 @@
 // new token's own row is patched into the staged slice from shared memory, so the early request need
 // not wait for the cache write); scores, running maximum and sums are 32-bit
 // (attn_decode.py:77-90), P is rounded to bfloat16 for the second product (attn_decode.py:12-14,89).
-// The warps' partial (m, l, acc) are combined through shared memory.  With several splits each block
-// leaves its partial in global memory and takes a ticket; the block that draws the last ticket of a
-// (row, kv head) combines all partials in split order, so the result does not depend on arrival
-// order, and puts the ticket counter back to zero.  No block waits for another: there is no spin.
+// The warps' partial (m, l, acc) are combined through shared memory.  Two to eight splits run as the blocks
+// of a cluster: a short sequence stays in its first block, else every block sends each other block a share of
+// its partial sums through distributed shared memory and adds up its own share over all splits, in split order
+// (two barriers of the cluster: one before anything is sent, one behind the sending).  More splits, or splits
+// outside a cluster, leave their partials in global memory and take a ticket; the block that draws the last
+// ticket of a (row, kv head) combines all partials in split order, so the result does not depend on arrival
+// order, and puts the ticket counter back to zero: there no block waits for another, and there is no spin.
 //
 // Code.  A decode step runs five kernels in turn on every SM, whose instruction cache holds 32 KB: what a launch executes is fetched
-// anew, at about 0.05 us a kilobyte (straight-line code of 16 KB: 2,700 cycles the first time, 1,040 the second).  So loops that run once
-// or twice a launch are not unrolled, and one piece of code serves queries, keys and values: 59 KB became 40.
+// anew, at about 0.05 us a kilobyte (a probe with straight-line code of 16 KB took 2,700 cycles the first time, 1,040 the second).  So loops
+// that run once or twice a launch are not unrolled, and one piece of code serves queries, keys and values: 59 KB became 40.
 //
 // A token with 40 keys, two kv heads, behind its projection's end: 7.1 us until the output product begins before, 4.4 now (one block
 // instead of a cluster of six, accumulators handed over without bank conflicts, less code); 540 keys, eight kv heads, clusters of six:
