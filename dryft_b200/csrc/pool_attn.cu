@@ -612,8 +612,9 @@ __global__ void __launch_bounds__(ROWS_WARPS * 32) pool_attn_rows_kernel(
       out[((size_t)t * H + head) * DV + c] = from_f32<T>(den > 0.f ? O * f / den * gate_at<T>(gate, gate_ld, t, head, c) : 0.f);
     } else {
       const size_t pi = ((size_t)t * H + head) * n_splits + sp;
-      part_o[pi * DV + c] = O;
-      if (c == 0) { part_ml[pi * 2] = M; part_ml[pi * 2 + 1] = L; }
+      // (scores that are all -inf give sums that are no numbers; the joining launch multiplies a split of weight zero, too)
+      part_o[pi * DV + c] = M == -INFINITY ? 0.f : O;
+      if (c == 0) { part_ml[pi * 2] = M; part_ml[pi * 2 + 1] = M == -INFINITY ? 0.f : L; }
     }
   }
 }
