@@ -640,10 +640,12 @@ int launch_rows(const float* q_lat, const void* q, int q_stride, int q_rot_off, 
                 const float* inv_freq_lo, int interleaved, void* o_lat, float* part, int n_splits, int n_tokens, int H, int kv_rank,
                 int rot, float scale, int window, const float* sink, cudaStream_t st) {
   int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  // twice the blocks, a key's row read from shared memory for half as many heads, while half of the multiprocessors would have none (the figures at the
-  // row kernel are with both: the line itself is where the second half still runs in the same wave)
+  cudaError_t ce = cudaGetDevice(&dev);
+  if (ce == cudaSuccess) ce = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (ce != cudaSuccess) return (int)ce;
+  // Twice the blocks, a key's row read from shared memory for half as many heads, while half of the multiprocessors would have none.  16 heads of
+  // 512 + 64, 1,300 keys, two / four heads a warp, both launches: one token (32 blocks of four heads a warp) 31.9 / 38.2 us, two 32.5 / 38.8;
+  // beyond the line, four tokens (128 blocks) 38.6 / 38.8, 16 tokens 101.8 / 69.9.
   const bool few = 2LL * n_tokens * ((H + HW_MOST * WPB - 1) / (HW_MOST * WPB)) * n_splits <= sms;
   int e = (few ? launch_rows_of<T, NR, HW_MOST / 2> : launch_rows_of<T, NR, HW_MOST>)(q_lat, q, q_stride, q_rot_off, k_pages, page_table, max_pages, page_size,
                                                                                     tok_slot, tok_pos, inv_freq, inv_freq_lo, interleaved, o_lat, part,
@@ -682,7 +684,7 @@ DRYFT_API int dryft_latent_attn_rows(int is_bf16, const float* q_lat, const void
                                      int interleaved, void* o_lat, float* part, int n_splits, int n_tokens, int H, int kv_rank,
                                      int rot, float scale, int window, const float* sink, cudaStream_t st) {
   if (n_tokens <= 0) return 0;
-  if (kv_rank <= 0 || kv_rank > 512 || rot < 0 || (rot & 1) || H <= 0 || H > 65535) return DRYFT_ERR_UNSUPPORTED;
+  if (kv_rank <= 0 || kv_rank > 512 || rot < 0 || (rot & 1) || H <= 0 || (H + HW_MOST * WPB - 1) / (HW_MOST * WPB) > 65535) return DRYFT_ERR_UNSUPPORTED;
   if (n_splits < 1 || n_splits > MAX_SPLITS || (n_splits > 1 && !part)) return DRYFT_ERR_UNSUPPORTED;
   typedef __nv_bfloat16 bf;
   const int nr = (kv_rank + 31) / 32;

@@ -34,3 +34,20 @@ def test_few_and_many_blocks(dtype, kv_rank, rot, H, n_splits):
     assert torch.isfinite(together).all()
     for t in (0, 1, 2, 3, 4, 77, 159):
         assert torch.equal(rows([t])[:, 0], together[:, t]), t
+
+
+def test_more_heads_than_a_grid_has_rows():
+    """65,537 heads in blocks of 16: the first, the last and some between against one head alone."""
+    torch.manual_seed(3)
+    kv_rank, H = 16, 65537
+    k_pages, table = torch.randn(1, 1, 64, kv_rank, device=DEV), i32([[0]])
+    q_lat, q = torch.randn(H, 1, kv_rank, device=DEV), torch.zeros(1, H, 1, device=DEV)
+
+    def rows(heads):
+        out = torch.full((len(heads), 1, kv_rank), float("nan"), device=DEV)
+        K.latent_attn_rows(q_lat[heads].contiguous(), q[:, heads].contiguous(), 1, k_pages, table, i32([0]), i32([40]), None, True, out, kv_rank, 0, 0.2, None)
+        return out
+
+    together = rows(list(range(H)))
+    for h in (0, 15, 16, 32767, 65535, 65536):
+        assert torch.equal(rows([h])[0], together[h]), h
