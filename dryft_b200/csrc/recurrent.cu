@@ -137,12 +137,15 @@ __global__ void __launch_bounds__(RT_THREADS) retention_scan_kernel(
 // 16 heads of 128 x 128, one token: 11.1 us a launch with the walk above, 9.7 here, of which half runs beside the product before it (5.2 us of
 // its own): a 1,300-token prompt + 16 steps, 6 such launches a step, 14,709 -> 14,266 us.  Sizes it does not take (rows that are no 16-byte words, more
 // than STEP_ROWS rows a thread, angles or partial sums beyond 48 KB of shared memory) are walked as longer steps are.
+// Few rows a thread have a kernel with registers for as many: 64 sequences, us with registers for 16 rows / now / the walk: 8 heads of
+// 64 x 64 (four rows a thread) 9.1 / 5.7 / 7.6, 32 heads of 16 x 32 (one) 25.8 / 11.4 / 12.3, 16 heads of 64 x 128 (eight) 25.2 / 18.0 / 23.4.
 constexpr int STEP_ROWS = 16;
+__host__ __device__ constexpr int step_rows(int dim, int vdim) { return (dim + RT_THREADS / (vdim / 4) - 1) / (RT_THREADS / (vdim / 4)); }
 __host__ __device__ constexpr bool step_fits(int dim, int vdim, int rot) {
-  return vdim % 4 == 0 && vdim <= 4 * RT_THREADS && (dim + RT_THREADS / (vdim / 4) - 1) / (RT_THREADS / (vdim / 4)) <= STEP_ROWS && rot <= 1024;
+  return vdim % 4 == 0 && vdim <= 4 * RT_THREADS && step_rows(dim, vdim) <= STEP_ROWS && rot <= 1024;
 }
 
-template <typename T>
+template <typename T, int ROWS>
 __global__ void __launch_bounds__(RT_THREADS) retention_step_kernel(
     const T* __restrict__ proj, int ld, int q_off, int k_off, int v_off, int g_off, const int* __restrict__ seq_slot, const int* __restrict__ tok_pos,
     const float* __restrict__ inv_freq, const float* __restrict__ inv_freq_lo, int rot, const double* __restrict__ decay, float* __restrict__ state,
@@ -163,10 +166,10 @@ __global__ void __launch_bounds__(RT_THREADS) retention_step_kernel(
   float2* const turn = reinterpret_cast<float2*>(vs + vdim);      // [rot / 2] sin, cos
   __shared__ float scratch[33];
   float4* const Sg = reinterpret_cast<float4*>(state + ((size_t)slot * H + hd) * dim * vdim);
-  float4 old[STEP_ROWS];
+  float4 old[ROWS];
   auto request = [&]() {      // (through L2: a state written while this launch was resident is no read-only data)
 #pragma unroll
-    for (int i = 0; i < STEP_ROWS; ++i) {
+    for (int i = 0; i < ROWS; ++i) {
       const int d = rg + i * groups;
       old[i] = rg < groups && d < dim ? __ldcg(Sg + (size_t)d * words + cv) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
@@ -206,7 +209,7 @@ __global__ void __launch_bounds__(RT_THREADS) retention_step_kernel(
     const float4 v = reinterpret_cast<const float4*>(vs)[cv];
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-    for (int i = 0; i < STEP_ROWS; ++i) {
+    for (int i = 0; i < ROWS; ++i) {
       const int d = rg + i * groups;
       if (d < dim) {
         const float k = ks[d], q = qs[d];
@@ -870,11 +873,14 @@ DRYFT_API int dryft_retention_scan(int is_bf16, const void* proj, int ld, int q_
     cfg.attrs = attr;
     cfg.numAttrs = pdl ? 1 : 0;
     if (cfg.dynamicSmemBytes <= 48 * 1024) {
-      const cudaError_t e =
-          is_bf16 ? cudaLaunchKernelEx(&cfg, retention_step_kernel<bf>, (const bf*)proj, ld, q_off, k_off, v_off, g_off, seq_slot, tok_pos, inv_freq,
-                                       inv_freq_lo, rot, decay, state, (bf*)out, H, dim, vdim, k_scale, eps, early_state || !pdl)
-                  : cudaLaunchKernelEx(&cfg, retention_step_kernel<float>, (const float*)proj, ld, q_off, k_off, v_off, g_off, seq_slot, tok_pos,
-                                       inv_freq, inv_freq_lo, rot, decay, state, (float*)out, H, dim, vdim, k_scale, eps, early_state || !pdl);
+      const int rows = step_rows(dim, vdim), early = early_state || !pdl;
+      auto run = [&](auto kernel, auto type) {
+        typedef decltype(type) T;
+        return cudaLaunchKernelEx(&cfg, kernel, (const T*)proj, ld, q_off, k_off, v_off, g_off, seq_slot, tok_pos, inv_freq, inv_freq_lo, rot, decay,
+                                  state, (T*)out, H, dim, vdim, k_scale, eps, early);
+      };
+      const cudaError_t e = is_bf16 ? run(rows <= 4 ? retention_step_kernel<bf, 4> : rows <= 8 ? retention_step_kernel<bf, 8> : retention_step_kernel<bf, STEP_ROWS>, bf())
+                                    : run(rows <= 4 ? retention_step_kernel<float, 4> : rows <= 8 ? retention_step_kernel<float, 8> : retention_step_kernel<float, STEP_ROWS>, 0.f);
       return e != cudaSuccess ? (int)e : launch_status();
     }
   }

@@ -40,3 +40,10 @@ def test_steps_of_one_token(dtype, H, d, dv, rot):
     assert torch.all(state[0] == 7.0)
     with pytest.raises(K.KernelError):
         K.retention_scan(proj, offs, i32([0, 4]), i32([1]), i32([0] * 4), inv, rot, dec, state, out, 1, H, d, dv, 1.0, eps, one_token=True)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H, d, dv, rot", [(2, 32, 128, 16), (1, 33, 128, 0), (2, 64, 128, 64), (1, 65, 128, 2)])
+def test_rows_a_thread_around_those_that_have_a_kernel(dtype, H, d, dv, rot):
+    """Four, five, eight and nine rows a thread."""
+    test_steps_of_one_token(dtype, H, d, dv, rot)
