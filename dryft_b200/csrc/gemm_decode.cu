@@ -252,8 +252,10 @@ __global__ void __launch_bounds__(GW * 32 * GROUPS, GW * GROUPS == 8 ? 2 : 1) ge
     if (rs < MP)
       for (int c = ctid; c < CHUNKS; c += CT) *reinterpret_cast<uint4*>(a_res + (size_t)rs * KA + c * 8) = zero;
     for (int m = ctid >> 5; m < MP; m += WARPS * GROUPS) {
-      // (requested together: one after the other they took 0.4 us of every launch with a norm)
-      constexpr int AT_ONCE = 5;
+      // Requested together: one after the other they took 0.4 us of every launch with a norm.  Eight a lane are the 256 blocks of a 4,096-wide
+      // stream, the most of the usual widths; with five those took three more trips (four layers of the 8B shape, 30 keys, a step: 318 us with
+      // five, 312 with eight; 1,024, 2,048 and 2,560 wide the same with both).
+      constexpr int AT_ONCE = 8;
       float s = 0.f, part[AT_ONCE];
 #pragma unroll
       for (int i = 0; i < AT_ONCE; ++i) part[i] = m < M && lane + 32 * i < ss_parts ? ld_prev(ss_in + (size_t)(lane + 32 * i) * SS_STRIDE + m) : 0.f;
