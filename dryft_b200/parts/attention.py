@@ -105,10 +105,11 @@ class Attention:
 
     def _decode_splits(self, max_kv: int, n_rows: int) -> int:
         """Splits of the one-launch decode attention.  Up to eight splits of a (row, kv head) run as one
-        thread-block cluster and are combined through distributed shared memory, which costs about a
-        microsecond, so a block may take as little as three pages (192 keys: one or two 16-key slices per
-        warp) -- as long as the grid stays within one block per SM: more blocks than that take the slots in
-        which the next launch's blocks start early, which costs more than the shorter walk saves.
+        thread-block cluster and are combined through distributed shared memory, a split for every three
+        pages that the context bucket may hold -- as long as the grid stays within one block per SM: more
+        blocks than that take the slots in which the next launch's blocks start early, which costs more than
+        the shorter walk saves.  A row shorter than its bucket is cut into as many splits, or, up to 256 keys
+        (192 with blocks of four warps), left to the cluster's first block (csrc/attn_decode.cu).
         Sequences too long for that split further and meet in memory (a block then takes up to 1,024 keys)."""
         pages = (max(1, max_kv) + self.rt.page_size - 1) // self.rt.page_size
         room = max(1, self.rt.sm_count // max(1, n_rows * self.n_kv))
