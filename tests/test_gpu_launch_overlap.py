@@ -1,32 +1,25 @@
 """The engine's switch for overlapped launches (``pdl``) reaches every kernel: a captured step holds programmatic edges with it and
 none without, and the results are the same bits."""
 
-import ctypes
-
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
 
-class _EdgeData(ctypes.Structure):
-    _fields_ = [("from_port", ctypes.c_ubyte), ("to_port", ctypes.c_ubyte), ("type", ctypes.c_ubyte), ("reserved", ctypes.c_ubyte * 5)]
-
-
 def programmatic_edges(fn) -> int:
-    """Edges of a captured ``fn()`` on which a launch may start before the one in front of it has ended (nothing is run).  The runtime is
-    asked with buffers of this function's own: the ones that the Python binding hands out are given back before they can be read."""
+    """Edges of a captured ``fn()`` on which a launch may start before the one in front of it has ended (nothing is run)."""
+    from cuda.bindings import runtime as R
+
     fn()
     torch.cuda.synchronize()
     graph = torch.cuda.CUDAGraph(keep_graph=True)
     with torch.cuda.graph(graph):
         keep = fn()
-    runtime, room = ctypes.CDLL("libcudart.so.12"), 20000
-    begins, ends, data, n = (ctypes.c_void_p * room)(), (ctypes.c_void_p * room)(), (_EdgeData * room)(), ctypes.c_size_t(room)
-    rc = runtime.cudaGraphGetEdges_v2(ctypes.c_void_p(int(graph.raw_cuda_graph())), begins, ends, data, ctypes.byref(n))
-    assert rc == 0 and 0 < n.value < room, (rc, n.value)
+    rc, _, _, data, n = R.cudaGraphGetEdges_v2(R.cudaGraph_t(graph.raw_cuda_graph()), 20000)
+    assert rc == R.cudaError_t.cudaSuccess and 0 < n < 20000, rc
     del keep
-    return sum(data[i].type == 1 for i in range(n.value))      # cudaGraphDependencyTypeProgrammatic
+    return sum(int(e.type) == int(R.cudaGraphDependencyType.cudaGraphDependencyTypeProgrammatic) for e in data[:n])
 
 
 @pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
