@@ -42,9 +42,10 @@ template <typename T> struct Smem {
   static constexpr size_t bytes() {
     return sizeof(float) * (G * D + G * PAGE + 3 * G) + sizeof(T) * (size_t)(PAGE * KSTRIDE + PAGE * D) + 32;
   }
-  // blocks a multiprocessor that the registers have to leave room for: as many as shared memory does, up to what costs few spills
+  // Blocks a multiprocessor that the registers have to leave room for: as many as shared memory does, up to what costs few spills.  16 heads on one
+  // kv head, 1,500 rows of 800 keys, us with room for 5 / 7: 32 dims, 32-bit 287 / 259, bfloat16 268 / 222, 64 dims, bfloat16 385 / 352.
   static constexpr int blocks() {
-    const size_t n = 227 * 1024 / (bytes() + 1024), most = G > 8 ? 5 : G > 2 ? 8 : 10;
+    const size_t n = 227 * 1024 / (bytes() + 1024), most = G > 8 ? 7 : G > 2 ? 8 : 10;
     return n < 1 ? 1 : (int)(n > most ? most : n);
   }
 };
@@ -115,15 +116,15 @@ __global__ void __launch_bounds__(THREADS, Smem<T>::blocks()) attn_rows_kernel(
 
   const int* pt = page_table + (size_t)slot * max_pages;
   constexpr int VPR = D / L::VEC;  // 16-byte vectors per row
-  // One page.  `whole`: all its keys are this block's, and every bound is a constant; else rows [r0, r1) are.  With bounds that only the launch
-  // knows, launches of many rows, which walk whole pages mostly, were up to 1.37 times as long: probabilities read one by one instead of four
-  // at a time, a division an item, registers for loads that no thread makes.  A part of a page is widened to groups of eight rows, zeros and
-  // probabilities of zero beside the block's own.
+  // One page, of whose keys rows [r0, r1) are this block's.  `whole`: it is walked from end to end with constant bounds, zeros and probabilities of
+  // zero beside the block's own; else only the groups of eight rows that hold some of them are.  With bounds that only the launch knows, launches
+  // of many rows were up to 1.37 times as long: probabilities read one by one instead of four at a time, a division an item, registers for
+  // loads that no thread makes.
   auto walk = [&](auto whole, int pg) {
     constexpr bool WHOLE = decltype(whole)::value;
     const int page = pt[pg];
     const int p0 = pg * PAGE;
-    const int r0 = WHOLE ? 0 : max(k_begin - p0, 0), r1 = WHOLE ? PAGE : min(k_end - p0, PAGE);
+    const int r0 = max(k_begin - p0, 0), r1 = min(k_end - p0, PAGE);
     const int ra = WHOLE ? 0 : r0 & ~7, rb = WHOLE ? PAGE : (r1 + 7) & ~7, rows = rb - ra;
     const T* kp = k_pages + ((size_t)page * nKV + kvh) * PAGE * D;
     const T* vp = v_pages + ((size_t)page * nKV + kvh) * PAGE * D;
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(THREADS, Smem<T>::blocks()) attn_rows_kernel(
       for (int u = 0; u < AHEAD; ++u) {
         const int i = i0 + u * THREADS, r = i / VPR, c = i % VPR;
         kv4[u] = vv4[u] = make_uint4(0, 0, 0, 0);
-        if (WHOLE ? i < PAGE * VPR : r >= r0 && r < r1) {
+        if (i < rb * VPR && r >= r0 && r < r1) {
           kv4[u] = reinterpret_cast<const uint4*>(kp + (size_t)r * D)[c];
           vv4[u] = reinterpret_cast<const uint4*>(vp + (size_t)r * D)[c];
         }
@@ -229,8 +230,10 @@ __global__ void __launch_bounds__(THREADS, Smem<T>::blocks()) attn_rows_kernel(
       }
     }
   };
+  // More than half a page of keys is walked as a whole one: 64 rows of 300 keys (the last page has 44), 8 heads of 64 in bfloat16, us as a
+  // part / as a whole page: one split 13.0 / 12.1, four 13.9 / 12.6.  A few keys are not: 200 rows of 130, 32-bit, 8 heads of 64 on four 13.8 / 14.6.
   for (int pg = k_begin / PAGE; pg * PAGE < k_end; ++pg) {
-    if (k_begin <= pg * PAGE && k_end >= (pg + 1) * PAGE) walk(std::true_type{}, pg);
+    if (min(k_end, (pg + 1) * PAGE) - max(k_begin, pg * PAGE) > PAGE / 2) walk(std::true_type{}, pg);
     else walk(std::false_type{}, pg);
   }
   __syncthreads();
