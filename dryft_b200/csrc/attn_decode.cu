@@ -497,8 +497,8 @@ __global__ void __launch_bounds__(NWARP * 32) attn_decode_kernel(const Params p)
     }
   }
   __syncthreads();
-  // A thread a warp and head: the warps' weights relative to the block's maximum, which go in the place of the maxima.  (With every warp working out all weights for itself, one head a kv head, 64 dims, 24 rows
-  // of 100 keys took 6.8 us; 6.05 so.)
+  // A thread a warp and head: the warps' weights relative to the block's maximum, which go in the place of the maxima.  (With every warp
+  // working out all weights for itself, one head a kv head, 64 dims, 24 rows of 100 keys took 6.8 us; 6.05 so.)
   if (tid < 16 * NWARP) {
     const int w = tid % NWARP, h = tid / NWARP;
     const float m = w < busy && h < NT * 8 ? wm[w * 16 + h] : -INFINITY;

@@ -123,7 +123,7 @@ template <> struct Vec16<__nv_bfloat16> {
 // staged row is read from shared memory once for all of them (16 bytes at a time where the row length allows): the loop is
 // bound by shared-memory reads, and this quarters them.  With one split the result goes to o_lat; with several, each block
 // leaves (max, sum, unnormalised weighted sum) in `part` and latent_combine joins them.
-// The block's queries come in together (asynchronous copies, the angles from one table, nine words of keys a thread on their way meanwhile):
+// The block's queries come in together (asynchronous copies, the angles from one table, a thread's first words of keys on their way meanwhile):
 // staged head by head they took half of a decode step's launch.  16 heads, rank 512 + 64, 1,300 keys, one token: 23.4 us before, 16.0 now;
 // whole request (3 layers x 16 steps) with the retention's steps as they are, 14,263 -> 13,785 us.
 template <typename T, int NR, int HW>
@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(WPB * 32) latent_attn_rows_kernel(
   const int hi = min(pos, lo + per_split * KT - 1);   // last key of this split
   const int nh = max(0, min(HW, H - hd0));            // live heads of this warp
   const float* qs = qs_all + (size_t)warp * HW * Dq;
-  const int first = blockIdx.y * HPB, live = min(HPB, H - first);      // the block's heads; one that does not exist stays zero, so that its sums stay finite
+  const int first = blockIdx.y * HPB, live = min(HPB, H - first);      // the block's heads; others are zeros, so that their sums stay finite
   for (int i = threadIdx.x; i < (HPB - live) * Dq; i += WPB * 32) qs_all[(size_t)live * Dq + i] = 0.f;
   const bool copied = (kv_rank & 3) == 0 && ((uintptr_t)q_lat & 15) == 0;
   const int quads = kv_rank / 4;

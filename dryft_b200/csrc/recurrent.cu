@@ -879,8 +879,12 @@ DRYFT_API int dryft_retention_scan(int is_bf16, const void* proj, int ld, int q_
         return cudaLaunchKernelEx(&cfg, kernel, (const T*)proj, ld, q_off, k_off, v_off, g_off, seq_slot, tok_pos, inv_freq, inv_freq_lo, rot, decay,
                                   state, (T*)out, H, dim, vdim, k_scale, eps, early);
       };
-      const cudaError_t e = is_bf16 ? run(rows <= 4 ? retention_step_kernel<bf, 4> : rows <= 8 ? retention_step_kernel<bf, 8> : retention_step_kernel<bf, STEP_ROWS>, bf())
-                                    : run(rows <= 4 ? retention_step_kernel<float, 4> : rows <= 8 ? retention_step_kernel<float, 8> : retention_step_kernel<float, STEP_ROWS>, 0.f);
+      const cudaError_t e = is_bf16 ? run(rows <= 4   ? retention_step_kernel<bf, 4>
+                                          : rows <= 8 ? retention_step_kernel<bf, 8>
+                                                      : retention_step_kernel<bf, STEP_ROWS>, bf())
+                                    : run(rows <= 4   ? retention_step_kernel<float, 4>
+                                          : rows <= 8 ? retention_step_kernel<float, 8>
+                                                      : retention_step_kernel<float, STEP_ROWS>, 0.f);
       return e != cudaSuccess ? (int)e : launch_status();
     }
   }
